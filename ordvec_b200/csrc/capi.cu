@@ -104,7 +104,15 @@ void grow_codes(Index& ix, uint64_t rows) {
   ix.codes.cap = cap;
 }
 
-void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w) {
+bool accepts_rows(const Index& ix, uint64_t n) {
+  return ix.n + n <= kMaxVectors && !(ix.kind == OVB_INDEX_KIND_FASTSCAN && ix.n) &&
+         !(ix.kind != OVB_INDEX_KIND_SIGN_BITMAP && ix.dim > kMaxDeviceRankDim);
+}
+
+// Appends n device rows.  With check, a row that is not finite refuses the add:
+// the encoders look at every value anyway, so they raise the flag, and the
+// rows they wrote lie past the index's end until ix.n moves.
+void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, bool check = false) {
   if (!n) return;
   if (ix.n + n > kMaxVectors)
     fail(ORDVEC_STATUS_BAD_ARGUMENT, "index would exceed MAX_VECTORS (67108864); had " + std::to_string(ix.n) +
@@ -115,9 +123,21 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w) {
   if (ix.kind != OVB_INDEX_KIND_SIGN_BITMAP && ix.dim > kMaxDeviceRankDim)
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "device rank transform supports dim <= 16384");
   grow_codes(ix, ix.n + n);
+  uint32_t *flag = nullptr, *h = nullptr;
+  if (check) {
+    flag = (uint32_t*)w.flag.ensure(4);
+    h = (uint32_t*)w.pinned.ensure(4);
+    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
+  }
   launch_encode((int)encode_kind(ix.kind), d_vecs, n, ix.dim, ix.bits, ix.n_top, ix.pairs_pad, ix.codes.p, ix.n,
-                w.stream);
+                flag, w.stream);
+  if (check) OVB_CUDA(cudaMemcpyAsync(h, flag, 4, cudaMemcpyDeviceToHost, w.stream));
   OVB_CUDA(cudaStreamSynchronize(w.stream));
+  if (check && *h) {
+    // FastScan's last block pads with zeros: a refused add leaves none of its rows there
+    if (ix.kind == OVB_INDEX_KIND_FASTSCAN) OVB_CUDA(cudaMemset(ix.codes.p, 0, ix.codes.cap));
+    fail(ORDVEC_STATUS_BAD_ARGUMENT, "ordvec: input contains non-finite (NaN or +-Inf) values");
+  }
   ix.n += n;
 }
 
@@ -576,14 +596,16 @@ ordvec_status_t ovb_index_add_device(ordvec_index_t* index, const float* d_vecto
     if (n && !d_vectors) fail(ORDVEC_STATUS_NULL_POINTER, "vectors pointer is NULL");
     if (!n) return;
     Workspace& w = workspace();
-    uint32_t* flag = (uint32_t*)w.flag.ensure(4);
-    uint32_t* h = (uint32_t*)w.pinned.ensure(4);
-    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
-    launch_finite_flag(d_vectors, n * ix.dim, flag, w.stream);
-    OVB_CUDA(cudaMemcpyAsync(h, flag, 4, cudaMemcpyDeviceToHost, w.stream));
-    OVB_CUDA(cudaStreamSynchronize(w.stream));
-    if (*h) fail(ORDVEC_STATUS_BAD_ARGUMENT, "ordvec: input contains non-finite (NaN or +-Inf) values");
-    add_device_rows(ix, d_vectors, n, w);
+    if (!accepts_rows(ix, n)) {  // non-finite input is reported before the other refusals
+      uint32_t* flag = (uint32_t*)w.flag.ensure(4);
+      uint32_t* h = (uint32_t*)w.pinned.ensure(4);
+      OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
+      launch_finite_flag(d_vectors, n * ix.dim, flag, w.stream);
+      OVB_CUDA(cudaMemcpyAsync(h, flag, 4, cudaMemcpyDeviceToHost, w.stream));
+      OVB_CUDA(cudaStreamSynchronize(w.stream));
+      if (*h) fail(ORDVEC_STATUS_BAD_ARGUMENT, "ordvec: input contains non-finite (NaN or +-Inf) values");
+    }
+    add_device_rows(ix, d_vectors, n, w, true);
   });
 }
 
@@ -736,7 +758,7 @@ ordvec_status_t ovb_sign_bitmap_score_all(const ordvec_index_t* sign, const floa
     Workspace& w = workspace();
     const float* d_q = upload_queries(w, query, 1, ix.dim, true);
     uint64_t* qb = (uint64_t*)w.qbits.ensure(ix.qpv() * 8);
-    launch_sign_query(d_q, 1, ix.dim, qb, w.stream);
+    launch_sign_encode(d_q, 1, ix.dim, qb, nullptr, w.stream);
     uint32_t* keys = (uint32_t*)w.keys.ensure(ix.n * 4);
     launch_popc_scan(0, ix.codes.as<uint64_t>(), ix.n, ix.qpv(), qb, 1, 0, keys, ix.n, w.stream);
     OVB_CUDA(cudaMemcpyAsync(scores, keys, ix.n * 4, cudaMemcpyDeviceToHost, w.stream));

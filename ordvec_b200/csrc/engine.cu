@@ -507,7 +507,7 @@ uint32_t engine_rankquant_symmetric(const Index& rq, const float* d_q, uint64_t 
   const uint32_t ke = (uint32_t)(k < rq.n ? k : rq.n);
   if (!ke || !nq) return ke;
   float* qc = (float*)w.q_unit.ensure(nq * rq.dim * 4);
-  launch_encode(6, d_q, nq, rq.dim, rq.bits, 0, 0, qc, 0, st);
+  launch_encode(6, d_q, nq, rq.dim, rq.bits, 0, 0, qc, 0, nullptr, st);
   const float norm = rankquant_norm_f32(rq.dim, rq.bits);
   const float inv_norm_sq = 1.0f / (norm * norm);
   // batches: split-BF16 candidates (the centred buckets are exact in BF16, so
@@ -540,7 +540,7 @@ uint32_t engine_rank_full(const Index& rk, const float* d_q, uint64_t nq, uint64
     });
   } else {
     uint16_t* qr = (uint16_t*)w.qbits.ensure(nq * dim * 2);
-    launch_encode(5, d_q, nq, dim, 0, 0, 0, qr, 0, st);
+    launch_encode(5, d_q, nq, dim, 0, 0, 0, qr, 0, nullptr, st);
     full_scan_select(w, nq, rk.n, ke, 32, ok, oi, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
       launch_rank_sym_scan(ranks, rk.n, dim, qr + q0 * dim, qn, keys, rk.n, st);
     });
@@ -580,7 +580,7 @@ uint32_t engine_candidates(const Index& s1, const float* d_q, uint64_t nq, uint6
       const int mode = s1.kind == OVB_INDEX_KIND_SIGN_BITMAP ? 0 : 1;
       uint64_t* qb = (uint64_t*)w.qbits.ensure(nq * s1.qpv() * 8);
       if (mode == 0)
-        launch_sign_query(d_q, nq, s1.dim, qb, st);
+        launch_sign_encode(d_q, nq, s1.dim, qb, nullptr, st);
       else
         launch_bitmap_query(d_q, nq, s1.dim, s1.n_top, qb, st);
       w.mark(st, 1);

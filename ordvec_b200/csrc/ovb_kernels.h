@@ -35,8 +35,9 @@ void launch_select_rows(const SelectArgs& a, uint64_t rows, uint64_t* scratch,
 // ---- K8 query preparation (prep.cu) ------------------------------------------
 void launch_l2_normalise(const float* q, uint64_t nq, uint32_t dim, float* out,
                          cudaStream_t stream);
-void launch_sign_query(const float* q, uint64_t nq, uint32_t dim, uint64_t* out,
-                       cudaStream_t stream);
+// sign bits of rows (bit j = v[j] > 0); *flag is set when a value is not finite (may be null)
+void launch_sign_encode(const float* vecs, uint64_t rows, uint32_t dim, uint64_t* out, uint32_t* flag,
+                        cudaStream_t stream);
 void launch_bitmap_query(const float* q, uint64_t nq, uint32_t dim, uint32_t n_top,
                          uint64_t* out, cudaStream_t stream);
 void launch_fastscan_lut(const float* q_unit, uint64_t nq, uint32_t dim, uint32_t pairs_pad,
@@ -175,7 +176,7 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
 // kind: 0 RankQuant packed codes, 1 sign bitmap, 2 const-weight bitmap, 3 FastScan
 // (device layout), 4 multi-bucket bitmaps.
 void launch_encode(int kind, const float* vecs, uint64_t n, uint32_t dim, uint32_t bits,
-                   uint32_t n_top, uint32_t pairs_pad, void* out, uint64_t first_doc,
+                   uint32_t n_top, uint32_t pairs_pad, void* out, uint64_t first_doc, uint32_t* flag,
                    cudaStream_t stream);
 uint32_t fastscan_pairs_pad(uint32_t dim);
 uint64_t fastscan_block_bytes(uint32_t pairs_pad);

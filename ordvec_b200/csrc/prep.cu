@@ -4,9 +4,7 @@
 //   -0.0, correctly rounded sqrt and reciprocal, elementwise multiply.  The
 //   sum is sequential on purpose: the FastScan LUT (and with it every
 //   candidate id) depends on q_unit bit for bit.
-// * sign query    (src/sign_bitmap.rs:204-214): bit j set iff q[j] > 0.
-// * bitmap query  (src/bitmap.rs:170-187): the n_top largest coordinates,
-//   stable descending sort (ties keep the lower index; -0.0 == +0.0).
+// * sign and bitmap query bits: the encoders of encode.cu.
 // * FastScan LUT  (src/fastscan.rs:130-173): v = qa*c[a] + qc*c[c] without
 //   contraction, global min/max with first-occurrence ties, affine u8
 //   quantisation with round-half-away-from-zero and clamp.
@@ -57,57 +55,6 @@ __global__ void l2_normalise_kernel(const float* __restrict__ q, uint64_t nq, ui
   } else {
     const float inv = __fdiv_rn(1.0f, norm);
     for (uint32_t j = lane; j < dim; j += 32) y[j] = __fmul_rn(x[j], inv);
-  }
-}
-
-__global__ void sign_query_kernel(const float* __restrict__ q, uint64_t nq, uint32_t dim,
-                                  uint64_t* __restrict__ out) {
-  const uint32_t qpv = dim / 64;
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq * qpv) return;
-  const uint64_t qi = t / qpv, w = t % qpv;
-  const float* x = q + qi * dim + w * 64;
-  uint64_t bits = 0;
-  for (int j = 0; j < 64; j++)
-    if (x[j] > 0.0f) bits |= 1ull << j;
-  out[t] = bits;
-}
-
-// Bitonic sort of `len` (power of two) u64 keys in shared memory.
-__device__ void block_bitonic(uint64_t* buf, uint32_t len) {
-  for (uint32_t size = 2; size <= len; size <<= 1)
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t t = threadIdx.x; t < len / 2; t += blockDim.x) {
-        uint32_t i = 2 * t - (t & (stride - 1)), j = i + stride;
-        bool up = (i & size) == 0;
-        uint64_t a = buf[i], b = buf[j];
-        if ((a > b) == up) {
-          buf[i] = b;
-          buf[j] = a;
-        }
-      }
-      __syncthreads();
-    }
-}
-
-__device__ __forceinline__ float canon_zero(float v) { return v == 0.0f ? 0.0f : v; }
-
-// n_top largest coordinates, stable: key = (desc value, index) ascending.
-__global__ void bitmap_query_kernel(const float* __restrict__ q, uint32_t dim, uint32_t n_top,
-                                    uint32_t len, uint64_t* __restrict__ out) {
-  extern __shared__ uint64_t skeys[];
-  const float* x = q + (uint64_t)blockIdx.x * dim;
-  for (uint32_t j = threadIdx.x; j < len; j += blockDim.x)
-    skeys[j] = j < dim ? ((uint64_t)desc_key(canon_zero(x[j])) << 32) | j : ~0ull;
-  __syncthreads();
-  block_bitonic(skeys, len);
-  const uint32_t qpv = dim / 64;
-  uint64_t* o = out + (uint64_t)blockIdx.x * qpv;
-  for (uint32_t w = threadIdx.x; w < qpv; w += blockDim.x) o[w] = 0;
-  __syncthreads();
-  for (uint32_t t = threadIdx.x; t < n_top; t += blockDim.x) {
-    uint32_t j = (uint32_t)skeys[t];
-    atomicOr((unsigned long long*)&o[j / 64], 1ull << (j % 64));
   }
 }
 
@@ -232,24 +179,11 @@ void launch_l2_normalise(const float* q, uint64_t nq, uint32_t dim, float* out,
   launched();
 }
 
-void launch_sign_query(const float* q, uint64_t nq, uint32_t dim, uint64_t* out,
-                       cudaStream_t stream) {
-  uint64_t total = nq * (dim / 64);
-  if (!total) return;
-  sign_query_kernel<<<ceil_div(total, 256), 256, 0, stream>>>(q, nq, dim, out);
-  launched();
-}
-
 void launch_bitmap_query(const float* q, uint64_t nq, uint32_t dim, uint32_t n_top,
                          uint64_t* out, cudaStream_t stream) {
   if (!nq) return;
-  uint32_t len = 1;
-  while (len < dim) len <<= 1;
-  size_t smem = (size_t)len * 8;
-  if (smem > 227 * 1024) throw std::invalid_argument("Bitmap query dim too large for the device path (dim <= 16384)");
-  allow_dynamic_smem(bitmap_query_kernel);
-  bitmap_query_kernel<<<(unsigned)nq, 512, smem, stream>>>(q, dim, n_top, len, out);
-  launched();
+  if (dim > 16384) throw std::invalid_argument("Bitmap query dim too large for the device path (dim <= 16384)");
+  launch_encode(7, q, nq, dim, 0, n_top, 0, out, 0, nullptr, stream);
 }
 
 void launch_fastscan_lut(const float* q_unit, uint64_t nq, uint32_t dim, uint32_t pairs_pad,
