@@ -220,7 +220,7 @@ void bitmap_tc_candidates(const Index& s1, const uint64_t* qb, uint32_t qpv, uin
   }
   if (bitmap_fp4_usable(qpv)) {
     q4 = (uint8_t*)w.q_nib.ensure(nq * row4);
-    launch_bitmap_fp4_query(qb, nq, qpv, q4, st);
+    launch_bitmap_fp4_query(qb, nq, qpv, key_kind == 2, q4, st);
   }
   filtered_select(
       w, n, nq, me, fp, key_bits, sk, si, st,

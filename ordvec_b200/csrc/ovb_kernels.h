@@ -87,7 +87,7 @@ void launch_fastscan_filter_tc(const uint8_t* blocks, uint64_t n, uint32_t pairs
 // Rows of qpv u64 words; key_kind 0: key32 = n_top - popcount(q AND d)
 // (constant-weight bitmap), 1: key32 = desc_key((float)popcount) (multi-bucket
 // with identity weights), 2: key32 = popcount(q XOR d) = |q| + |d| - 2 |q AND d|
-// (sign bitmap; qpop = |q| per query).  The query operand is the query bits
+// (sign bitmap; qpop = |q| per query, query bytes +-1).  The query operand is the query bits
 // expanded to 0/1 bytes (launch_bitmap_tc_query, which also writes qpop when
 // given), bitmap_tc_kblocks(qpv) * 128 per query.
 uint32_t bitmap_tc_kblocks(uint32_t qpv);
@@ -102,7 +102,8 @@ void launch_bitmap_scan_tc(const uint64_t* words, uint64_t n, uint32_t qpv, uint
 // whether the filter below may take it (OVB_BITMAP_FP4=0 says no).
 uint32_t bitmap_fp4_kblocks(uint32_t qpv);
 bool bitmap_fp4_usable(uint32_t qpv);
-void launch_bitmap_fp4_query(const uint64_t* qbits, uint64_t nq, uint32_t qpv, uint8_t* out, cudaStream_t stream);
+void launch_bitmap_fp4_query(const uint64_t* qbits, uint64_t nq, uint32_t qpv, bool sign, uint8_t* out,
+                             cudaStream_t stream);
 // Filter with a tie bound: keeps (key32, doc) <= (thr, tdoc) in (key, doc)
 // order, tdoc = the doc of sample position thr_pos[q * thr_stride] of a sample
 // taken with block stride smp_stride (every doc at key < thr when thr_pos is null).

@@ -202,7 +202,9 @@ __device__ __forceinline__ void tc_scan_body(const CUtensorMap& lut_map, const T
     // ---- MMA issuer ----------------------------------------------------------
     if (lane == 0) {
       // D s32, A/B u8, both K-major, N = nt, M = 128
-      const uint32_t idesc = (2u << 4) | ((nt >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+      // (sign bitmaps' queries are +-1: both operands s8)
+      const uint32_t i8fmt = (MODE == 1 && a.key_kind == 2) ? (1u << 7) | (1u << 10) : 0u;
+      const uint32_t idesc = (2u << 4) | i8fmt | ((nt >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       uint32_t done = 0;
       for (uint32_t kb = 0; kb < n_kb; kb++) {
         const uint32_t s = kb % kTcStages, it = kb / kTcStages;
@@ -272,13 +274,10 @@ __device__ __forceinline__ void tc_scan_body(const CUtensorMap& lut_map, const T
           __syncwarp();
         }
 #pragma unroll
-        for (uint32_t c = 0; c < 4; c++) {  // 16 coordinates per 16-byte chunk
-          const uint32_t h = (uint32_t)(wd >> (16 * c));
-          uint32_t o[4];
-#pragma unroll
-          for (uint32_t i = 0; i < 4; i++)  // 4 bits -> 4 bytes (the shifted copies never overlap)
-            o[i] = (((h >> (4 * i)) & 15u) * 0x00204081u) & 0x01010101u;
-          st_shared_v4(dst[c] + base, o[0], o[1], o[2], o[3]);
+        for (uint32_t c = 0; c < 4; c++) {  // half a word per 32 bytes, in expand_query_bits_kernel's order
+          const uint32_t h = (uint32_t)(wd >> (32 * (c >> 1))) >> (4 * (c & 1));
+          st_shared_v4(dst[c] + base, h & 0x01010101u, (h >> 1) & 0x01010101u, (h >> 2) & 0x01010101u,
+                       (h >> 3) & 0x01010101u);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -379,7 +378,6 @@ __device__ __forceinline__ void tc_scan_body(const CUtensorMap& lut_map, const T
       const uint64_t doc = pb * 32 + lane;
       const uint64_t u = (uint64_t)blockIdx.x * kTcM + row;
       const bool valid = pb < n_blocks && doc < a.n;
-      const uint32_t dpop = (MODE == 1 && a.key_kind == 2) ? row_popcount(a, doc, valid) : 0u;
       const uint32_t taddr = tmem + ((lq * 32) << 16) + h * kAcc1Col;
       const bool any_exact = S.any_exact != 0;
       // filter list: the A stages are dead once acc_full has fired; each warp
@@ -395,7 +393,7 @@ __device__ __forceinline__ void tc_scan_body(const CUtensorMap& lut_map, const T
         tmem_ld32(taddr + cb, v);
         if (MODE == 1 && a.key_kind == 2) {
 #pragma unroll
-          for (uint32_t j = 0; j < 32; j++) v[j] = ham_y(v[j], dpop);
+          for (uint32_t j = 0; j < 32; j++) v[j] += kHamBias;
         }
         if (dense) {
 #pragma unroll
@@ -509,22 +507,28 @@ __global__ void query_popcount_kernel(const uint64_t* __restrict__ qbits, uint64
   out[q] = c;
 }
 
-// query bits (qpv u64 words per query) -> 0/1 bytes, row_bytes per query
+// Query bits (qpv u64 words per query) -> bytes of 1 and `clear` (0, or -1 for
+// sign bitmaps), row_bytes per query, zeros past the row.  Byte p of each half
+// word's 32 holds bit 8 (p % 4) + p / 4: the order in which the builders expand
+// doc rows with one shift and one mask per four bytes.
 __global__ void expand_query_bits_kernel(const uint64_t* __restrict__ qbits, uint64_t nq, uint32_t qpv,
-                                         uint32_t row_bytes, uint8_t* __restrict__ out) {
+                                         uint32_t row_bytes, uint8_t clear, uint8_t* __restrict__ out) {
   const uint64_t total = nq * (uint64_t)row_bytes;
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t q = t / row_bytes;
-    const uint32_t j = (uint32_t)(t % row_bytes);
-    out[t] = (j / 64 < qpv) ? (uint8_t)((qbits[q * qpv + j / 64] >> (j % 64)) & 1ull) : 0;
+    const uint32_t j = (uint32_t)(t % row_bytes), p = j % 32, bit = (j / 32 % 2) * 32 + 8 * (p % 4) + p / 4;
+    out[t] = j / 64 >= qpv ? 0 : ((qbits[q * qpv + j / 64] >> bit) & 1ull) ? 1 : clear;
   }
 }
 
-// query bits -> packed e2m1 nibbles (byte j: coordinate 2 j in the low nibble,
-// 2 j + 1 in the high one; 0b0010 = 1.0 where the bit is set), row_bytes per query
+// Query bits -> packed e2m1 nibbles, row_bytes per query, zeros past the row.
+// Nibble n of each half word's 32 holds bit 4 (n % 8) + n / 8, as the builders'
+// rows (st_nibbles), with the reciprocal of the value a set doc bit has there:
+// 2.0 (0b0100), 1.0 (0b0010), 0.5 (0b0001), 1.0 for n / 8 = 0..3.  A clear bit is
+// 0, or with `sign` the negative value (0b1000 set).
 __global__ void expand_query_nibbles_kernel(const uint64_t* __restrict__ qbits, uint64_t nq, uint32_t qpv,
-                                            uint32_t row_bytes, uint8_t* __restrict__ out) {
+                                            uint32_t row_bytes, bool sign, uint8_t* __restrict__ out) {
   const uint64_t total = nq * (uint64_t)row_bytes;
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -532,8 +536,12 @@ __global__ void expand_query_nibbles_kernel(const uint64_t* __restrict__ qbits, 
     const uint32_t j = (uint32_t)(t % row_bytes);
     uint32_t v = 0;
     if (j / 32 < qpv) {
-      const uint32_t two = (uint32_t)(qbits[q * qpv + j / 32] >> ((2 * j) % 64)) & 3u;
-      v = ((two & 1u) ? 0x02u : 0u) | ((two & 2u) ? 0x20u : 0u);
+      const uint32_t h = (uint32_t)(qbits[q * qpv + j / 32] >> (32 * (j / 16 % 2)));
+#pragma unroll
+      for (uint32_t i = 0; i < 2; i++) {
+        const uint32_t n = 2 * (j % 16) + i, one = (0x2124u >> (4 * (n / 8))) & 15u;
+        v |= (((h >> (4 * (n % 8) + n / 8)) & 1u) ? one : sign ? one | 8u : 0u) << (4 * i);
+      }
     }
     out[t] = (uint8_t)v;
   }
@@ -656,20 +664,21 @@ void launch_fastscan_filter_tc(const uint8_t* blocks, uint64_t n, uint32_t pairs
 uint32_t bitmap_tc_kblocks(uint32_t qpv) { return (qpv + 1) / 2; }
 uint32_t bitmap_fp4_kblocks(uint32_t qpv) { return (qpv + 3) / 4; }
 
-// The bitmap filter runs on the FP4 tensor cores when its rows fit the FP4
-// form and the bitmap family runs on CTA pairs; OVB_BITMAP_FP4=0 keeps int8.
+// The bitmap filter runs on the FP4 tensor cores when the bitmap family runs on
+// CTA pairs; OVB_BITMAP_FP4=0 keeps int8.
 bool bitmap_fp4_usable(uint32_t qpv) {
   const char* e = getenv("OVB_BITMAP_FP4");
   if (e && e[0] == '0') return false;
   return qpv >= 1 && qpv <= tc_fp4_max_words() && tc_form(1) == TcForm::kPair;
 }
 
-void launch_bitmap_fp4_query(const uint64_t* qbits, uint64_t nq, uint32_t qpv, uint8_t* out, cudaStream_t stream) {
+void launch_bitmap_fp4_query(const uint64_t* qbits, uint64_t nq, uint32_t qpv, bool sign, uint8_t* out,
+                             cudaStream_t stream) {
   if (!nq) return;
   const uint32_t row = bitmap_fp4_kblocks(qpv) * kTcKBytes;
   uint64_t blocks = (nq * row + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  expand_query_nibbles_kernel<<<(unsigned)blocks, 256, 0, stream>>>(qbits, nq, qpv, row, out);
+  expand_query_nibbles_kernel<<<(unsigned)blocks, 256, 0, stream>>>(qbits, nq, qpv, row, sign, out);
   launched();
 }
 
@@ -679,7 +688,7 @@ void launch_bitmap_tc_query(const uint64_t* qbits, uint64_t nq, uint32_t qpv, ui
   const uint32_t row = bitmap_tc_kblocks(qpv) * kTcKBytes;
   uint64_t blocks = (nq * row + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  expand_query_bits_kernel<<<(unsigned)blocks, 256, 0, stream>>>(qbits, nq, qpv, row, out);
+  expand_query_bits_kernel<<<(unsigned)blocks, 256, 0, stream>>>(qbits, nq, qpv, row, qpop ? 0xFF : 0, out);
   launched();
   if (qpop) {
     query_popcount_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, stream>>>(qbits, nq, qpv, qpop);

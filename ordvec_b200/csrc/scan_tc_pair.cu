@@ -15,17 +15,20 @@
 // t % q_tiles (query tiles inner: a doc tile's codes are reused from L2).
 //
 // Warp roles (704 threads per CTA):
-//   warp 0, lane 0   TMA producer: this CTA's nt/2 B rows of K-block kb ->
-//                    stage s (waits its own empty[s]; complete_tx on the
-//                    leader's full_b[s], whose expect_tx the leader posts for
-//                    both halves)
-//   warp 1           TMEM allocation for the pair (both CTAs); on the leader,
-//                    lane 0 issues the MMAs: waits the leader's full_a[s] /
-//                    full_b[s], 4 MMAs per K-block, commits to both CTAs'
-//                    empty[s]; after a tile's last K-block commits to both
-//                    CTAs' acc_full[b]; before a tile waits acc_empty[b]
-//   warps 2..5       A builders (both CTAs): a thread per doc row, 8 chunks
-//                    per K-block, one arrive per warp on the leader's full_a[s]
+//   warp 0, lane 0   TMA producer: this CTA's nt/2 B rows of K-block kb -> its
+//                    stage (waits its own empty_b; complete_tx on the leader's
+//                    full_b, whose expect_tx the leader posts for both halves)
+//   warp 1           TMEM allocation for the pair (both CTAs); on the leader the
+//                    warp walks the K-blocks and one elected lane issues: 4 MMAs
+//                    and a commit to both CTAs' empty_b per K-block, a commit to
+//                    both CTAs' acc_full[b] per tile; before a tile it waits
+//                    acc_empty[b].  The warp, not one lane, runs the loop: the
+//                    descriptors then stay in uniform registers (a lane's own
+//                    loop spends 990 clocks a K-block issuing, this one 350)
+//   warps 2..5       A builders (both CTAs).  Bitmap rows: a warp a K-block, four
+//                    K-blocks at a time; FastScan: all four warps every K-block.
+//                    Ring mode: A slot and B stage of a K-block share the leader's
+//                    full_b and empty_b; resident A has its own full_a / empty_a
 //   warps 6..21      epilogue (both CTAs): TMEM lane quarter warp % 4, column
 //                    quarter (warp - 6) / 4; after reading the accumulator one
 //                    arrive per warp on the leader's acc_empty[b]
@@ -36,15 +39,18 @@
 // Results are the one-CTA kernel's (scan_fastscan_tc.cu), bit for bit: same
 // integer accumulators, same key functions and filter rules.
 //
-// The bitmap filter also runs on the FP4 tensor cores (MODE 2): a set bit is
-// the e2m1 value 1.0 (nibble 0b0010), a clear one 0, so an MMA of K=64 packed
-// nibbles (kind::mxf4, every ue8m0 block scale 1) sums 64 products of 0/1 into
-// an f32 accumulator, exact for overlaps below 2^24, at twice the int8 rate and
-// with half the operand bytes.  The scale factors sit in tensor-memory columns
+// The bitmap filter also runs on the FP4 tensor cores (MODE 2): a set bit is an
+// e2m1 value and the query's the reciprocal one, a clear one 0 (-1 times it in a
+// sign query), so an MMA of K=64 packed nibbles (kind::mxf4, every ue8m0 block
+// scale 1) sums 64 products of 0 and +-1 into an f32 accumulator, exact for sums
+// below 2^24, at twice the int8 rate and with half the operand bytes.
+// Measured (filter scan, before this form of issuer, builders and epilogue and
+// now): 10M docs x 768 bits x 1,024 queries 6.79 -> 5.29 ms, epilogue-bound; 1M x
+// 1,024 x 61 (sign) 507 -> 143 us and 1M x 3,072 x 256 (multi-bucket, int8 before)
+// 790 -> 553 us, both bound by the ring's round trip; FastScan 171,332 x 1,024 x
+// 1,000 1.01 -> 0.83 ms.  The scale factors sit in tensor-memory columns
 // [224, 256) (A) and [480, 512) (B), all bytes 127, past the two accumulators
-// of N <= 224 query columns; non-negative f32 values order like their bit
-// patterns, so the epilogue compares the accumulator bits with the f32 bits of
-// each query's integer threshold.
+// of N <= 224 query columns.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -62,13 +68,13 @@ namespace {
 using namespace tc;
 using namespace tcs;
 
-constexpr int kPBuildWarps = 4;  // warps 2..5: one thread per doc row
+constexpr int kPBuildWarps = 4;  // warps 2..5
 constexpr int kPEpiWarps = 16;   // warps 6..21: four per TMEM lane quarter
 constexpr int kPThreads = 32 * (2 + kPBuildWarps + kPEpiWarps);
 constexpr int kPEpiThreads = kPEpiWarps * 32;
 constexpr uint32_t kPMaxN = 256;
 constexpr uint32_t kPMaxQ = 1024;        // queries per launch of the pair form (per-query parameters staged once)
-constexpr uint32_t kPRowCacheWords = 16;  // bitmap rows of up to 16 words stay in the builders' registers
+constexpr uint32_t kPF4MaxWords = 4096;   // FP4 form: row length (f32 sums stay exact far beyond)
 constexpr uint32_t kPKBytes = 128;
 constexpr uint32_t kPTmemCols = 512;
 constexpr uint32_t kPF4MaxN = 224;                  // FP4 form: query columns per tile (scale factors above)
@@ -81,25 +87,31 @@ constexpr uint32_t kUnitScales = 0x7F7F7F7Fu;       // four ue8m0 bytes of 2^0
 // PAIR: CTA pairs, 128 doc rows per CTA, two 256-column accumulators.
 // !PAIR: one CTA per SM, 256 doc rows (two M=128 halves) in one 512-column
 // accumulator; the next tile's MMAs wait for the epilogue's TMEM reads only.
-template <bool PAIR>
+template <bool PAIR, bool F4 = false>
 struct PT {
   static constexpr uint32_t kRows = PAIR ? 128 : 256;  // doc rows per CTA per tile
   // A: K-block slots (pair form: a bitmap doc tile's whole row when it fits,
   // built once and read by all its query tiles; otherwise a ring); B: a ring
   static constexpr int kASlots = PAIR ? 6 : 3;
   static constexpr int kBStages = PAIR ? 4 : 3;
+  // FP4: B stages as deep as the tile's columns leave room for, up to the A slots
+  static constexpr int kMaxStages = F4 ? kASlots : kBStages;
   static constexpr uint32_t kSegCap = PAIR ? 128 : 192;  // kept entries per epilogue warp per tile
   static constexpr uint32_t kAStage = kRows * kPKBytes;
-  static constexpr uint32_t kBStage = (PAIR ? kPMaxN / 2 : kPMaxN) * kPKBytes;
+  static constexpr uint32_t kBStage = (F4 ? kPF4MaxN / 2 : PAIR ? kPMaxN / 2 : kPMaxN) * kPKBytes;
   static constexpr uint32_t kAccBufs = PAIR ? 2 : 1;
+  // bitmap rows: a K-block is kWords words of each row, kItems 16-byte pieces a
+  // lane of the warp that builds it
+  static constexpr uint32_t kWords = F4 ? 4 : 2;
+  static constexpr uint32_t kItems = kRows * (kWords / 2) / 32;
   static constexpr uint32_t kRowsPerThread = kRows / (kPBuildWarps * 32);
 };
 
-template <bool PAIR>
+template <bool PAIR, bool F4 = false>
 struct PSmem {
-  uint8_t a[PT<PAIR>::kASlots][PT<PAIR>::kAStage];
-  uint8_t b[PT<PAIR>::kBStages][PT<PAIR>::kBStage];
-  uint2 list[kPEpiWarps][PT<PAIR>::kSegCap];  // (accumulator, q | slot << 8 | row << 16)
+  uint8_t a[PT<PAIR, F4>::kASlots][PT<PAIR, F4>::kAStage];
+  uint8_t b[PT<PAIR, F4>::kBStages][PT<PAIR, F4>::kBStage];
+  uint2 list[kPEpiWarps][PT<PAIR, F4>::kSegCap];  // (accumulator, q | slot << 8 | row << 16)
   // one-CTA form: per-query parameters of the current tile
   static constexpr uint32_t kTileQ = PAIR ? 1 : kPMaxN;
   float bias[kTileQ];
@@ -113,14 +125,12 @@ struct PSmem {
   // pair form: per-query parameters of the launch, [amin | tdoc or bias | thr | qpop or invq]
   uint32_t qp[PAIR ? 4 * kPMaxQ : 1];
   uint32_t wamin[PAIR ? kPEpiWarps : 1][64];  // pair form: each epilogue warp's 64 column thresholds
-  // pair form, bitmap rows of <= kPRowCacheWords words: each builder thread's row
-  // of the current doc tile (pitch kPRowCacheWords + 1 words: a warp's 8-byte reads
-  // take the minimum two wavefronts)
-  uint64_t rowc[PAIR ? 128 : 1][kPRowCacheWords + 1];
-  uint64_t full_a[PT<PAIR>::kASlots];
-  uint64_t empty_a[PT<PAIR>::kASlots];
-  uint64_t full_b[PT<PAIR>::kBStages];
-  uint64_t empty_b[PT<PAIR>::kBStages];
+  // pair form: the row words of each builder warp's next K-block
+  uint4 raw[PAIR ? kPBuildWarps : 1][PAIR ? PT<PAIR, F4>::kItems : 1][PAIR ? 32 : 1];
+  uint64_t full_a[PT<PAIR, F4>::kASlots];
+  uint64_t empty_a[PT<PAIR, F4>::kASlots];
+  uint64_t full_b[PT<PAIR, F4>::kMaxStages];
+  uint64_t empty_b[PT<PAIR, F4>::kMaxStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem;
@@ -160,14 +170,14 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // waiter suspended for long wakes late and the tensor pipe idles meanwhile)
 __device__ __forceinline__ bool mbar_wait_issuer(uint64_t* bar, uint32_t parity) { return mbar_wait_spin(bar, parity); }
 
-template <bool PAIR>
-__device__ __forceinline__ bool aborted(const PSmem<PAIR>& S) {
+template <bool PAIR, bool F4>
+__device__ __forceinline__ bool aborted(const PSmem<PAIR, F4>& S) {
   return *reinterpret_cast<const volatile uint32_t*>(&S.abort) != 0;
 }
 
 // Sets the abort flag of the CTA (and of its pair) and bit 0 of *err.
-template <bool PAIR>
-__device__ __forceinline__ void raise_abort(PSmem<PAIR>& S, uint32_t* err) {
+template <bool PAIR, bool F4>
+__device__ __forceinline__ void raise_abort(PSmem<PAIR, F4>& S, uint32_t* err) {
   atomicExch(&S.abort, 1u);
   if (PAIR)
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_addr(smem_u32(&S.abort), cta_rank() ^ 1)), "r"(1u)
@@ -217,15 +227,21 @@ __device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t w) {
       : "memory");
 }
 
-// Bits 0..7 of x -> eight nibbles, nibble i = e2m1 1.0 (0b0010) where bit i is
-// set and 0 elsewhere (bit i moves to bit 4 i + 1; the shifted copies never
-// overlap, so no carries).
-__device__ __forceinline__ uint32_t fp4_ones8(uint32_t x) {
-  uint32_t v = x & 0xFFu;
-  v = (v | (v << 12)) & 0x000F000Fu;
-  v = (v | (v << 6)) & 0x03030303u;
-  v = (v | (v << 3)) & 0x11111111u;
-  return v << 1;
+// Half a word (32 bits of a bitmap row) -> 32 e2m1 nibbles (16 bytes): word s of
+// the four holds bits 4 y + s (y = 0..7) in its nibbles, each bit left in place
+// where it can be: set, it reads 0.5 (s = 0), 1.0 (s = 1, 3) or 2.0 (s = 2).  The
+// query operand is laid out the same way with the reciprocal values
+// (expand_query_nibbles_kernel), so every product is 0 or +-1, and a dot product
+// does not depend on the order of its terms.
+__device__ __forceinline__ void st_nibbles(uint32_t addr, uint32_t h) {
+  st_shared_v4(addr, h & 0x11111111u, h & 0x22222222u, h & 0x44444444u, (h >> 2) & 0x22222222u);
+}
+
+// Chunk k (0, 1) of half a word's 32 bytes of 0/1: byte p of the 32 holds bit
+// 8 (p % 4) + p / 4 (expand_query_bits_kernel's order).
+__device__ __forceinline__ void st_bytes(uint32_t addr, uint32_t h, uint32_t k) {
+  h >>= 4 * k;
+  st_shared_v4(addr, h & 0x01010101u, (h >> 1) & 0x01010101u, (h >> 2) & 0x01010101u, (h >> 3) & 0x01010101u);
 }
 
 // v[j] by a 5-level select tree on the bits of j (no local-memory indexing)
@@ -242,10 +258,15 @@ __device__ __forceinline__ uint32_t pick32(const uint32_t (&v)[32], uint32_t j) 
   return (j & 16) ? t2[1] : t2[0];
 }
 
-// The integer value of an f32 accumulator holding an integer in [0, 2^23)
-// (add 2^23: the integer lands in the mantissa bits).
-__device__ __forceinline__ uint32_t f4_int(uint32_t bits) {
-  return __float_as_uint(__fadd_rn(__uint_as_float(bits), 8388608.0f)) & 0x7FFFFFu;
+// The f32 an FP4 accumulator is compared with for an integer bound (exact: the
+// sums stay below 2^23; sign bitmaps carry kHamBias).
+__device__ __forceinline__ float f4_bound(const TcArgs& a, uint32_t am) {
+  return (float)((int)am - (a.key_kind == 2 ? (int)kHamBias : 0));
+}
+
+// The (biased) integer of an FP4 accumulator.
+__device__ __forceinline__ uint32_t f4_int(const TcArgs& a, uint32_t bits) {
+  return (uint32_t)__float2int_rn(__uint_as_float(bits)) + (a.key_kind == 2 ? kHamBias : 0u);
 }
 
 // Arrive-one on the barrier at the same shared-memory offset in both CTAs of
@@ -307,42 +328,51 @@ struct TileCursor {
 
 template <int MODE, bool PAIR>
 __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs& a, const PairGrid g) {
-  using T = PT<PAIR>;
   constexpr bool BM = MODE != 0, F4 = MODE == 2;  // bitmap rows; on the FP4 tensor cores
+  using T = PT<PAIR, F4>;
   static_assert(!F4 || PAIR, "the FP4 bitmap form runs on CTA pairs");
-  constexpr int kASlots = T::kASlots, kBStages = T::kBStages;
+  constexpr int kASlots = T::kASlots;
   constexpr uint32_t kPRows = T::kRows, kPSegCap = T::kSegCap, kBufs = T::kAccBufs;
   extern __shared__ uint8_t smem_raw[];
-  PSmem<PAIR>& S =
-      *reinterpret_cast<PSmem<PAIR>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  PSmem<PAIR, F4>& S =
+      *reinterpret_cast<PSmem<PAIR, F4>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int t = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, t >> 5, 0), lane = t & 31;
   const uint32_t rank = PAIR ? cta_rank() : 0u;
   // a "cluster" is a pair of CTAs, or one CTA
   const uint32_t cluster = PAIR ? blockIdx.x >> 1 : blockIdx.x, n_clusters = PAIR ? gridDim.x >> 1 : gridDim.x;
   const uint32_t nt = a.nt, half = nt / 2;
   const uint32_t n_kb = a.n_kb;
+  // B stages: a ring that wide tiles fill with kBStages, narrow FP4 tiles with more
+  const uint32_t b_stage = F4 ? nt / 2 * kPKBytes : T::kBStage;
+  const uint32_t n_st = F4 ? min((uint32_t)T::kMaxStages, (uint32_t)sizeof(S.b) / b_stage) : (uint32_t)T::kBStages;
+  auto b_addr = [&](uint32_t st) -> uint8_t* { return &S.b[0][0] + st * b_stage; };
   const uint64_t n_blocks = (a.n + 31) / 32;
   const bool dense = a.keys != nullptr;
-  // FP4 form: filter only, rows held in the builders' row cache (host-checked;
-  // a launch that breaks either does no work and sets bit 0 of *err)
-  if (F4 && (dense || a.qpv > kPRowCacheWords || nt > kPF4MaxN)) {
+  // FP4 form: filter only (host-checked; a launch that breaks a limit does no
+  // work and sets bit 0 of *err)
+  if (F4 && (dense || a.qpv > kPF4MaxWords || nt > kPF4MaxN)) {
     if (t == 0 && blockIdx.x == 0) atomicOr(a.err, 1u);
     return;
   }
   // A resident per doc tile: built once, read by the doc tile's q_tiles
-  // consecutive tiles (whole doc tiles per cluster, rows of <= 12 words)
-  const bool resA = PAIR && BM && g.doc_major && n_kb <= (uint32_t)kASlots && a.qpv <= kPRowCacheWords;
+  // consecutive tiles (whole doc tiles per cluster, rows that fit the slots).
+  // A lone query tile takes the ring: its K-blocks free one by one.
+  const bool resA = PAIR && BM && g.doc_major && g.q_tiles > 1 && n_kb <= (uint32_t)kASlots;
   // resident A in two halves when two doc tiles fit: the builders build the
   // next doc tile's rows while the MMAs read the current one's
   const bool resA2 = resA && 2 * n_kb <= (uint32_t)kASlots;
 
+  // builder warps that arrive for a K-block: one a CTA (bitmap rows), or all
+  const uint32_t build_arrivals = (PAIR ? 2 : 1) * (BM ? 1 : kPBuildWarps);
   if (t == 32) {
     for (int s = 0; s < kASlots; s++) {
-      mbar_init(&S.full_a[s], (PAIR ? 2 : 1) * kPBuildWarps);  // builder warps of both CTAs
-      mbar_init(&S.empty_a[s], 1);                             // the leader's MMA commit
+      mbar_init(&S.full_a[s], build_arrivals);  // resident A: builder warps of both CTAs
+      mbar_init(&S.empty_a[s], 1);              // ... and the leader's MMA commit
     }
-    for (int s = 0; s < kBStages; s++) {
-      mbar_init(&S.full_b[s], 1);   // the leader's expect_tx
+    for (uint32_t s = 0; s < n_st; s++) {
+      // the leader's expect_tx, and in ring mode the builder warps: A slot s and
+      // B stage s of a K-block share both barriers (one wait, one commit)
+      mbar_init(&S.full_b[s], 1 + (resA ? 0 : build_arrivals));
       mbar_init(&S.empty_b[s], 1);  // the leader's MMA commit
     }
     for (int b = 0; b < 2; b++) {
@@ -390,128 +420,135 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
   if (warp == 0) {
     // ---- TMA producer (both CTAs) ----------------------------------------------
     if (lane == 0) {
-      uint64_t it = 0;  // K-blocks issued
+      uint32_t st = 0, use = 0, issued = 0;  // stage of the next K-block, rounds of the ring, K-blocks issued
       TileCursor tc_;
       for (tc_.start(g, cluster); tc_.valid(g) && !aborted(S); tc_.next(g, n_clusters)) {
         const uint64_t q0 = (uint64_t)tc_.qt * nt;
-        for (uint32_t kb = 0; kb < n_kb; kb++, it++) {
-          const uint32_t s = (uint32_t)(it % kBStages);
+        for (uint32_t kb = 0; kb < n_kb; kb++) {
           if (aborted(S)) break;
-          if (it >= (uint64_t)kBStages && !mbar_wait_issuer(&S.empty_b[s], (uint32_t)((it / kBStages - 1) & 1))) {
+          if (use && !mbar_wait_issuer(&S.empty_b[st], (use - 1) & 1)) {
             raise_abort(S, a.err);
             break;
           }
-          if (rank == 0) mbar_expect_tx(&S.full_b[s], nt * kPKBytes);  // both halves
+          if (rank == 0) mbar_expect_tx(&S.full_b[st], nt * kPKBytes);  // both halves
           if (PAIR)
-            tma_load_2d_pair(S.b[s], &b_map, (int)(kb * kPKBytes), (int)(q0 + rank * half),
-                             peer_addr(smem_u32(&S.full_b[s]), 0));
+            tma_load_2d_pair(b_addr(st), &b_map, (int)(kb * kPKBytes), (int)(q0 + rank * half),
+                             peer_addr(smem_u32(&S.full_b[st]), 0));
           else
-            tma_load_2d(S.b[s], &b_map, (int)(kb * kPKBytes), (int)q0, &S.full_b[s]);
+            tma_load_2d(b_addr(st), &b_map, (int)(kb * kPKBytes), (int)q0, &S.full_b[st]);
+          if (issued < n_st) issued++;
+          if (++st == n_st) {
+            st = 0;
+            use++;
+          }
         }
       }
       // the leader waits (bounded) until its last copies, and the peer's, landed
       if (rank == 0)
-        for (uint64_t j = it > (uint64_t)kBStages ? it - kBStages : 0; j < it; j++)
-          mbar_wait_cluster(&S.full_b[j % kBStages], (uint32_t)((j / kBStages) & 1));
+        for (; issued; issued--) {
+          const bool prev = st < issued;  // the stage's last K-block was in the previous round
+          const uint32_t s2 = prev ? st + n_st - issued : st - issued;
+          mbar_wait_cluster(&S.full_b[s2], (prev ? use - 1 : use) & 1);
+        }
     }
   } else if (warp == 1) {
-    // ---- MMA issuer (leader) ------------------------------------------------------
-    if (lane == 0 && rank == 0) {
+    // ---- MMA issuer (leader): the whole warp walks, one lane issues ----------------
+    if (rank == 0) {
+      const bool el = elect_one();
       // i8: D s32, A/B u8, K-major, N = nt; M = 256 across the pair, or two M = 128 halves.
       // FP4: A/B e2m1 (format 1), K-major, ue8m0 scales (bit 23), scale ids 0, K = 64, D f32
+      // sign bitmaps' queries are +-1: both operands s8
+      const uint32_t i8fmt = (BM && a.key_kind == 2) ? (1u << 7) | (1u << 10) : 0u;
       const uint32_t idesc = F4 ? (1u << 7) | (1u << 10) | ((nt >> 3) << 17) | (1u << 23) | (16u << 24)
-                                : (2u << 4) | ((nt >> 3) << 17) | ((uint32_t)((PAIR ? 256 : 128) >> 4) << 24);
-      uint64_t it = 0, issued = 0;  // B K-blocks issued, last issued B K-block + 1
-      uint32_t rb_s = 0, rb_p = 0, ra_s = 0, ra_p = 0;  // B ring / A ring: slot and phase of the next K-block
+                                : (2u << 4) | i8fmt | ((nt >> 3) << 17) | ((uint32_t)((PAIR ? 256 : 128) >> 4) << 24);
+      // a slot, and a 32-byte K step (2), advance the descriptors' start-address
+      // field (16-byte units; shared addresses stay below its 2^18 bytes)
+      const uint64_t a_desc0 = sw128_desc(smem_u32(S.a[0])), b_desc0 = sw128_desc(smem_u32(b_addr(0)));
+      auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+        return __all_sync(0xFFFFFFFFu, mbar_wait_issuer(bar, parity));
+      };
+      uint32_t rs = 0, rp = 0;  // B stage (ring mode: and A slot) of the next K-block, and its phase
       uint32_t tcount = 0;
-      bool ok = true;
+      bool ok = true, any = false;
       TileCursor tc_;
       for (tc_.start(g, cluster); tc_.valid(g) && ok; tc_.next(g, n_clusters), tcount++) {
         const uint32_t b = tcount % kBufs;
         // resident A: this doc tile's slots and their phase
         const uint32_t a_base = resA2 ? (tc_.di & 1) * n_kb : 0u;
-        const uint32_t pa_res = (resA2 ? tc_.di >> 1 : tc_.di) & 1;
-        const bool last_q = tc_.qt + 1 == g.q_tiles;  // resident A: its last reader
-        if (tcount >= kBufs && !mbar_wait_issuer(&S.acc_empty[b], (tcount / kBufs - 1) & 1)) ok = false;
+        const uint32_t pa = (resA2 ? tc_.di >> 1 : tc_.di) & 1;
+        // resident A: after the doc tile's first query tile its slots are known
+        // full (nothing refills them before its last query tile frees them)
+        const bool need_a = resA && tc_.qt == 0, free_a = resA && tc_.qt + 1 == g.q_tiles;
+        if ((tcount >= kBufs && !wait(&S.acc_empty[b], (tcount / kBufs - 1) & 1)) ||
+            __any_sync(0xFFFFFFFFu, aborted(S))) {
+          ok = false;
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem + b * 256;
-        for (uint32_t kb = 0; kb < n_kb && ok; kb++, it++) {
-          const uint32_t sb = rb_s, pb = rb_p;
-          const uint32_t sa = resA ? a_base + kb : ra_s;
-          const uint32_t pa = resA ? pa_res : ra_p;
-          // resident A: after the doc tile's first query tile its slots are known
-          // full (nothing refills them before its last query tile frees them)
-          const bool need_a = !resA || tc_.qt == 0;
-          if ((kb == 0 && aborted(S)) || !mbar_wait_issuer(&S.full_b[sb], pb) ||
-              (need_a && !mbar_wait_issuer(&S.full_a[sa], pa))) {
+        for (uint32_t kb = 0; kb < n_kb; kb++) {
+          const uint32_t sa = resA ? a_base + kb : rs;
+          if (!wait(&S.full_b[rs], rp) || (need_a && !wait(&S.full_a[sa], pa))) {
             ok = false;
             break;
           }
           // (operands arrive by TMA, or by builder stores behind a proxy fence and
           // the barrier: no tcgen05 fence is needed before reading them)
-          if (!PAIR) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a0 = smem_u32(S.a[sa]), b0 = smem_u32(S.b[sb]);
-          const bool free_a = !resA || last_q;
-          if (PAIR) {
-            // a 32-byte K step adds 2 to the descriptor's start-address field (16-byte units)
-            const uint64_t ad = sw128_desc(a0), bd = sw128_desc(b0);
-            if constexpr (F4) {
-#pragma unroll
-              for (uint32_t j = 0; j < 4; j++)
-                mma_mxf4_pair(d, ad + 2 * j, bd + 2 * j, idesc, (kb | j) != 0, tmem + kSfaCol, tmem + kSfbCol);
-            } else {
-#pragma unroll
-              for (uint32_t j = 0; j < 4; j++) mma_i8_pair(d, ad + 2 * j, bd + 2 * j, idesc, (kb | j) != 0);
-            }
-            commit_both(smem_u32(&S.empty_b[sb]));
-            if (free_a) commit_both(smem_u32(&S.empty_a[sa]));
-          } else {
+          const uint64_t ad = a_desc0 + sa * (T::kAStage >> 4), bd = b_desc0 + rs * (b_stage >> 4);
+          if (el) {
 #pragma unroll
             for (uint32_t j = 0; j < 4; j++) {
-              const uint64_t bd = sw128_desc(b0 + 32 * j);
-              mma_i8(d, sw128_desc(a0 + 32 * j), bd, idesc, (kb | j) != 0);
-              mma_i8(d + 256, sw128_desc(a0 + kPRows / 2 * kPKBytes + 32 * j), bd, idesc, (kb | j) != 0);
+              if constexpr (F4) {
+                mma_mxf4_pair(d, ad + 2 * j, bd + 2 * j, idesc, (kb | j) != 0, tmem + kSfaCol, tmem + kSfbCol);
+              } else if constexpr (PAIR) {
+                mma_i8_pair(d, ad + 2 * j, bd + 2 * j, idesc, (kb | j) != 0);
+              } else {
+                mma_i8(d, ad + 2 * j, bd + 2 * j, idesc, (kb | j) != 0);
+                mma_i8(d + 256, ad + (kPRows / 2 * kPKBytes >> 4) + 2 * j, bd + 2 * j, idesc, (kb | j) != 0);
+              }
             }
-            mma_commit(&S.empty_b[sb]);
-            mma_commit(&S.empty_a[sa]);
+            if (PAIR) {
+              commit_both(smem_u32(&S.empty_b[rs]));
+              if (free_a) commit_both(smem_u32(&S.empty_a[sa]));
+            } else {
+              mma_commit(&S.empty_b[rs]);
+            }
           }
-          if (!resA && ++ra_s == (uint32_t)kASlots) {
-            ra_s = 0;
-            ra_p ^= 1;
+          __syncwarp();
+          any = true;
+          if (++rs == n_st) {
+            rs = 0;
+            rp ^= 1;
           }
-          if (++rb_s == (uint32_t)kBStages) {
-            rb_s = 0;
-            rb_p ^= 1;
-          }
-          issued = it + 1;
         }
         if (!ok) break;
-        if (PAIR) {
-          commit_both(smem_u32(&S.acc_full[b]));
-        } else {
-          mma_commit(&S.acc_full[b]);
+        if (el) {
+          if (PAIR)
+            commit_both(smem_u32(&S.acc_full[b]));
+          else
+            mma_commit(&S.acc_full[b]);
         }
+        __syncwarp();
       }
       if (!ok) {
-        if (!aborted(S)) raise_abort(S, a.err);
+        if (el && !aborted(S)) raise_abort(S, a.err);
         // no MMA in flight when the pair frees its tensor memory
-        if (issued > 0)
-          mbar_wait(&S.empty_b[(issued - 1) % kBStages], (uint32_t)(((issued - 1) / kBStages) & 1));
+        if (any) mbar_wait(&S.empty_b[rs ? rs - 1 : n_st - 1], rs ? rp : rp ^ 1);
+        __syncwarp();
       }
     }
   } else if (warp < 2 + kPBuildWarps) {
     // ---- A builders: thread r builds doc rows r + 128 i (i < kRowsPerThread), chunks 0..7
     constexpr uint32_t R = T::kRowsPerThread;
     const uint32_t r = (uint32_t)t - 64;  // 0..127
-    // leader's full_a[0] (a cluster address; the CTA's own barrier when alone)
-    const uint32_t full_a0 = PAIR ? peer_addr(smem_u32(&S.full_a[0]), 0) : 0u;
-    uint64_t it = 0;
-    bool ok = true;
-    // wait for A ring slot s to be free, or stop (warp-uniform)
-    auto acquire = [&](uint32_t s) -> bool {
+    // leader's barriers of slot 0 (cluster addresses; the CTA's own when alone)
+    uint64_t* const full0 = resA ? &S.full_a[0] : &S.full_b[0];
+    const uint32_t full0_peer = PAIR ? peer_addr(smem_u32(full0), 0) : 0u;
+    // wait for A ring slot s to be free of its `use` earlier K-blocks, or stop (warp-uniform)
+    auto acquire = [&](uint32_t s, uint32_t use) -> bool {
       bool w = true;
-      if (it >= (uint64_t)kASlots) {
-        if (lane == 0) w = !aborted(S) && mbar_wait_issuer(&S.empty_a[s], (uint32_t)((it / kASlots - 1) & 1));
+      if (use) {
+        if (lane == 0) w = !aborted(S) && mbar_wait_issuer(&S.empty_b[s], (use - 1) & 1);
         w = __shfl_sync(0xFFFFFFFFu, w, 0);
         if (!w && lane == 0 && !aborted(S)) raise_abort(S, a.err);
         __syncwarp();
@@ -523,156 +560,196 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
       __syncwarp();
       if (lane == 0) {
         if (PAIR)
-          arrive_remote(full_a0 + 8 * s);
+          arrive_remote(full0_peer + 8 * s);
         else
-          mbar_arrive(&S.full_a[s]);
+          mbar_arrive(full0 + s);
       }
     };
-    uint64_t cached_dt = ~0ull;  // pair form, bitmap rows <= 16 words: doc tile of S.rowc
+    if constexpr (BM) {
+      // K-block kb = words [WPK kb, +WPK) of the rows.  A K-block is built whole by
+      // one warp: its chain of wait, loads, stores, fence and arrival takes about
+      // 1,100 clocks whatever the rows, and four K-blocks are in that chain at once.
+      // A parity wait must not be two phases ahead of its barrier.  In ring mode
+      // the warps take turns: K-block i waits for i - n_st, and the warp's previous
+      // one (i - 4) waited for i - 4 - n_st, at or after the phase before (i - 2 n_st)
+      // as long as there are no more warps than stages.  Resident slots belong to
+      // a warp each (slot % 4).  In the pair form the words of a warp's next K-block
+      // come by cp.async, which neither holds registers nor is waited for by the
+      // fences and arrivals, and L2 is warmed with the tile after.
+      constexpr uint32_t WPK = T::kWords, P = WPK / 2, ITEMS = T::kItems;
+      const bool vec = a.qpv % 2 == 0;  // rows start 16-byte aligned
+      const uint32_t bw = (uint32_t)warp - 2;
+      // Item i of a lane: row i * 32 / P + lane / P, 16-byte piece lane % P of the
+      // K-block.  Rows of a 32-doc block are contiguous, blocks block_stride apart.
+      const uint32_t lane_row = lane / P, piece = lane % P;
+      const uint64_t row_bytes = (uint64_t)a.qpv * 8, blk_bytes = 32 * row_bytes * a.block_stride;
+      const uint32_t blk_docs = 32 * a.block_stride;
+      // this CTA's first doc of a tile, and the docs left from there (0: none)
+      auto tile_docs = [&](uint64_t dt, uint64_t& first) -> uint32_t {
+        first = (dt * 8 + rank * (kPRows / 32)) * blk_docs;
+        return first < a.n ? (uint32_t)(a.n - first < 0xFFFFFFFFull ? a.n - first : 0xFFFFFFFFull) : 0u;
+      };
+      // rows are built once per doc tile when A is resident
+      auto step = [&](TileCursor& c) {
+        if (resA) {
+          c.dt += n_clusters;
+          c.di++;
+        } else {
+          c.next(g, n_clusters);
+        }
+      };
+      constexpr uint32_t NBW = PAIR ? kPBuildWarps : 3;  // warps that take turns in ring mode
+      static_assert(NBW <= (uint32_t)T::kBStages && NBW <= (uint32_t)kPBuildWarps, "ring mode: turns");
+      // The warp's walk over its K-blocks: ring slot, the slot's earlier uses.
+      struct Walk {
+        TileCursor c;
+        uint32_t kb, slot, use;
+      };
+      auto settle = [&](Walk& w) {  // kb past the row: on to the tile it falls into
+        while (w.kb >= n_kb && w.c.valid(g)) {
+          step(w.c);
+          w.kb = resA ? (bw + 4 * 16 - (resA2 ? (w.c.di & 1) * n_kb : 0u)) % kPBuildWarps : w.kb - n_kb;
+        }
+      };
+      auto advance = [&](Walk& w) {
+        w.kb += resA ? (uint32_t)kPBuildWarps : NBW;
+        w.slot += NBW;
+        if (w.slot >= n_st) {
+          w.slot -= n_st;
+          w.use++;
+        }
+        settle(w);
+      };
+      Walk bk, lk;  // build walk and load walk
+      bk.c.start(g, cluster);
+      bk.kb = bk.slot = bw;
+      bk.use = 0;
+      if (!resA && bw >= NBW) bk.c.dt = g.n_doc_tiles;  // no turns
+      settle(bk);
+      uint64_t warmed = ~0ull;
+      auto load = [&]() {  // the load walk's K-block; words past the row are zero
+        if (lk.c.valid(g)) {
+          uint64_t first;
+          const uint32_t left = tile_docs(lk.c.dt, first), wi = lk.kb * WPK + 2 * piece;
+          const uint8_t* base = a.blocks + first * row_bytes + lane_row * row_bytes + wi * 8;
+          const uint32_t dst = smem_u32(&S.raw[bw][0][lane]);
+#pragma unroll
+          for (uint32_t i = 0; i < ITEMS; i++) {
+            const uint32_t blk = i / P, in_blk = i % P * (32 / P);  // rows before this item's
+            const bool row_ok = blk * blk_docs + in_blk + lane_row < left;
+            const uint8_t* p = base + blk * blk_bytes + in_blk * row_bytes;
+            if (vec) {
+              const bool any = row_ok && wi < a.qpv;
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * 512),
+                           "l"(any ? p : a.blocks), "r"(any ? 16u : 0u)
+                           : "memory");
+            } else {
+#pragma unroll
+              for (uint32_t y = 0; y < 2; y++) {
+                const bool any = row_ok && wi + y < a.qpv;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + i * 512 + 8 * y),
+                             "l"(any ? p + 8 * y : a.blocks), "r"(any ? 8u : 0u)
+                             : "memory");
+              }
+            }
+          }
+          if (lk.c.dt != warmed) {  // the next tile's rows, a block a warp
+            warmed = lk.c.dt;
+            TileCursor nx = lk.c;
+            step(nx);
+            if (nx.valid(g) && nx.dt != lk.c.dt) {
+              const uint32_t nleft = tile_docs(nx.dt, first);
+#pragma unroll
+              for (uint32_t blk = bw; blk < kPRows / 32; blk += kPBuildWarps) {
+                if (blk * blk_docs + lane >= nleft) break;
+                const uint8_t* p = a.blocks + (first + (uint64_t)blk * blk_docs + lane) * row_bytes;
+                for (uint32_t o = 0; o < a.qpv * 8; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
+              }
+            }
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      if (PAIR) {
+        lk = bk;
+        load();
+      }
+      for (; bk.c.valid(g); advance(bk)) {
+        const uint32_t s = resA ? (resA2 ? (bk.c.di & 1) * n_kb : 0u) + bk.kb : bk.slot;
+        bool got = true;
+        if (resA) {
+          // earlier uses of this doc tile's slots (doc tiles this cluster
+          // started before, or of the same parity with two halves)
+          const uint32_t dc = resA2 ? bk.c.di >> 1 : bk.c.di;
+          if (dc > 0) {  // the slot's previous doc tile has been read by its last query tile
+            // (with two halves the builders run a doc tile ahead: they sleep
+            // rather than poll, leaving the issue slots to the epilogue and MMA warps)
+            if (lane == 0)
+              got = !aborted(S) && (resA2 ? mbar_wait(&S.empty_a[s], (dc - 1) & 1)
+                                          : mbar_wait_issuer(&S.empty_a[s], (dc - 1) & 1));
+            got = __shfl_sync(0xFFFFFFFFu, got, 0);
+            if (!got && lane == 0 && !aborted(S)) raise_abort(S, a.err);
+            __syncwarp();
+          }
+        } else {
+          got = acquire(s, bk.use);
+        }
+        if (!got) break;
+        if (PAIR) asm volatile("cp.async.wait_all;" ::: "memory");
+        // 128 bytes a row (8-row atoms of 1,024 bytes), 16-byte chunks swizzled by
+        // the row's low bits, which are the same for all of a lane's items
+        const uint32_t at = smem_u32(S.a[s]) + lane_row * 128, rr = lane_row & 7;
+#pragma unroll
+        for (uint32_t i = 0; i < ITEMS; i++) {
+          uint4 v;
+          if (PAIR) {
+            v = S.raw[bw][i][lane];
+          } else {
+            uint64_t first;
+            const uint32_t left = tile_docs(bk.c.dt, first), blk = i / P, in_blk = i % P * (32 / P);
+            const bool row_ok = blk * blk_docs + in_blk + lane_row < left;
+            const uint32_t wi = bk.kb * WPK + 2 * piece;
+            const uint64_t* p = reinterpret_cast<const uint64_t*>(
+                a.blocks + (first + (uint64_t)blk * blk_docs + in_blk + lane_row) * row_bytes + wi * 8);
+            const uint64_t x = row_ok && wi < a.qpv ? __ldg(p) : 0ull;
+            const uint64_t y = row_ok && wi + 1 < a.qpv ? __ldg(p + 1) : 0ull;
+            v = make_uint4((uint32_t)x, (uint32_t)(x >> 32), (uint32_t)y, (uint32_t)(y >> 32));
+          }
+          const uint32_t h[4] = {v.x, v.y, v.z, v.w};
+          const uint32_t to = at + i * (32 / P) * 128;
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++) {
+            const uint32_t half = 4 * piece + j;
+            if (F4) {
+              st_nibbles(to + ((half ^ rr) << 4), h[j]);
+            } else {
+              st_bytes(to + (((2 * half) ^ rr) << 4), h[j], 0);
+              st_bytes(to + (((2 * half + 1) ^ rr) << 4), h[j], 1);
+            }
+          }
+        }
+        publish(s);
+        if (PAIR) {  // after the words were read, and off the K-block's way to the MMAs
+          advance(lk);
+          load();
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+    uint32_t st = 0, use = 0;
+    bool ok = true;
     TileCursor tc_;
     for (tc_.start(g, cluster); tc_.valid(g) && ok; tc_.next(g, n_clusters)) {
       const uint64_t dt = tc_.dt;
-      const uint32_t qt_ = tc_.qt;
-      uint64_t pb[R], doc[R];
+      uint64_t pb[R];
       uint32_t a_row[R];  // row offset in a stage: 8-row atoms of 1024 bytes, 128 bytes a row
 #pragma unroll
       for (uint32_t i = 0; i < R; i++) {
         const uint32_t row = r + 128 * i;
         pb[i] = (dt * 8 + rank * (kPRows / 32) + (row >> 5)) * a.block_stride;
-        doc[i] = pb[i] * 32 + (row & 31);
         a_row[i] = (row >> 3) * 1024 + (row & 7) * 128;
       }
-      if constexpr (BM && PAIR) {
-        if (a.qpv <= kPRowCacheWords) {
-          // the row's words stay in registers while the doc tile's query tiles pass
-          if (dt != cached_dt) {
-            const bool row_ok = pb[0] < n_blocks && doc[0] < a.n;
-            const uint64_t* wp = reinterpret_cast<const uint64_t*>(a.blocks) + (row_ok ? doc[0] : 0) * (uint64_t)a.qpv;
-            // global -> shared without registers; words past the row (or of an
-            // invalid row) are zero-filled (source size 0)
-#pragma unroll
-            for (uint32_t j = 0; j < kPRowCacheWords; j++) {
-              const uint32_t src_bytes = (row_ok && j < a.qpv) ? 8u : 0u;
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(&S.rowc[r][j])),
-                           "l"(wp + (src_bytes ? j : 0)), "r"(src_bytes)
-                           : "memory");
-            }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            cached_dt = dt;
-            // warm L2 with the row of this cluster's next doc tile
-            const uint64_t nd = dt + n_clusters;
-            if (nd < g.n_doc_tiles) {
-              const uint64_t npb = (nd * 8 + rank * (kPRows / 32) + (r >> 5)) * a.block_stride;
-              const uint64_t ndoc = npb * 32 + (r & 31);
-              if (npb < n_blocks && ndoc < a.n)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint64_t*>(a.blocks) +
-                                                             ndoc * (uint64_t)a.qpv));
-            }
-          }
-          if (resA && qt_ != 0) continue;  // the doc tile's A is resident: built at its first query tile
-          // resident A: earlier uses of this doc tile's slots (doc tiles this
-          // cluster started before, or of the same parity with two halves)
-          const uint64_t dc = resA2 ? tc_.di >> 1 : tc_.di;
-          const uint32_t s_base = resA2 ? (tc_.di & 1) * n_kb : 0u;
-          const uint32_t base0 = a_row[0], rr = r & 7;
-          constexpr uint32_t kWordsPerKb = F4 ? 4 : 2;  // 128 bytes: 256 nibbles or 128 bytes of 0/1
-#pragma unroll
-          for (uint32_t kb = 0; kb < kPRowCacheWords / kWordsPerKb; kb++) {
-            if (kb >= n_kb) break;
-            uint32_t s;
-            if (resA) {
-              s = s_base + kb;
-              if (dc > 0) {  // the slot's previous doc tile has been read by its last query tile
-                // (with two halves the builders run a doc tile ahead: they sleep
-                // rather than poll, leaving the issue slots to the epilogue and MMA warps)
-                bool w = true;
-                if (lane == 0)
-                  w = !aborted(S) && (resA2 ? mbar_wait(&S.empty_a[s], (uint32_t)((dc - 1) & 1))
-                                            : mbar_wait_issuer(&S.empty_a[s], (uint32_t)((dc - 1) & 1)));
-                w = __shfl_sync(0xFFFFFFFFu, w, 0);
-                if (!w && lane == 0 && !aborted(S)) raise_abort(S, a.err);
-                __syncwarp();
-                if (!w) {
-                  ok = false;
-                  break;
-                }
-              }
-            } else {
-              s = (uint32_t)(it % kASlots);
-              if (!acquire(s)) {
-                ok = false;
-                break;
-              }
-            }
-            const uint32_t base = smem_u32(S.a[s]) + base0;
-            if constexpr (F4) {
-#pragma unroll
-              for (uint32_t c = 0; c < 8; c++) {  // 32 coordinates (half a word) per 16-byte chunk
-                const uint32_t h = (uint32_t)(S.rowc[r][4 * kb + (c >> 1)] >> (32 * (c & 1)));
-                st_shared_v4(base + ((c ^ rr) << 4), fp4_ones8(h), fp4_ones8(h >> 8), fp4_ones8(h >> 16),
-                             fp4_ones8(h >> 24));
-              }
-            } else {
-              const uint64_t w0 = S.rowc[r][2 * kb], w1 = S.rowc[r][2 * kb + 1];
-#pragma unroll
-              for (uint32_t c = 0; c < 8; c++) {  // 16 coordinates per 16-byte chunk
-                const uint32_t h = (uint32_t)((c < 4 ? w0 : w1) >> (16 * (c & 3)));
-                uint32_t o[4];
-#pragma unroll
-                for (uint32_t q = 0; q < 4; q++) o[q] = (((h >> (4 * q)) & 15u) * 0x00204081u) & 0x01010101u;
-                st_shared_v4(base + ((c ^ rr) << 4), o[0], o[1], o[2], o[3]);
-              }
-            }
-            publish(s);
-            it++;
-          }
-          continue;
-        }
-      }
-      if constexpr (MODE == 1) {
-        const uint64_t* words[R];
-        bool row_ok[R];
-        uint64_t w[R][4];  // K-block kb = words 2 kb, 2 kb + 1; two K-blocks of words in flight
-#pragma unroll
-        for (uint32_t i = 0; i < R; i++) {
-          row_ok[i] = pb[i] < n_blocks && doc[i] < a.n;
-          words[i] = reinterpret_cast<const uint64_t*>(a.blocks) + (row_ok[i] ? doc[i] : 0) * (uint64_t)a.qpv;
-#pragma unroll
-          for (uint32_t j = 0; j < 4; j++) w[i][j] = (row_ok[i] && j < a.qpv) ? __ldg(words[i] + j) : 0ull;
-        }
-        for (uint32_t kb = 0; kb < n_kb; kb++, it++) {
-          uint64_t lo[R], hi[R];
-#pragma unroll
-          for (uint32_t i = 0; i < R; i++) {
-            lo[i] = w[i][0];
-            hi[i] = w[i][1];
-            w[i][0] = w[i][2];
-            w[i][1] = w[i][3];
-            const uint32_t wi = 2 * kb + 4;
-            w[i][2] = (row_ok[i] && wi < a.qpv) ? __ldg(words[i] + wi) : 0ull;
-            w[i][3] = (row_ok[i] && wi + 1 < a.qpv) ? __ldg(words[i] + wi + 1) : 0ull;
-          }
-          const uint32_t s = (uint32_t)(it % kASlots);
-          if (!acquire(s)) {
-            ok = false;
-            break;
-          }
-#pragma unroll
-          for (uint32_t i = 0; i < R; i++) {
-            const uint32_t base = smem_u32(S.a[s]) + a_row[i], rr = (r + 128 * i) & 7;
-#pragma unroll
-            for (uint32_t c = 0; c < 8; c++) {  // 16 coordinates per 16-byte chunk
-              const uint32_t h = (uint32_t)((c < 4 ? lo[i] : hi[i]) >> (16 * (c & 3)));
-              uint32_t o[4];
-#pragma unroll
-              for (uint32_t q = 0; q < 4; q++)  // 4 bits -> 4 bytes (the shifted copies never overlap)
-                o[q] = (((h >> (4 * q)) & 15u) * 0x00204081u) & 0x01010101u;
-              st_shared_v4(base + ((c ^ rr) << 4), o[0], o[1], o[2], o[3]);
-            }
-          }
-          publish(s);
-        }
-      } else if constexpr (MODE == 0) {
+      {
         const uint8_t* row_codes[R];
         bool row_valid[R];
         uint4 next[R];
@@ -692,8 +769,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
           }
 #pragma unroll
           for (uint32_t j = 0; j < 4; j++) {
-            const uint32_t s = (uint32_t)(it % kASlots);
-            if (!acquire(s)) {
+            const uint32_t s = st;
+            if (!acquire(s, use)) {
               ok = false;
               break;
             }
@@ -708,10 +785,14 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
               }
             }
             publish(s);
-            it++;
+            if (++st == n_st) {
+              st = 0;
+              use++;
+            }
           }
         }
       }
+    }
     }
   } else if constexpr (PAIR) {
     // ---- epilogue of the pair form: every warp works alone -----------------------
@@ -792,51 +873,41 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
       __syncwarp();  // the list is reused by the next tile
     };
     if constexpr (F4) {
-      // FP4 form: the f32 sums of constant-weight and multi-bucket keys are
-      // compared as bits with the f32 bits of each column's integer threshold
-      // (non-negative floats order like their bit patterns); sign bitmaps take
-      // the integer sums.  Both 32-column chunks are read back to back (one
-      // tensor-memory latency) and the buffer released before any compare; the
-      // slots of a tile's kept entries are reserved by atomics whose results are
-      // first used during the next tile.
-      uint32_t* wam = S.wamin[e];
-      const bool fbits = a.key_kind != 2;
-      // this lane's entry of the previous tile, its slot reserved
-      bool pend = false;
-      uint32_t p_pos = 0, p_key = 0, p_id = 0;
-      uint64_t p_q = 0;
-      auto finish = [&]() {
-        if (pend && p_pos < a.cap) {
-          a.f_keys[p_q * a.cap + p_pos] = p_key;
-          a.f_ids[p_q * a.cap + p_pos] = p_id;
+      // FP4 form: the f32 sums are compared with the f32 of each query's integer
+      // threshold, read straight from the launch's parameters (a tile stages
+      // nothing); docs at the threshold itself are settled by the tie bound when
+      // their entry is made.  The buffer is released once the last chunk is in
+      // registers.  Kept entries stay in the warp's list over the tiles until it
+      // is nearly full, then every lane reserves and writes one at a time: staging
+      // thresholds and reserving slots tile by tile took 1,900 of a tile's 4,200
+      // clocks.
+      float* amf = reinterpret_cast<float*>(&P_am(0));
+      for (uint32_t i = et; i < kPMaxQ; i += kPEpiThreads)
+        amf[i] = i < a.nq ? f4_bound(a, P_am(i)) : __int_as_float(0x7f800000);
+      epi_sync();
+      uint32_t held = 0;  // entries in the list: (doc, biased sum | query << 21)
+      auto drain = [&]() {
+        __syncwarp();
+        for (uint32_t j = lane; j < held; j += 32) {
+          const uint2 en = list[j];
+          const uint32_t q = en.y >> 21;
+          const uint32_t pos = atomicAdd(&a.cnt[q], 1u);
+          if (pos < a.cap) {
+            a.f_keys[(uint64_t)q * a.cap + pos] = bm_key_q(a, P_pop(q), en.y & 0x1FFFFFu);
+            a.f_ids[(uint64_t)q * a.cap + pos] = en.x;
+          }
         }
-        pend = false;
+        __syncwarp();
+        held = 0;
       };
       uint32_t tcount = 0;
       TileCursor tc_;
       for (tc_.start(g, cluster); tc_.valid(g); tc_.next(g, n_clusters), tcount++) {
-        const uint64_t dt = tc_.dt;
-        const uint64_t q0 = (uint64_t)tc_.qt * nt;
-        const uint32_t nqt = (uint32_t)((a.nq - q0) < nt ? (a.nq - q0) : nt);
+        const uint32_t q0 = tc_.qt * nt;
+        const uint32_t nqt = (uint32_t)a.nq - q0 < nt ? (uint32_t)a.nq - q0 : nt;
         const uint32_t b = tcount % kBufs;
-        const uint64_t first = dt * 256 + rank * kPRows;
-        // thresholds of this warp's columns for this tile
-#pragma unroll
-        for (uint32_t h2 = 0; h2 < 2; h2++) {
-          const uint32_t c = col0 + 32 * h2 + lane;
-          uint32_t am = kNeverPasses;
-          if (c < nqt) {
-            am = P_am(q0 + c);
-            if (a.thr_pos) {
-              const uint32_t td = P_td(q0 + c);
-              am = td >= first + kPRows - 1 ? am : td < first ? am + 1 : kExactCompare;
-            }
-            if (fbits && am < kNeverPasses) am = __float_as_uint((float)am);  // exact: am <= 2^24
-          }
-          wam[32 * h2 + lane] = am;
-        }
-        const bool any_exact = __any_sync(0xFFFFFFFFu, wam[lane] == kExactCompare || wam[32 + lane] == kExactCompare);
-        __syncwarp();
+        const uint32_t doc = tc_.dt * 256 + rank * kPRows + row;  // filter: block stride 1
+        const bool valid = doc < a.n;
         bool ready = false;
         if (lane == 0) ready = !aborted(S) && mbar_wait_cluster(&S.acc_full[b], (tcount / kBufs) & 1);
         ready = __shfl_sync(0xFFFFFFFFu, ready, 0);
@@ -845,11 +916,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t doc = first + row;  // filter: block stride 1
-        const bool valid = doc < a.n;
         const uint32_t taddr = tmem + ((lq * 32) << 16) + b * 256 + col0;
-        const uint32_t dpop = fbits ? 0u : row_popcount(a, doc, valid);
-        uint32_t wcount = 0;
         if (nch == 0) {  // nothing to read: release the accumulator at once
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
@@ -865,63 +932,33 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
             __syncwarp();
             if (lane == 0) arrive_remote(acc_empty0 + 8 * b);
           }
-          if (c == 0) finish();  // the previous tile's slots have long been reserved
-          if (!fbits) {
-#pragma unroll
-            for (uint32_t j = 0; j < 32; j++) v[j] = ham_y(f4_int(v[j]), dpop);
-          }
           uint32_t hm = 0;  // the columns (queries) this lane's doc passes
-          if (!any_exact) {
 #pragma unroll
-            for (uint32_t j = 0; j < 32; j += 4) {
-              const uint4 am = *reinterpret_cast<const uint4*>(&wam[32 * c + j]);
-              hm |= ((uint32_t)(v[j] >= am.x) << j) | ((uint32_t)(v[j + 1] >= am.y) << (j + 1)) |
-                    ((uint32_t)(v[j + 2] >= am.z) << (j + 2)) | ((uint32_t)(v[j + 3] >= am.w) << (j + 3));
-            }
-          } else {
-#pragma unroll
-            for (uint32_t j = 0; j < 32; j++) {
-              const uint32_t q = (uint32_t)q0 + cb + j;
-              const uint32_t am = wam[32 * c + j];
-              const uint32_t tq = fbits ? __float_as_uint((float)P_thr(q)) : P_thr(q);
-              const bool pass = am != kExactCompare ? v[j] >= am : v[j] > tq || (v[j] == tq && doc <= P_td(q));
-              hm |= (uint32_t)pass << j;
-            }
+          for (uint32_t j = 0; j < 32; j += 4) {
+            const float4 am = *reinterpret_cast<const float4*>(&amf[q0 + cb + j]);
+            hm |= ((uint32_t)(__uint_as_float(v[j]) >= am.x) << j) |
+                  ((uint32_t)(__uint_as_float(v[j + 1]) >= am.y) << (j + 1)) |
+                  ((uint32_t)(__uint_as_float(v[j + 2]) >= am.z) << (j + 2)) |
+                  ((uint32_t)(__uint_as_float(v[j + 3]) >= am.w) << (j + 3));
           }
           // columns past the tile's queries (never written by the MMAs) keep nothing
           if (!valid) hm = 0;
           const uint32_t ncols = nqt > cb ? nqt - cb : 0u;
           hm &= ncols >= 32 ? 0xFFFFFFFFu : (1u << ncols) - 1u;
           while (__any_sync(0xFFFFFFFFu, hm != 0)) {
-            const bool has = hm != 0;
-            const uint32_t j = has ? (uint32_t)(__ffs(hm) - 1) : 0u;
-            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, has);
-            const uint32_t pos = wcount + __popc(bal & lt);
-            if (has && pos < kPSegCap) {
-              const uint32_t x = pick32(v, j);
-              list[pos] = make_uint2(fbits ? (uint32_t)__uint_as_float(x) : x, (cb + j) | (row << 16));
-            }
-            wcount += __popc(bal);
+            const uint32_t j = hm ? (uint32_t)(__ffs(hm) - 1) : 0u;
+            const uint32_t q = q0 + cb + j, y = f4_int(a, pick32(v, j));
+            // (key, doc) <= (thr, tdoc): at the threshold, docs up to the tie bound
+            const bool keep = hm != 0 && !(a.thr_pos && y == P_thr(q) && doc > P_td(q));
+            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, keep);
+            if (held + __popc(bal) > kPSegCap) drain();
+            if (keep) list[held + __popc(bal & lt)] = make_uint2(doc, y | (q << 21));
+            held += __popc(bal);
             hm &= hm - 1;
           }
         }
-        if (nch == 0) finish();
-        __syncwarp();
-        if (wcount > 32) {
-          flush(wcount, q0, dt, nqt);  // more than one entry per lane (or lost ones): reserve and write now
-        } else if (lane < wcount) {
-          // reserve this lane's slot now, write the entry during the next tile
-          const uint2 en = list[lane];
-          const uint32_t q = en.y & 0xFFFFu, rw_ = en.y >> 16;
-          p_q = q0 + q;
-          p_pos = atomicAdd(&a.cnt[p_q], 1u);
-          p_key = bm_key_q(a, P_pop(p_q), en.x);
-          p_id = (uint32_t)(first + rw_);
-          pend = true;
-        }
-        __syncwarp();  // the list is reused by the next tile
       }
-      finish();
+      drain();
     } else {
       uint32_t* wam = S.wamin[e];
       uint32_t tcount = 0;
@@ -961,7 +998,6 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
         const uint64_t doc = pb * 32 + lane;
         const uint64_t u = dt * 256 + rank * kPRows + row;
         const bool valid = pb < n_blocks && doc < a.n;
-        const uint32_t dpop = (BM && a.key_kind == 2) ? row_popcount(a, doc, valid) : 0u;
         const uint32_t taddr = tmem + ((lq * 32) << 16) + b * 256 + col0;
         uint32_t wcount = 0;
         if (nch == 0) {  // nothing to read: release the accumulator at once
@@ -981,7 +1017,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
           }
           if (BM && a.key_kind == 2) {
 #pragma unroll
-            for (uint32_t j = 0; j < 32; j++) v[j] = ham_y(v[j], dpop);
+            for (uint32_t j = 0; j < 32; j++) v[j] += kHamBias;
           }
           if (dense) {
 #pragma unroll
@@ -1118,7 +1154,6 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
       const uint64_t doc = pb * 32 + lane;
       const uint64_t u = dt * 256 + rank * kPRows + row;
       const bool valid = pb < n_blocks && doc < a.n;
-      const uint32_t dpop = (MODE == 1 && a.key_kind == 2) ? row_popcount(a, doc, valid) : 0u;
       const uint32_t taddr = tmem + ((lq * 32) << 16) + (b + h) * 256;
       const bool any_exact = S.any_exact != 0;
       uint32_t wcount = 0;
@@ -1130,7 +1165,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
         tmem_ld32(taddr + cb, v);
         if (MODE == 1 && a.key_kind == 2) {
 #pragma unroll
-          for (uint32_t j = 0; j < 32; j++) v[j] = ham_y(v[j], dpop);
+          for (uint32_t j = 0; j < 32; j++) v[j] += kHamBias;
         }
         if (dense) {
 #pragma unroll
@@ -1301,9 +1336,7 @@ TcForm tc_form(int mode) {
 // kept entries one epilogue warp of the persistent one-CTA form may hold per tile
 uint32_t tc_persist_seg_cap() { return PT<false>::kSegCap; }
 
-// The FP4 form of the bitmap filter takes rows the builders keep whole in
-// shared memory.
-uint32_t tc_fp4_max_words() { return kPRowCacheWords; }
+uint32_t tc_fp4_max_words() { return kPF4MaxWords; }
 
 template <int MODE>
 void launch_tc_pair(TcArgs a, const uint8_t* b_rows, cudaStream_t stream, bool pair) {
@@ -1334,8 +1367,8 @@ void launch_tc_pair(TcArgs a, const uint8_t* b_rows, cudaStream_t stream, bool p
   if (!a.n_kb || (MODE == 0 && a.n_kb % 4)) throw std::invalid_argument(std::string(what) + ": bad K extent");
   if (MODE == 2) {
     // query tiles of at most kPF4TileN columns (OVB_FP4_TILE_N: 16..224), balanced: a multiple of 16
-    if (!pair || a.keys || a.qpv > kPRowCacheWords || 4ull * a.n_kb < a.qpv)
-      throw std::invalid_argument(std::string(what) + ": needs CTA pairs, a filter and rows of <= 16 words");
+    if (!pair || a.keys || a.qpv > kPF4MaxWords || 4ull * a.n_kb < a.qpv)
+      throw std::invalid_argument(std::string(what) + ": needs CTA pairs, a filter and rows of <= 4096 words");
     uint32_t tile_n = kPF4TileN;
     if (const char* e = getenv("OVB_FP4_TILE_N")) {
       const long v = strtol(e, nullptr, 10);
@@ -1372,7 +1405,8 @@ void launch_tc_pair(TcArgs a, const uint8_t* b_rows, cudaStream_t stream, bool p
   const uint64_t total = doc_tiles * q_tiles;
   if (pair) {
     auto kernel = MODE == 0 ? fastscan_pair_kernel : MODE == 1 ? bitmap_pair_kernel : bitmap_fp4_pair_kernel;
-    const size_t smem = sizeof(PSmem<true>) + 1024;
+    const size_t smem = sizeof(PSmem<true, MODE == 2>) + 1024;
+    static_assert(sizeof(PSmem<true, MODE == 2>) + 1024 <= 227 * 1024, "pair form: shared memory");
     OVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     uint64_t clusters = resident_pairs((const void*)kernel, smem);
     // whole doc tiles per cluster once every cluster gets at least two of them

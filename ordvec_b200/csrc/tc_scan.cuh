@@ -110,13 +110,12 @@ __device__ inline uint32_t bm_amin(const TcArgs& a, uint32_t thr) {
   return lo;
 }
 
-// Sign bitmaps (key_kind 2): Hamming(q, d) = |q| + |d| - 2 |q AND d|.  The
-// epilogue compares y = 2 acc + kHamBias - |d| (per doc row) against
-// |q| + kHamBias - thr (per query), so the threshold test stays one compare
-// per (doc, query) and key <= thr <=> y >= that bound.
+// Sign bitmaps (key_kind 2): the doc operand is 0/1, the query operand +1 where
+// its bit is set and -1 where it is clear, so the accumulator is
+// |q AND d| - |d AND NOT q| = |q| - Hamming(q, d): no popcount of the docs.
+// The epilogue adds kHamBias to keep it an unsigned integer y (dim < 2^20);
+// key <= thr <=> y >= |q| + kHamBias - thr.
 constexpr uint32_t kHamBias = 1u << 20;
-
-__device__ __forceinline__ uint32_t ham_y(uint32_t acc, uint32_t dpop) { return 2 * acc + kHamBias - dpop; }
 
 // key of a (possibly transformed) accumulator for a query with popcount qpop
 __device__ __forceinline__ uint32_t bm_key_q(const TcArgs& a, uint32_t qpop, uint32_t y) {
@@ -126,16 +125,6 @@ __device__ __forceinline__ uint32_t bm_key_q(const TcArgs& a, uint32_t qpop, uin
 // smallest (transformed) accumulator whose key is <= thr
 __device__ __forceinline__ uint32_t bm_amin_q(const TcArgs& a, uint32_t qpop, uint32_t thr) {
   return a.key_kind == 2 ? qpop + kHamBias - thr : bm_amin(a, thr);
-}
-
-// popcount of a bitmap row (qpv words), 0 for an invalid row
-__device__ __forceinline__ uint32_t row_popcount(const TcArgs& a, uint64_t doc, bool valid) {
-  uint32_t c = 0;
-  if (valid) {
-    const uint64_t* w = reinterpret_cast<const uint64_t*>(a.blocks) + doc * (uint64_t)a.qpv;
-    for (uint32_t i = 0; i < a.qpv; i++) c += __popcll(__ldg(w + i));
-  }
-  return c;
 }
 
 __device__ __forceinline__ uint4 load_codes(const uint8_t* p) {
