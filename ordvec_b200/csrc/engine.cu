@@ -237,6 +237,12 @@ void bitmap_tc_candidates(const Index& s1, const uint64_t* qb, uint32_t qpv, uin
       dense);
 }
 
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  OVB_CUDA(cudaStreamIsCapturing(st, &s));
+  return s != cudaStreamCaptureStatusNone;
+}
+
 void require_kind(const Index& ix, uint32_t kind, const char* what) {
   if (ix.kind != kind) fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, std::string(what) + ": wrong index kind");
 }
@@ -264,14 +270,25 @@ uint64_t default_candidate_count(uint64_t k, uint64_t space) {
   return c < space ? c : space;
 }
 
-// Batched full scans use the split-BF16 tensor-core scan (with the exact FP64
-// rescoring below) from 64 queries on eligible shapes; OVB_RANK_TC=0/1 forces.
-bool use_rank_tc(const Index& rq, uint64_t nq) {
+// Batched full scans use the tensor-core candidate scan (with the exact FP64
+// rescoring below) from 64 queries on eligible shapes, and smaller batches where
+// the sampled filter runs and the FP64 table scan's work, nq n dim bits, is
+// above 1e9 + 800 n.  Measured with both forms (us, tables / tensor cores): n = 1M
+// dim 768 b=1: 236 / 263 at 2 queries, 285 / 262 at 3; b=2: 271 / 272 at 1, 413 /
+// 274 at 2, 4,673 / 301 at 32; n = 200k dim 1024 b=1: 140 / 149 at 4, 175 / 144 at 6;
+// n = 40k dim 384 b=2: 82 / 113 at 16, 132 / 114 at 32.  A capturing stream keeps
+// the table scan below 64 queries (the candidate form reads a flag on the host).
+// OVB_RANK_TC=0/1 forces.
+bool use_rank_tc(const Index& rq, uint64_t nq, uint64_t k, cudaStream_t st) {
   const char* e = getenv("OVB_RANK_TC");
   if (!rank_tc_eligible(rq.dim, rq.bits)) return false;
   if (e && e[0] == '0') return false;
   if (e && e[0] == '1') return true;
-  return nq >= 64 && rq.n >= 4096;
+  if (nq >= 64) return rq.n >= 4096;
+  const uint64_t n = rq.n, ke = k < n ? k : n, kp = std::min<uint64_t>(std::max<uint64_t>(2 * ke, ke + 64), n);
+  FilterPlan fp;
+  return nq * n * rq.dim * rq.bits >= 1000000000ull + 800 * n && score_rankquant_eligible(rq.dim, rq.bits) &&
+         kp <= kSelectSmemCap && filter_plan(n, (uint32_t)kp, fp) && !capturing(st);
 }
 
 // Split-BF16 filter for rows of kp candidates: the sample-threshold plan with
@@ -286,24 +303,75 @@ static uint64_t split_filter_bytes_per_query(const FilterPlan& fp, uint64_t kp) 
   return fp.n_s * 4 + (uint64_t)fp.r * 8 + (uint64_t)fp.cap * 8 + 4 + kp * 12 + 8;
 }
 
-// Enqueues the filtered split-BF16 pipeline for qn queries (no host
+// The tensor-core candidate scores of an exact RankQuant search over prepared
+// query rows: integer fixed-point scores (scan_score_pair.cu), or split-BF16 where
+// 16-bit fixed point would overflow the accumulators.  prepare() builds the query
+// operand and the per-query error bounds of qn rows (stream-ordered: one chunk of
+// rows at a time).
+struct CandScores {
+  const Index& rq;
+  float inv_norm;
+  bool fixed, half_steps;  // half_steps: the rows are multiples of 1/2 (symmetric search)
+  uint32_t q_per_tile;
+  ScoreOperand op{};
+  double* bound = nullptr;
+  uint16_t* qs = nullptr;
+  float* l1 = nullptr;
+  CandScores(const Index& ix, float inv, bool half, uint32_t qpt)
+      : rq(ix), inv_norm(inv), fixed(score_rankquant_eligible(ix.dim, ix.bits)), half_steps(half), q_per_tile(qpt) {}
+  void prepare(const float* qu, uint64_t qn, Workspace& w, cudaStream_t st) {
+    if (fixed) {
+      op = score_operand(rq.bits, qn, rq.dim, q_per_tile);
+      op.rows = w.q_fix.ensure(op.bytes);
+      bound = (double*)w.q_bound.ensure(qn * 16);
+      launch_fix_rankquant(qu, qn, rq.dim, rq.bits, half_steps, op, bound, st);
+    } else {
+      qs = (uint16_t*)w.q_split.ensure(qn * 2 * rq.dim * 2);
+      l1 = (float*)w.q_l1.ensure(qn * 4);
+      launch_split_queries(qu, qn, rq.dim, qs, l1, st);
+    }
+  }
+  void scan(uint64_t qn, uint32_t stride, uint32_t* keys, uint64_t ld, uint32_t* err, cudaStream_t st) const {
+    const uint8_t* codes = rq.codes.as<uint8_t>();
+    if (fixed)
+      launch_score_scan(codes, rq.n, rq.dim, rq.bits, op, qn, stride, keys, ld, err, st);
+    else
+      launch_rank_scan_tc(codes, rq.n, rq.dim, rq.bits, qs, qn, inv_norm, stride, keys, ld, q_per_tile, err, st);
+  }
+  void filter(uint64_t qn, const uint32_t* thr, uint64_t thr_stride, uint32_t* cnt, uint32_t cap, uint32_t* fk,
+              uint32_t* fi, uint32_t* err, cudaStream_t st) const {
+    const uint8_t* codes = rq.codes.as<uint8_t>();
+    if (fixed)
+      launch_score_filter(codes, rq.n, rq.dim, rq.bits, op, qn, thr, thr_stride, cnt, cap, fk, fi, err, st);
+    else
+      launch_rank_filter_tc(codes, rq.n, rq.dim, rq.bits, qs, qn, inv_norm, thr, thr_stride, cnt, cap, fk, fi,
+                            q_per_tile, err, st);
+  }
+  void margin(const uint32_t* sel, uint64_t qn, uint32_t kp, uint32_t ke, uint32_t* flag, cudaStream_t st) const {
+    if (fixed)
+      launch_score_margin(sel, qn, kp, ke, bound, rq.bits, flag, st);
+    else
+      launch_split_margin(sel, qn, kp, ke, l1, split_error_bound(rq.dim, rq.bits, inv_norm), flag, st);
+  }
+};
+
+// Enqueues a filtered candidate pipeline for qn queries (no host
 // synchronisation, graph-capturable): sample scan, each query's r-th sample
-// key as threshold, filtered scan, top-kp of the kept docs by split score,
-// margin test, FP64 rescoring of the kp, top-ke into out_keys / out_ids.
-// *d_flag |= 1 when some query kept fewer than kp or more than cap docs, or
-// its kp-th split score is within twice the error bound of its k-th: the
-// result is then not known to be exact and the caller redoes the rows.
-// Kept sets are prefixes of the split-key order, so their top-kp is the
+// key as threshold, filtered scan, top-kp of the kept docs by candidate score,
+// margin test, exact rescoring of the kp (rescore(candidate ids) -> keys), top-ke
+// into out_keys / out_ids.  *d_flag |= 1 when some query kept fewer than kp or
+// more than cap docs, or its kp-th candidate score is within the error bounds of
+// its k-th: the result is then not known to be exact and the caller redoes the
+// rows.  Kept sets are prefixes of the candidate order, so their top-kp is the
 // whole index's.
-static void split_filtered(const Index& rq, const uint16_t* qs, const float* qu, const float* l1, float inv_norm,
-                           uint64_t qn, uint32_t ke, uint32_t kp, const FilterPlan& fp, uint32_t q_per_tile,
-                           uint32_t* d_flag, uint32_t* out_keys, uint32_t* out_ids, Workspace& w, cudaStream_t st) {
-  const uint64_t n = rq.n;
-  const uint32_t dim = rq.dim, bits = rq.bits, id_bits = bits_for(n - 1);
-  const uint8_t* codes = rq.codes.as<uint8_t>();
+template <class Scores, class Rescore>
+static void filtered_candidates(const Scores& sc, uint64_t n, uint64_t qn, uint32_t ke, uint32_t kp,
+                                const FilterPlan& fp, uint32_t* d_flag, uint32_t* out_keys, uint32_t* out_ids,
+                                Workspace& w, cudaStream_t st, Rescore&& rescore) {
+  const uint32_t id_bits = bits_for(n - 1);
   uint32_t* err = w.tc_err_word(st);
   uint32_t* smp = (uint32_t*)w.smp_keys.ensure(qn * fp.n_s * 4);
-  launch_rank_scan_tc(codes, n, dim, bits, qs, qn, inv_norm, fp.stride, smp, fp.n_s, q_per_tile, err, st);
+  sc.scan(qn, fp.stride, smp, fp.n_s, err, st);
   uint32_t* tk = (uint32_t*)w.thr_keys.ensure(qn * fp.r * 4);
   uint32_t* ti = (uint32_t*)w.thr_ids.ensure(qn * fp.r * 4);
   select_rows(w, smp, nullptr, nullptr, fp.n_s, fp.n_s, qn, fp.r, 32, bits_for(fp.n_s - 1), tk, ti, st);
@@ -312,41 +380,45 @@ static void split_filtered(const Index& rq, const uint16_t* qs, const float* qu,
   uint32_t* fk = (uint32_t*)w.f_keys.ensure(qn * fp.cap * 4);
   uint32_t* fi = (uint32_t*)w.f_ids.ensure(qn * fp.cap * 4);
   OVB_CUDA(cudaMemsetAsync(cnt, 0, qn * 4, st));
-  launch_rank_filter_tc(codes, n, dim, bits, qs, qn, inv_norm, tk + (fp.r - 1), fp.r, cnt, fp.cap, fk, fi, q_per_tile,
-                        err, st);
+  sc.filter(qn, tk + (fp.r - 1), fp.r, cnt, fp.cap, fk, fi, err, st);
   launch_filter_check(cnt, qn, kp, fp.cap, d_flag, st);
   w.mark(st, 2);
   uint32_t* ck = (uint32_t*)w.sel_keys.ensure(qn * kp * 4);
   uint32_t* ci = (uint32_t*)w.sel_ids.ensure(qn * kp * 4);
   select_rows(w, fk, fi, nullptr, fp.cap, fp.cap, qn, kp, 32, id_bits, ck, ci, st, cnt);
   launch_clamp_ids(ci, qn * kp, (uint32_t)n, st);  // a row that kept < kp docs ends in sentinels
-  launch_split_margin(ck, qn, kp, ke, l1, split_error_bound(dim, bits, inv_norm), d_flag, st);
+  sc.margin(ck, qn, kp, ke, d_flag, st);
   w.mark(st, 3);
-  uint64_t* off = (uint64_t*)w.off.ensure((qn + 1) * 8);
-  launch_uniform_offsets(off, qn, kp, st);
   uint32_t* k2 = (uint32_t*)w.keys2.ensure(qn * kp * 4);
-  launch_asym_subset(codes, dim, bits, qu, qn, off, ci, kp, inv_norm, k2, st);
+  rescore(ci, k2);
   w.mark(st, 4);
-  select_rows(w, k2, ci, off, 0, 0, qn, ke, 32, id_bits, out_keys, out_ids, st);
+  select_rows(w, k2, ci, nullptr, kp, kp, qn, ke, 32, id_bits, out_keys, out_ids, st);
   w.mark(st, 5);
 }
 
-// Split-BF16 search of prepared query rows qu (nq x dim f32) scored as
+// The FP64 rescoring of an exact RankQuant search's kp candidates per query.
+static void rescore_rankquant(const Index& rq, const float* qu, float inv_norm, uint64_t qn, uint32_t kp,
+                              const uint32_t* ids, uint32_t* keys, Workspace& w, cudaStream_t st) {
+  uint64_t* off = (uint64_t*)w.off.ensure((qn + 1) * 8);
+  launch_uniform_offsets(off, qn, kp, st);
+  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, qn, off, ids, kp, inv_norm, keys, st);
+}
+
+// Tensor-core search of prepared query rows qu (nq x dim f32) scored as
 // sum_j qu[j] (code_j - c) * inv_norm: the unit query and 1/norm for
 // search_asymmetric, the centred query buckets and 1/norm^2 for the symmetric
-// search.  The error bound is linear in |qu|_1 and inv_norm, so both share it.
-static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, uint64_t nq, uint64_t k, bool exact,
-                             Workspace& w, cudaStream_t st, uint32_t q_per_tile) {
+// search (half_steps).  exact: candidates by CandScores, rescored in FP64; else the
+// split-BF16 scores themselves.
+static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, bool half_steps, uint64_t nq,
+                             uint64_t k, bool exact, Workspace& w, cudaStream_t st, uint32_t q_per_tile) {
   if (!rank_tc_eligible(rq.dim, rq.bits))
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "split-BF16 scan needs dim to be a multiple of 64");
   const uint64_t n = rq.n;
   const uint32_t ke = (uint32_t)(k < n ? k : n);
   if (!ke || !nq) return ke;
-  const uint32_t dim = rq.dim, bits = rq.bits;
-  const float bound = split_error_bound(dim, bits, inv_norm);
-  uint16_t* qs = (uint16_t*)w.q_split.ensure(nq * 2 * dim * 2);
-  float* l1 = (float*)w.q_l1.ensure(nq * 4);
-  launch_split_queries(qu, nq, dim, qs, l1, st);
+  const uint32_t dim = rq.dim;
+  CandScores sc(rq, inv_norm, half_steps, q_per_tile);
+  if (!exact) sc.fixed = false;
   uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
   uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
   uint32_t* flag = (uint32_t*)w.f_flag.ensure(4);
@@ -364,8 +436,11 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, u
     for (uint64_t q0 = 0; q0 < nq; q0 += fc) {
       const uint64_t qn = nq - q0 < fc ? nq - q0 : fc;
       OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
-      split_filtered(rq, qs + q0 * 2 * dim, qu + q0 * dim, l1 + q0, inv_norm, qn, ke, (uint32_t)kp0, fp, q_per_tile,
-                     flag, ok + q0 * ke, oi + q0 * ke, w, st);
+      sc.prepare(qu + q0 * dim, qn, w, st);
+      filtered_candidates(sc, n, qn, ke, (uint32_t)kp0, fp, flag, ok + q0 * ke, oi + q0 * ke, w, st,
+                          [&](const uint32_t* ids, uint32_t* keys) {
+                            rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp0, ids, keys, w, st);
+                          });
       OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
       OVB_CUDA(cudaStreamSynchronize(st));
       if (!*flag_h) {
@@ -383,16 +458,16 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, u
     if (!done.empty() && std::all_of(done.begin() + q0, done.begin() + q0 + qn, [](char c) { return c != 0; }))
       continue;
     if (!keys) keys = (uint32_t*)w.keys.ensure(qc * n * 4);
-    launch_rank_scan_tc(rq.codes.as<uint8_t>(), n, dim, bits, qs + q0 * 2 * dim, qn, inv_norm, 1, keys, n,
-                        q_per_tile, w.tc_err_word(st), st);
+    sc.prepare(qu + q0 * dim, qn, w, st);
+    sc.scan(qn, 1, keys, n, w.tc_err_word(st), st);
     w.mark(st, 2);
     if (!exact) {
       select_rows(w, keys, nullptr, nullptr, n, n, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st);
       w.mark(st, 3);
       continue;
     }
-    // candidates: the top kp by split score, kp grown until the kp-th is more
-    // than twice the bound below the k-th, so every doc whose exact score can
+    // candidates: the top kp by candidate score, kp grown until the kp-th is more
+    // than the error bounds below the k-th, so every doc whose exact score can
     // reach the exact top-k is a candidate; the key matrix is reused
     uint64_t kp = std::max<uint64_t>(2ull * ke, ke + 64ull);
     for (;;) {
@@ -402,19 +477,17 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, u
       select_rows(w, keys, nullptr, nullptr, n, n, qn, (uint32_t)kp, 32, id_bits, tk, ti, st);
       if (kp == n) break;
       OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
-      launch_split_margin(tk, qn, (uint32_t)kp, ke, l1 + q0, bound, flag, st);
+      sc.margin(tk, qn, (uint32_t)kp, ke, flag, st);
       OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
       OVB_CUDA(cudaStreamSynchronize(st));
       if (!*flag_h) break;
       kp *= 4;
     }
     w.split_kp = std::max<uint64_t>(w.split_kp, kp);
-    uint64_t* off = (uint64_t*)w.off.ensure((qn + 1) * 8);
-    launch_uniform_offsets(off, qn, (uint32_t)kp, st);
     uint32_t* k2 = (uint32_t*)w.keys2.ensure(qn * kp * 4);
     const uint32_t* ti = w.thr_ids.as<uint32_t>();
-    launch_asym_subset(rq.codes.as<uint8_t>(), dim, bits, qu + q0 * dim, qn, off, ti, kp, inv_norm, k2, st);
-    select_rows(w, k2, ti, off, 0, 0, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st);
+    rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp, ti, k2, w, st);
+    select_rows(w, k2, ti, w.off.as<uint64_t>(), 0, 0, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st);
     w.mark(st, 3);
   }
   return ke;
@@ -428,7 +501,7 @@ uint32_t engine_rankquant_full_split(const Index& rq, const float* d_q, uint64_t
   const uint64_t ke = k < rq.n ? k : rq.n;
   if (!ke || !nq) return (uint32_t)ke;
   const float* qu = normalised(w, d_q, nq, rq.dim, st);
-  return split_search(rq, qu, inv_rankquant_norm(rq.dim, rq.bits), nq, k, exact, w, st, q_per_tile);
+  return split_search(rq, qu, inv_rankquant_norm(rq.dim, rq.bits), false, nq, k, exact, w, st, q_per_tile);
 }
 
 bool split_fixed_fits(const Index& rq, uint64_t nq, uint64_t k) {
@@ -454,34 +527,33 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   const uint32_t dim = rq.dim, bits = rq.bits, id_bits = bits_for(n - 1);
   const float* qu = normalised(w, d_q, nq, dim, st);
   const float inv_norm = inv_rankquant_norm(dim, bits);
-  uint16_t* qs = (uint16_t*)w.q_split.ensure(nq * 2 * dim * 2);
-  float* l1 = (float*)w.q_l1.ensure(nq * 4);
-  launch_split_queries(qu, nq, dim, qs, l1, st);
+  CandScores sc(rq, inv_norm, false, q_per_tile);
+  sc.prepare(qu, nq, w, st);
   uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
   uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
   if (filtered) {
-    split_filtered(rq, qs, qu, l1, inv_norm, nq, ke, (uint32_t)kp, fp, q_per_tile, d_flag, ok, oi, w, st);
+    filtered_candidates(sc, n, nq, ke, (uint32_t)kp, fp, d_flag, ok, oi, w, st,
+                        [&](const uint32_t* ids, uint32_t* keys) {
+                          rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ids, keys, w, st);
+                        });
     return ke;
   }
   uint32_t* keys = (uint32_t*)w.keys.ensure(nq * n * 4);
-  launch_rank_scan_tc(rq.codes.as<uint8_t>(), n, dim, bits, qs, nq, inv_norm, 1, keys, n, q_per_tile,
-                      w.tc_err_word(st), st);
+  sc.scan(nq, 1, keys, n, w.tc_err_word(st), st);
   uint32_t* tk = (uint32_t*)w.thr_keys.ensure(nq * kp * 4);
   uint32_t* ti = (uint32_t*)w.thr_ids.ensure(nq * kp * 4);
   select_rows(w, keys, nullptr, nullptr, n, n, nq, (uint32_t)kp, 32, id_bits, tk, ti, st);
-  if (kp < n) launch_split_margin(tk, nq, (uint32_t)kp, ke, l1, split_error_bound(dim, bits, inv_norm), d_flag, st);
-  uint64_t* off = (uint64_t*)w.off.ensure((nq + 1) * 8);
-  launch_uniform_offsets(off, nq, (uint32_t)kp, st);
+  if (kp < n) sc.margin(tk, nq, (uint32_t)kp, ke, d_flag, st);
   uint32_t* k2 = (uint32_t*)w.keys2.ensure(nq * kp * 4);
-  launch_asym_subset(rq.codes.as<uint8_t>(), dim, bits, qu, nq, off, ti, kp, inv_norm, k2, st);
-  select_rows(w, k2, ti, off, 0, 0, nq, ke, 32, id_bits, ok, oi, st);
+  rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ti, k2, w, st);
+  select_rows(w, k2, ti, w.off.as<uint64_t>(), 0, 0, nq, ke, 32, id_bits, ok, oi, st);
   return ke;
 }
 
 uint32_t engine_rankquant_full(const Index& rq, const float* d_q, uint64_t nq, uint64_t k,
                                Workspace& w, cudaStream_t st) {
   require_kind(rq, ORDVEC_INDEX_KIND_RANK_QUANT, "search_asymmetric");
-  if (use_rank_tc(rq, nq)) return engine_rankquant_full_split(rq, d_q, nq, k, true, w, st);
+  if (use_rank_tc(rq, nq, k, st)) return engine_rankquant_full_split(rq, d_q, nq, k, true, w, st);
   const uint32_t ke = (uint32_t)(k < rq.n ? k : rq.n);
   if (!ke || !nq) return ke;
   const float* qu = normalised(w, d_q, nq, rq.dim, st);
@@ -512,7 +584,7 @@ uint32_t engine_rankquant_symmetric(const Index& rq, const float* d_q, uint64_t 
   const float inv_norm_sq = 1.0f / (norm * norm);
   // batches: split-BF16 candidates (the centred buckets are exact in BF16, so
   // lo = 0) rescored exactly
-  if (use_rank_tc(rq, nq)) return split_search(rq, qc, inv_norm_sq, nq, k, true, w, st, 0);
+  if (use_rank_tc(rq, nq, k, st)) return split_search(rq, qc, inv_norm_sq, true, nq, k, true, w, st, 0);
   uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
   uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
   full_scan_select(w, nq, rq.n, ke, 32, ok, oi, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
@@ -520,6 +592,43 @@ uint32_t engine_rankquant_symmetric(const Index& rq, const float* d_q, uint64_t 
                      st);
   });
   return ke;
+}
+
+// The integer candidate scores of a Rank search (scan_score_pair.cu).
+struct RankScores {
+  const Index& rk;
+  ScoreOperand op{};
+  double* bound = nullptr;
+  void prepare(bool sym, const void* q, uint64_t qn, Workspace& w, cudaStream_t st) {
+    op = score_operand(16, qn, rk.dim, 0);
+    op.rows = w.q_fix.ensure(op.bytes);
+    bound = (double*)w.q_bound.ensure(qn * 16);
+    launch_fix_rank(sym, q, qn, rk.dim, op, bound, st);
+  }
+  void scan(uint64_t qn, uint32_t stride, uint32_t* keys, uint64_t ld, uint32_t* err, cudaStream_t st) const {
+    launch_score_scan(rk.codes.p, rk.n, rk.dim, 16, op, qn, stride, keys, ld, err, st);
+  }
+  void filter(uint64_t qn, const uint32_t* thr, uint64_t thr_stride, uint32_t* cnt, uint32_t cap, uint32_t* fk,
+              uint32_t* fi, uint32_t* err, cudaStream_t st) const {
+    launch_score_filter(rk.codes.p, rk.n, rk.dim, 16, op, qn, thr, thr_stride, cnt, cap, fk, fi, err, st);
+  }
+  void margin(const uint32_t* sel, uint64_t qn, uint32_t kp, uint32_t ke, uint32_t* flag, cudaStream_t st) const {
+    launch_score_margin(sel, qn, kp, ke, bound, 16, flag, st);
+  }
+};
+
+// Rank searches on the tensor cores: batches whose kp candidates take the sampled
+// filter, from two queries and nq n dim = 9e8 (OVB_RANK_TC=0/1 forces as for
+// RankQuant).  Measured with both forms, symmetric (us, CUDA cores / tensor
+// cores): n = 1M dim 768: 429 / 381 at 1 query, 639 / 384 at 2, 733 / 385 at 8, 3,911
+// / 412 at 48; n = 200k dim 1024: 191 / 222 at 4, 289 / 229 at 6; n = 40k dim 384:
+// 84 / 113 at 16, 142 / 124 at 48.
+static bool use_rank_scores(const Index& rk, uint64_t nq, uint64_t kp, cudaStream_t st, FilterPlan& fp) {
+  const char* e = getenv("OVB_RANK_TC");
+  if (e && e[0] == '0') return false;
+  if (capturing(st)) return false;  // the margin flag is read on the host
+  if (!score_rank_eligible(rk.dim) || !split_filter_plan(rk.n, kp, fp)) return false;
+  return (e && e[0] == '1') || (nq >= 2 && nq * rk.n * rk.dim >= 900000000ull);
 }
 
 // Rank::search / Rank::search_asymmetric (src/rank.rs:364-482).
@@ -532,18 +641,52 @@ uint32_t engine_rank_full(const Index& rk, const float* d_q, uint64_t nq, uint64
   const uint32_t dim = rk.dim;
   uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
   uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
+  const float* qu = nullptr;
+  float* qsum = nullptr;
+  uint16_t* qr = nullptr;
   if (asymmetric) {
-    const float* qu = normalised(w, d_q, nq, dim, st);
-    float* qsum = (float*)w.invq.ensure(nq * 4);
-    full_scan_select(w, nq, rk.n, ke, 32, ok, oi, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
-      launch_rank_asym_scan(ranks, rk.n, dim, qu + q0 * dim, qsum + q0, qn, keys, rk.n, st);
-    });
+    qu = normalised(w, d_q, nq, dim, st);
+    qsum = (float*)w.invq.ensure(nq * 4);
+    launch_rank_row_sum(qu, nq, dim, qsum, st);
   } else {
-    uint16_t* qr = (uint16_t*)w.qbits.ensure(nq * dim * 2);
+    qr = (uint16_t*)w.qbits.ensure(nq * dim * 2);
     launch_encode(5, d_q, nq, dim, 0, 0, 0, qr, 0, nullptr, st);
-    full_scan_select(w, nq, rk.n, ke, 32, ok, oi, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
-      launch_rank_sym_scan(ranks, rk.n, dim, qr + q0 * dim, qn, keys, rk.n, st);
-    });
+  }
+  // rows [q0, q0 + qn) through the key matrix of exact scores
+  auto full = [&](uint64_t qa, uint64_t qn) {
+    full_scan_select(w, qn, rk.n, ke, 32, ok + qa * ke, oi + qa * ke, st,
+                     [&](uint64_t q0, uint64_t qm, uint32_t* keys) {
+                       const uint64_t q = qa + q0;
+                       if (asymmetric)
+                         launch_rank_asym_scan(ranks, rk.n, dim, qu + q * dim, qsum + q, qm, keys, rk.n, st);
+                       else
+                         launch_rank_sym_scan(ranks, rk.n, dim, qr + q * dim, qm, keys, rk.n, st);
+                     });
+  };
+  const uint64_t kp = std::min<uint64_t>(std::max<uint64_t>(2ull * ke, ke + 64ull), rk.n);
+  FilterPlan fp;
+  if (!use_rank_scores(rk, nq, kp, st, fp)) {
+    full(0, nq);
+    return ke;
+  }
+  uint32_t* flag = (uint32_t*)w.f_flag.ensure(4);
+  uint32_t* flag_h = (uint32_t*)w.f_flag_host.ensure(4);
+  uint64_t fc = keys_budget() / split_filter_bytes_per_query(fp, kp);
+  if (fc < 1) fc = 1;
+  RankScores sc{rk};
+  for (uint64_t q0 = 0; q0 < nq; q0 += fc) {
+    const uint64_t qn = nq - q0 < fc ? nq - q0 : fc;
+    const void* q = asymmetric ? (const void*)(qu + q0 * dim) : (const void*)(qr + q0 * dim);
+    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
+    sc.prepare(!asymmetric, q, qn, w, st);
+    filtered_candidates(sc, rk.n, qn, ke, (uint32_t)kp, fp, flag, ok + q0 * ke, oi + q0 * ke, w, st,
+                        [&](const uint32_t* ids, uint32_t* keys) {
+                          launch_rank_subset(!asymmetric, ranks, dim, q, asymmetric ? qsum + q0 : nullptr, qn, ids,
+                                             (uint32_t)kp, keys, st);
+                        });
+    OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
+    OVB_CUDA(cudaStreamSynchronize(st));
+    if (*flag_h) full(q0, qn);
   }
   return ke;
 }

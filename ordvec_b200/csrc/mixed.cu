@@ -66,7 +66,7 @@ float inv_norm_of(uint32_t dim, uint32_t bits) {
 }
 
 // The autotuner: event-time the scan at 32 / 64 / 128 queries per tile over
-// the first (up to) 64K rows with the plan's split queries, keep the fastest.
+// the first (up to) 64K rows with the plan's prepared queries, keep the fastest.
 uint32_t autotune_tile(Plan& p) {
   Workspace& w = *p.w;
   const Index& ix = *p.ix;
@@ -80,12 +80,25 @@ uint32_t autotune_tile(Plan& p) {
   float best_ms = std::numeric_limits<float>::infinity();
   for (uint32_t qpt : {32u, 64u, 128u}) {
     if (qpt > 32 && (uint64_t)qpt / 2 >= p.nq) break;  // larger tiles than the batch change nothing
-    launch_rank_scan_tc(ix.codes.as<uint8_t>(), rows, ix.dim, ix.bits, w.q_split.p, p.nq, inv_norm, 1, keys, rows,
-                        qpt, w.tc_err_word(w.stream), w.stream);
+    const bool fixed = score_rankquant_eligible(ix.dim, ix.bits);
+    ScoreOperand op;
+    if (fixed) {  // the operand is laid out for its tile
+      op = score_operand(ix.bits, p.nq, ix.dim, qpt);
+      op.rows = w.q_fix.ensure(op.bytes);
+      launch_fix_rankquant(w.q_unit.as<float>(), p.nq, ix.dim, ix.bits, false, op,
+                           (double*)w.q_bound.ensure(p.nq * 16), w.stream);
+    }
+    auto scan = [&] {
+      if (fixed)
+        launch_score_scan(ix.codes.p, rows, ix.dim, ix.bits, op, p.nq, 1, keys, rows, w.tc_err_word(w.stream),
+                          w.stream);
+      else
+        launch_rank_scan_tc(ix.codes.as<uint8_t>(), rows, ix.dim, ix.bits, w.q_split.p, p.nq, inv_norm, 1, keys, rows,
+                            qpt, w.tc_err_word(w.stream), w.stream);
+    };
+    scan();
     OVB_CUDA(cudaEventRecord(e0, w.stream));
-    for (int r = 0; r < 2; r++)
-      launch_rank_scan_tc(ix.codes.as<uint8_t>(), rows, ix.dim, ix.bits, w.q_split.p, p.nq, inv_norm, 1, keys, rows,
-                          qpt, w.tc_err_word(w.stream), w.stream);
+    for (int r = 0; r < 2; r++) scan();
     OVB_CUDA(cudaEventRecord(e1, w.stream));
     OVB_CUDA(cudaEventSynchronize(e1));
     float ms = 0.0f;

@@ -102,6 +102,8 @@ struct Workspace {
   DevBuf smp_keys, thr_keys, thr_ids, f_keys, f_ids, f_cnt, f_flag;
   // split-BF16 rank scan: [hi; lo] query rows and |q|_1
   DevBuf q_split, q_l1;
+  // integer score scans: the queries' byte planes and their error bounds
+  DevBuf q_fix, q_bound;
   // bitmap filter on FP4 tensor cores: the query bits as e2m1 nibbles
   DevBuf q_nib;
   // split-BF16 rerank: top-kp split keys / ids per query, their FP64 keys, the margin flag

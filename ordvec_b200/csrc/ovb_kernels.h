@@ -162,7 +162,7 @@ float rank_norm_f32(uint32_t dim);
 void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const uint16_t* q_ranks, uint64_t nq,
                           uint32_t* keys, uint64_t ld, cudaStream_t stream);
 // Rank::search_asymmetric: q_unit rows; q_sum (nq floats) is scratch the launch fills
-void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, float* q_sum,
+void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, const float* q_sum,
                            uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream);
 
 // ---- K4/K5 asymmetric RankQuant scoring (scan_asym.cu) ---------------------------
@@ -172,6 +172,41 @@ void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t b
 void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const float* q_unit,
                         uint64_t nq, const uint64_t* offsets, const uint32_t* cands,
                         uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream);
+
+// ---- integer score scans on CTA pairs (scan_score_pair.cu) ---------------------------
+// src: 1, 2, 4 = RankQuant bits, 16 = Rank.  The operand's rows (bytes of device
+// memory the caller provides) hold the queries in tiles of nqt.
+struct ScoreOperand {
+  void* rows;
+  uint64_t bytes;
+  uint32_t nqt, k_bytes, planes;
+};
+bool score_rankquant_eligible(uint32_t dim, uint32_t bits);
+bool score_rank_eligible(uint32_t dim);
+// shape of the operand for nq queries (rows unset); q_per_tile (RankQuant): at most this many, 0 = 128
+ScoreOperand score_operand(uint32_t src, uint64_t nq, uint32_t dim, uint32_t q_per_tile);
+// fill the operand and bound[2 nq] (launch_score_margin's); q: what the scores sum;
+// half_steps: multiples of 1/2, which a power-of-two scale holds exactly
+void launch_fix_rankquant(const float* q, uint64_t nq, uint32_t dim, uint32_t bits, bool half_steps,
+                          const ScoreOperand& b, double* bound, cudaStream_t stream);
+// sym: q = u16 query ranks, else f32 unit queries
+void launch_fix_rank(bool sym, const void* q, uint64_t nq, uint32_t dim, const ScoreOperand& b, double* bound,
+                     cudaStream_t stream);
+// keys[q * ld + u] of the (sampled) documents; smaller is better
+void launch_score_scan(const void* rows, uint64_t n, uint32_t dim, uint32_t src, const ScoreOperand& b, uint64_t nq,
+                       uint32_t block_stride, uint32_t* keys, uint64_t ld, uint32_t* err, cudaStream_t stream);
+// (key, doc) with key <= thr[q * thr_stride] appended to row q (cnt, cap)
+void launch_score_filter(const void* rows, uint64_t n, uint32_t dim, uint32_t src, const ScoreOperand& b, uint64_t nq,
+                         const uint32_t* thr, uint64_t thr_stride, uint32_t* cnt, uint32_t cap, uint32_t* f_keys,
+                         uint32_t* f_ids, uint32_t* err, cudaStream_t stream);
+// *flag |= 1 when a document outside some query's kp selected keys could belong to its top k
+void launch_score_margin(const uint32_t* sel_keys, uint64_t nq, uint32_t kp, uint32_t k, const double* bound,
+                         uint32_t src, uint32_t* flag, cudaStream_t stream);
+// exact Rank scores of kp candidates per query (ids below n): keys[q * kp + i]
+void launch_rank_subset(bool sym, const uint16_t* ranks, uint32_t dim, const void* q, const float* q_sum, uint64_t nq,
+                        const uint32_t* cands, uint32_t kp, uint32_t* keys, cudaStream_t stream);
+float rank_norm_f32(uint32_t dim);
+void launch_rank_row_sum(const float* q, uint64_t nq, uint32_t dim, float* out, cudaStream_t stream);
 
 // ---- encoders (encode.cu) ----------------------------------------------------------
 // kind: 0 RankQuant packed codes, 1 sign bitmap, 2 const-weight bitmap, 3 FastScan

@@ -174,13 +174,33 @@ __global__ void __launch_bounds__(kRfThreads)
   }
 }
 
-// q_sum = sequential f32 sum of each q_unit row (Iterator::sum order)
+// q_sum = sequential f32 sum of each q_unit row (Iterator::sum order).  A warp per
+// row stages it in shared memory; lane 0 adds in order, bound by the add latency
+// (a thread per row read its row from global memory one value at a time).
 __global__ void row_sum_kernel(const float* __restrict__ q, uint64_t nq, uint32_t dim, float* __restrict__ out) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ __align__(16) float row[4][1024];
+  const uint32_t wid = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const uint64_t i = (uint64_t)blockIdx.x * 4 + wid;
   if (i >= nq) return;
   float s = -0.0f;
-  for (uint32_t j = 0; j < dim; j++) s = __fadd_rn(s, q[i * dim + j]);
-  out[i] = s;
+  for (uint32_t c0 = 0; c0 < dim; c0 += 1024) {
+    const uint32_t cn = dim - c0 < 1024 ? dim - c0 : 1024;
+    for (uint32_t j = lane; j < cn; j += 32) row[wid][j] = q[i * dim + c0 + j];
+    __syncwarp();
+    if (lane == 0) {
+      uint32_t j = 0;
+      for (; j + 4 <= cn; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&row[wid][j]);
+        s = __fadd_rn(s, v.x);
+        s = __fadd_rn(s, v.y);
+        s = __fadd_rn(s, v.z);
+        s = __fadd_rn(s, v.w);
+      }
+      for (; j < cn; j++) s = __fadd_rn(s, row[wid][j]);
+    }
+    __syncwarp();
+  }
+  if (lane == 0) out[i] = s;
 }
 
 unsigned rf_grid(uint64_t units, uint64_t per_cta) {
@@ -240,6 +260,12 @@ float rank_norm_f32(uint32_t dim) {
   return (float)std::sqrt(d * (d * d - 1.0) / 12.0);
 }
 
+void launch_rank_row_sum(const float* q, uint64_t nq, uint32_t dim, float* out, cudaStream_t stream) {
+  if (!nq) return;
+  row_sum_kernel<<<(unsigned)((nq + 3) / 4), 128, 0, stream>>>(q, nq, dim, out);
+  launched();
+}
+
 void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const uint16_t* q_ranks, uint64_t nq,
                           uint32_t* keys, uint64_t ld, cudaStream_t stream) {
   if (!n || !nq) return;
@@ -263,11 +289,9 @@ void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const
   }
 }
 
-void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, float* q_sum,
+void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, const float* q_sum,
                            uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream) {
   if (!n || !nq) return;
-  row_sum_kernel<<<(unsigned)((nq + 127) / 128), 128, 0, stream>>>(q_unit, nq, dim, q_sum);
-  launched();
   const float inv_norm = 1.0f / rank_norm_f32(dim);
   const float mean = ((float)dim - 1.0f) / 2.0f;
   if (dim % 8 == 0) {
