@@ -40,6 +40,7 @@ void select_rows(Workspace& w, const uint32_t* keys, const uint32_t* ids, const 
   SelectArgs a{keys, ids, row_off, ld, n, k, key_bits, id_bits, out_keys, out_ids, row_len, ordered ? 0u : 1u};
   size_t se = select_rows_scratch_elems(rows, k, row_off ? 0 : n);
   uint64_t* scratch = se ? (uint64_t*)w.scratch.ensure(se * 8) : nullptr;
+  if (select_takes_grid(a, rows, scratch)) a.err = w.tc_err_word(st);
   launch_select_rows(a, rows, scratch, st);
 }
 

@@ -23,12 +23,15 @@ struct SelectArgs {
   uint32_t* out_keys;
   uint32_t* out_ids;
   const uint32_t* row_len;  // optional: row r holds min(row_len[r], n) entries at r*ld
-  uint32_t unordered;       // 1: a row's k_eff winners in any order (the set only; per-row and cluster forms)
+  uint32_t unordered;       // 1: a row's k_eff winners in any order (the set only)
+  uint32_t* err;            // whole-GPU form: |= 1 when a barrier wait gave up (may be null)
 };
 // u64 scratch elements launch_select_rows may use for `rows` rows of length n
 // (0 for ragged rows): global sort buffers for k > kSelectSmemCap, and the
-// whole-GPU form's histograms and winners for a few rows of >= 2^20 keys.
+// whole-GPU form's histograms and candidates for a few rows of >= 32,768 keys.
 size_t select_rows_scratch_elems(uint64_t rows, uint32_t k, uint64_t n);
+// whether launch_select_rows runs the whole-GPU form (and so may set *a.err)
+bool select_takes_grid(const SelectArgs& a, uint64_t rows, const uint64_t* scratch);
 void launch_select_rows(const SelectArgs& a, uint64_t rows, uint64_t* scratch,
                         cudaStream_t stream);
 

@@ -438,62 +438,94 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kSelThrea
   }
 }
 
-// Whole-GPU form for a few very long rows (one query per call over millions
-// of docs): each digit pass is one launch whose CTAs histogram grid-stride
-// slices of every row into a global histogram; the last CTA of a row to
-// finish (atomic arrival count after a fence) scans it, fixes the digit and
-// resets the histogram.  A collect launch gathers the winners the same way and
-// its last CTA per row sorts and writes them.  No CTA waits for another.
-constexpr uint32_t kWideRows = 16;
-constexpr uint64_t kWideMinN = 1u << 20;
-constexpr int kWideThreads = 512;
+// Whole-GPU form for a few long rows (one query per call): a cooperative launch of
+// C CTAs per row.  Each CTA stages its slice of the row in shared memory once and
+// histograms it there digit by digit; the histograms are added up in global
+// memory, and after a grid barrier every CTA finds the bin of the k-th key.  The
+// digits stop as soon as the keys up to that bin are few enough for one CTA to
+// order: the CTAs append them to a global list, and the last CTA to finish takes
+// the k best.  Barrier waits are bounded; one that gives up sets *a.err and the
+// row's CTAs return.
+// What bounds it: the barriers and the histogram's round trips, about 4 us a
+// digit.  Measured, one row (us, the 8-CTA cluster form or, from 2^20 keys, a launch
+// per digit over the whole GPU before, and this form): 100k Hamming keys top-320 17.9
+// -> 9.9; 171k float keys top-1,000 27.3 -> 13.7; 1M float keys top-10 101 -> 16.7; 5M
+// overlaps top-2,000 92 -> 33.
+constexpr uint32_t kGridRows = 16;
+constexpr uint64_t kGridMinN = 32768;
+constexpr int kGridThreads = 512;
+constexpr uint32_t kGridSlice = 4096;   // keys a CTA takes before more CTAs join
+constexpr uint32_t kGridCtas = 148;     // all CTAs of a launch are resident at once
+constexpr uint32_t kGridDigits = 6;     // 32 key bits and 32 id bits, 11 at a time
+constexpr size_t kGridStageBytes = 176 * 1024;
 
-struct WideState {
-  uint64_t prefix, fixed;
-  uint32_t need, done, arrive, below, tie, pad;
+struct GridState {
+  uint32_t arrive, cands, done, pad;
 };
-static_assert(sizeof(WideState) == 40, "WideState layout");
 
-struct WideScratch {
-  uint32_t* hist;    // rows x kHistBins
-  WideState* state;  // rows
-  uint64_t* win;     // rows x k
+struct GridScratch {
+  GridState* state;  // rows, zeroed by the launcher
+  uint32_t* hist;    // rows x kGridDigits x kHistBins, zeroed by the launcher
+  uint64_t* cand;    // rows x kSelectSmemCap
 };
 
-__host__ __device__ inline uint64_t wide_state_elems(uint64_t rows) { return (rows * sizeof(WideState) + 7) / 8; }
-
-__host__ inline WideScratch wide_scratch(uint64_t* scratch, uint64_t rows) {
-  WideScratch w;
-  w.hist = reinterpret_cast<uint32_t*>(scratch);
-  w.state = reinterpret_cast<WideState*>(scratch + rows * (kHistBins / 2));
-  w.win = scratch + rows * (kHistBins / 2) + wide_state_elems(rows);
-  return w;
+__host__ __device__ inline uint64_t grid_zero_bytes(uint64_t rows) {
+  return rows * (sizeof(GridState) + (uint64_t)kGridDigits * kHistBins * 4);
 }
 
-__global__ void wide_init_kernel(SelectArgs a, WideScratch w) {
-  const uint64_t row = blockIdx.x;
-  for (uint32_t b = threadIdx.x; b < kHistBins; b += blockDim.x) w.hist[row * kHistBins + b] = 0;
+__host__ inline GridScratch grid_scratch(uint64_t* scratch, uint64_t rows) {
+  GridScratch g;
+  g.state = reinterpret_cast<GridState*>(scratch);
+  g.hist = reinterpret_cast<uint32_t*>(g.state + rows);
+  g.cand = scratch + grid_zero_bytes(rows) / 8;
+  return g;
+}
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Barrier over a row's CTAs; `target` arrivals in all.  False when it gave up
+// (about a second) or another CTA did.
+__device__ bool grid_barrier(GridState* st, uint32_t target, uint32_t* err) {
+  __shared__ uint32_t s_ok;
+  __threadfence();
+  __syncthreads();
   if (threadIdx.x == 0) {
-    WideState& st = w.state[row];
-    st.prefix = 0;
-    st.fixed = 0;
-    st.need = (uint32_t)(a.n < a.k ? a.n : a.k);
-    st.done = st.need == a.n;  // every key is a winner
-    st.arrive = st.below = st.tie = st.pad = 0;
+    atomicAdd(&st->arrive, 1u);
+    uint32_t ok = 0;
+    uint64_t t0 = 0;
+    for (uint32_t it = 0; it < (1u << 24); it++) {
+      if (ld_acquire(&st->arrive) >= target) {
+        ok = 1;
+        break;
+      }
+      if ((it & 1023) == 1023) {
+        uint64_t now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (!t0)
+          t0 = now;
+        else if (now - t0 > 1000000000ull)
+          break;
+      }
+    }
+    if (!ok && err) atomicOr(err, 1u);
+    s_ok = ok;
   }
+  __syncthreads();
+  const bool ok = s_ok != 0;
+  __syncthreads();
+  return ok;
 }
 
-// Exclusive scan of hist[0..kHistBins) by kWideThreads threads (4 bins each);
+// Exclusive scan of hist[0..kHistBins) by kGridThreads threads (4 bins each);
 // the thread whose bins hold the need-th key writes (bin, before, in_bin).
-__device__ void wide_find_bin(const uint32_t* hist, uint32_t need, uint32_t* out3) {
-  __shared__ uint32_t warp_tot[kWideThreads / 32];
+__device__ void grid_find_bin(const uint32_t (&h)[4], uint32_t need, uint32_t* out3) {
+  __shared__ uint32_t warp_tot[kGridThreads / 32];
   const uint32_t t = threadIdx.x, lane = t & 31, wp = t >> 5;
-  uint32_t h[4], sum = 0;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    h[j] = hist[4 * t + j];
-    sum += h[j];
-  }
+  const uint32_t sum = h[0] + h[1] + h[2] + h[3];
   uint32_t incl = sum;
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
@@ -502,13 +534,13 @@ __device__ void wide_find_bin(const uint32_t* hist, uint32_t need, uint32_t* out
   if (lane == 31) warp_tot[wp] = incl;
   __syncthreads();
   if (wp == 0) {
-    const uint32_t v = lane < kWideThreads / 32 ? warp_tot[lane] : 0;
+    const uint32_t v = lane < kGridThreads / 32 ? warp_tot[lane] : 0;
     uint32_t x = v;
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
       if (lane >= o) x += y;
     }
-    if (lane < kWideThreads / 32) warp_tot[lane] = x - v;
+    if (lane < kGridThreads / 32) warp_tot[lane] = x - v;
   }
   __syncthreads();
   uint32_t before = warp_tot[wp] + incl - sum;
@@ -527,139 +559,181 @@ __device__ void wide_find_bin(const uint32_t* hist, uint32_t need, uint32_t* out
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kWideThreads) wide_hist_kernel(SelectArgs a, WideScratch w, uint32_t shift,
-                                                                 uint32_t width) {
-  __shared__ uint32_t hist[kHistBins];
-  __shared__ uint32_t s_last, s_pick[3];
-  const uint64_t row = blockIdx.y;
-  WideState& st = w.state[row];
-  if (*reinterpret_cast<volatile uint32_t*>(&st.done)) return;  // uniform per row
-  const uint64_t prefix = st.prefix, fixed = st.fixed;
-  const uint32_t mask = (1u << width) - 1;
-  for (uint32_t b = threadIdx.x; b < kHistBins; b += blockDim.x) hist[b] = 0;
+__global__ void __launch_bounds__(kGridThreads) grid_select_kernel(SelectArgs a, GridScratch w, uint32_t ctas,
+                                                                   uint32_t stage) {
+  // this CTA's candidates, then the row's; during the digits four copies of the
+  // histogram (the first digits of float scores fall into few bins)
+  __shared__ __align__(16) uint64_t buf[kSelectSmemCap];
+  uint32_t* hist = reinterpret_cast<uint32_t*>(buf);
+  static_assert(sizeof(uint64_t) * kSelectSmemCap >= 4 * kHistBins * 4, "histogram copies");
+  __shared__ uint32_t s_pick[3], s_cnt, s_base, s_last;
+  extern __shared__ __align__(16) uint32_t st_keys[];  // [per] keys, then [per] ids when explicit
+  const uint64_t row = blockIdx.x / ctas;
+  const uint32_t c = blockIdx.x % ctas, t = threadIdx.x;
+  GridState* st = w.state + row;
+  const uint64_t n = a.n, per = (n + ctas - 1) / ctas;
+  const uint64_t lo = c * per < n ? c * per : n, hi = lo + per < n ? lo + per : n;
+  const uint32_t cnt = (uint32_t)(hi - lo);
+  const uint32_t* keys = a.keys + row * a.ld + lo;
+  const uint32_t* ids = a.ids ? a.ids + row * a.ld + lo : nullptr;
+  uint32_t* st_ids = st_keys + per;
+  const uint32_t k_eff = (uint32_t)(n < a.k ? n : a.k);
+  // few enough for one CTA: a sort of at most k + k/4 + 64, or, when the order does
+  // not matter, a last bin of at most 256 whose lowest are found by rank
+  auto enough = [&](uint32_t need, uint32_t in_bin) -> bool {
+    const uint32_t total = k_eff - need + in_bin;
+    if (in_bin == need) return true;
+    return total <= kSelectSmemCap && (a.unordered ? in_bin <= 256 : total <= k_eff + k_eff / 4 + 64);
+  };
+  if (stage) {  // eight loads in flight per thread
+    for (uint32_t i0 = t; i0 < cnt; i0 += 8 * kGridThreads) {
+      uint32_t v[8], u[8];
+#pragma unroll
+      for (uint32_t j = 0; j < 8; j++) {
+        const uint32_t i = i0 + j * kGridThreads;
+        v[j] = i < cnt ? keys[i] : 0u;
+        u[j] = i < cnt && ids ? ids[i] : 0u;
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < 8; j++) {
+        const uint32_t i = i0 + j * kGridThreads;
+        if (i < cnt) {
+          st_keys[i] = v[j];
+          if (ids) st_ids[i] = u[j];
+        }
+      }
+    }
+  }
+  auto key_at = [&](uint32_t i) -> uint64_t {
+    const uint32_t k = stage ? st_keys[i] : keys[i];
+    const uint32_t id = ids ? (stage ? st_ids[i] : ids[i]) : (uint32_t)(lo + i);
+    return ((uint64_t)k << 32) | id;
+  };
+  uint64_t prefix = 0, fixed = 0;
+  uint32_t need = k_eff, in_bin = (uint32_t)n, phase = 0;
+  uint32_t left[2] = {a.key_bits, a.id_bits};
+  uint32_t part = left[0] ? 0 : 1;
+  while (!enough(need, in_bin) && part < 2) {
+    const uint32_t width = left[part] < 11 ? left[part] : 11;
+    left[part] -= width;
+    const uint32_t shift = (part ? 0 : 32) + left[part], mask = (1u << width) - 1;
+    if (!left[part]) part++;
+    if (part == 1 && !left[1]) part = 2;
+    for (uint32_t b = t; b < 4 * kHistBins; b += kGridThreads) hist[b] = 0;
+    __syncthreads();
+    uint32_t* mine = hist + (t & 3) * kHistBins;
+    for (uint32_t i = t; i < cnt; i += kGridThreads) {
+      const uint64_t key = key_at(i);
+      if ((key & fixed) == prefix) atomicAdd(&mine[(uint32_t)(key >> shift) & mask], 1u);
+    }
+    __syncthreads();
+    uint32_t* gh = w.hist + (row * kGridDigits + phase) * kHistBins;
+    for (uint32_t b = t; b <= mask; b += kGridThreads) {
+      const uint32_t v = hist[b] + hist[b + kHistBins] + hist[b + 2 * kHistBins] + hist[b + 3 * kHistBins];
+      if (v) atomicAdd(&gh[b], v);
+    }
+    phase++;
+    if (!grid_barrier(st, phase * ctas, a.err)) return;
+    uint32_t h[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) h[j] = 4 * t + j <= mask ? __ldcg(&gh[4 * t + j]) : 0u;
+    grid_find_bin(h, need, s_pick);
+    need -= s_pick[1];
+    in_bin = s_pick[2];
+    prefix |= (uint64_t)s_pick[0] << shift;
+    fixed |= (uint64_t)mask << shift;
+    __syncthreads();
+  }
+  // candidates: every key up to the prefix's bin (k_eff - need + in_bin of them)
+  if (t == 0) s_cnt = 0;
   __syncthreads();
-  const uint32_t* keys = a.keys + row * a.ld;
-  const uint32_t* ids = a.ids ? a.ids + row * a.ld : nullptr;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t key = load_key(keys, ids, i);
-    if ((key & fixed) == prefix) atomicAdd(&hist[(uint32_t)(key >> shift) & mask], 1u);
+  for (uint32_t i = t; i < cnt; i += kGridThreads) {
+    const uint64_t key = key_at(i);
+    if ((key & fixed) <= prefix) {
+      const uint32_t at = atomicAdd(&s_cnt, 1u);
+      if (at < kSelectSmemCap) buf[at] = key;
+    }
   }
   __syncthreads();
-  uint32_t* gh = w.hist + row * kHistBins;
-  for (uint32_t b = threadIdx.x; b <= mask; b += blockDim.x)
-    if (hist[b]) atomicAdd(&gh[b], hist[b]);
+  const uint32_t total = k_eff - need + in_bin < kSelectSmemCap ? k_eff - need + in_bin : kSelectSmemCap;
+  if (t == 0) s_base = s_cnt ? atomicAdd(&st->cands, s_cnt) : 0u;
+  __syncthreads();
+  uint64_t* cand = w.cand + row * kSelectSmemCap;
+  for (uint32_t j = t; j < s_cnt && j < kSelectSmemCap; j += kGridThreads)
+    if (s_base + j < kSelectSmemCap) cand[s_base + j] = buf[j];
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&st.arrive, 1u) == gridDim.x - 1;
+  if (t == 0) s_last = atomicAdd(&st->done, 1u) == ctas - 1;
   __syncthreads();
   if (!s_last) return;
-  // last CTA of this row: every other CTA's histogram is in gh
   __threadfence();
-  for (uint32_t b = threadIdx.x; b < kHistBins; b += blockDim.x) {
-    hist[b] = b <= mask ? *reinterpret_cast<volatile uint32_t*>(&gh[b]) : 0u;
-    gh[b] = 0;
-  }
-  __syncthreads();
-  const uint32_t need = st.need;
-  wide_find_bin(hist, need, s_pick);
-  if (threadIdx.x == 0) {
-    st.need = need - s_pick[1];
-    st.prefix = prefix | ((uint64_t)s_pick[0] << shift);
-    st.fixed = fixed | ((uint64_t)mask << shift);
-    st.done = s_pick[2] == need - s_pick[1];  // the whole bin is taken
-    st.arrive = 0;
-  }
-}
-
-// Collect: keys strictly below the prefix, then `need` keys inside it; the last
-// CTA of a row sorts the k winners and writes them.
-__global__ void __launch_bounds__(kWideThreads) wide_collect_kernel(SelectArgs a, WideScratch w) {
-  __shared__ uint64_t buf[kSelectSmemCap];
-  __shared__ uint32_t s_last;
-  const uint64_t row = blockIdx.y;
-  WideState& st = w.state[row];
-  const uint64_t prefix = st.prefix, fixed = st.fixed;
-  const uint32_t k_eff = (uint32_t)(a.n < a.k ? a.n : a.k), need = st.need;
-  const uint32_t below_total = k_eff - need;
-  const uint32_t* keys = a.keys + row * a.ld;
-  const uint32_t* ids = a.ids ? a.ids + row * a.ld : nullptr;
-  uint64_t* win = w.win + row * (uint64_t)a.k;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  // warp-uniform trip count so the ballots see every lane
-  const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-  for (uint64_t base = first; base < a.n; base += stride) {
-    const uint64_t i = base + lane;
-    uint64_t key = 0;
-    bool lo = false, eq = false;
-    if (i < a.n) {
-      key = load_key(keys, ids, i);
-      const uint64_t m = key & fixed;
-      lo = m < prefix;
-      eq = m == prefix;
-    }
-    uint32_t lt;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-    const uint32_t bl = __ballot_sync(0xFFFFFFFFu, lo), be = __ballot_sync(0xFFFFFFFFu, eq);
-    uint32_t b0 = 0, e0 = 0;
-    if (lane == 0) {
-      if (bl) b0 = atomicAdd(&st.below, (uint32_t)__popc(bl));
-      if (be) e0 = atomicAdd(&st.tie, (uint32_t)__popc(be));
-    }
-    b0 = __shfl_sync(0xFFFFFFFFu, b0, 0);
-    e0 = __shfl_sync(0xFFFFFFFFu, e0, 0);
-    if (lo) {
-      const uint32_t slot = b0 + __popc(bl & lt);
-      if (slot < below_total) win[slot] = key;
-    } else if (eq) {
-      const uint32_t slot = e0 + __popc(be & lt);
-      if (slot < need) win[below_total + slot] = key;
-    }
-  }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&st.arrive, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  uint32_t len = 1;
-  while (len < k_eff) len <<= 1;
-  for (uint32_t j = threadIdx.x; j < len; j += blockDim.x)
-    buf[j] = j < k_eff ? *reinterpret_cast<volatile uint64_t*>(&win[j]) : ~0ull;
-  __syncthreads();
-  bitonic_sort(buf, len);
   uint32_t* out_k = a.out_keys + row * (uint64_t)a.k;
   uint32_t* out_i = a.out_ids + row * (uint64_t)a.k;
-  for (uint32_t j = threadIdx.x; j < a.k; j += blockDim.x) {
-    out_k[j] = j < k_eff ? (uint32_t)(buf[j] >> 32) : kSentinelKey;
-    out_i[j] = j < k_eff ? (uint32_t)buf[j] : kSentinelId;
+  for (uint32_t j = k_eff + t; j < a.k; j += kGridThreads) {
+    out_k[j] = kSentinelKey;
+    out_i[j] = kSentinelId;
   }
-}
-
-void launch_select_wide(const SelectArgs& a, uint64_t rows, uint64_t* scratch, cudaStream_t stream) {
-  const WideScratch w = wide_scratch(scratch, rows);
-  wide_init_kernel<<<(unsigned)rows, 256, 0, stream>>>(a, w);
-  uint64_t per_row = (a.n + kWideThreads * 32 - 1) / (kWideThreads * 32);  // ~32 keys per thread
-  const uint64_t cap = (148ull * 4 + rows - 1) / rows;
-  if (per_row > cap) per_row = cap;
-  if (per_row < 1) per_row = 1;
-  const dim3 grid((unsigned)per_row, (unsigned)rows);
-  for (int part = 0; part < 2; part++) {  // key bits, then id bits, 11 at a time from the top
-    uint32_t bits = part == 0 ? a.key_bits : a.id_bits;
-    uint32_t top = (part == 0 ? 32u : 0u) + bits;
-    while (bits > 0) {
-      const uint32_t wd = bits < 11 ? bits : 11;
-      top -= wd;
-      wide_hist_kernel<<<grid, kWideThreads, 0, stream>>>(a, w, top, wd);
-      bits -= wd;
+  if (a.unordered) {
+    // keys below the bin are in; the bin's `need` lowest are found by rank among
+    // the bin (at most 256 of them unless the digits ran out on equal keys)
+    if (t == 0) s_cnt = s_base = 0;
+    __syncthreads();
+    for (uint32_t j = t; j < total; j += kGridThreads) {
+      const uint64_t key = __ldcg(&cand[j]);
+      if ((key & fixed) < prefix) {
+        const uint32_t at = atomicAdd(&s_cnt, 1u);
+        out_k[at] = (uint32_t)(key >> 32);
+        out_i[at] = (uint32_t)key;
+      } else {
+        buf[atomicAdd(&s_base, 1u)] = key;
+      }
     }
+    __syncthreads();
+    const uint32_t bin_n = s_base;
+    for (uint32_t j = t; j < bin_n; j += kGridThreads) {
+      const uint64_t key = buf[j];
+      uint32_t r = 0;
+      if (in_bin != need)
+        for (uint32_t e = 0; e < bin_n; e++) r += buf[e] < key || (buf[e] == key && e < j) ? 1u : 0u;
+      else
+        r = j;
+      if (r < need) {
+        out_k[k_eff - need + r] = (uint32_t)(key >> 32);
+        out_i[k_eff - need + r] = (uint32_t)key;
+      }
+    }
+    return;
   }
-  wide_collect_kernel<<<grid, kWideThreads, 0, stream>>>(a, w);
-  launched();
+  uint32_t len = 1;
+  while (len < total) len <<= 1;
+  for (uint32_t j = t; j < len; j += kGridThreads) buf[j] = j < total ? __ldcg(&cand[j]) : ~0ull;
+  __syncthreads();
+  bitonic_sort(buf, len);
+  for (uint32_t j = t; j < k_eff; j += kGridThreads) {
+    out_k[j] = (uint32_t)(buf[j] >> 32);
+    out_i[j] = (uint32_t)buf[j];
+  }
 }
 
-bool use_select_wide(const SelectArgs& a, uint64_t rows, const uint64_t* scratch) {
-  return scratch && !a.row_off && !a.row_len && rows <= kWideRows && a.n >= kWideMinN && a.k <= kSelectSmemCap;
+bool use_select_grid(const SelectArgs& a, uint64_t rows, const uint64_t* scratch) {
+  return scratch && !a.row_off && !a.row_len && rows <= kGridRows && a.n >= kGridMinN && a.n < (1ull << 32) &&
+         a.k >= 1 && a.k <= kSelectSmemCap;
+}
+
+void launch_select_grid(const SelectArgs& a, uint64_t rows, uint64_t* scratch, cudaStream_t stream) {
+  const GridScratch w = grid_scratch(scratch, rows);
+  OVB_CUDA(cudaMemsetAsync(scratch, 0, grid_zero_bytes(rows), stream));
+  uint64_t ctas = (a.n + kGridSlice - 1) / kGridSlice;
+  if (ctas > kGridCtas / rows) ctas = kGridCtas / rows;
+  const uint64_t per = (a.n + ctas - 1) / ctas, bytes = per * (a.ids ? 8 : 4);
+  uint32_t stage = bytes <= kGridStageBytes ? 1u : 0u, c32 = (uint32_t)ctas;
+  allow_dynamic_smem(grid_select_kernel);
+  SelectArgs args = a;
+  GridScratch ws = w;
+  void* p[] = {&args, &ws, &c32, &stage};
+  OVB_CUDA(cudaLaunchCooperativeKernel((const void*)grid_select_kernel, dim3((unsigned)(rows * ctas)),
+                                       dim3(kGridThreads), p, stage ? (size_t)bytes : 0, stream));
+  launched();
 }
 
 }  // namespace
@@ -668,19 +742,23 @@ size_t select_rows_scratch_elems(uint64_t rows, uint32_t k, uint64_t n) {
   uint64_t len = 1;
   while (len < k) len <<= 1;
   uint64_t e = k <= kSelectSmemCap ? 0 : rows * len;
-  if (rows <= kWideRows && k <= kSelectSmemCap && n >= kWideMinN) {  // the whole-GPU form for few long rows
-    const uint64_t wide = rows * (kHistBins / 2) + wide_state_elems(rows) + rows * (uint64_t)k;
-    if (wide > e) e = wide;
+  if (rows <= kGridRows && k <= kSelectSmemCap && n >= kGridMinN) {  // the whole-GPU form for few long rows
+    const uint64_t grid = grid_zero_bytes(rows) / 8 + rows * (uint64_t)kSelectSmemCap;
+    if (grid > e) e = grid;
   }
   return e;
+}
+
+bool select_takes_grid(const SelectArgs& a, uint64_t rows, const uint64_t* scratch) {
+  const char* env = getenv("OVB_SELECT_WIDE");  // "0" keeps the cluster / per-row forms
+  return !(env && env[0] == '0') && use_select_grid(a, rows, scratch);
 }
 
 void launch_select_rows(const SelectArgs& a, uint64_t rows, uint64_t* scratch,
                         cudaStream_t stream) {
   if (rows == 0) return;
-  const char* wide_env = getenv("OVB_SELECT_WIDE");  // "0" keeps the cluster / per-row forms
-  if (!(wide_env && wide_env[0] == '0') && use_select_wide(a, rows, scratch)) {
-    launch_select_wide(a, rows, scratch, stream);
+  if (select_takes_grid(a, rows, scratch)) {
+    launch_select_grid(a, rows, scratch, stream);
     return;
   }
   // few long rows: one 8-CTA cluster per row (below two rows per SM the
