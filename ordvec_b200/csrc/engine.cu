@@ -399,10 +399,8 @@ static void filtered_candidates(const Scores& sc, uint64_t n, uint64_t qn, uint3
 
 // The FP64 rescoring of an exact RankQuant search's kp candidates per query.
 static void rescore_rankquant(const Index& rq, const float* qu, float inv_norm, uint64_t qn, uint32_t kp,
-                              const uint32_t* ids, uint32_t* keys, Workspace& w, cudaStream_t st) {
-  uint64_t* off = (uint64_t*)w.off.ensure((qn + 1) * 8);
-  launch_uniform_offsets(off, qn, kp, st);
-  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, qn, off, ids, kp, inv_norm, keys, st);
+                              const uint32_t* ids, uint32_t* keys, cudaStream_t st) {
+  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, qn, nullptr, ids, kp, inv_norm, keys, st);
 }
 
 // Tensor-core search of prepared query rows qu (nq x dim f32) scored as
@@ -440,7 +438,7 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, b
       sc.prepare(qu + q0 * dim, qn, w, st);
       filtered_candidates(sc, n, qn, ke, (uint32_t)kp0, fp, flag, ok + q0 * ke, oi + q0 * ke, w, st,
                           [&](const uint32_t* ids, uint32_t* keys) {
-                            rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp0, ids, keys, w, st);
+                            rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp0, ids, keys, st);
                           });
       OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
       OVB_CUDA(cudaStreamSynchronize(st));
@@ -487,8 +485,8 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, b
     w.split_kp = std::max<uint64_t>(w.split_kp, kp);
     uint32_t* k2 = (uint32_t*)w.keys2.ensure(qn * kp * 4);
     const uint32_t* ti = w.thr_ids.as<uint32_t>();
-    rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp, ti, k2, w, st);
-    select_rows(w, k2, ti, w.off.as<uint64_t>(), 0, 0, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st);
+    rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp, ti, k2, st);
+    select_rows(w, k2, ti, nullptr, kp, kp, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st);
     w.mark(st, 3);
   }
   return ke;
@@ -535,7 +533,7 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   if (filtered) {
     filtered_candidates(sc, n, nq, ke, (uint32_t)kp, fp, d_flag, ok, oi, w, st,
                         [&](const uint32_t* ids, uint32_t* keys) {
-                          rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ids, keys, w, st);
+                          rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ids, keys, st);
                         });
     return ke;
   }
@@ -546,8 +544,8 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   select_rows(w, keys, nullptr, nullptr, n, n, nq, (uint32_t)kp, 32, id_bits, tk, ti, st);
   if (kp < n) sc.margin(tk, nq, (uint32_t)kp, ke, d_flag, st);
   uint32_t* k2 = (uint32_t*)w.keys2.ensure(nq * kp * 4);
-  rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ti, k2, w, st);
-  select_rows(w, k2, ti, w.off.as<uint64_t>(), 0, 0, nq, ke, 32, id_bits, ok, oi, st);
+  rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ti, k2, st);
+  select_rows(w, k2, ti, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st);
   return ke;
 }
 
@@ -893,10 +891,8 @@ static bool split_rerank(const Index& rq, const float* qu, uint64_t nq, uint32_t
   select_rows(w, keys, cand, nullptr, me, me, nq, kp, 32, id_bits, ck, ci, st);
   OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
   launch_split_margin(ck, nq, kp, ke, l1, split_error_bound(dim, bits, inv_norm), flag, st);
-  uint64_t* off = (uint64_t*)w.off.ensure((nq + 1) * 8);
-  launch_uniform_offsets(off, nq, kp, st);
   uint32_t* k2 = (uint32_t*)w.rr_keys2.ensure(nq * kp * 4);
-  launch_asym_subset(codes, dim, bits, qu, nq, off, ci, kp, inv_norm, k2, st);
+  launch_asym_subset(codes, dim, bits, qu, nq, nullptr, ci, kp, inv_norm, k2, st);
   select_rows(w, k2, ci, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st);
   w.mark(st, 5);
   OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
@@ -934,10 +930,8 @@ uint32_t engine_two_stage(const Index& rq, const Index& s1, const float* d_q, ui
   const uint32_t mode = rerank_mode(w, rq, nq, me, ke);
   if (mode != OVB_RERANK_FP64 && split_rerank(rq, qu, nq, me, ke, inv_norm, mode == OVB_RERANK_SPLIT_RAW, w, st))
     return ke;
-  uint64_t* off = (uint64_t*)w.off.ensure((nq + 1) * 8);
-  launch_uniform_offsets(off, nq, me, st);
   uint32_t* keys = (uint32_t*)w.keys2.ensure(nq * me * 4);
-  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, nq, off, cand, me, inv_norm, keys, st);
+  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, nq, nullptr, cand, me, inv_norm, keys, st);
   w.mark(st, 4);
   // rows are uniform (me candidates each): the strided form, not offsets
   select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st);

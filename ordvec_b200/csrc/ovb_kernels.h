@@ -172,6 +172,8 @@ void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, cons
 void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t bits,
                       const float* q_unit, uint64_t nq, float inv_norm, uint32_t* keys,
                       uint64_t ld, cudaStream_t stream);
+// rows: query i's candidates cands[offsets[i] .. offsets[i + 1]) (at most max_row), or
+// with offsets null exactly max_row each; keys[] like cands[]
 void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const float* q_unit,
                         uint64_t nq, const uint64_t* offsets, const uint32_t* cands,
                         uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream);
@@ -223,8 +225,7 @@ uint64_t fastscan_block_bytes(uint32_t pairs_pad);
 // sets *flag (device u32, caller-zeroed) if any value is non-finite
 void launch_finite_flag(const float* x, uint64_t count, uint32_t* flag, cudaStream_t stream);
 
-// helper: key32 -> float score / sentinel mapping and uniform offsets
-void launch_uniform_offsets(uint64_t* off, uint64_t nq, uint64_t m, cudaStream_t stream);
+// helper: key32 -> float score / sentinel mapping
 // CSR rows from prefixes: row q of dst (at off[q]) = the first off[q+1] - off[q]
 // entries of row q of src (row stride ld)
 void launch_prefix_compact(const uint32_t* src, uint64_t ld, const uint64_t* off, uint64_t nq, uint32_t* dst,

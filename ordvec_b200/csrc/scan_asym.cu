@@ -127,11 +127,11 @@ __global__ void __launch_bounds__(kThreads)
 template <int BITS, int W>
 __global__ void __launch_bounds__(kThreads)
     asym_subset_kernel(const uint8_t* __restrict__ codes, uint32_t dim,
-                       const float* __restrict__ q_unit, const uint64_t* __restrict__ off,
+                       const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                        const uint32_t* __restrict__ cands, float inv_norm,
                        uint32_t* __restrict__ keys) {
   const uint64_t qi = blockIdx.y;
-  const uint64_t s = off[qi], e = off[qi + 1];
+  const uint64_t s = off ? off[qi] : qi * row_len, e = off ? off[qi + 1] : s + row_len;
   const uint32_t words = dim * BITS / 32;
   const int lane = threadIdx.x & 31;
   double qs[W][32 / BITS];
@@ -191,14 +191,15 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(kThreads)
     asym_subset_generic(const uint8_t* __restrict__ codes, uint32_t dim, uint32_t bits,
-                        const float* __restrict__ q_unit, const uint64_t* __restrict__ off,
+                        const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                         const uint32_t* __restrict__ cands, float inv_norm,
                         uint32_t* __restrict__ keys) {
   const uint64_t qi = blockIdx.y;
+  const uint64_t s = off ? off[qi] : qi * row_len, e = off ? off[qi + 1] : s + row_len;
   const uint32_t bpv = dim * bits / 8;
   const uint64_t gw = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) / 32;
   const uint64_t nw = (uint64_t)gridDim.x * kThreads / 32;
-  for (uint64_t i = off[qi] + gw; i < off[qi + 1]; i += nw) {
+  for (uint64_t i = s + gw; i < e; i += nw) {
     const double dot = generic_row_dot(codes + (uint64_t)cands[i] * bpv, dim, bits, q_unit + qi * dim);
     if ((threadIdx.x & 31) == 0) keys[i] = desc_key((float)(dot * (double)inv_norm));
   }
@@ -219,6 +220,37 @@ __global__ void __launch_bounds__(kThreads)
 constexpr int kTabThreads = 256;
 constexpr uint32_t kTabMaxBytes = 200 * 1024;
 
+// T[16 g + v] by the CTA's THREADS threads: a thread takes four values v of a group
+// (its high two bits fixed), so that each product and each conversion to double is
+// made once for them (16 queries x 1,000 rows, dim 1024 b=2: 13.8 -> 11.9 us).  Sums
+// run in the order of the codes.
+template <int BITS, int THREADS>
+__device__ __forceinline__ void build_table(double* T, const float* __restrict__ q, uint32_t dim) {
+  constexpr int G = 4 / BITS;
+  for (uint32_t e = threadIdx.x; e < dim * BITS; e += THREADS) {
+    const uint32_t g = e >> 2, i = e & 3;
+    const float* x = q + g * G;
+    double t[4];
+    if constexpr (BITS == 4) {  // v = 4 i + j: q (v - 7.5)
+      const double q0 = x[0], c = (double)(float)(4 * i) - 7.5;
+#pragma unroll
+      for (int j = 0; j < 4; j++) t[j] = 0.0 + q0 * (c + j);
+    } else if constexpr (BITS == 2) {  // codes i, j
+      const double q0 = x[0], q1 = x[1], a = 0.0 + q0 * ((double)(float)i - 1.5);
+#pragma unroll
+      for (int j = 0; j < 4; j++) t[j] = a + q1 * (j - 1.5);
+    } else {  // codes i >> 1, i & 1, j >> 1, j & 1
+      const double q0 = x[0], q1 = x[1], q2 = x[2], q3 = x[3];
+      const double a = (0.0 + q0 * ((i & 2) ? 0.5 : -0.5)) + q1 * ((i & 1) ? 0.5 : -0.5);
+#pragma unroll
+      for (int j = 0; j < 4; j++) t[j] = (a + q2 * ((j & 2) ? 0.5 : -0.5)) + q3 * ((j & 1) ? 0.5 : -0.5);
+    }
+    double2* out = reinterpret_cast<double2*>(T + 16 * g + 4 * i);
+    out[0] = make_double2(t[0], t[1]);
+    out[1] = make_double2(t[2], t[3]);
+  }
+}
+
 __device__ __forceinline__ double lds_f64(uint32_t addr) {
   double v;
   asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr));
@@ -228,34 +260,21 @@ __device__ __forceinline__ double lds_f64(uint32_t addr) {
 template <int BITS, bool SUBSET>
 __global__ void __launch_bounds__(kTabThreads)
     asym_table_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
-                      const float* __restrict__ q_unit, const uint64_t* __restrict__ off,
+                      const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                       const uint32_t* __restrict__ cands, float inv_norm, uint32_t* __restrict__ keys,
                       uint64_t ld) {
-  constexpr int G = 4 / BITS;
-  constexpr uint32_t MASK = (1u << BITS) - 1;
-  constexpr double C = ((double)(1u << BITS) - 1.0) * 0.5;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
   double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
   const uint64_t qi = blockIdx.y;
   const float* q = q_unit + qi * dim;
-  const uint32_t n_nib = dim * BITS / 4;
-  for (uint32_t e = threadIdx.x; e < n_nib * 16; e += kTabThreads) {
-    const uint32_t g = e >> 4, v = e & 15;
-    double acc = 0.0;
-#pragma unroll
-    for (int i = 0; i < G; i++) {
-      const uint32_t code = (v >> (BITS * (G - 1 - i))) & MASK;
-      acc += (double)q[g * G + i] * ((double)code - C);
-    }
-    T[e] = acc;
-  }
+  build_table<BITS, kTabThreads>(T, q, dim);
   __syncthreads();
 
   uint64_t start, end;
   if (SUBSET) {
-    start = off[qi];
-    end = off[qi + 1];
+    start = off ? off[qi] : qi * row_len;
+    end = off ? off[qi + 1] : start + row_len;
   } else {
     start = 0;
     end = n;
@@ -300,6 +319,63 @@ __global__ void __launch_bounds__(kTabThreads)
   }
 }
 
+// The table form for a handful of candidate rows (one query per call): four lanes a
+// row, one per accumulator of the lane-per-row form (nibbles = lane mod 4, the same
+// order), added up in the same tree, so the score is the same bit for bit.  A
+// lane's chain of dependent loads and adds is a quarter as long and four times as
+// many warps are in flight; with many rows the lane-per-row form is faster (its
+// 32 lookups stay in one 128-byte group, these take two to four wavefronts).
+constexpr int kTab4Threads = 512;
+constexpr uint64_t kTab4Rows = 8192;  // candidate rows of a launch that take this form
+template <int BITS>
+__global__ void __launch_bounds__(kTab4Threads)
+    asym_table4_kernel(const uint8_t* __restrict__ codes, uint32_t dim, const float* __restrict__ q_unit,
+                       const uint64_t* __restrict__ off, uint64_t row_len, const uint32_t* __restrict__ cands,
+                       float inv_norm, uint32_t* __restrict__ keys) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
+  double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
+  const uint64_t qi = blockIdx.y;
+  const float* q = q_unit + qi * dim;
+  const uint64_t start = off ? off[qi] : qi * row_len, end = off ? off[qi + 1] : start + row_len;
+  const uint32_t bpv = dim * BITS / 8, chunks = bpv / 16, r = threadIdx.x & 3;
+  const uint64_t i = start + (uint64_t)blockIdx.x * (kTab4Threads / 4) + threadIdx.x / 4;
+  const bool valid = i < end;
+  // the row's first pieces are on their way while the table is built
+  const uint4* rp = reinterpret_cast<const uint4*>(codes + (valid ? (uint64_t)cands[i] : 0) * bpv);
+  uint4 x[4];
+#pragma unroll
+  for (uint32_t u = 0; u < 4; u++) x[u] = valid && u < chunks ? __ldg(rp + u) : make_uint4(0, 0, 0, 0);
+  build_table<BITS, kTab4Threads>(T, q, dim);
+  __syncthreads();
+  // nibble 8 k + 2 b + h of a piece (h = 0: high) belongs to accumulator 2 (b & 1) + h
+  const uint32_t b0 = r >> 1, h = r & 1, sh = 8 * b0 + (h ? 0 : 4), at = t_base + (2 * b0 + h) * 128;
+  double acc = 0.0;
+  for (uint32_t c0 = 0; c0 < chunks; c0 += 4) {
+    uint4 nx[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++)
+      nx[u] = valid && c0 + 4 + u < chunks ? __ldg(rp + c0 + 4 + u) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      if (c0 + u < chunks) {
+        const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, tb = at + (c0 + u) * 4096;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t n0 = (w[k] >> sh) & 15u, n1 = (w[k] >> (sh + 16)) & 15u;
+          acc += lds_f64(tb + k * 1024 + n0 * 8);
+          acc += lds_f64(tb + k * 1024 + 512 + n1 * 8);
+        }
+      }
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) x[u] = nx[u];
+  }
+  acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
+  acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
+  if (valid && r == 0) keys[i] = desc_key((float)(acc * (double)inv_norm));
+}
+
 size_t table_smem(uint32_t dim, uint32_t bits) { return (size_t)dim * bits * 32 + 4096; }
 
 bool table_ok(uint32_t dim, uint32_t bits) {
@@ -310,13 +386,13 @@ bool table_ok(uint32_t dim, uint32_t bits) {
 
 template <bool SUBSET>
 void launch_table(uint32_t bits, dim3 grid, size_t smem, cudaStream_t st, const uint8_t* codes, uint64_t n,
-                  uint32_t dim, const float* qu, const uint64_t* off, const uint32_t* cands, float inv_norm,
-                  uint32_t* keys, uint64_t ld) {
+                  uint32_t dim, const float* qu, const uint64_t* off, uint64_t row_len, const uint32_t* cands,
+                  float inv_norm, uint32_t* keys, uint64_t ld) {
 #define OVB_TAB(B)                                                                                     \
   do {                                                                                                 \
     allow_dynamic_smem(asym_table_kernel<B, SUBSET>);                                                  \
-    asym_table_kernel<B, SUBSET><<<grid, kTabThreads, smem, st>>>(codes, n, dim, qu, off, cands, inv_norm, \
-                                                                  keys, ld);                           \
+    asym_table_kernel<B, SUBSET><<<grid, kTabThreads, smem, st>>>(codes, n, dim, qu, off, row_len, cands, \
+                                                                  inv_norm, keys, ld);                           \
   } while (0)
   if (bits == 1)
     OVB_TAB(1);
@@ -347,11 +423,11 @@ int plan_w(uint32_t dim, uint32_t bits) {
 template <int BITS>
 void dispatch_bits(int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t* codes, uint64_t n,
                    uint32_t dim, const float* qu, float inv_norm, uint32_t* keys, uint64_t ld,
-                   const uint64_t* off, const uint32_t* cands) {
+                   const uint64_t* off, uint64_t row_len, const uint32_t* cands) {
 #define OVB_ASYM_CASE(WV)                                                                                  \
   if (W == WV) {                                                                                           \
     if (subset)                                                                                            \
-      asym_subset_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, dim, qu, off, cands, inv_norm, keys); \
+      asym_subset_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, dim, qu, off, row_len, cands, inv_norm, keys); \
     else                                                                                                   \
       asym_scan_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, n, dim, qu, inv_norm, keys, ld);        \
     return;                                                                                                \
@@ -371,13 +447,13 @@ void dispatch_bits(int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t
 
 void dispatch(uint32_t bits, int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t* codes,
               uint64_t n, uint32_t dim, const float* qu, float inv_norm, uint32_t* keys, uint64_t ld,
-              const uint64_t* off, const uint32_t* cands) {
+              const uint64_t* off, uint64_t row_len, const uint32_t* cands) {
   if (bits == 1)
-    dispatch_bits<1>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, cands);
+    dispatch_bits<1>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands);
   else if (bits == 2)
-    dispatch_bits<2>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, cands);
+    dispatch_bits<2>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands);
   else
-    dispatch_bits<4>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, cands);
+    dispatch_bits<4>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands);
 }
 
 }  // namespace
@@ -392,7 +468,7 @@ void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t b
       unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
       dim3 grid(grid_x(1024, n), gy);
       launch_table<false>(bits, grid, table_smem(dim, bits), stream, codes, n, dim, q_unit + q0 * dim, nullptr,
-                          nullptr, inv_norm, keys + q0 * ld, ld);
+                           0, nullptr, inv_norm, keys + q0 * ld, ld);
       launched();
     }
     return;
@@ -403,7 +479,7 @@ void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t b
     dim3 grid(grid_x(kThreads / 32, n), gy);
     if (W)
       dispatch(bits, W, false, grid, stream, codes, n, dim, q_unit + q0 * dim, inv_norm, keys + q0 * ld, ld,
-               nullptr, nullptr);
+               nullptr, 0, nullptr);
     else
       asym_scan_generic<<<grid, kThreads, 0, stream>>>(codes, n, dim, bits, q_unit + q0 * dim, inv_norm,
                                                        keys + q0 * ld, ld);
@@ -418,13 +494,36 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
   // one arithmetic for every batch size, so a query scores the same alone and
   // inside a batch
   if (table_ok(dim, bits)) {
+    // few rows in all: four lanes a row (us, lane per row / four lanes, one query x 1,000
+    // rows: dim 1024 b=2 12.1 / 9.6, dim 768 b=2 13.9 / 8.3, dim 1024 b=1 7.7 / 6.0; 16
+    // x 1,000 at dim 1024 b=2 takes 11.9 a lane per row)
+    if (nq * max_row <= kTab4Rows) {
+      const dim3 grid((unsigned)((max_row + kTab4Threads / 4 - 1) / (kTab4Threads / 4)), (unsigned)nq);
+      const size_t smem = table_smem(dim, bits);
+#define OVB_TAB4(B)                                                                                             \
+  do {                                                                                                          \
+    allow_dynamic_smem(asym_table4_kernel<B>);                                                                  \
+    asym_table4_kernel<B><<<grid, kTab4Threads, smem, stream>>>(codes, dim, q_unit, offsets, max_row, cands,    \
+                                                                inv_norm, keys);                                \
+  } while (0)
+      if (bits == 1)
+        OVB_TAB4(1);
+      else if (bits == 2)
+        OVB_TAB4(2);
+      else
+        OVB_TAB4(4);
+#undef OVB_TAB4
+      launched();
+      return;
+    }
     // 512 rows per CTA (two per lane) with many queries, fewer with few
     const uint64_t rows_per_cta = nq >= 64 ? 512 : 128;
     for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
       unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
       dim3 grid(grid_x(rows_per_cta, max_row), gy);
       launch_table<true>(bits, grid, table_smem(dim, bits), stream, codes, 0, dim, q_unit + q0 * dim,
-                         offsets + q0, cands, inv_norm, keys, 0);
+                         offsets ? offsets + q0 : nullptr, max_row, cands + (offsets ? 0 : q0 * max_row), inv_norm,
+                         keys + (offsets ? 0 : q0 * max_row), 0);
       launched();
     }
     return;
@@ -436,12 +535,14 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
     dim3 grid(grid_x((kThreads / 32) * rows_per_warp, max_row), gy);
+    const uint64_t* off = offsets ? offsets + q0 : nullptr;
+    const uint32_t* c = cands + (offsets ? 0 : q0 * max_row);
+    uint32_t* k = keys + (offsets ? 0 : q0 * max_row);
     if (W)
-      dispatch(bits, W, true, grid, stream, codes, 0, dim, q_unit + q0 * dim, inv_norm, keys, 0, offsets + q0,
-               cands);
+      dispatch(bits, W, true, grid, stream, codes, 0, dim, q_unit + q0 * dim, inv_norm, k, 0, off, max_row, c);
     else
-      asym_subset_generic<<<grid, kThreads, 0, stream>>>(codes, dim, bits, q_unit + q0 * dim, offsets + q0,
-                                                         cands, inv_norm, keys);
+      asym_subset_generic<<<grid, kThreads, 0, stream>>>(codes, dim, bits, q_unit + q0 * dim, off, max_row, c,
+                                                         inv_norm, k);
     launched();
   }
 }
