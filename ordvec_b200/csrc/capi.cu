@@ -7,6 +7,7 @@
 // order by (score desc, row asc) and truncate, :959-981).  Exceptions never
 // cross the boundary: they become statuses the way ffi_boundary turns panics
 // into ORDVEC_STATUS_PANIC (:224-239).
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -193,26 +194,87 @@ void check_tc(Workspace& w) {
   }
 }
 
-// results of the last pipeline (w.out_keys / w.out_ids, count entries) -> host
-void download_results(Workspace& w, uint64_t count, int mode, uint32_t n_top, float* scores, int64_t* ids) {
+// Results of up to this many bytes are written by the device straight into pinned
+// host memory (with the tensor-core error word), so that a call ends in one
+// synchronisation and a memcpy; each copy into the caller's pageable memory
+// costs a staged transfer and a wait (a one-query call: three of them, ~25 us).
+constexpr uint64_t kPinnedResults = 128u << 10;
+
+// The sink of a host call with at most `max_count` results; clear it by download_results
+// or, when the pipeline throws, by the guard.
+struct HostSink {
+  Workspace& w;
+  bool pinned = false;
+  HostSink(Workspace& ws, uint64_t max_count, int mode, uint32_t n_top) : w(ws) {
+    w.sink = Workspace::Sink();
+    w.sink.mode = mode;
+    w.sink.n_top = n_top;
+    if (!max_count) return;
+    pinned = max_count <= kPinnedResults / 12;
+    if (pinned) {
+      uint8_t* p = (uint8_t*)w.results.ensure(kPinnedResults + 16);
+      *(volatile uint32_t*)p = 1;  // overwritten when the results are
+      w.sink.err_dst = (uint32_t*)p;
+      w.sink.ids = (int64_t*)(p + 16);
+      w.sink.scores = (float*)(p + 16 + max_count * 8);
+    } else {
+      w.sink.scores = (float*)w.scores.ensure(max_count * 4);
+      w.sink.ids = (int64_t*)w.ids.ensure(max_count * 8);
+    }
+  }
+  ~HostSink() { w.sink = Workspace::Sink(); }
+};
+
+// The sink of a device-pointer call: the final select writes the caller's buffers,
+// or finish() converts the keys.
+struct DeviceSink {
+  Workspace& w;
+  DeviceSink(Workspace& ws, float* scores, int64_t* ids, int mode, uint32_t n_top) : w(ws) {
+    w.sink = Workspace::Sink();
+    w.sink.scores = scores;
+    w.sink.ids = ids;
+    w.sink.mode = mode;
+    w.sink.n_top = n_top;
+  }
+  void finish(uint64_t count, cudaStream_t st) {
+    const Workspace::Sink& s = w.sink;
+    if (!s.used)
+      launch_keys_to_results(w.out_keys.as<uint32_t>(), w.out_ids.as<uint32_t>(), count, s.mode, s.n_top, s.scores,
+                             s.ids, st);
+  }
+  ~DeviceSink() { w.sink = Workspace::Sink(); }
+};
+
+[[noreturn]] void tc_timeout(Workspace& w) {
+  OVB_CUDA(cudaMemsetAsync(w.tc_err.p, 0, 4, w.stream));
+  OVB_CUDA(cudaStreamSynchronize(w.stream));
+  fail(ORDVEC_STATUS_INTERNAL, "tensor-core FastScan scan: a bounded wait timed out; results discarded");
+}
+
+// results of the last pipeline (in the sink, or keys in w.out_keys / w.out_ids; count entries) -> host
+void download_results(HostSink& out, uint64_t count, float* scores, int64_t* ids) {
   if (!count) return;
-  float* ds = (float*)w.scores.ensure(count * 4);
-  int64_t* di = (int64_t*)w.ids.ensure(count * 8);
-  launch_keys_to_results(w.out_keys.as<uint32_t>(), w.out_ids.as<uint32_t>(), count, mode, n_top, ds, di, w.stream);
-  OVB_CUDA(cudaMemcpyAsync(scores, ds, count * 4, cudaMemcpyDeviceToHost, w.stream));
-  OVB_CUDA(cudaMemcpyAsync(ids, di, count * 8, cudaMemcpyDeviceToHost, w.stream));
+  Workspace& w = out.w;
+  const Workspace::Sink s = w.sink;
+  if (!s.used)
+    launch_keys_to_results(w.out_keys.as<uint32_t>(), w.out_ids.as<uint32_t>(), count, s.mode, s.n_top, s.scores,
+                           s.ids, w.stream, w.tc_used ? w.tc_err.as<uint32_t>() : nullptr, s.err_dst);
+  if (out.pinned) {
+    OVB_CUDA(cudaStreamSynchronize(w.stream));
+    w.tc_used = false;
+    if (*(volatile uint32_t*)s.err_dst) tc_timeout(w);
+    memcpy(scores, s.scores, count * 4);
+    memcpy(ids, s.ids, count * 8);
+    return;
+  }
+  OVB_CUDA(cudaMemcpyAsync(scores, s.scores, count * 4, cudaMemcpyDeviceToHost, w.stream));
+  OVB_CUDA(cudaMemcpyAsync(ids, s.ids, count * 8, cudaMemcpyDeviceToHost, w.stream));
   // the tensor-core error word comes back with the results: one synchronisation
   uint32_t* h_err = w.tc_used ? (uint32_t*)w.pinned.ensure(4) : nullptr;
   if (h_err) OVB_CUDA(cudaMemcpyAsync(h_err, w.tc_err.p, 4, cudaMemcpyDeviceToHost, w.stream));
   OVB_CUDA(cudaStreamSynchronize(w.stream));
-  if (h_err) {
-    w.tc_used = false;
-    if (*h_err) {
-      OVB_CUDA(cudaMemsetAsync(w.tc_err.p, 0, 4, w.stream));
-      OVB_CUDA(cudaStreamSynchronize(w.stream));
-      fail(ORDVEC_STATUS_INTERNAL, "tensor-core FastScan scan: a bounded wait timed out; results discarded");
-    }
-  }
+  w.tc_used = false;
+  if (h_err && *h_err) tc_timeout(w);
 }
 
 void need_queries(const float* q, uint64_t nq) {
@@ -428,6 +490,7 @@ ordvec_status_t ordvec_index_search(const ordvec_index_t* index, const ordvec_se
       Workspace& w = workspace();
       const float* d_q = upload_queries(w, p.query, 1, ix.dim, false);
       uint32_t ke = 0;
+      HostSink out(w, required, ix.kind == ORDVEC_INDEX_KIND_RANK_QUANT ? 0 : 1, ix.n_top);
       if (!rows) {
         ke = ix.kind == ORDVEC_INDEX_KIND_RANK_QUANT ? engine_rankquant_full(ix, d_q, 1, required, w, w.stream)
                                                      : engine_bitmap_full(ix, d_q, 1, required, w, w.stream);
@@ -443,7 +506,7 @@ ordvec_status_t ordvec_index_search(const ordvec_index_t* index, const ordvec_se
       }
       std::vector<float> sc(ke);
       std::vector<int64_t> id(ke);
-      download_results(w, ke, ix.kind == ORDVEC_INDEX_KIND_RANK_QUANT ? 0 : 1, ix.n_top, sc.data(), id.data());
+      download_results(out, ke, sc.data(), id.data());
       for (uint32_t s = 0; s < ke; s++) {
         if (id[s] < 0) break;
         hits_out[s].row_id = (uint64_t)id[s];
@@ -657,8 +720,9 @@ ordvec_status_t ovb_rankquant_search(const ordvec_index_t* rq, const float* quer
     if (!scores || !ids) fail(ORDVEC_STATUS_NULL_POINTER, "output pointer is NULL");
     Workspace& w = workspace();
     const float* d_q = upload_queries(w, queries, nq, ix.dim, true);
+    HostSink out(w, nq * ke, 0, 0);
     uint32_t got = engine_rankquant_full(ix, d_q, nq, ke, w, w.stream);
-    download_results(w, nq * got, 0, 0, scores, ids);
+    download_results(out, nq * got, scores, ids);
   });
 }
 
@@ -672,8 +736,9 @@ ordvec_status_t ovb_rankquant_search_split(const ordvec_index_t* rq, const float
     if (!scores || !ids) fail(ORDVEC_STATUS_NULL_POINTER, "output pointer is NULL");
     Workspace& w = workspace();
     const float* d_q = upload_queries(w, queries, nq, ix.dim, true);
+    HostSink out(w, nq * ke, 0, 0);
     uint32_t got = engine_rankquant_full_split(ix, d_q, nq, ke, exact != 0, w, w.stream);
-    download_results(w, nq * got, 0, 0, scores, ids);
+    download_results(out, nq * got, scores, ids);
   });
 }
 
@@ -710,8 +775,9 @@ ordvec_status_t ovb_rankquant_search_subset(const ordvec_index_t* rq, const floa
     uint32_t* d_c = (uint32_t*)w.sel_ids.ensure((total ? total : 1) * 4);
     OVB_CUDA(cudaMemcpyAsync(d_off, offsets, (nq + 1) * 8, cudaMemcpyHostToDevice, w.stream));
     if (total) OVB_CUDA(cudaMemcpyAsync(d_c, candidates, total * 4, cudaMemcpyHostToDevice, w.stream));
+    HostSink out(w, nq * ke, 0, 0);
     uint32_t got = engine_rankquant_subset(ix, d_q, nq, d_off, d_c, max_row, ke, w, w.stream);
-    download_results(w, nq * got, 0, 0, scores, ids);
+    download_results(out, nq * got, scores, ids);
   });
 }
 
@@ -777,8 +843,9 @@ ordvec_status_t ovb_bitmap_search(const ordvec_index_t* bm, const float* queries
     if (!scores || !ids) fail(ORDVEC_STATUS_NULL_POINTER, "output pointer is NULL");
     Workspace& w = workspace();
     const float* d_q = upload_queries(w, queries, nq, ix.dim, true);
+    HostSink out(w, nq * ke, 1, ix.n_top);
     uint32_t got = engine_bitmap_full(ix, d_q, nq, ke, w, w.stream);
-    download_results(w, nq * got, 1, ix.n_top, scores, ids);
+    download_results(out, nq * got, scores, ids);
   });
 }
 
@@ -801,8 +868,9 @@ ordvec_status_t ovb_fastscan_search(const ordvec_index_t* fs, const float* queri
     if (!scores || !ids) fail(ORDVEC_STATUS_NULL_POINTER, "output pointer is NULL");
     Workspace& w = workspace();
     const float* d_q = upload_queries(w, queries, nq, ix.dim, true);
+    HostSink out(w, nq * ke, 0, 0);
     uint32_t got = engine_fastscan_full(ix, d_q, nq, ke, w, w.stream);
-    download_results(w, nq * got, 0, 0, scores, ids);
+    download_results(out, nq * got, scores, ids);
   });
 }
 
@@ -819,9 +887,10 @@ static void rank_query_search(const ordvec_index_t* h, uint32_t kind, const char
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "device rank search supports dim <= 16384");
   Workspace& w = workspace();
   const float* d_q = upload_queries(w, queries, nq, ix.dim, true);
+  HostSink out(w, nq * ke, 0, 0);
   uint32_t got = variant == 2 ? engine_rankquant_symmetric(ix, d_q, nq, ke, w, w.stream)
                               : engine_rank_full(ix, d_q, nq, ke, variant == 1, w, w.stream);
-  download_results(w, nq * got, 0, 0, scores, ids);
+  download_results(out, nq * got, scores, ids);
 }
 
 ordvec_status_t ovb_rank_search(const ordvec_index_t* rank, const float* queries, uint64_t nq, uint64_t k,
@@ -863,8 +932,10 @@ ordvec_status_t ovb_two_stage_search(const ordvec_index_t* rq, const ordvec_inde
     if (!scores || !ids) fail(ORDVEC_STATUS_NULL_POINTER, "output pointer is NULL");
     Workspace& w = workspace();
     const float* d_q = upload_queries(w, queries, nq, r.dim, true);
+    const uint64_t me = std::min<uint64_t>(m ? m : default_candidate_count(k, r.n), r.n);
+    HostSink out(w, nq * std::min<uint64_t>(k, me), 0, 0);
     uint32_t got = engine_two_stage(r, s, d_q, nq, m, k, w, w.stream);
-    download_results(w, nq * got, 0, 0, scores, ids);
+    download_results(out, nq * got, scores, ids);
   });
 }
 
@@ -879,8 +950,9 @@ ordvec_status_t ovb_two_stage_search_device(const ordvec_index_t* rq, const ordv
     if (!d_scores || !d_ids) fail(ORDVEC_STATUS_NULL_POINTER, "output pointer is NULL");
     Workspace& w = workspace();
     cudaStream_t st = (cudaStream_t)stream;
+    DeviceSink out(w, d_scores, d_ids, 0, 0);
     uint32_t got = engine_two_stage(r, s, d_queries, nq, m, k, w, st);
-    launch_keys_to_results(w.out_keys.as<uint32_t>(), w.out_ids.as<uint32_t>(), nq * got, 0, 0, d_scores, d_ids, st);
+    out.finish(nq * got, st);
   });
 }
 
@@ -901,8 +973,9 @@ ordvec_status_t ovb_two_stage_search_device_ex(const ordvec_index_t* rq, const o
       Mode(Workspace& ws, uint32_t m_) : w(ws) { w.rerank_mode = m_; }
       ~Mode() { w.rerank_mode = OVB_RERANK_AUTO; }
     } guard(w, rerank_mode);
+    DeviceSink out(w, d_scores, d_ids, 0, 0);
     uint32_t got = engine_two_stage(r, s, d_queries, nq, m, k, w, st);
-    launch_keys_to_results(w.out_keys.as<uint32_t>(), w.out_ids.as<uint32_t>(), nq * got, 0, 0, d_scores, d_ids, st);
+    out.finish(nq * got, st);
   });
 }
 
@@ -950,7 +1023,7 @@ ordvec_status_t ovb_index_search_device(const ordvec_index_t* index, uint32_t me
     Workspace& w = workspace();
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t got = 0;
-    int mode = 0;
+    DeviceSink out(w, d_scores, d_ids, ix.kind == ORDVEC_INDEX_KIND_BITMAP ? 1 : 0, ix.n_top);
     switch (ix.kind) {
       case ORDVEC_INDEX_KIND_RANK_QUANT:
         got = asym ? engine_rankquant_full(ix, d_queries, nq, ke, w, st)
@@ -961,13 +1034,11 @@ ordvec_status_t ovb_index_search_device(const ordvec_index_t* index, uint32_t me
         break;
       case ORDVEC_INDEX_KIND_BITMAP:
         got = engine_bitmap_full(ix, d_queries, nq, ke, w, st);
-        mode = 1;
         break;
       default:
         got = engine_fastscan_full(ix, d_queries, nq, ke, w, st);
     }
-    launch_keys_to_results(w.out_keys.as<uint32_t>(), w.out_ids.as<uint32_t>(), nq * got, mode, ix.n_top, d_scores,
-                           d_ids, st);
+    out.finish(nq * got, st);
   });
 }
 

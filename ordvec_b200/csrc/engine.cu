@@ -36,11 +36,24 @@ float inv_rankquant_norm(uint32_t dim, uint32_t bits) { return 1.0f / rankquant_
 void select_rows(Workspace& w, const uint32_t* keys, const uint32_t* ids, const uint64_t* row_off,
                  uint64_t ld, uint64_t n, uint64_t rows, uint32_t k, uint32_t key_bits,
                  uint32_t id_bits, uint32_t* out_keys, uint32_t* out_ids, cudaStream_t st,
-                 const uint32_t* row_len = nullptr, bool ordered = true) {
+                 const uint32_t* row_len = nullptr, bool ordered = true, bool final = false) {
   SelectArgs a{keys, ids, row_off, ld, n, k, key_bits, id_bits, out_keys, out_ids, row_len, ordered ? 0u : 1u};
+  if (final && w.sink.scores) {  // the rows' place in the results is their place in w.out_keys
+    const uint64_t at = out_keys - w.out_keys.as<uint32_t>();
+    a.res_scores = w.sink.scores + at;
+    a.res_ids = w.sink.ids + at;
+    a.res_mode = w.sink.mode;
+    a.res_n_top = w.sink.n_top;
+    a.err_src = w.tc_used ? w.tc_err.as<uint32_t>() : nullptr;
+    a.err_dst = w.sink.err_dst;
+    w.sink.used = true;
+  }
   size_t se = select_rows_scratch_elems(rows, k, row_off ? 0 : n);
   uint64_t* scratch = se ? (uint64_t*)w.scratch.ensure(se * 8) : nullptr;
-  if (select_takes_grid(a, rows, scratch)) a.err = w.tc_err_word(st);
+  if (select_takes_grid(a, rows, scratch)) {
+    a.err = w.tc_err_word(st);
+    if (a.res_scores) a.err_src = a.err;
+  }
   launch_select_rows(a, rows, scratch, st);
 }
 
@@ -48,6 +61,8 @@ void select_rows(Workspace& w, const uint32_t* keys, const uint32_t* ids, const 
 template <class F>
 void full_scan_select(Workspace& w, uint64_t nq, uint64_t n, uint32_t k, uint32_t key_bits,
                       uint32_t* out_keys, uint32_t* out_ids, cudaStream_t st, F&& scan) {
+  const bool final = out_keys >= w.out_keys.as<uint32_t>() &&
+                     out_keys < (uint32_t*)((char*)w.out_keys.p + w.out_keys.cap);  // else stage-1 candidates
   const uint64_t per_q = n * 4;
   uint64_t qc = keys_budget() / per_q;
   if (qc < 1) qc = 1;
@@ -59,7 +74,7 @@ void full_scan_select(Workspace& w, uint64_t nq, uint64_t n, uint32_t k, uint32_
     scan(q0, qn, keys);
     w.mark(st, 2);
     select_rows(w, keys, nullptr, nullptr, n, n, qn, k, key_bits, id_bits, out_keys + q0 * k,
-                out_ids + q0 * k, st, nullptr, !w.cand_unordered);
+                out_ids + q0 * k, st, nullptr, !w.cand_unordered, final);
     w.mark(st, 3);
   }
 }
@@ -393,7 +408,7 @@ static void filtered_candidates(const Scores& sc, uint64_t n, uint64_t qn, uint3
   uint32_t* k2 = (uint32_t*)w.keys2.ensure(qn * kp * 4);
   rescore(ci, k2);
   w.mark(st, 4);
-  select_rows(w, k2, ci, nullptr, kp, kp, qn, ke, 32, id_bits, out_keys, out_ids, st);
+  select_rows(w, k2, ci, nullptr, kp, kp, qn, ke, 32, id_bits, out_keys, out_ids, st, nullptr, true, true);
   w.mark(st, 5);
 }
 
@@ -461,7 +476,8 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, b
     sc.scan(qn, 1, keys, n, w.tc_err_word(st), st);
     w.mark(st, 2);
     if (!exact) {
-      select_rows(w, keys, nullptr, nullptr, n, n, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st);
+      select_rows(w, keys, nullptr, nullptr, n, n, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st, nullptr, true,
+                  true);
       w.mark(st, 3);
       continue;
     }
@@ -486,7 +502,7 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, b
     uint32_t* k2 = (uint32_t*)w.keys2.ensure(qn * kp * 4);
     const uint32_t* ti = w.thr_ids.as<uint32_t>();
     rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp, ti, k2, st);
-    select_rows(w, k2, ti, nullptr, kp, kp, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st);
+    select_rows(w, k2, ti, nullptr, kp, kp, qn, ke, 32, id_bits, ok + q0 * ke, oi + q0 * ke, st, nullptr, true, true);
     w.mark(st, 3);
   }
   return ke;
@@ -545,7 +561,7 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   if (kp < n) sc.margin(tk, nq, (uint32_t)kp, ke, d_flag, st);
   uint32_t* k2 = (uint32_t*)w.keys2.ensure(nq * kp * 4);
   rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ti, k2, st);
-  select_rows(w, k2, ti, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st);
+  select_rows(w, k2, ti, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true);
   return ke;
 }
 
@@ -704,7 +720,7 @@ uint32_t engine_rankquant_subset(const Index& rq, const float* d_q, uint64_t nq,
                      keys, st);
   uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
   uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
-  select_rows(w, keys, d_cands, d_off, 0, 0, nq, ke, 32, bits_for(rq.n - 1), ok, oi, st);
+  select_rows(w, keys, d_cands, d_off, 0, 0, nq, ke, 32, bits_for(rq.n - 1), ok, oi, st, nullptr, true, true);
   return ke;
 }
 
@@ -879,7 +895,7 @@ static bool split_rerank(const Index& rq, const float* qu, uint64_t nq, uint32_t
   uint32_t* ok = w.out_keys.as<uint32_t>();
   uint32_t* oi = w.out_ids.as<uint32_t>();
   if (raw) {
-    select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st);
+    select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true);
     w.mark(st, 5);
     return true;
   }
@@ -893,7 +909,7 @@ static bool split_rerank(const Index& rq, const float* qu, uint64_t nq, uint32_t
   launch_split_margin(ck, nq, kp, ke, l1, split_error_bound(dim, bits, inv_norm), flag, st);
   uint32_t* k2 = (uint32_t*)w.rr_keys2.ensure(nq * kp * 4);
   launch_asym_subset(codes, dim, bits, qu, nq, nullptr, ci, kp, inv_norm, k2, st);
-  select_rows(w, k2, ci, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st);
+  select_rows(w, k2, ci, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true);
   w.mark(st, 5);
   OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
   OVB_CUDA(cudaStreamSynchronize(st));
@@ -934,7 +950,7 @@ uint32_t engine_two_stage(const Index& rq, const Index& s1, const float* d_q, ui
   launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, nq, nullptr, cand, me, inv_norm, keys, st);
   w.mark(st, 4);
   // rows are uniform (me candidates each): the strided form, not offsets
-  select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st);
+  select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true);
   w.mark(st, 5);
   return ke;
 }

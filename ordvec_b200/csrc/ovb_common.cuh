@@ -89,6 +89,11 @@ __host__ __device__ __forceinline__ float desc_key_to_float(uint32_t k) {
 #endif
 }
 
+// The score of a key: a float score (mode 0) or a bitmap overlap (mode 1).
+__device__ __forceinline__ float key_score(uint32_t key, int mode, uint32_t n_top) {
+  return mode == 0 ? desc_key_to_float(key) : (float)(n_top - key);
+}
+
 constexpr uint32_t kSentinelKey = 0xFFFFFFFFu;
 constexpr uint32_t kSentinelId = 0xFFFFFFFFu;
 

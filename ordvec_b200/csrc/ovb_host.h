@@ -117,6 +117,18 @@ struct Workspace {
   uint64_t split_kp = 0;  // largest candidate count the last exact split search settled on
   bool cand_unordered = false;  // set while a two-stage search selects its stage-1 set
   HostBuf pinned, f_flag_host;
+  // Where the calling entry point wants its results: set before the pipeline runs,
+  // it lets the final select write scores and ids (and the error word's copy)
+  // itself; `used` says it did.  scores null: keys in out_keys / out_ids only.
+  struct Sink {
+    float* scores = nullptr;
+    int64_t* ids = nullptr;
+    uint32_t* err_dst = nullptr;
+    int mode = 0;
+    uint32_t n_top = 0;
+    bool used = false;
+  } sink;
+  HostBuf results;  // small results: device-written pinned memory
   // error word of the tensor-core kernels (zeroed once; checked by host APIs)
   DevBuf tc_err;
   bool tc_used = false;

@@ -25,6 +25,14 @@ struct SelectArgs {
   const uint32_t* row_len;  // optional: row r holds min(row_len[r], n) entries at r*ld
   uint32_t unordered;       // 1: a row's k_eff winners in any order (the set only)
   uint32_t* err;            // whole-GPU form: |= 1 when a barrier wait gave up (may be null)
+  // final results instead of keys (per-row forms; else they follow by
+  // launch_keys_to_results): row r at r * k
+  float* res_scores;
+  int64_t* res_ids;
+  int res_mode;
+  uint32_t res_n_top;
+  const uint32_t* err_src;  // copied to *err_dst once the results are written (either may be null)
+  uint32_t* err_dst;
 };
 // u64 scratch elements launch_select_rows may use for `rows` rows of length n
 // (0 for ragged rows): global sort buffers for k > kSelectSmemCap, and the
@@ -232,8 +240,9 @@ void launch_prefix_compact(const uint32_t* src, uint64_t ld, const uint64_t* off
                            cudaStream_t stream);
 // ids[i] >= n (sentinels of underfull select rows) -> 0, so a gather stays in bounds
 void launch_clamp_ids(uint32_t* ids, uint64_t count, uint32_t n, cudaStream_t stream);
+// (with err_dst, *err_dst = err_src ? *err_src : 0)
 void launch_keys_to_results(const uint32_t* keys, const uint32_t* ids, uint64_t count,
                             int mode, uint32_t n_top, float* scores, int64_t* out_ids,
-                            cudaStream_t stream);
+                            cudaStream_t stream, const uint32_t* err_src = nullptr, uint32_t* err_dst = nullptr);
 
 }  // namespace ovb

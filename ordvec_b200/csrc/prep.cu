@@ -40,7 +40,7 @@ __device__ __forceinline__ float ordered_sum(float s, const float* v, uint32_t n
 
 // One warp per query.  The warp squares the query into shared memory in
 // 1024-element chunks; lane 0 then adds the squares in index order (the
-// reference's sequential f32 sum).  One query of dim 1,024: 7.4 -> 5.0 us with the
+// reference's sequential f32 sum).  One query of dim 1,024: 7.4 -> 6.4 us with the
 // values loaded 32 ahead (four before).
 __global__ void l2_normalise_kernel(const float* __restrict__ q, uint64_t nq, uint32_t dim,
                                     float* __restrict__ out) {
@@ -132,17 +132,14 @@ __global__ void finite_flag_kernel(const float* __restrict__ x, uint64_t count,
 __global__ void keys_to_results_kernel(const uint32_t* __restrict__ keys,
                                        const uint32_t* __restrict__ ids, uint64_t count,
                                        int mode, uint32_t n_top, float* __restrict__ scores,
-                                       int64_t* __restrict__ out_ids) {
+                                       int64_t* __restrict__ out_ids, const uint32_t* err_src, uint32_t* err_dst) {
   uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0 && err_dst) *err_dst = err_src ? *err_src : 0u;
   if (t >= count) return;
-  uint32_t k = keys[t], id = ids[t];
-  if (id == kSentinelId) {
-    scores[t] = __int_as_float(0xff800000);
-    out_ids[t] = -1;
-    return;
-  }
-  scores[t] = mode == 0 ? desc_key_to_float(k) : (float)(n_top - k);
-  out_ids[t] = (int64_t)id;
+  const uint32_t id = ids[t];
+  const bool none = id == kSentinelId;
+  scores[t] = none ? __int_as_float(0xff800000) : key_score(keys[t], mode, n_top);
+  out_ids[t] = none ? -1 : (int64_t)id;
 }
 
 }  // namespace
@@ -211,9 +208,10 @@ void launch_prefix_compact(const uint32_t* src, uint64_t ld, const uint64_t* off
 
 void launch_keys_to_results(const uint32_t* keys, const uint32_t* ids, uint64_t count,
                             int mode, uint32_t n_top, float* scores, int64_t* out_ids,
-                            cudaStream_t stream) {
+                            cudaStream_t stream, const uint32_t* err_src, uint32_t* err_dst) {
   if (!count) return;
-  keys_to_results_kernel<<<ceil_div(count, 256), 256, 0, stream>>>(keys, ids, count, mode, n_top, scores, out_ids);
+  keys_to_results_kernel<<<ceil_div(count, 256), 256, 0, stream>>>(keys, ids, count, mode, n_top, scores, out_ids,
+                                                                   err_src, err_dst);
   launched();
 }
 

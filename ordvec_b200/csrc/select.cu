@@ -84,10 +84,20 @@ __global__ void __launch_bounds__(T)
   uint32_t* out_k = a.out_keys + row * (uint64_t)a.k;
   uint32_t* out_i = a.out_ids + row * (uint64_t)a.k;
 
-  for (uint32_t j = k_eff + threadIdx.x; j < a.k; j += blockDim.x) {
-    out_k[j] = kSentinelKey;
-    out_i[j] = kSentinelId;
-  }
+  // entry j of the row, as key and id or as the final result
+  auto put = [&](uint32_t j, uint32_t key, uint32_t id) {
+    if (a.res_scores) {
+      const uint64_t at = row * (uint64_t)a.k + j;
+      const bool none = id == kSentinelId;
+      a.res_scores[at] = none ? __int_as_float(0xff800000) : key_score(key, a.res_mode, a.res_n_top);
+      a.res_ids[at] = none ? -1 : (int64_t)id;
+    } else {
+      out_k[j] = key;
+      out_i[j] = id;
+    }
+  };
+  if (a.err_dst && row == 0 && threadIdx.x == 0) *a.err_dst = a.err_src ? *a.err_src : 0u;
+  for (uint32_t j = k_eff + threadIdx.x; j < a.k; j += blockDim.x) put(j, kSentinelKey, kSentinelId);
   if (k_eff == 0) return;
 
   uint64_t* buf = (k_eff <= CAP) ? sbuf : gbuf + row * (uint64_t)gbuf_stride;
@@ -196,8 +206,7 @@ __global__ void __launch_bounds__(T)
   }
   for (uint32_t j = threadIdx.x; j < k_eff; j += blockDim.x) {
     uint64_t key = buf[j];
-    out_k[j] = (uint32_t)(key >> 32);
-    out_i[j] = (uint32_t)key;
+    put(j, (uint32_t)(key >> 32), (uint32_t)key);
   }
 }
 
@@ -757,8 +766,14 @@ bool select_takes_grid(const SelectArgs& a, uint64_t rows, const uint64_t* scrat
 void launch_select_rows(const SelectArgs& a, uint64_t rows, uint64_t* scratch,
                         cudaStream_t stream) {
   if (rows == 0) return;
+  auto results = [&] {  // for the forms that leave keys
+    if (a.res_scores)
+      launch_keys_to_results(a.out_keys, a.out_ids, rows * a.k, a.res_mode, a.res_n_top, a.res_scores, a.res_ids,
+                             stream, a.err_src, a.err_dst);
+  };
   if (select_takes_grid(a, rows, scratch)) {
     launch_select_grid(a, rows, scratch, stream);
+    results();
     return;
   }
   // few long rows: one 8-CTA cluster per row (below two rows per SM the
@@ -772,6 +787,7 @@ void launch_select_rows(const SelectArgs& a, uint64_t rows, uint64_t* scratch,
     if (smem) allow_dynamic_smem(select_rows_cluster_kernel);  // static 32 KiB + the stage
     select_rows_cluster_kernel<<<(unsigned)(rows * kClusterCtas), kSelThreads, smem, stream>>>(a, stage);
     launched();
+    results();
     return;
   }
   // short uniform rows: 256 threads per row, several rows per SM

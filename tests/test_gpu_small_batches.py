@@ -56,3 +56,23 @@ def test_fastscan_tables_of_unusual_queries(orc, dim):
     ws, wi = orc.fastscan_search(orc.fastscan_pack(docs, dim), n, dim, qs, 50)
     assert np.array_equal(got.indices.reshape(5, -1), wi)
     assert np.array_equal(got.scores.reshape(5, -1).view(np.uint32), np.asarray(ws, np.float32).reshape(5, -1).view(np.uint32))
+
+
+def test_results_around_the_pinned_limit(orc):
+    """10,922 results are the most that come back in pinned memory: one more and one
+    less give the same prefix, and the oracle's order."""
+    n, dim = 11_000, 64
+    docs = ob.synth_docs(3, n, dim)
+    q, _ = ob.synth_queries(3, n, 1, dim)
+    rq = ob.RankQuant(dim, 2)
+    rq.add(docs)
+    bm = ob.Bitmap(dim, 16)
+    bm.add(docs)
+    words = orc.bitmap_encode(docs, dim, 16)
+    for ix in (rq, bm):
+        search = rq.search_asymmetric if ix is rq else bm.search
+        a, b = search(q, 10_922), search(q, 10_923)
+        assert np.array_equal(a.indices, b.indices[:10_922])
+        assert np.array_equal(a.scores.view(np.uint32), b.scores[:10_922].view(np.uint32))
+    ws, wi = orc.bitmap_search(words, n, dim, 16, q, 10_922)
+    assert np.array_equal(bm.search(q, 10_922).indices, np.asarray(wi).reshape(-1))
