@@ -36,8 +36,10 @@ float inv_rankquant_norm(uint32_t dim, uint32_t bits) { return 1.0f / rankquant_
 void select_rows(Workspace& w, const uint32_t* keys, const uint32_t* ids, const uint64_t* row_off,
                  uint64_t ld, uint64_t n, uint64_t rows, uint32_t k, uint32_t key_bits,
                  uint32_t id_bits, uint32_t* out_keys, uint32_t* out_ids, cudaStream_t st,
-                 const uint32_t* row_len = nullptr, bool ordered = true, bool final = false) {
+                 const uint32_t* row_len = nullptr, bool ordered = true, bool final = false,
+                 const uint32_t* gate = nullptr) {
   SelectArgs a{keys, ids, row_off, ld, n, k, key_bits, id_bits, out_keys, out_ids, row_len, ordered ? 0u : 1u};
+  a.gate = gate;
   if (final && w.sink.scores) {  // the rows' place in the results is their place in w.out_keys
     const uint64_t at = out_keys - w.out_keys.as<uint32_t>();
     a.res_scores = w.sink.scores + at;
@@ -57,10 +59,12 @@ void select_rows(Workspace& w, const uint32_t* keys, const uint32_t* ids, const 
   launch_select_rows(a, rows, scratch, st);
 }
 
-// scan(q0, qn, keys) writes keys[qn][n]; rows are selected into out[nq][k].
+// scan(q0, qn, keys) writes keys[qn][n]; rows are selected into out[nq][k].  gate (may
+// be null; scan's launches take the same): nothing happens when *gate is 0.
 template <class F>
 void full_scan_select(Workspace& w, uint64_t nq, uint64_t n, uint32_t k, uint32_t key_bits,
-                      uint32_t* out_keys, uint32_t* out_ids, cudaStream_t st, F&& scan) {
+                      uint32_t* out_keys, uint32_t* out_ids, cudaStream_t st, F&& scan,
+                      const uint32_t* gate = nullptr) {
   const bool final = out_keys >= w.out_keys.as<uint32_t>() &&
                      out_keys < (uint32_t*)((char*)w.out_keys.p + w.out_keys.cap);  // else stage-1 candidates
   const uint64_t per_q = n * 4;
@@ -72,10 +76,10 @@ void full_scan_select(Workspace& w, uint64_t nq, uint64_t n, uint32_t k, uint32_
   for (uint64_t q0 = 0; q0 < nq; q0 += qc) {
     const uint64_t qn = nq - q0 < qc ? nq - q0 : qc;
     scan(q0, qn, keys);
-    w.mark(st, 2);
+    if (!gate) w.mark(st, 2);
     select_rows(w, keys, nullptr, nullptr, n, n, qn, k, key_bits, id_bits, out_keys + q0 * k,
-                out_ids + q0 * k, st, nullptr, !w.cand_unordered, final);
-    w.mark(st, 3);
+                out_ids + q0 * k, st, nullptr, !w.cand_unordered, final, gate);
+    if (!gate) w.mark(st, 3);
   }
 }
 
@@ -286,25 +290,15 @@ uint64_t default_candidate_count(uint64_t k, uint64_t space) {
   return c < space ? c : space;
 }
 
-// Batched full scans use the tensor-core candidate scan (with the exact FP64
-// rescoring below) from 64 queries on eligible shapes, and smaller batches where
-// the sampled filter runs and the FP64 table scan's work, nq n dim bits, is
-// above 1e9 + 800 n.  Measured with both forms (us, tables / tensor cores): n = 1M
-// dim 768 b=1: 236 / 263 at 2 queries, 285 / 262 at 3; b=2: 271 / 272 at 1, 413 /
-// 274 at 2, 4,673 / 301 at 32; n = 200k dim 1024 b=1: 140 / 149 at 4, 175 / 144 at 6;
-// n = 40k dim 384 b=2: 82 / 113 at 16, 132 / 114 at 32.  A capturing stream keeps
-// the table scan below 64 queries (the candidate form reads a flag on the host).
+// Batches of at least 64 queries use the tensor-core candidate scan (with the exact
+// FP64 rescoring below) on eligible shapes; smaller ones choose by small_form.
 // OVB_RANK_TC=0/1 forces.
-bool use_rank_tc(const Index& rq, uint64_t nq, uint64_t k, cudaStream_t st) {
+bool use_rank_tc(const Index& rq, uint64_t nq) {
   const char* e = getenv("OVB_RANK_TC");
   if (!rank_tc_eligible(rq.dim, rq.bits)) return false;
   if (e && e[0] == '0') return false;
   if (e && e[0] == '1') return true;
-  if (nq >= 64) return rq.n >= 4096;
-  const uint64_t n = rq.n, ke = k < n ? k : n, kp = std::min<uint64_t>(std::max<uint64_t>(2 * ke, ke + 64), n);
-  FilterPlan fp;
-  return nq * n * rq.dim * rq.bits >= 1000000000ull + 800 * n && score_rankquant_eligible(rq.dim, rq.bits) &&
-         kp <= kSelectSmemCap && filter_plan(n, (uint32_t)kp, fp) && !capturing(st);
+  return nq >= 64 && rq.n >= 4096;
 }
 
 // Split-BF16 filter for rows of kp candidates: the sample-threshold plan with
@@ -416,6 +410,19 @@ static void filtered_candidates(const Scores& sc, uint64_t n, uint64_t qn, uint3
 static void rescore_rankquant(const Index& rq, const float* qu, float inv_norm, uint64_t qn, uint32_t kp,
                               const uint32_t* ids, uint32_t* keys, cudaStream_t st) {
   launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, qn, nullptr, ids, kp, inv_norm, keys, st);
+}
+
+// The end of a candidate pipeline outside the filtered form: margin test of the kp
+// candidates ck / ci of each query (*d_flag |= 1: the result is not known to be exact),
+// FP64 rescoring, top-ke into w.out_keys / out_ids.
+static void rescored_top_k(const CandScores& sc, const Index& rq, const float* qu, float inv_norm, uint64_t nq,
+                           uint32_t kp, uint32_t ke, const uint32_t* ck, const uint32_t* ci, uint32_t* d_flag,
+                           Workspace& w, cudaStream_t st) {
+  sc.margin(ck, nq, kp, ke, d_flag, st);
+  uint32_t* k2 = (uint32_t*)w.rr_keys2.ensure(nq * kp * 4);
+  rescore_rankquant(rq, qu, inv_norm, nq, kp, ci, k2, st);
+  select_rows(w, k2, ci, nullptr, kp, kp, nq, ke, 32, bits_for(rq.n - 1), w.out_keys.as<uint32_t>(),
+              w.out_ids.as<uint32_t>(), st, nullptr, true, true);
 }
 
 // Tensor-core search of prepared query rows qu (nq x dim f32) scored as
@@ -565,20 +572,88 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   return ke;
 }
 
+// How an exact search of fewer than 64 queries scores the documents.  W = nq n dim bits is
+// what the FP64 table scan's time goes with.
+//   kRows: integer scores on the CUDA cores into the key matrix, the best kp rescored, from
+//     W = 8e8 on: below, the select of the kp, the margin test and the rescoring cost
+//     more than the scan saves.
+//   kFilter: integer scores on the tensor cores behind the sampled filter, for more than
+//     four queries (kRows takes a pass over the rows for each four) where W is above
+//     1e9 + 800 n.
+// Measured (us, tables / rows / filter): n = 1M dim 768 b=1: 98 / 117 / 230 at one query
+// (7.7e8), 156 / 145 / 231 at 2, 264 / 199 / 233 at 4, 319 / 307 / 235 at 5; b=2: 189 /
+// 129 / 251 at 1, 608 / 216 / 250 at 4, 745 / 334 / 256 at 5, 6,913 / 1,920 / 271 at 48; n =
+// 200k dim 1024 b=1: 91 / 109 / 129 at 3 (6.1e8), 154 / 141 / 136 at 6; b=2: 86 / 90 / 129
+// at 1 (4.1e8), 113 / 99 / 129 at 2 (8.2e8), 266 / 147 / 140 at 6; n = 40k dim 384 b=2: 112
+// / 107 / 103 at 24 (7.4e8), b=4: 89 / 79 / 98 at 8 (4.9e8), 181 / 110 / 106 at 24; n = 10k
+// dim 256: 40 / 80 / 80.
+// A capturing stream keeps the tables, whose buffers every search of the size has.
+// OVB_ROW_SCORES=0/1 forces kRows, here and for candidate rows; OVB_RANK_TC=0 leaves
+// kFilter out.
+enum class SmallForm { kTables, kRows, kFilter };
+static SmallForm small_form(const Index& rq, uint64_t nq, uint64_t kp, cudaStream_t st, FilterPlan& fp) {
+  const char* rows_env = getenv("OVB_ROW_SCORES");
+  const char* tc_env = getenv("OVB_RANK_TC");
+  const uint64_t n = rq.n, work = nq * n * rq.dim * rq.bits;
+  if (nq >= 64 || kp > kSelectSmemCap || !score_rankquant_eligible(rq.dim, rq.bits) || capturing(st))
+    return SmallForm::kTables;
+  const bool rows = score_rows_eligible(rq.dim, rq.bits) && kp * 4 <= n && nq * n * 4 <= keys_budget() &&
+                    !(rows_env && rows_env[0] == '0');
+  if (rows && rows_env && rows_env[0] == '1') return SmallForm::kRows;
+  if ((nq > 4 || !rows) && work >= 1000000000ull + 800 * n && !(tc_env && tc_env[0] == '0') &&
+      rank_tc_eligible(rq.dim, rq.bits) && split_filter_plan(n, kp, fp))
+    return SmallForm::kFilter;
+  return rows && work >= 800000000ull ? SmallForm::kRows : SmallForm::kTables;
+}
+
+// Exact search of prepared query rows qu (as in split_search).  The candidate forms are
+// followed by the FP64 table scan of every document behind their flag: it does nothing
+// unless the margin test failed for some query, so no form waits on the host.
+static void exact_search(const Index& rq, const float* qu, float inv_norm, bool half_steps, uint64_t nq, uint32_t ke,
+                         Workspace& w, cudaStream_t st) {
+  const uint64_t n = rq.n, kp64 = std::max<uint64_t>(2ull * ke, ke + 64ull);
+  const uint32_t kp = (uint32_t)kp64;
+  uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
+  uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
+  FilterPlan fp;
+  const SmallForm form = small_form(rq, nq, kp64, st, fp);
+  uint32_t* flag = nullptr;
+  if (form != SmallForm::kTables) {
+    flag = (uint32_t*)w.f_flag.ensure(4);
+    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
+    CandScores sc(rq, inv_norm, half_steps, 0);
+    sc.prepare(qu, nq, w, st);
+    if (form == SmallForm::kRows) {
+      uint32_t* keys = (uint32_t*)w.keys.ensure(nq * n * 4);
+      launch_score_rows(rq.codes.p, n, rq.dim, rq.bits, sc.op, nq, keys, n, st);
+      w.mark(st, 2);
+      uint32_t* ck = (uint32_t*)w.thr_keys.ensure(nq * kp * 4);
+      uint32_t* ci = (uint32_t*)w.thr_ids.ensure(nq * kp * 4);
+      select_rows(w, keys, nullptr, nullptr, n, n, nq, kp, 32, bits_for(n - 1), ck, ci, st);
+      w.mark(st, 3);
+      rescored_top_k(sc, rq, qu, inv_norm, nq, kp, ke, ck, ci, flag, w, st);
+    } else {
+      filtered_candidates(sc, n, nq, ke, kp, fp, flag, ok, oi, w, st, [&](const uint32_t* ids, uint32_t* keys) {
+        rescore_rankquant(rq, qu, inv_norm, nq, kp, ids, keys, st);
+      });
+    }
+  }
+  full_scan_select(
+      w, nq, n, ke, 32, ok, oi, st,
+      [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
+        launch_asym_scan(rq.codes.as<uint8_t>(), n, rq.dim, rq.bits, qu + q0 * rq.dim, qn, inv_norm, keys, n, st, flag);
+      },
+      flag);
+}
+
 uint32_t engine_rankquant_full(const Index& rq, const float* d_q, uint64_t nq, uint64_t k,
                                Workspace& w, cudaStream_t st) {
   require_kind(rq, ORDVEC_INDEX_KIND_RANK_QUANT, "search_asymmetric");
-  if (use_rank_tc(rq, nq, k, st)) return engine_rankquant_full_split(rq, d_q, nq, k, true, w, st);
+  if (use_rank_tc(rq, nq)) return engine_rankquant_full_split(rq, d_q, nq, k, true, w, st);
   const uint32_t ke = (uint32_t)(k < rq.n ? k : rq.n);
   if (!ke || !nq) return ke;
   const float* qu = normalised(w, d_q, nq, rq.dim, st);
-  const float inv_norm = inv_rankquant_norm(rq.dim, rq.bits);
-  uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
-  uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
-  full_scan_select(w, nq, rq.n, ke, 32, ok, oi, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
-    launch_asym_scan(rq.codes.as<uint8_t>(), rq.n, rq.dim, rq.bits, qu + q0 * rq.dim, qn, inv_norm, keys,
-                     rq.n, st);
-  });
+  exact_search(rq, qu, inv_rankquant_norm(rq.dim, rq.bits), false, nq, ke, w, st);
   return ke;
 }
 
@@ -597,15 +672,8 @@ uint32_t engine_rankquant_symmetric(const Index& rq, const float* d_q, uint64_t 
   launch_encode(6, d_q, nq, rq.dim, rq.bits, 0, 0, qc, 0, nullptr, st);
   const float norm = rankquant_norm_f32(rq.dim, rq.bits);
   const float inv_norm_sq = 1.0f / (norm * norm);
-  // batches: split-BF16 candidates (the centred buckets are exact in BF16, so
-  // lo = 0) rescored exactly
-  if (use_rank_tc(rq, nq, k, st)) return split_search(rq, qc, inv_norm_sq, true, nq, k, true, w, st, 0);
-  uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
-  uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
-  full_scan_select(w, nq, rq.n, ke, 32, ok, oi, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
-    launch_asym_scan(rq.codes.as<uint8_t>(), rq.n, rq.dim, rq.bits, qc + q0 * rq.dim, qn, inv_norm_sq, keys, rq.n,
-                     st);
-  });
+  if (use_rank_tc(rq, nq)) return split_search(rq, qc, inv_norm_sq, true, nq, k, true, w, st, 0);
+  exact_search(rq, qc, inv_norm_sq, true, nq, ke, w, st);
   return ke;
 }
 
@@ -635,13 +703,13 @@ struct RankScores {
 // Rank searches on the tensor cores: batches whose kp candidates take the sampled
 // filter, from two queries and nq n dim = 9e8 (OVB_RANK_TC=0/1 forces as for
 // RankQuant).  Measured with both forms, symmetric (us, CUDA cores / tensor
-// cores): n = 1M dim 768: 429 / 381 at 1 query, 639 / 384 at 2, 733 / 385 at 8, 3,911
-// / 412 at 48; n = 200k dim 1024: 191 / 222 at 4, 289 / 229 at 6; n = 40k dim 384:
-// 84 / 113 at 16, 142 / 124 at 48.
+// cores): n = 1M dim 768: 324 / 363 at 1 query, 567 / 364 at 2, 692 / 369 at 8, 3,939
+// / 376 at 48; n = 200k dim 1024: 180 / 216 at 4, 277 / 217 at 5; n = 100k dim 768: 123 /
+// 160 at 8, 192 / 162 at 12; n = 40k dim 384: 107 / 110 at 24, 139 / 111 at 48.
 static bool use_rank_scores(const Index& rk, uint64_t nq, uint64_t kp, cudaStream_t st, FilterPlan& fp) {
   const char* e = getenv("OVB_RANK_TC");
   if (e && e[0] == '0') return false;
-  if (capturing(st)) return false;  // the margin flag is read on the host
+  if (capturing(st)) return false;  // as in small_form
   if (!score_rank_eligible(rk.dim) || !split_filter_plan(rk.n, kp, fp)) return false;
   return (e && e[0] == '1') || (nq >= 2 && nq * rk.n * rk.dim >= 900000000ull);
 }
@@ -668,24 +736,25 @@ uint32_t engine_rank_full(const Index& rk, const float* d_q, uint64_t nq, uint64
     launch_encode(5, d_q, nq, dim, 0, 0, 0, qr, 0, nullptr, st);
   }
   // rows [q0, q0 + qn) through the key matrix of exact scores
-  auto full = [&](uint64_t qa, uint64_t qn) {
-    full_scan_select(w, qn, rk.n, ke, 32, ok + qa * ke, oi + qa * ke, st,
-                     [&](uint64_t q0, uint64_t qm, uint32_t* keys) {
-                       const uint64_t q = qa + q0;
-                       if (asymmetric)
-                         launch_rank_asym_scan(ranks, rk.n, dim, qu + q * dim, qsum + q, qm, keys, rk.n, st);
-                       else
-                         launch_rank_sym_scan(ranks, rk.n, dim, qr + q * dim, qm, keys, rk.n, st);
-                     });
+  auto full = [&](uint64_t qa, uint64_t qn, const uint32_t* gate) {
+    full_scan_select(
+        w, qn, rk.n, ke, 32, ok + qa * ke, oi + qa * ke, st,
+        [&](uint64_t q0, uint64_t qm, uint32_t* keys) {
+          const uint64_t q = qa + q0;
+          if (asymmetric)
+            launch_rank_asym_scan(ranks, rk.n, dim, qu + q * dim, qsum + q, qm, keys, rk.n, st, gate);
+          else
+            launch_rank_sym_scan(ranks, rk.n, dim, qr + q * dim, qm, keys, rk.n, st, gate);
+        },
+        gate);
   };
   const uint64_t kp = std::min<uint64_t>(std::max<uint64_t>(2ull * ke, ke + 64ull), rk.n);
   FilterPlan fp;
   if (!use_rank_scores(rk, nq, kp, st, fp)) {
-    full(0, nq);
+    full(0, nq, nullptr);
     return ke;
   }
   uint32_t* flag = (uint32_t*)w.f_flag.ensure(4);
-  uint32_t* flag_h = (uint32_t*)w.f_flag_host.ensure(4);
   uint64_t fc = keys_budget() / split_filter_bytes_per_query(fp, kp);
   if (fc < 1) fc = 1;
   RankScores sc{rk};
@@ -699,9 +768,7 @@ uint32_t engine_rank_full(const Index& rk, const float* d_q, uint64_t nq, uint64
                           launch_rank_subset(!asymmetric, ranks, dim, q, asymmetric ? qsum + q0 : nullptr, qn, ids,
                                              (uint32_t)kp, keys, st);
                         });
-    OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
-    OVB_CUDA(cudaStreamSynchronize(st));
-    if (*flag_h) full(q0, qn);
+    full(q0, qn, flag);  // does nothing unless the flag is set
   }
   return ke;
 }
@@ -872,6 +939,24 @@ static uint32_t rerank_mode(const Workspace& w, const Index& rq, uint64_t nq, ui
   return nq >= 16 && (uint64_t)me >= 4ull * ke + 64 ? OVB_RERANK_SPLIT : OVB_RERANK_FP64;
 }
 
+// Whether a rerank scores its candidates in integers first (scan_score_rows.cu) and
+// only the best kp in FP64: from 2-bit codes and nq me dim bits >= 5e8 on, where the FP64
+// rerank's time is more than the select, margin test and rescoring add.  Measured on
+// whole two-stage calls (us, FP64 / integers first): n = 171,332 dim 1024 b=2: 230 / 250
+// at 61 x 1,600 candidates (2.0e8), 342 / 327 at 256 x 1,000 (5.2e8), 618 / 551 at 1,000 x
+// 1,000, 948 / 775 at 1,024 x 2,000; n = 1M dim 768 b=2: 453 / 464 at 256 x 1,000 (3.9e8),
+// 558 / 538 at 256 x 2,000 (7.9e8), 1,352 / 1,221 at 1,024 x 2,000; n = 1M dim 1024 b=4: 260
+// / 291 at 32 x 1,000 (1.3e8), 368 / 356 at 128 x 1,000 (5.2e8), 762 / 606 at 256 x 2,000;
+// one-bit rows, whose FP64 form reads few tables, stay: 751 / 754 at 1,024 x 2,000 of dim
+// 1024.
+static bool use_subset_scores(const Index& rq, uint64_t nq, uint32_t me, uint32_t ke, cudaStream_t st) {
+  const char* e = getenv("OVB_ROW_SCORES");
+  if (e && e[0] == '0') return false;
+  const uint64_t kp = std::max<uint64_t>(2ull * ke, ke + 64ull);
+  if (!score_rows_eligible(rq.dim, rq.bits) || nq > 65535 || me < 4 * kp || capturing(st)) return false;
+  return (e && e[0] == '1') || (rq.bits >= 2 && nq * me * rq.dim * rq.bits >= 500000000ull);
+}
+
 // Split-BF16 rerank of the uniform candidate rows in w.sel_ids (me per query):
 // split queries, the tensor-core rerank (keys2), then either the raw top-ke of
 // the split scores (raw) or the exact form -- the top-kp by split score with
@@ -947,10 +1032,26 @@ uint32_t engine_two_stage(const Index& rq, const Index& s1, const float* d_q, ui
   if (mode != OVB_RERANK_FP64 && split_rerank(rq, qu, nq, me, ke, inv_norm, mode == OVB_RERANK_SPLIT_RAW, w, st))
     return ke;
   uint32_t* keys = (uint32_t*)w.keys2.ensure(nq * me * 4);
-  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, nq, nullptr, cand, me, inv_norm, keys, st);
+  const uint32_t* gate = nullptr;
+  if (w.rerank_mode == OVB_RERANK_AUTO && use_subset_scores(rq, nq, me, ke, st)) {
+    // integer scores of all candidates, FP64 scores of the best kp; the FP64 rerank of all
+    // of them below runs only where the margin test failed for some query
+    const uint32_t kp = std::max<uint32_t>(2 * ke, ke + 64);
+    uint32_t* flag = (uint32_t*)w.rr_flag.ensure(4);
+    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
+    CandScores sc(rq, inv_norm, false, 0);
+    sc.prepare(qu, nq, w, st);
+    launch_score_subset(rq.codes.p, rq.dim, rq.bits, sc.op, nq, cand, me, keys, st);
+    uint32_t* ck = (uint32_t*)w.rr_keys.ensure(nq * kp * 4);
+    uint32_t* ci = (uint32_t*)w.rr_ids.ensure(nq * kp * 4);
+    select_rows(w, keys, cand, nullptr, me, me, nq, kp, 32, id_bits, ck, ci, st);
+    rescored_top_k(sc, rq, qu, inv_norm, nq, kp, ke, ck, ci, flag, w, st);
+    gate = flag;
+  }
+  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, nq, nullptr, cand, me, inv_norm, keys, st, gate);
   w.mark(st, 4);
   // rows are uniform (me candidates each): the strided form, not offsets
-  select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true);
+  select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true, gate);
   w.mark(st, 5);
   return ke;
 }

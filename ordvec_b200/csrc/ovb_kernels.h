@@ -33,6 +33,7 @@ struct SelectArgs {
   uint32_t res_n_top;
   const uint32_t* err_src;  // copied to *err_dst once the results are written (either may be null)
   uint32_t* err_dst;
+  const uint32_t* gate;  // the launch does nothing when *gate is 0 (may be null)
 };
 // u64 scratch elements launch_select_rows may use for `rows` rows of length n
 // (0 for ragged rows): global sort buffers for k > kSelectSmemCap, and the
@@ -169,22 +170,25 @@ void launch_wait_probe(uint32_t* d_out, cudaStream_t stream);
 
 // ---- K9 Rank (u16) index scans (scan_rank_full.cu) -> key32 [nq][ld] ------------
 float rank_norm_f32(uint32_t dim);
+// gate (here and below, may be null): the launch does nothing when *gate is 0 on the device
 // Rank::search: q_ranks = the queries' u16 ranks (nq x dim)
 void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const uint16_t* q_ranks, uint64_t nq,
-                          uint32_t* keys, uint64_t ld, cudaStream_t stream);
+                          uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate = nullptr);
 // Rank::search_asymmetric: q_unit rows; q_sum (nq floats) is scratch the launch fills
 void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, const float* q_sum,
-                           uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream);
+                           uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream,
+                           const uint32_t* gate = nullptr);
 
 // ---- K4/K5 asymmetric RankQuant scoring (scan_asym.cu) ---------------------------
 void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t bits,
                       const float* q_unit, uint64_t nq, float inv_norm, uint32_t* keys,
-                      uint64_t ld, cudaStream_t stream);
+                      uint64_t ld, cudaStream_t stream, const uint32_t* gate = nullptr);
 // rows: query i's candidates cands[offsets[i] .. offsets[i + 1]) (at most max_row), or
 // with offsets null exactly max_row each; keys[] like cands[]
 void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const float* q_unit,
                         uint64_t nq, const uint64_t* offsets, const uint32_t* cands,
-                        uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream);
+                        uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream,
+                        const uint32_t* gate = nullptr);
 
 // ---- integer score scans on CTA pairs (scan_score_pair.cu) ---------------------------
 // src: 1, 2, 4 = RankQuant bits, 16 = Rank.  The operand's rows (bytes of device
@@ -212,6 +216,14 @@ void launch_score_scan(const void* rows, uint64_t n, uint32_t dim, uint32_t src,
 void launch_score_filter(const void* rows, uint64_t n, uint32_t dim, uint32_t src, const ScoreOperand& b, uint64_t nq,
                          const uint32_t* thr, uint64_t thr_stride, uint32_t* cnt, uint32_t cap, uint32_t* f_keys,
                          uint32_t* f_ids, uint32_t* err, cudaStream_t stream);
+// The same keys on the CUDA cores (scan_score_rows.cu; dim * bits % 128 == 0, at most
+// 65,535 queries): every document for a few queries, or row_len candidates of each
+// query (ids below n), keys[q * row_len + i].
+bool score_rows_eligible(uint32_t dim, uint32_t bits);
+void launch_score_rows(const void* codes, uint64_t n, uint32_t dim, uint32_t bits, const ScoreOperand& b, uint64_t nq,
+                       uint32_t* keys, uint64_t ld, cudaStream_t stream);
+void launch_score_subset(const void* codes, uint32_t dim, uint32_t bits, const ScoreOperand& b, uint64_t nq,
+                         const uint32_t* cands, uint64_t row_len, uint32_t* keys, cudaStream_t stream);
 // *flag |= 1 when a document outside some query's kp selected keys could belong to its top k
 void launch_score_margin(const uint32_t* sel_keys, uint64_t nq, uint32_t kp, uint32_t k, const double* bound,
                          uint32_t src, uint32_t* flag, cudaStream_t stream);
@@ -243,6 +255,7 @@ void launch_clamp_ids(uint32_t* ids, uint64_t count, uint32_t n, cudaStream_t st
 // (with err_dst, *err_dst = err_src ? *err_src : 0)
 void launch_keys_to_results(const uint32_t* keys, const uint32_t* ids, uint64_t count,
                             int mode, uint32_t n_top, float* scores, int64_t* out_ids,
-                            cudaStream_t stream, const uint32_t* err_src = nullptr, uint32_t* err_dst = nullptr);
+                            cudaStream_t stream, const uint32_t* err_src = nullptr, uint32_t* err_dst = nullptr,
+                            const uint32_t* gate = nullptr);
 
 }  // namespace ovb

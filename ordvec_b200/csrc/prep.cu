@@ -132,7 +132,9 @@ __global__ void finite_flag_kernel(const float* __restrict__ x, uint64_t count,
 __global__ void keys_to_results_kernel(const uint32_t* __restrict__ keys,
                                        const uint32_t* __restrict__ ids, uint64_t count,
                                        int mode, uint32_t n_top, float* __restrict__ scores,
-                                       int64_t* __restrict__ out_ids, const uint32_t* err_src, uint32_t* err_dst) {
+                                       int64_t* __restrict__ out_ids, const uint32_t* err_src, uint32_t* err_dst,
+                                       const uint32_t* gate) {
+  if (gate && !*gate) return;
   uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t == 0 && err_dst) *err_dst = err_src ? *err_src : 0u;
   if (t >= count) return;
@@ -208,10 +210,10 @@ void launch_prefix_compact(const uint32_t* src, uint64_t ld, const uint64_t* off
 
 void launch_keys_to_results(const uint32_t* keys, const uint32_t* ids, uint64_t count,
                             int mode, uint32_t n_top, float* scores, int64_t* out_ids,
-                            cudaStream_t stream, const uint32_t* err_src, uint32_t* err_dst) {
+                            cudaStream_t stream, const uint32_t* err_src, uint32_t* err_dst, const uint32_t* gate) {
   if (!count) return;
   keys_to_results_kernel<<<ceil_div(count, 256), 256, 0, stream>>>(keys, ids, count, mode, n_top, scores, out_ids,
-                                                                   err_src, err_dst);
+                                                                   err_src, err_dst, gate);
   launched();
 }
 

@@ -109,7 +109,8 @@ template <int BITS, int W>
 __global__ void __launch_bounds__(kThreads)
     asym_scan_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
                      const float* __restrict__ q_unit, float inv_norm,
-                     uint32_t* __restrict__ keys, uint64_t ld) {
+                     uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
+  if (gate && !*gate) return;
   const uint64_t qi = blockIdx.y;
   const uint32_t words = dim * BITS / 32;
   const int lane = threadIdx.x & 31;
@@ -129,7 +130,8 @@ __global__ void __launch_bounds__(kThreads)
     asym_subset_kernel(const uint8_t* __restrict__ codes, uint32_t dim,
                        const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                        const uint32_t* __restrict__ cands, float inv_norm,
-                       uint32_t* __restrict__ keys) {
+                       uint32_t* __restrict__ keys, const uint32_t* gate) {
+  if (gate && !*gate) return;
   const uint64_t qi = blockIdx.y;
   const uint64_t s = off ? off[qi] : qi * row_len, e = off ? off[qi + 1] : s + row_len;
   const uint32_t words = dim * BITS / 32;
@@ -178,7 +180,8 @@ __device__ __forceinline__ double generic_row_dot(const uint8_t* row, uint32_t d
 __global__ void __launch_bounds__(kThreads)
     asym_scan_generic(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim, uint32_t bits,
                       const float* __restrict__ q_unit, float inv_norm,
-                      uint32_t* __restrict__ keys, uint64_t ld) {
+                      uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
+  if (gate && !*gate) return;
   const uint64_t qi = blockIdx.y;
   const uint32_t bpv = dim * bits / 8;
   const uint64_t gw = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) / 32;
@@ -193,7 +196,8 @@ __global__ void __launch_bounds__(kThreads)
     asym_subset_generic(const uint8_t* __restrict__ codes, uint32_t dim, uint32_t bits,
                         const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                         const uint32_t* __restrict__ cands, float inv_norm,
-                        uint32_t* __restrict__ keys) {
+                        uint32_t* __restrict__ keys, const uint32_t* gate) {
+  if (gate && !*gate) return;
   const uint64_t qi = blockIdx.y;
   const uint64_t s = off ? off[qi] : qi * row_len, e = off ? off[qi + 1] : s + row_len;
   const uint32_t bpv = dim * bits / 8;
@@ -262,7 +266,8 @@ __global__ void __launch_bounds__(kTabThreads)
     asym_table_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
                       const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                       const uint32_t* __restrict__ cands, float inv_norm, uint32_t* __restrict__ keys,
-                      uint64_t ld) {
+                      uint64_t ld, const uint32_t* gate) {
+  if (gate && !*gate) return;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
   double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
@@ -331,7 +336,8 @@ template <int BITS>
 __global__ void __launch_bounds__(kTab4Threads)
     asym_table4_kernel(const uint8_t* __restrict__ codes, uint32_t dim, const float* __restrict__ q_unit,
                        const uint64_t* __restrict__ off, uint64_t row_len, const uint32_t* __restrict__ cands,
-                       float inv_norm, uint32_t* __restrict__ keys) {
+                       float inv_norm, uint32_t* __restrict__ keys, const uint32_t* gate) {
+  if (gate && !*gate) return;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
   double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
@@ -387,12 +393,12 @@ bool table_ok(uint32_t dim, uint32_t bits) {
 template <bool SUBSET>
 void launch_table(uint32_t bits, dim3 grid, size_t smem, cudaStream_t st, const uint8_t* codes, uint64_t n,
                   uint32_t dim, const float* qu, const uint64_t* off, uint64_t row_len, const uint32_t* cands,
-                  float inv_norm, uint32_t* keys, uint64_t ld) {
+                  float inv_norm, uint32_t* keys, uint64_t ld, const uint32_t* gate) {
 #define OVB_TAB(B)                                                                                     \
   do {                                                                                                 \
     allow_dynamic_smem(asym_table_kernel<B, SUBSET>);                                                  \
     asym_table_kernel<B, SUBSET><<<grid, kTabThreads, smem, st>>>(codes, n, dim, qu, off, row_len, cands, \
-                                                                  inv_norm, keys, ld);                           \
+                                                                  inv_norm, keys, ld, gate);                     \
   } while (0)
   if (bits == 1)
     OVB_TAB(1);
@@ -403,10 +409,13 @@ void launch_table(uint32_t bits, dim3 grid, size_t smem, cudaStream_t st, const 
 #undef OVB_TAB
 }
 
-unsigned grid_x(uint64_t rows_per_cta, uint64_t n) {
+// CTAs a query.  A gated launch, which most often does nothing, takes two CTAs an SM
+// in all (or one a query): the rows loop.
+unsigned grid_x(uint64_t rows_per_cta, uint64_t n, const uint32_t* gate, uint64_t queries) {
   uint64_t g = (n + rows_per_cta - 1) / rows_per_cta;
+  const uint64_t most = gate ? 148 * 2 / queries : 148 * 8;
+  if (g > most) g = most;
   if (g < 1) g = 1;
-  if (g > 148 * 8) g = 148 * 8;
   return (unsigned)g;
 }
 
@@ -423,13 +432,14 @@ int plan_w(uint32_t dim, uint32_t bits) {
 template <int BITS>
 void dispatch_bits(int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t* codes, uint64_t n,
                    uint32_t dim, const float* qu, float inv_norm, uint32_t* keys, uint64_t ld,
-                   const uint64_t* off, uint64_t row_len, const uint32_t* cands) {
+                   const uint64_t* off, uint64_t row_len, const uint32_t* cands, const uint32_t* gate) {
 #define OVB_ASYM_CASE(WV)                                                                                  \
   if (W == WV) {                                                                                           \
     if (subset)                                                                                            \
-      asym_subset_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, dim, qu, off, row_len, cands, inv_norm, keys); \
+      asym_subset_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, dim, qu, off, row_len, cands,         \
+                                                              inv_norm, keys, gate);                       \
     else                                                                                                   \
-      asym_scan_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, n, dim, qu, inv_norm, keys, ld);        \
+      asym_scan_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, n, dim, qu, inv_norm, keys, ld, gate);  \
     return;                                                                                                \
   }
   if constexpr (BITS == 1) {
@@ -447,28 +457,28 @@ void dispatch_bits(int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t
 
 void dispatch(uint32_t bits, int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t* codes,
               uint64_t n, uint32_t dim, const float* qu, float inv_norm, uint32_t* keys, uint64_t ld,
-              const uint64_t* off, uint64_t row_len, const uint32_t* cands) {
+              const uint64_t* off, uint64_t row_len, const uint32_t* cands, const uint32_t* gate) {
   if (bits == 1)
-    dispatch_bits<1>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands);
+    dispatch_bits<1>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, gate);
   else if (bits == 2)
-    dispatch_bits<2>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands);
+    dispatch_bits<2>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, gate);
   else
-    dispatch_bits<4>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands);
+    dispatch_bits<4>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, gate);
 }
 
 }  // namespace
 
 void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t bits,
                       const float* q_unit, uint64_t nq, float inv_norm, uint32_t* keys,
-                      uint64_t ld, cudaStream_t stream) {
+                      uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
   if (!n || !nq) return;
   if (table_ok(dim, bits)) {
     // ~1024 rows per CTA: the table build stays a few percent of the scoring
     for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
       unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-      dim3 grid(grid_x(1024, n), gy);
+      dim3 grid(grid_x(1024, n, gate, gy), gy);
       launch_table<false>(bits, grid, table_smem(dim, bits), stream, codes, n, dim, q_unit + q0 * dim, nullptr,
-                           0, nullptr, inv_norm, keys + q0 * ld, ld);
+                           0, nullptr, inv_norm, keys + q0 * ld, ld, gate);
       launched();
     }
     return;
@@ -476,20 +486,21 @@ void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t b
   const int W = plan_w(dim, bits);
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-    dim3 grid(grid_x(kThreads / 32, n), gy);
+    dim3 grid(grid_x(kThreads / 32, n, gate, gy), gy);
     if (W)
       dispatch(bits, W, false, grid, stream, codes, n, dim, q_unit + q0 * dim, inv_norm, keys + q0 * ld, ld,
-               nullptr, 0, nullptr);
+               nullptr, 0, nullptr, gate);
     else
       asym_scan_generic<<<grid, kThreads, 0, stream>>>(codes, n, dim, bits, q_unit + q0 * dim, inv_norm,
-                                                       keys + q0 * ld, ld);
+                                                       keys + q0 * ld, ld, gate);
     launched();
   }
 }
 
 void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const float* q_unit,
                         uint64_t nq, const uint64_t* offsets, const uint32_t* cands,
-                        uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream) {
+                        uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream,
+                        const uint32_t* gate) {
   if (!nq || !max_row) return;
   // one arithmetic for every batch size, so a query scores the same alone and
   // inside a batch
@@ -504,7 +515,7 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
   do {                                                                                                          \
     allow_dynamic_smem(asym_table4_kernel<B>);                                                                  \
     asym_table4_kernel<B><<<grid, kTab4Threads, smem, stream>>>(codes, dim, q_unit, offsets, max_row, cands,    \
-                                                                inv_norm, keys);                                \
+                                                                inv_norm, keys, gate);                          \
   } while (0)
       if (bits == 1)
         OVB_TAB4(1);
@@ -520,10 +531,10 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
     const uint64_t rows_per_cta = nq >= 64 ? 512 : 128;
     for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
       unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-      dim3 grid(grid_x(rows_per_cta, max_row), gy);
+      dim3 grid(grid_x(rows_per_cta, max_row, gate, gy), gy);
       launch_table<true>(bits, grid, table_smem(dim, bits), stream, codes, 0, dim, q_unit + q0 * dim,
                          offsets ? offsets + q0 : nullptr, max_row, cands + (offsets ? 0 : q0 * max_row), inv_norm,
-                         keys + (offsets ? 0 : q0 * max_row), 0);
+                         keys + (offsets ? 0 : q0 * max_row), 0, gate);
       launched();
     }
     return;
@@ -534,15 +545,16 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
   const uint64_t rows_per_warp = nq >= 64 ? 32 : 4;
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-    dim3 grid(grid_x((kThreads / 32) * rows_per_warp, max_row), gy);
+    dim3 grid(grid_x((kThreads / 32) * rows_per_warp, max_row, gate, gy), gy);
     const uint64_t* off = offsets ? offsets + q0 : nullptr;
     const uint32_t* c = cands + (offsets ? 0 : q0 * max_row);
     uint32_t* k = keys + (offsets ? 0 : q0 * max_row);
     if (W)
-      dispatch(bits, W, true, grid, stream, codes, 0, dim, q_unit + q0 * dim, inv_norm, k, 0, off, max_row, c);
+      dispatch(bits, W, true, grid, stream, codes, 0, dim, q_unit + q0 * dim, inv_norm, k, 0, off, max_row, c,
+               gate);
     else
       asym_subset_generic<<<grid, kThreads, 0, stream>>>(codes, dim, bits, q_unit + q0 * dim, off, max_row, c,
-                                                         inv_norm, k);
+                                                         inv_norm, k, gate);
     launched();
   }
 }

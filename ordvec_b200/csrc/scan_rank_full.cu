@@ -43,7 +43,8 @@ template <bool SYM, int QT, bool WIDE>
 __global__ void __launch_bounds__(kRfThreads)
     rank_tile_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim, const void* __restrict__ q,
                      const float* __restrict__ q_sum, uint64_t nq, float mean, float scale,
-                     uint32_t* __restrict__ keys, uint64_t ld) {
+                     uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
+  if (gate && !*gate) return;
   using Acc = typename std::conditional<WIDE, unsigned long long, uint32_t>::type;
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* rows = smem;                            // [warp][32][kRowWords]
@@ -137,7 +138,8 @@ __global__ void __launch_bounds__(kRfThreads)
 __global__ void __launch_bounds__(kRfThreads)
     rank_sym_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim,
                     const uint16_t* __restrict__ q_ranks, float inv_norm_sq, uint32_t* __restrict__ keys,
-                    uint64_t ld) {
+                    uint64_t ld, const uint32_t* gate) {
+  if (gate && !*gate) return;
   extern __shared__ int32_t qc[];  // 2 q_r - (D - 1)
   const uint64_t qi = blockIdx.y;
   const int32_t m2 = (int32_t)dim - 1;
@@ -159,7 +161,8 @@ __global__ void __launch_bounds__(kRfThreads)
 __global__ void __launch_bounds__(kRfThreads)
     rank_asym_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim,
                      const float* __restrict__ q_unit, const float* __restrict__ q_sum, float mean,
-                     float inv_norm, uint32_t* __restrict__ keys, uint64_t ld) {
+                     float inv_norm, uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
+  if (gate && !*gate) return;
   extern __shared__ float qs[];
   const uint64_t qi = blockIdx.y;
   for (uint32_t j = threadIdx.x; j < dim; j += blockDim.x) qs[j] = q_unit[qi * dim + j];
@@ -203,10 +206,12 @@ __global__ void row_sum_kernel(const float* __restrict__ q, uint64_t nq, uint32_
   if (lane == 0) out[i] = s;
 }
 
-unsigned rf_grid(uint64_t units, uint64_t per_cta) {
+// CTAs a query; a gated launch, which most often does nothing, takes two an SM in all
+unsigned rf_grid(uint64_t units, uint64_t per_cta, const uint32_t* gate, uint64_t queries) {
   uint64_t g = (units + per_cta - 1) / per_cta;
+  const uint64_t most = gate ? 148 * 2 / queries : 148 * 16;
+  if (g > most) g = most;
   if (g < 1) g = 1;
-  if (g > 148 * 16) g = 148 * 16;
   return (unsigned)g;
 }
 
@@ -220,14 +225,14 @@ int rank_qt(uint64_t nq, uint32_t dim) {
 
 template <bool SYM, int QT, bool WIDE>
 void launch_tile(const uint16_t* ranks, uint64_t n, uint32_t dim, const void* q, const float* q_sum, uint64_t nq,
-                 float mean, float scale, uint32_t* keys, uint64_t ld, cudaStream_t stream) {
+                 float mean, float scale, uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
   const size_t smem = ((size_t)kRfWarps * 32 * kRowWords + (size_t)dim * QT) * 4;
   auto kern = rank_tile_kernel<SYM, QT, WIDE>;
   allow_dynamic_smem(kern);
   const uint64_t groups = (nq + QT - 1) / QT;
   uint64_t gy = (n + kRfWarps * 32 - 1) / (kRfWarps * 32);
   // enough CTAs to fill every SM several times over; documents beyond that loop
-  const uint64_t want = 148ull * 32;
+  const uint64_t want = gate ? 148 * 2 : 148 * 32;
   if (gy * groups > want) gy = (want + groups - 1) / groups;
   if (gy < 1) gy = 1;
   if (gy > 65535) gy = 65535;
@@ -236,20 +241,22 @@ void launch_tile(const uint16_t* ranks, uint64_t n, uint32_t dim, const void* q,
     const uint64_t q0 = g0 * QT;
     const void* qp = SYM ? (const void*)((const uint16_t*)q + q0 * dim) : (const void*)((const float*)q + q0 * dim);
     kern<<<dim3((unsigned)gn, (unsigned)gy), kRfThreads, smem, stream>>>(
-        ranks, n, dim, qp, q_sum ? q_sum + q0 : nullptr, nq - q0, mean, scale, keys + q0 * ld, ld);
+        ranks, n, dim, qp, q_sum ? q_sum + q0 : nullptr, nq - q0, mean, scale, keys + q0 * ld, ld,
+        gate);
     launched();
   }
 }
 
 template <bool SYM, bool WIDE>
 void launch_tiled(int qt, const uint16_t* ranks, uint64_t n, uint32_t dim, const void* q, const float* q_sum,
-                  uint64_t nq, float mean, float scale, uint32_t* keys, uint64_t ld, cudaStream_t stream) {
+                  uint64_t nq, float mean, float scale, uint32_t* keys, uint64_t ld, cudaStream_t stream,
+                  const uint32_t* gate) {
   if (qt == 8)
-    launch_tile<SYM, 8, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream);
+    launch_tile<SYM, 8, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, gate);
   else if (qt == 4)
-    launch_tile<SYM, 4, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream);
+    launch_tile<SYM, 4, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, gate);
   else
-    launch_tile<SYM, 1, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream);
+    launch_tile<SYM, 1, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, gate);
 }
 
 }  // namespace
@@ -267,43 +274,46 @@ void launch_rank_row_sum(const float* q, uint64_t nq, uint32_t dim, float* out, 
 }
 
 void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const uint16_t* q_ranks, uint64_t nq,
-                          uint32_t* keys, uint64_t ld, cudaStream_t stream) {
+                          uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
   if (!n || !nq) return;
   const float norm = rank_norm_f32(dim);
   const float inv_norm_sq = 1.0f / (norm * norm);
   if (dim % 8 == 0) {
     const int qt = rank_qt(nq, dim);
     if (dim <= 2048)
-      launch_tiled<true, false>(qt, ranks, n, dim, q_ranks, nullptr, nq, 0.0f, inv_norm_sq, keys, ld, stream);
+      launch_tiled<true, false>(qt, ranks, n, dim, q_ranks, nullptr, nq, 0.0f, inv_norm_sq, keys, ld, stream,
+                                gate);
     else
-      launch_tiled<true, true>(qt, ranks, n, dim, q_ranks, nullptr, nq, 0.0f, inv_norm_sq, keys, ld, stream);
+      launch_tiled<true, true>(qt, ranks, n, dim, q_ranks, nullptr, nq, 0.0f, inv_norm_sq, keys, ld, stream,
+                                gate);
     return;
   }
   const size_t smem = (size_t)dim * 4;
   allow_dynamic_smem(rank_sym_kernel);
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     const unsigned gy = (unsigned)(nq - q0 < 65535 ? nq - q0 : 65535);
-    rank_sym_kernel<<<dim3(rf_grid(n, kRfThreads / 32), gy), kRfThreads, smem, stream>>>(
-        ranks, n, dim, q_ranks + q0 * dim, inv_norm_sq, keys + q0 * ld, ld);
+    rank_sym_kernel<<<dim3(rf_grid(n, kRfThreads / 32, gate, gy), gy), kRfThreads, smem, stream>>>(
+        ranks, n, dim, q_ranks + q0 * dim, inv_norm_sq, keys + q0 * ld, ld, gate);
     launched();
   }
 }
 
 void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, const float* q_sum,
-                           uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream) {
+                           uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
   if (!n || !nq) return;
   const float inv_norm = 1.0f / rank_norm_f32(dim);
   const float mean = ((float)dim - 1.0f) / 2.0f;
   if (dim % 8 == 0) {
-    launch_tiled<false, false>(rank_qt(nq, dim), ranks, n, dim, q_unit, q_sum, nq, mean, inv_norm, keys, ld, stream);
+    launch_tiled<false, false>(rank_qt(nq, dim), ranks, n, dim, q_unit, q_sum, nq, mean, inv_norm, keys, ld, stream,
+                               gate);
     return;
   }
   const size_t smem = (size_t)dim * 4;
   allow_dynamic_smem(rank_asym_kernel);
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     const unsigned gy = (unsigned)(nq - q0 < 65535 ? nq - q0 : 65535);
-    rank_asym_kernel<<<dim3(rf_grid(n, kRfThreads), gy), kRfThreads, smem, stream>>>(
-        ranks, n, dim, q_unit + q0 * dim, q_sum + q0, mean, inv_norm, keys + q0 * ld, ld);
+    rank_asym_kernel<<<dim3(rf_grid(n, kRfThreads, gate, gy), gy), kRfThreads, smem, stream>>>(
+        ranks, n, dim, q_unit + q0 * dim, q_sum + q0, mean, inv_norm, keys + q0 * ld, ld, gate);
     launched();
   }
 }

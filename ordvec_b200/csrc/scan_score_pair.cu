@@ -527,7 +527,10 @@ __device__ __forceinline__ uint64_t b_row(uint64_t q, uint32_t nqt, uint32_t pla
 // - q^| + the rounding of S q): an upper bound, in units of T, of what rounding q
 // changes a document's c-centred sum by; bound[2q + 1] = c sum q^, the centre.  A
 // query with NaN or infinity gets an infinite bound (no candidate set is enough).
-// half_steps: S is a power of two, so that multiples of 1/2 have no rounding at all.
+// half_steps: S is a power of two, so that multiples of 1/2 have no rounding at all:
+// T orders documents as their sums do, and those, multiples of 1/4 below 2^20, stay
+// distinct in the final f32 rounding, so the best kp by (T, id) begin with the answer
+// whatever ties there are: a bound of minus infinity passes the margin test.
 __global__ void fix_rankquant_kernel(const float* __restrict__ qu, uint32_t dim, uint32_t bits, bool half_steps,
                                      uint32_t nqt, uint32_t k_bytes, int8_t* __restrict__ out, double* __restrict__ bound) {
   __shared__ float fpart[32];
@@ -565,7 +568,7 @@ __global__ void fix_rankquant_kernel(const float* __restrict__ qu, uint32_t dim,
   if (threadIdx.x == 0) {
     const double c = ((double)(1u << bits) - 1.0) * 0.5;
     // |fl(S q) - S q| <= 32640 * 2^-24 < 0.002
-    bound[2 * q] = bad || flat ? (double)INFINITY : 2.0 * c * (off + 0.002 * dim);
+    bound[2 * q] = bad || flat ? (double)INFINITY : half_steps ? -(double)INFINITY : 2.0 * c * (off + 0.002 * dim);
     bound[2 * q + 1] = c * sum;
   }
 }
