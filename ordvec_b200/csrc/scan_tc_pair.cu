@@ -45,9 +45,9 @@
 // scale 1) sums 64 products of 0 and +-1 into an f32 accumulator, exact for sums
 // below 2^24, at twice the int8 rate and with half the operand bytes.
 // Measured (filter scan, before this form of issuer, builders and epilogue and
-// now): 10M docs x 768 bits x 1,024 queries 6.79 -> 5.29 ms, epilogue-bound; 1M x
-// 1,024 x 61 (sign) 507 -> 143 us and 1M x 3,072 x 256 (multi-bucket, int8 before)
-// 790 -> 553 us, both bound by the ring's round trip; FastScan 171,332 x 1,024 x
+// now): 10M docs x 768 bits x 1,024 queries 6.79 -> 3.86 ms, epilogue-bound; 1M x
+// 1,024 x 61 (sign) 507 -> 131 us and 1M x 3,072 x 256 (multi-bucket, int8 before)
+// 790 -> 543 us, both bound by the ring's round trip; FastScan 171,332 x 1,024 x
 // 1,000 1.01 -> 0.83 ms.  The scale factors sit in tensor-memory columns
 // [224, 256) (A) and [480, 512) (B), all bytes 127, past the two accumulators
 // of N <= 224 query columns.
@@ -84,6 +84,16 @@ constexpr uint32_t kPF4MaxN = 224;                  // FP4 form: query columns p
 constexpr uint32_t kPF4TileN = kPF4MaxN;
 constexpr uint32_t kSfaCol = 224, kSfbCol = 480;    // FP4 form: scale-factor columns of A and B
 constexpr uint32_t kUnitScales = 0x7F7F7F7Fu;       // four ue8m0 bytes of 2^0
+// FP4 form, rows of at most 255 words: every accumulator starts at 2^23 + 2^22 +
+// 2^15, the product of a constant tile with itself (385 a 32-element block, twice, at
+// a scale of 2^14).  Its f32 pattern then holds 2^15 + sum in the low 16 bits, which is
+// what the epilogue loads, two columns a register (one more MMA a tile, 104 clocks of
+// 208 columns; longer rows compare f32 sums).
+// (bounds and sums stay within +-(kPackMax + 1), so that no difference of two leaves 16 bits)
+constexpr uint32_t kPackWords = 255, kPackMax = 64 * kPackWords;
+constexpr uint32_t kBiasScales = 0x8D8D8D8Du;       // 2^14
+constexpr uint32_t kSfaBiasCol = kSfaCol + 16;
+constexpr uint32_t kBiasTile = 4096;                // 128 rows of 32 bytes, every 16 bytes the same
 
 // PAIR: CTA pairs, 128 doc rows per CTA, two 256-column accumulators.
 // !PAIR: one CTA per SM, 256 doc rows (two M=128 halves) in one 512-column
@@ -125,7 +135,9 @@ struct PSmem {
   uint32_t base[kTileQ];
   // pair form: per-query parameters of the launch, [amin | tdoc or bias | thr | qpop or invq]
   uint32_t qp[PAIR ? 4 * kPMaxQ : 1];
-  uint32_t wamin[PAIR ? kPEpiWarps : 1][64];  // pair form: each epilogue warp's 64 column thresholds
+  // pair form: each epilogue warp's 64 column thresholds; FP4: the launch's, two a word
+  uint32_t wamin[PAIR ? kPEpiWarps : 1][64];
+  alignas(128) uint32_t unit[F4 ? kBiasTile / 4 : 1];  // FP4: the constant tile
   // pair form: the row words of each builder warp's next K-block
   uint4 raw[PAIR ? kPBuildWarps : 1][PAIR ? PT<PAIR, F4>::kItems : 1][PAIR ? 32 : 1];
   uint64_t full_a[PT<PAIR, F4>::kASlots];
@@ -174,14 +186,42 @@ __device__ __forceinline__ void mma_mxf4_pair(uint32_t d_tmem, uint64_t a_desc, 
       : "memory");
 }
 
-// Stores the word w into 32 consecutive columns from taddr in every lane of the
+// Stores the word w into 16 consecutive columns from taddr in every lane of the
 // calling warp's tensor-memory lane quarter.
-__device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t w) {
+__device__ __forceinline__ void tmem_fill16(uint32_t taddr, uint32_t w) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
       "r"(w)
       : "memory");
+}
+
+// The low 16 bits of 16, 32 or 64 columns, two a register (column 2 i in the low half of v[i]).
+__device__ __forceinline__ void tmem_ld_pack(uint32_t taddr, uint32_t (&v)[32], uint32_t groups) {
+  if (groups <= 1)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.pack::16b.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+  else if (groups == 2)
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+  else
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.pack::16b.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr)
+        : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // Half a word (32 bits of a bitmap row) -> 32 e2m1 nibbles (16 bytes): word s of
@@ -221,6 +261,12 @@ __device__ __forceinline__ float f4_bound(const TcArgs& a, uint32_t am) {
   return (float)((int)am - (a.key_kind == 2 ? (int)kHamBias : 0));
 }
 
+// The same bound for a packed sum, within what 16 bits hold (sums are within +-kPackMax).
+__device__ __forceinline__ int f4_bound16(const TcArgs& a, uint32_t am) {
+  const int x = (int)am - (a.key_kind == 2 ? (int)kHamBias : 0);
+  return min(max(x, -(int)kPackMax), (int)kPackMax + 1);
+}
+
 // The (biased) integer of an FP4 accumulator.
 __device__ __forceinline__ uint32_t f4_int(const TcArgs& a, uint32_t bits) {
   return (uint32_t)__float2int_rn(__uint_as_float(bits)) + (a.key_kind == 2 ? kHamBias : 0u);
@@ -251,6 +297,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
   auto b_addr = [&](uint32_t st) -> uint8_t* { return &S.b[0][0] + st * b_stage; };
   const uint64_t n_blocks = (a.n + 31) / 32;
   const bool dense = a.keys != nullptr;
+  const bool packed = F4 && a.qpv <= kPackWords;
   // FP4 form: filter only (host-checked; a launch that breaks a limit does no
   // work and sets bit 0 of *err)
   if (F4 && (dense || a.qpv > kPF4MaxWords || nt > kPF4MaxN)) {
@@ -311,10 +358,16 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
     // per tensor-memory lane quarter (warp % 4)
     if (warp >= 2 + kPBuildWarps && warp < 6 + kPBuildWarps) {
       const uint32_t lanes = ((uint32_t)(warp & 3) * 32) << 16;
-      tmem_fill32(tmem + lanes + kSfaCol, kUnitScales);
-      tmem_fill32(tmem + lanes + kSfbCol, kUnitScales);
+      tmem_fill16(tmem + lanes + kSfaCol, kUnitScales);
+      tmem_fill16(tmem + lanes + kSfaBiasCol, kBiasScales);
+      tmem_fill16(tmem + lanes + kSfbCol, kUnitScales);
+      tmem_fill16(tmem + lanes + kSfbCol + 16, kUnitScales);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
+    // ten 6s, a 4 and a 3 in each 32 elements: squares that sum to 385
+    for (uint32_t i = t; i < kBiasTile / 4; i += kPThreads)
+      S.unit[i] = i % 4 == 0 ? 0x77777777u : i % 4 == 1 ? 0x00005677u : 0u;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster_sync_all();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -367,6 +420,9 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
       // a slot, and a 32-byte K step (2), advance the descriptors' start-address
       // field (16-byte units; shared addresses stay below its 2^18 bytes)
       const uint64_t a_desc0 = sw128_desc(smem_u32(S.a[0])), b_desc0 = sw128_desc(smem_u32(b_addr(0)));
+      // the constant tile: no swizzle, 8 rows x 16 bytes next to each other, 256 bytes every 8 rows
+      const uint64_t bias_desc = (uint64_t)((smem_u32(S.unit) & 0x3FFFF) >> 4) | ((uint64_t)(128 >> 4) << 16) |
+                                 ((uint64_t)(256 >> 4) << 32) | ((uint64_t)1 << 46);
       auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
         return __all_sync(0xFFFFFFFFu, mbar_wait_issuer(bar, parity));
       };
@@ -389,6 +445,12 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = tmem + b * 256;
+        if constexpr (F4) {
+          if (packed) {
+            if (el) mma_mxf4_pair(d, bias_desc, bias_desc, idesc, 0, tmem + kSfaBiasCol, tmem + kSfbCol);
+            __syncwarp();
+          }
+        }
         for (uint32_t kb = 0; kb < n_kb; kb++) {
           const uint32_t sa = resA ? a_base + kb : rs;
           if (!wait(&S.full_b[rs], rp) || (need_a && !wait(&S.full_a[sa], pa))) {
@@ -402,7 +464,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
 #pragma unroll
             for (uint32_t j = 0; j < 4; j++) {
               if constexpr (F4) {
-                mma_mxf4_pair(d, ad + 2 * j, bd + 2 * j, idesc, (kb | j) != 0, tmem + kSfaCol, tmem + kSfbCol);
+                mma_mxf4_pair(d, ad + 2 * j, bd + 2 * j, idesc, packed || (kb | j) != 0, tmem + kSfaCol, tmem + kSfbCol);
               } else if constexpr (PAIR) {
                 mma_i8_pair(d, ad + 2 * j, bd + 2 * j, idesc, (kb | j) != 0);
               } else {
@@ -775,7 +837,113 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
       }
       __syncwarp();  // the list is reused by the next tile
     };
-    if constexpr (F4) {
+    if (F4 && packed) {
+      // FP4 form, 16-bit sums: a subtraction gives two columns' compares (bit 15 of a
+      // half: sum >= bound; neither half can borrow), eight of them 16 queries', and
+      // one vote says whether any of the warp's 32 docs is kept for them.  Groups of 16
+      // columns go round the four warps of a lane quarter.  A warp's accumulator
+      // columns are in registers after one load, and the buffer is released.  Kept
+      // entries stay in the warp's list over the tiles until it is nearly full, then
+      // every lane reserves and writes four at once; docs at the threshold itself are
+      // settled by the tie bound there.  Measured (scan, f32 compares and one atomic in
+      // flight a lane / this): 10M docs x 768 bits x 1,024 queries 5.27 / 3.86 ms, 2M
+      // 1.25 / 1.02, 1M x 1,024 x 1,024 (sign) 0.65 / 0.53, 1M x 1,024 x 61 137 / 131
+      // us.  Slower: a pair of writer warps fed by rings (4.1 ms, and 1.77 at 2M, where
+      // more is kept), two teams of eight warps on alternate tiles (4.5 ms).
+      uint32_t* am2 = &S.wamin[0][0];
+      static_assert(sizeof(S.wamin) >= (kPMaxQ + kPMaxN) * 2, "two bounds a word, past the last tile");
+      for (uint32_t i = et; i < (kPMaxQ + kPMaxN) / 2; i += kPEpiThreads) {
+        const int lo = 2 * i < a.nq ? f4_bound16(a, P_am(2 * i)) : (int)kPackMax + 1;
+        const int hi = 2 * i + 1 < a.nq ? f4_bound16(a, P_am(2 * i + 1)) : (int)kPackMax + 1;
+        am2[i] = (uint32_t)(hi * 65536 + lo);
+      }
+      epi_sync();
+      const uint32_t n_grp = nt / 16, part = e >> 2;
+      const uint32_t my_grp = n_grp / 4 + (part < n_grp % 4 ? 1 : 0);  // up to 4 groups of this warp
+      const uint32_t c0 = 16 * (part * (n_grp / 4) + min(part, n_grp % 4));
+      uint32_t held = 0;  // entries in the list: (doc, 2^15 + sum - bound | query << 16)
+      auto drain = [&]() {
+        __syncwarp();
+        // every lane's atomics in flight together
+        uint32_t pos[kPSegCap / 32], key[kPSegCap / 32];
+#pragma unroll
+        for (uint32_t i = 0; i < kPSegCap / 32; i++) {
+          pos[i] = 0xFFFFFFFFu;
+          if (32 * i + lane >= held) continue;
+          const uint2 en = list[32 * i + lane];
+          const uint32_t q = en.y >> 16;
+          const uint32_t y = (uint32_t)((int)(en.y & 0xFFFFu) - 0x8000 + f4_bound16(a, P_am(q))) +
+                             (a.key_kind == 2 ? kHamBias : 0u);
+          key[i] = bm_key_q(a, P_pop(q), y);
+          // (key, doc) <= (thr, tdoc): at the threshold, docs up to the tie bound
+          if (!(a.thr_pos && y == P_thr(q) && en.x > P_td(q))) pos[i] = atomicAdd(&a.cnt[q], 1u);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kPSegCap / 32; i++) {
+          if (pos[i] >= a.cap) continue;
+          const uint2 en = list[32 * i + lane];
+          const uint64_t at = (uint64_t)(en.y >> 16) * a.cap + pos[i];
+          a.f_keys[at] = key[i];
+          a.f_ids[at] = en.x;
+        }
+        __syncwarp();
+        held = 0;
+      };
+      uint32_t tcount = 0;
+      TileCursor tc_;
+      for (tc_.start(g, cluster); tc_.valid(g); tc_.next(g, n_clusters), tcount++) {
+        const uint32_t q0 = tc_.qt * nt;
+        const uint32_t b = tcount % kBufs;
+        const uint32_t doc = tc_.dt * 256 + rank * kPRows + row;  // filter: block stride 1
+        const uint32_t pass = doc < a.n ? 0x80008000u : 0u;
+        bool ready = false;
+        if (lane == 0) ready = !aborted(S) && mbar_wait_cluster(&S.acc_full[b], (tcount / kBufs) & 1);
+        ready = __shfl_sync(0xFFFFFFFFu, ready, 0);
+        if (!ready) {
+          if (lane == 0 && !aborted(S)) raise_abort(S, a.err);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t v[32];
+        __syncwarp();
+        if (my_grp) tmem_ld_pack(tmem + ((lq * 32) << 16) + b * 256 + c0, v, my_grp);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive_remote(acc_empty0 + 8 * b);  // the columns are in registers
+#pragma unroll
+        for (uint32_t gr = 0; gr < 4; gr++) {
+          if (gr >= my_grp) break;
+          const uint4* bp = reinterpret_cast<const uint4*>(am2 + (q0 + c0) / 2 + 8 * gr);
+          const uint4 b0 = bp[0], b1 = bp[1];
+          const uint32_t bd[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+          uint32_t x[8], any = 0;
+#pragma unroll
+          for (uint32_t r = 0; r < 8; r++) {
+            x[r] = v[8 * gr + r] - bd[r];
+            any |= x[r];
+          }
+          if (!__any_sync(0xFFFFFFFFu, (any & pass) != 0)) continue;
+          uint32_t hm = 0;  // bit r: column 2 r, bit 16 + r: column 2 r + 1
+#pragma unroll
+          for (uint32_t r = 0; r < 8; r++) hm |= (x[r] >> (15 - r)) & (0x00010001u << r);
+          if (!pass) hm = 0;
+          for (uint32_t bal = __ballot_sync(0xFFFFFFFFu, hm != 0); bal; bal = __ballot_sync(0xFFFFFFFFu, hm != 0)) {
+            if (held + __popc(bal) > kPSegCap) drain();
+            if (hm) {
+              const uint32_t j = (uint32_t)__ffs(hm) - 1, odd = j >> 4;
+              const uint32_t y01 = j & 1 ? x[1] : x[0], y23 = j & 1 ? x[3] : x[2], y45 = j & 1 ? x[5] : x[4],
+                             y67 = j & 1 ? x[7] : x[6];
+              const uint32_t y03 = j & 2 ? y23 : y01, y47 = j & 2 ? y67 : y45, w2 = j & 4 ? y47 : y03;
+              const uint32_t q = q0 + c0 + 16 * gr + 2 * (j & 7) + odd;
+              list[held + __popc(bal & lt)] = make_uint2(doc, (odd ? w2 >> 16 : w2 & 0xFFFFu) | (q << 16));
+              hm &= hm - 1;
+            }
+            held += __popc(bal);
+          }
+        }
+      }
+      drain();
+    } else if constexpr (F4) {
       // FP4 form: the f32 sums are compared with the f32 of each query's integer
       // threshold, read straight from the launch's parameters (a tile stages
       // nothing); docs at the threshold itself are settled by the tie bound when
