@@ -45,8 +45,8 @@
 // scale 1) sums 64 products of 0 and +-1 into an f32 accumulator, exact for sums
 // below 2^24, at twice the int8 rate and with half the operand bytes.
 // Measured (filter scan, before this form of issuer, builders and epilogue and
-// now): 10M docs x 768 bits x 1,024 queries 6.79 -> 3.86 ms, epilogue-bound; 1M x
-// 1,024 x 61 (sign) 507 -> 131 us and 1M x 3,072 x 256 (multi-bucket, int8 before)
+// now): 10M docs x 768 bits x 1,024 queries 6.79 -> 3.42 ms, epilogue-bound; 1M x
+// 1,024 x 61 (sign) 507 -> 122 us and 1M x 3,072 x 256 (multi-bucket, int8 before)
 // 790 -> 543 us, both bound by the ring's round trip; FastScan 171,332 x 1,024 x
 // 1,000 1.01 -> 0.83 ms.  The scale factors sit in tensor-memory columns
 // [224, 256) (A) and [480, 512) (B), all bytes 127, past the two accumulators
@@ -55,6 +55,7 @@
 #include <cudaTypedefs.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "ovb_common.cuh"
 #include "ovb_kernels.h"
@@ -107,7 +108,7 @@ struct PT {
   static constexpr int kBStages = PAIR ? 4 : 3;
   // FP4: B stages as deep as the tile's columns leave room for, up to the A slots
   static constexpr int kMaxStages = F4 ? kASlots : kBStages;
-  static constexpr uint32_t kSegCap = PAIR ? 128 : 192;  // kept entries per epilogue warp per tile
+  static constexpr uint32_t kSegCap = F4 ? 96 : PAIR ? 128 : 192;  // kept entries per epilogue warp (per tile)
   static constexpr uint32_t kAStage = kRows * kPKBytes;
   static constexpr uint32_t kBStage = (F4 ? kPF4MaxN / 2 : PAIR ? kPMaxN / 2 : kPMaxN) * kPKBytes;
   static constexpr uint32_t kAccBufs = PAIR ? 2 : 1;
@@ -138,6 +139,9 @@ struct PSmem {
   // pair form: each epilogue warp's 64 column thresholds; FP4: the launch's, two a word
   uint32_t wamin[PAIR ? kPEpiWarps : 1][64];
   alignas(128) uint32_t unit[F4 ? kBiasTile / 4 : 1];  // FP4: the constant tile
+  // FP4, 16-bit sums: docs kept for some of 16 columns, (doc, first query) and the columns' words
+  uint4 raw_words[F4 ? kPEpiWarps : 1][F4 ? 32 : 1][2];
+  uint2 raw_head[F4 ? kPEpiWarps : 1][F4 ? 32 : 1];
   // pair form: the row words of each builder warp's next K-block
   uint4 raw[PAIR ? kPBuildWarps : 1][PAIR ? PT<PAIR, F4>::kItems : 1][PAIR ? 32 : 1];
   uint64_t full_a[PT<PAIR, F4>::kASlots];
@@ -270,6 +274,78 @@ __device__ __forceinline__ int f4_bound16(const TcArgs& a, uint32_t am) {
 // The (biased) integer of an FP4 accumulator.
 __device__ __forceinline__ uint32_t f4_int(const TcArgs& a, uint32_t bits) {
   return (uint32_t)__float2int_rn(__uint_as_float(bits)) + (a.key_kind == 2 ? kHamBias : 0u);
+}
+
+// The list of an epilogue warp of the FP4 form (16-bit sums), held <= kF4List entries (doc,
+// 2^15 + sum - bound | query << 16), -> the candidate rows: every lane's atomics in flight
+// together.  qp: the launch's parameters.  Out of line, as is f4_unpack: the tile loop's
+// instructions then stay in the cache (inlined four times over, 5.1 ms for 3.5).
+constexpr uint32_t kF4List = PT<true, true>::kSegCap;
+struct F4Out {
+  uint32_t *cnt, *f_keys, *f_ids;
+  uint32_t cap, key_kind, n_top, ties;
+};
+__device__ __noinline__ void f4_drain(const F4Out o, const uint32_t* qp, const uint2* list, uint32_t held) {
+  const uint32_t lane = threadIdx.x & 31;
+  TcArgs a{};  // what the key functions read
+  a.key_kind = o.key_kind;
+  a.n_top = o.n_top;
+  __syncwarp();
+  uint32_t pos[kF4List / 32], key[kF4List / 32];
+#pragma unroll
+  for (uint32_t i = 0; i < kF4List / 32; i++) {
+    pos[i] = 0xFFFFFFFFu;
+    if (32 * i + lane >= held) continue;
+    const uint2 en = list[32 * i + lane];
+    const uint32_t q = en.y >> 16;
+    const uint32_t y = (uint32_t)((int)(en.y & 0xFFFFu) - 0x8000 + f4_bound16(a, qp[q])) +
+                       (a.key_kind == 2 ? kHamBias : 0u);
+    key[i] = bm_key_q(a, qp[3 * kPMaxQ + q], y);
+    // (key, doc) <= (thr, tdoc): at the threshold, docs up to the tie bound
+    if (!(o.ties && y == qp[2 * kPMaxQ + q] && en.x > qp[kPMaxQ + q])) pos[i] = atomicAdd(&o.cnt[q], 1u);
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < kF4List / 32; i++) {
+    if (pos[i] >= o.cap) continue;
+    const uint2 en = list[32 * i + lane];
+    const uint64_t at = (uint64_t)(en.y >> 16) * o.cap + pos[i];
+    o.f_keys[at] = key[i];
+    o.f_ids[at] = en.x;
+  }
+  __syncwarp();
+}
+
+// The kept columns of up to 32 docs, a lane a doc: head = (doc, first query), words = the 16
+// columns' 2^15 + sum - bound -> the list; returns its entries.
+__device__ __noinline__ uint32_t f4_unpack(const F4Out o, const uint32_t* qp, const uint4* words, const uint2* head,
+                                           uint2* list, uint32_t n, uint32_t held) {
+  const uint32_t lane = threadIdx.x & 31;
+  __syncwarp();
+  uint32_t hm = 0;  // bit r: column 2 r, bit 16 + r: column 2 r + 1
+  uint2 hd = make_uint2(0, 0);
+  const uint32_t* x = reinterpret_cast<const uint32_t*>(words + 2 * lane);
+  if (lane < n) {
+    hd = head[lane];
+    const uint4 w0 = words[2 * lane], w1 = words[2 * lane + 1];
+    const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+    for (uint32_t r = 0; r < 8; r++) hm |= (w[r] >> (15 - r)) & (0x00010001u << r);
+  }
+  for (uint32_t bal = __ballot_sync(0xFFFFFFFFu, hm != 0); bal; bal = __ballot_sync(0xFFFFFFFFu, hm != 0)) {
+    if (held + __popc(bal) > kF4List) {
+      f4_drain(o, qp, list, held);
+      held = 0;
+    }
+    if (hm) {
+      const uint32_t j = (uint32_t)__ffs(hm) - 1, r = j & 7, odd = j >> 4;
+      list[held + __popc(bal & ((1u << lane) - 1))] =
+          make_uint2(hd.x, (odd ? x[r] >> 16 : x[r] & 0xFFFFu) | ((hd.y + 2 * r + odd) << 16));
+      hm &= hm - 1;
+    }
+    held += __popc(bal);
+  }
+  __syncwarp();
+  return held;
 }
 
 // named barrier 1 over the epilogue warps
@@ -842,14 +918,18 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
       // half: sum >= bound; neither half can borrow), eight of them 16 queries', and
       // one vote says whether any of the warp's 32 docs is kept for them.  Groups of 16
       // columns go round the four warps of a lane quarter.  A warp's accumulator
-      // columns are in registers after one load, and the buffer is released.  Kept
-      // entries stay in the warp's list over the tiles until it is nearly full, then
-      // every lane reserves and writes four at once; docs at the threshold itself are
-      // settled by the tie bound there.  Measured (scan, f32 compares and one atomic in
-      // flight a lane / this): 10M docs x 768 bits x 1,024 queries 5.27 / 3.86 ms, 2M
-      // 1.25 / 1.02, 1M x 1,024 x 1,024 (sign) 0.65 / 0.53, 1M x 1,024 x 61 137 / 131
-      // us.  Slower: a pair of writer warps fed by rings (4.1 ms, and 1.77 at 2M, where
-      // more is kept), two teams of eight warps on alternate tiles (4.5 ms).
+      // columns are in registers after one load, and the buffer is released; the
+      // subtractions and votes of all its groups come first, without a branch.  A doc kept
+      // for some of a group's queries is put aside as it is (the 16 words); 32 of those are
+      // taken apart together (f4_unpack, a lane each) into the warp's list, and a full list
+      // is written with three slot reservations in flight a lane; docs at the threshold
+      // itself are settled by the tie bound there.  Bound by the epilogue's latency
+      // (tensor pipe 50 % busy before the last of this): scan of 10M docs x 768 bits x
+      // 1,024 queries 5.27 ms with f32 compares, a mask bit a query and one reservation
+      // in flight, 3.86 with the 16-bit sums, 3.42 with the rest; 2M 1.25 / 1.02 / 0.80; 1M x
+      // 1,024 x 1,024 (sign) 650 / 525 / 455 us, x 61 137 / 131 / 122.  Without what is kept
+      // (no entries made) it would be 2.59.  Slower: warps of their own to take the lists to
+      // memory (4.1 to 5.9 ms), two teams of eight warps on alternate tiles (4.5).
       uint32_t* am2 = &S.wamin[0][0];
       static_assert(sizeof(S.wamin) >= (kPMaxQ + kPMaxN) * 2, "two bounds a word, past the last tile");
       for (uint32_t i = et; i < (kPMaxQ + kPMaxN) / 2; i += kPEpiThreads) {
@@ -861,33 +941,14 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
       const uint32_t n_grp = nt / 16, part = e >> 2;
       const uint32_t my_grp = n_grp / 4 + (part < n_grp % 4 ? 1 : 0);  // up to 4 groups of this warp
       const uint32_t c0 = 16 * (part * (n_grp / 4) + min(part, n_grp % 4));
-      uint32_t held = 0;  // entries in the list: (doc, 2^15 + sum - bound | query << 16)
-      auto drain = [&]() {
-        __syncwarp();
-        // every lane's atomics in flight together
-        uint32_t pos[kPSegCap / 32], key[kPSegCap / 32];
-#pragma unroll
-        for (uint32_t i = 0; i < kPSegCap / 32; i++) {
-          pos[i] = 0xFFFFFFFFu;
-          if (32 * i + lane >= held) continue;
-          const uint2 en = list[32 * i + lane];
-          const uint32_t q = en.y >> 16;
-          const uint32_t y = (uint32_t)((int)(en.y & 0xFFFFu) - 0x8000 + f4_bound16(a, P_am(q))) +
-                             (a.key_kind == 2 ? kHamBias : 0u);
-          key[i] = bm_key_q(a, P_pop(q), y);
-          // (key, doc) <= (thr, tdoc): at the threshold, docs up to the tie bound
-          if (!(a.thr_pos && y == P_thr(q) && en.x > P_td(q))) pos[i] = atomicAdd(&a.cnt[q], 1u);
-        }
-#pragma unroll
-        for (uint32_t i = 0; i < kPSegCap / 32; i++) {
-          if (pos[i] >= a.cap) continue;
-          const uint2 en = list[32 * i + lane];
-          const uint64_t at = (uint64_t)(en.y >> 16) * a.cap + pos[i];
-          a.f_keys[at] = key[i];
-          a.f_ids[at] = en.x;
-        }
-        __syncwarp();
-        held = 0;
+      uint32_t held = 0;  // entries in the list
+      uint2* raw_head = S.raw_head[e];
+      uint4* raw_words = &S.raw_words[e][0][0];
+      uint32_t n_raw = 0;
+      const F4Out out{a.cnt, a.f_keys, a.f_ids, a.cap, (uint32_t)a.key_kind, (uint32_t)a.n_top, a.thr_pos ? 1u : 0u};
+      auto unpack = [&]() {
+        held = f4_unpack(out, S.qp, raw_words, raw_head, list, n_raw, held);
+        n_raw = 0;
       };
       uint32_t tcount = 0;
       TileCursor tc_;
@@ -896,9 +957,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
         const uint32_t b = tcount % kBufs;
         const uint32_t doc = tc_.dt * 256 + rank * kPRows + row;  // filter: block stride 1
         const uint32_t pass = doc < a.n ? 0x80008000u : 0u;
-        bool ready = false;
-        if (lane == 0) ready = !aborted(S) && mbar_wait_cluster(&S.acc_full[b], (tcount / kBufs) & 1);
-        ready = __shfl_sync(0xFFFFFFFFu, ready, 0);
+        const bool ready = __all_sync(0xFFFFFFFFu, mbar_wait_spin(&S.acc_full[b], (tcount / kBufs) & 1));
         if (!ready) {
           if (lane == 0 && !aborted(S)) raise_abort(S, a.err);
           break;
@@ -910,39 +969,47 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& b_map, const TcArgs
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) arrive_remote(acc_empty0 + 8 * b);  // the columns are in registers
+        // N groups' subtractions and votes first (no branch between them), then the hits
+        auto compare = [&](auto n_const) {
+          constexpr uint32_t N = decltype(n_const)::value;
+          const uint4* bp = reinterpret_cast<const uint4*>(am2 + (q0 + c0) / 2);
+          uint32_t bal[N];
 #pragma unroll
-        for (uint32_t gr = 0; gr < 4; gr++) {
-          if (gr >= my_grp) break;
-          const uint4* bp = reinterpret_cast<const uint4*>(am2 + (q0 + c0) / 2 + 8 * gr);
-          const uint4 b0 = bp[0], b1 = bp[1];
-          const uint32_t bd[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-          uint32_t x[8], any = 0;
+          for (uint32_t gr = 0; gr < N; gr++) {
+            const uint4 b0 = bp[2 * gr], b1 = bp[2 * gr + 1];
+            const uint32_t bd[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            uint32_t any = 0;
 #pragma unroll
-          for (uint32_t r = 0; r < 8; r++) {
-            x[r] = v[8 * gr + r] - bd[r];
-            any |= x[r];
-          }
-          if (!__any_sync(0xFFFFFFFFu, (any & pass) != 0)) continue;
-          uint32_t hm = 0;  // bit r: column 2 r, bit 16 + r: column 2 r + 1
-#pragma unroll
-          for (uint32_t r = 0; r < 8; r++) hm |= (x[r] >> (15 - r)) & (0x00010001u << r);
-          if (!pass) hm = 0;
-          for (uint32_t bal = __ballot_sync(0xFFFFFFFFu, hm != 0); bal; bal = __ballot_sync(0xFFFFFFFFu, hm != 0)) {
-            if (held + __popc(bal) > kPSegCap) drain();
-            if (hm) {
-              const uint32_t j = (uint32_t)__ffs(hm) - 1, odd = j >> 4;
-              const uint32_t y01 = j & 1 ? x[1] : x[0], y23 = j & 1 ? x[3] : x[2], y45 = j & 1 ? x[5] : x[4],
-                             y67 = j & 1 ? x[7] : x[6];
-              const uint32_t y03 = j & 2 ? y23 : y01, y47 = j & 2 ? y67 : y45, w2 = j & 4 ? y47 : y03;
-              const uint32_t q = q0 + c0 + 16 * gr + 2 * (j & 7) + odd;
-              list[held + __popc(bal & lt)] = make_uint2(doc, (odd ? w2 >> 16 : w2 & 0xFFFFu) | (q << 16));
-              hm &= hm - 1;
+            for (uint32_t r = 0; r < 8; r++) {
+              v[8 * gr + r] -= bd[r];
+              any |= v[8 * gr + r];
             }
-            held += __popc(bal);
+            bal[gr] = __ballot_sync(0xFFFFFFFFu, (any & pass) != 0);
           }
-        }
+#pragma unroll
+          for (uint32_t gr = 0; gr < N; gr++) {
+            if (!bal[gr]) continue;
+            if (n_raw + __popc(bal[gr]) > 32) unpack();
+            if (bal[gr] >> lane & 1) {
+              const uint32_t slot = n_raw + __popc(bal[gr] & lt);
+              raw_head[slot] = make_uint2(doc, q0 + c0 + 16 * gr);
+              raw_words[2 * slot] = make_uint4(v[8 * gr], v[8 * gr + 1], v[8 * gr + 2], v[8 * gr + 3]);
+              raw_words[2 * slot + 1] = make_uint4(v[8 * gr + 4], v[8 * gr + 5], v[8 * gr + 6], v[8 * gr + 7]);
+            }
+            n_raw += __popc(bal[gr]);
+          }
+        };
+        if (my_grp == 4)
+          compare(std::integral_constant<uint32_t, 4>());
+        else if (my_grp == 3)
+          compare(std::integral_constant<uint32_t, 3>());
+        else if (my_grp == 2)
+          compare(std::integral_constant<uint32_t, 2>());
+        else if (my_grp == 1)
+          compare(std::integral_constant<uint32_t, 1>());
       }
-      drain();
+      unpack();
+      f4_drain(out, S.qp, list, held);
     } else if constexpr (F4) {
       // FP4 form: the f32 sums are compared with the f32 of each query's integer
       // threshold, read straight from the launch's parameters (a tile stages
