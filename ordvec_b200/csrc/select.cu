@@ -24,6 +24,7 @@ namespace {
 
 constexpr int kSelThreads = 1024;
 constexpr int kHistBins = 2048;
+constexpr uint32_t kSelTies = 256;     // entries of the last bin that are ranked one against another
 constexpr uint64_t kShortRow = 16384;  // rows up to this many keys take the 256-thread form
 constexpr uint32_t kShortCap = 2048;   // ... when k is at most this
 
@@ -59,6 +60,20 @@ __device__ void bitonic_sort(uint64_t* buf, uint32_t len) {
 
 // T threads per row (1024; 256 for rows of at most kShortRow keys, so that
 // several rows share an SM), CAP sorted entries in shared memory.
+//
+// The k-th smallest (key, id) is found by histograms of 2,048 bins that divide the
+// row's own range of keys evenly: the first pass over the row takes its minimum and
+// maximum (keys of at most 11 bits need none), the second the histogram, and where the
+// bin of the k-th entry then holds at most kSelTies entries a third collects what lies
+// below it and ranks the bin's.  A fuller bin is divided again, by keys and, where they
+// are all equal, by ids.  Bound by the passes over the row and the final sort; four loads
+// are in flight a thread, and a histogram of few bins has copies for the lanes.  Fixed
+// digits of 11 bits put most float keys of a row into a few bins (atomics on one
+// address) and took four to seven passes.  All launches of a call, us, then and now:
+// FastScan two-stage of 1,000 queries 146 / 106, multi-bucket 106 / 59, three RankQuant
+// searches of 1,024 / 2,048 / 1,024 queries 808 / 552, Rank of 64 59 / 48; integer keys of a
+// 10M-document bitmap batch (1,024 rows of 39,063 and of 10,000) 298 / 322, with the
+// reranks' 361 / 370.
 template <int T, uint32_t CAP>
 __global__ void __launch_bounds__(T)
     select_rows_kernel(SelectArgs a, uint64_t* gbuf, uint32_t gbuf_stride) {
@@ -67,7 +82,8 @@ __global__ void __launch_bounds__(T)
   __shared__ uint32_t hist[kHistBins];
   __shared__ uint32_t warp_tot[T / 32];
   __shared__ uint64_t sbuf[CAP];
-  __shared__ uint32_t s_bin, s_before, s_in_bin, s_cnt_below, s_cnt_tie;
+  __shared__ uint32_t s_bin, s_before, s_in_bin, s_cnt_below, s_cnt_tie, s_min, s_max;
+  __shared__ uint64_t tbuf[kSelTies];
 
   const uint64_t row = blockIdx.x;
   uint64_t start, n;
@@ -103,101 +119,179 @@ __global__ void __launch_bounds__(T)
 
   uint64_t* buf = (k_eff <= CAP) ? sbuf : gbuf + row * (uint64_t)gbuf_stride;
 
-  // digit schedule: key32 bits [32+key_bits-1, 32], then id bits [id_bits-1, 0]
-  Digit digits[8];
-  int nd = 0;
-  for (int part = 0; part < 2; part++) {
-    uint32_t bits = part == 0 ? a.key_bits : a.id_bits;
-    uint32_t top = (part == 0 ? 32u : 0u) + bits;
-    while (bits > 0) {
-      uint32_t w = bits < 11 ? bits : 11;
-      top -= w;
-      digits[nd++] = Digit{top, w};
-      bits -= w;
-    }
-  }
-
-  uint64_t prefix = 0, fixed = 0;
-  uint32_t need = k_eff;
-  bool take_all = (k_eff == n);
-  for (int d = 0; d < nd && !take_all; d++) {
-    const uint32_t shift = digits[d].shift, width = digits[d].width;
-    const uint32_t nbins = 1u << width;
-    for (uint32_t b = threadIdx.x; b < kHistBins; b += blockDim.x) hist[b] = 0;
-    __syncthreads();
-    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
-      uint64_t key = load_key(keys, ids, i);
-      if ((key & fixed) == prefix) atomicAdd(&hist[(uint32_t)(key >> shift) & (nbins - 1)], 1u);
-    }
-    __syncthreads();
-    // block scan over bins (BPT consecutive bins per thread) to find the bin
-    // holding the need-th key
-    const uint32_t t = threadIdx.x;
-    uint32_t hv[BPT];
-    uint32_t s = 0;
+  // f(key, id) for every entry of the row (id only with want_ids), four loads in flight;
+  // whole warps call f together
+  auto each = [&](bool want_ids, auto&& f) {
+    const uint64_t padded = (n + 31) / 32 * 32;
+    for (uint64_t i0 = threadIdx.x; i0 < padded; i0 += 4 * T) {
+      uint32_t kk[4], ii[4];
 #pragma unroll
-    for (int b = 0; b < BPT; b++) {
-      hv[b] = hist[BPT * t + b];
-      s += hv[b];
-    }
-    uint32_t incl = s;
-    const int lane = t & 31, w = t >> 5;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_tot[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-      uint32_t v = lane < T / 32 ? warp_tot[lane] : 0u, x = v;
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
+      for (uint32_t j = 0; j < 4; j++) {
+        const uint64_t i = i0 + j * T;
+        kk[j] = i < n ? keys[i] : 0u;
+        ii[j] = want_ids && i < n ? (ids ? ids[i] : (uint32_t)i) : 0u;
       }
-      if (lane < T / 32) warp_tot[lane] = x - v;  // exclusive warp offsets
+#pragma unroll
+      for (uint32_t j = 0; j < 4; j++)
+        if (i0 + j * T < padded) f(kk[j], ii[j], i0 + j * T < n);
     }
-    __syncthreads();
-    const uint32_t excl = warp_tot[w] + incl - s;
-    if (excl < need && need <= excl + s) {
-      uint32_t before = excl;
+  };
+  const uint32_t t = threadIdx.x;
+  const int lane = t & 31, w = t >> 5;
+  const bool take_all = k_eff == n;
+  // part 0: keys in [base, base + 2^sh) hold the need-th of the entries not below them;
+  // part 1: so do ids, of the entries whose key is `same`
+  uint32_t part = 0, base = 0, same = 0, sh = 0, need = k_eff;
+  if (!take_all) {
+    uint32_t used = 1u << (a.key_bits < 11 ? a.key_bits : 11);  // bins that can be hit
+    if (a.key_bits > 11) {
+      uint32_t mn = 0xFFFFFFFFu, mx = 0;
+      each(false, [&](uint32_t key, uint32_t, bool in) {
+        mn = in && key < mn ? key : mn;
+        mx = in && key > mx ? key : mx;
+      });
+      mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+      mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+      if (t == 0) {
+        s_min = 0xFFFFFFFFu;
+        s_max = 0;
+      }
+      __syncthreads();
+      if (lane == 0) {
+        atomicMin(&s_min, mn);
+        atomicMax(&s_max, mx);
+      }
+      __syncthreads();
+      base = s_min;
+      const int range_bits = 32 - __clz(s_max - s_min);
+      sh = range_bits > 11 ? range_bits - 11 : 0;
+      used = ((s_max - s_min) >> sh) + 1;
+    }
+    for (;;) {
+      for (uint32_t b = t; b < kHistBins; b += T) hist[b] = 0;
+      __syncthreads();
+      // few bins: 2^copies of each, the lanes in turn, so that equal keys of a warp meet less
+      const uint32_t copies = used <= kHistBins / 4 ? min(31 - __clz(kHistBins / used), 5) : 0;
+      const uint32_t copy = lane & ((1u << copies) - 1);
+      each(part != 0, [&](uint32_t key, uint32_t id, bool in) {
+        const uint32_t x = part ? id : key, bin = (x - base) >> sh;
+        if (in && (!part || key == same) && x >= base && bin < kHistBins) atomicAdd(&hist[bin << copies | copy], 1u);
+      });
+      __syncthreads();
+      if (copies) {  // used <= 512
+        uint32_t sum[2] = {0, 0};
+#pragma unroll
+        for (uint32_t j = 0; j < 2; j++)
+          for (uint32_t c = 0; t + j * T < used && c < 1u << copies; c++)
+            sum[j] += hist[(t + j * T) << copies | ((c + t) & ((1u << copies) - 1))];
+        __syncthreads();
+        for (uint32_t b = t; b < kHistBins; b += T) hist[b] = 0;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < 2; j++)
+          if (t + j * T < used) hist[t + j * T] = sum[j];
+        __syncthreads();
+      }
+      used = kHistBins;
+      // block scan over bins (BPT consecutive bins per thread) to find the bin
+      // holding the need-th entry
+      uint32_t hv[BPT];
+      uint32_t s = 0;
 #pragma unroll
       for (int b = 0; b < BPT; b++) {
-        if (need <= before + hv[b]) {
-          s_bin = BPT * t + b;
-          s_before = before;
-          s_in_bin = hv[b];
-          break;
+        hv[b] = hist[BPT * t + b];
+        s += hv[b];
+      }
+      uint32_t incl = s;
+      for (int o = 1; o < 32; o <<= 1) {
+        uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) warp_tot[w] = incl;
+      __syncthreads();
+      if (w == 0) {
+        uint32_t v = lane < T / 32 ? warp_tot[lane] : 0u, x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+          if (lane >= o) x += y;
         }
-        before += hv[b];
+        if (lane < T / 32) warp_tot[lane] = x - v;  // exclusive warp offsets
+      }
+      __syncthreads();
+      const uint32_t excl = warp_tot[w] + incl - s;
+      if (excl < need && need <= excl + s) {
+        uint32_t before = excl;
+#pragma unroll
+        for (int b = 0; b < BPT; b++) {
+          if (need <= before + hv[b]) {
+            s_bin = BPT * t + b;
+            s_before = before;
+            s_in_bin = hv[b];
+            break;
+          }
+          before += hv[b];
+        }
+      }
+      __syncthreads();
+      need -= s_before;
+      base += s_bin << sh;
+      const uint32_t in_bin = s_in_bin;
+      __syncthreads();
+      if (in_bin == need || in_bin <= kSelTies) break;
+      if (sh) {
+        sh = sh > 11 ? sh - 11 : 0;
+      } else if (!part) {
+        part = 1;
+        same = base;
+        base = 0;
+        sh = a.id_bits > 11 ? a.id_bits - 11 : 0;
+      } else {
+        break;  // equal entries: any of them
       }
     }
-    __syncthreads();
-    need -= s_before;
-    prefix |= (uint64_t)s_bin << shift;
-    fixed |= (uint64_t)(nbins - 1) << shift;
-    if (s_in_bin == need) take_all = true;  // the whole bin is taken
-    __syncthreads();
   }
 
-  // collect: keys strictly below the prefix, then `need` keys inside it
-  if (threadIdx.x == 0) {
+  // collect: what lies below the bin, then the bin's `need` smallest
+  if (t == 0) {
     s_cnt_below = 0;
     s_cnt_tie = 0;
   }
   __syncthreads();
-  const uint32_t below_total = k_eff - need;
-  for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    uint64_t key = load_key(keys, ids, i);
-    uint64_t m = key & fixed;
-    if (m < prefix) {
-      uint32_t slot = atomicAdd(&s_cnt_below, 1u);
-      if (slot < below_total) buf[slot] = key;
-    } else if (m == prefix) {
-      uint32_t tk = atomicAdd(&s_cnt_tie, 1u);
-      if (tk < need) buf[below_total + tk] = key;
+  const uint32_t below_total = take_all ? k_eff : k_eff - need;
+  const bool rank_ties = !take_all && s_in_bin <= kSelTies && s_in_bin != need;
+  uint32_t lt;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+  each(true, [&](uint32_t key, uint32_t id, bool in) {
+    const uint32_t x = part ? id : key;
+    const bool here = !part || key == same;  // the bin's range applies
+    const bool below = in && (take_all || (here ? x < base : key < same));
+    const bool tie = in && !take_all && here && x >= base && (x - base) >> sh == 0;
+    const uint32_t bb = __ballot_sync(0xFFFFFFFFu, below);
+    if (bb) {
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&s_cnt_below, (uint32_t)__popc(bb));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(bb & lt);
+      if (below && at < below_total) buf[at] = ((uint64_t)key << 32) | id;
     }
-  }
+    if (tie) {
+      const uint32_t tk = atomicAdd(&s_cnt_tie, 1u);
+      if (rank_ties)
+        tbuf[tk] = ((uint64_t)key << 32) | id;  // tk < s_in_bin <= kSelTies
+      else if (tk < need)
+        buf[below_total + tk] = ((uint64_t)key << 32) | id;
+    }
+  });
   __syncthreads();
+  if (rank_ties) {
+    const uint32_t c = s_in_bin;
+    if (t < c) {
+      const uint64_t mine = tbuf[t];
+      uint32_t rank = 0;
+      for (uint32_t i = 0; i < c; i++) rank += tbuf[i] < mine || (tbuf[i] == mine && i < t);
+      if (rank < need) buf[below_total + rank] = mine;
+    }
+    __syncthreads();
+  }
   if (!a.unordered) {  // a caller that needs only the set skips the sort
     uint32_t len = 1;
     while (len < k_eff) len <<= 1;
