@@ -294,7 +294,7 @@ def mixed_run(ob, nq: int, steps: int):
     """The mixed-k / mixed-bits batch configuration: N=1,000,000 synthetic docs,
     dim 1024, RankQuant indices at bits 1, 2 and 4 over the same corpus, nq
     queries each with its own bits and k in {10, 50, 100}, one call per step
-    (ovb_rankquant_search_mixed: split-BF16 tensor-core scan + exact FP64
+    (ovb_rankquant_search_mixed: integer tensor-core candidate scan + exact FP64
     rescoring, plans with autotuned tiles and CUDA-graph replay).  Host
     buffers in and out; wall time per call after the first (tuning) call."""
     n, dim, seed = 1_000_000, 1024, 0x0DD5EED3
@@ -330,7 +330,7 @@ def mixed_run(ob, nq: int, steps: int):
     return {"workload": f"N={n} dim={dim} bits {{1,2,4}} k {{10,50,100}}, {nq} mixed queries per call",
             "qps": nq / sec, "s_per_call": sec, "first_call_s": first_s, "calls": reps,
             "split_bf16_tflops_effective": flops / sec / 1e12, "identical_across_calls": same, "plans": plans,
-            "form": "host buffers; split-BF16 tcgen05 scan + exact FP64 rescoring; CUDA-graph replay"}
+            "form": "host buffers; 16-bit fixed-point tcgen05 (s8 planes) candidate scan + exact FP64 rescoring; CUDA-graph replay"}
 
 
 # ------------------------------------------------------ sign -> b=1, plain
@@ -658,7 +658,7 @@ def profile_case(case: str):
                 queries per call (rank_tile_kernel)
       multibucket MultiBucketBitmap(768, 2) N=2M: diagonal-weight top-2000 of 1
                 query per call (multibucket_rows_kernel), 3 calls
-      encode    RankQuant(768, 2).add of 1M docs, twice (rank_encode_kernel)
+      encode    RankQuant(768, 2).add of 1M docs, twice (rank_bins_kernel)
       rerank    Bitmap(768, 192) top-2000 -> RankQuant b=2 top-100 of 1024 queries,
                 N=2M, twice (rerank_tc_kernel, asym_table_kernel rescoring)
     Each search runs more than once so captures can skip the first call."""

@@ -184,9 +184,10 @@ ordvec_status_t ovb_rankquant_search(const ordvec_index_t *rq, const float *quer
 /* The same full search scored by the split-BF16 tensor-core scan (no
  * counterpart in the reference): rank codes exact in BF16, the query split
  * into hi + lo BF16 parts, f32 accumulation; dim must be a multiple of 64.
- * exact = 1 rescores in FP64 every candidate within twice the split error
- * bound of the k-th split score, giving ovb_rankquant_search's results
- * (ovb_rankquant_search itself takes this path for >= 64 queries);
+ * exact = 1 rescores in FP64 every candidate within twice the error bound of
+ * the k-th candidate score, giving ovb_rankquant_search's results (with
+ * 16-bit fixed-point integer candidate scores where they fit, as
+ * ovb_rankquant_search itself does for >= 64 queries);
  * exact = 0 returns the split-BF16 scores and their top-k. */
 ordvec_status_t ovb_rankquant_search_split(const ordvec_index_t *rq, const float *queries,
                                            uint64_t nq, uint64_t k, uint32_t exact,
@@ -234,7 +235,7 @@ ordvec_status_t ovb_rank_search_asymmetric(const ordvec_index_t *rank, const flo
  * call.  Output rows hold k_max entries: row i's first min(k_of_query[i], n)
  * are its top-k (score desc, id asc, the results ovb_rankquant_search gives),
  * the rest (-inf, -1).  Queries are grouped by index; each group on the
- * split-BF16 tensor-core path runs through a plan cached per (index, group
+ * tensor-core candidate path runs through a plan cached per (index, group
  * size, k): its first call tunes the scan's tile shape and records the
  * pipeline as a CUDA graph, later calls replay it (falling back to the exact
  * pipeline when the fixed candidate count is too small for a query).
@@ -295,7 +296,8 @@ ordvec_status_t ovb_two_stage_search_device(const ordvec_index_t *rq,
                                             void *stream);
 /* How the two-stage pipelines rerank (no counterpart in the reference, whose
  * rerank is its asymmetric subset scorer, src/quant.rs:1126-1281):
- *   OVB_RERANK_AUTO       FP64 (the faster form at the measured shapes); with the
+ *   OVB_RERANK_AUTO       FP64's ids and scores (large reranks score candidates in
+ *                         integers first and only the best in FP64); with the
  *                         environment variable OVB_RERANK_TC=1, the split form
  *                         where the shape allows it (dim % 64 == 0,
  *                         16 <= dim*bits/8 <= 256 and a multiple of 16, >= 16

@@ -925,7 +925,8 @@ uint32_t engine_fastscan_full(const Index& fs, const float* d_q, uint64_t nq, ui
 
 // How a two-stage search reranks its uniform candidate rows (me per query,
 // top-ke): the caller's OVB_RERANK_* mode; OVB_RERANK_AUTO takes the FP64
-// per-query tables, measured faster than the exact split-BF16 form at the
+// per-query tables (large ones behind integer scores, use_subset_scores),
+// measured faster than the exact split-BF16 form at the
 // benchmark shapes (N=10M dim 768 b=2, 1,024 x 2,000 candidates: 0.38 vs
 // 0.61 ms; N=171,332 dim 1024: 0.23 vs 0.36 ms), unless OVB_RERANK_TC=1 asks
 // for the split-BF16 tensor-core rerank (eligible shapes, >= 16 queries, rows

@@ -5,12 +5,12 @@
 // the group's largest k and each query's row keeps its own first k (the top-k
 // is a prefix of the top-k_max, ties by id included), padded with (-inf, -1).
 //
-// A group on the split-BF16 tensor-core path whose key matrix fits one chunk
+// A group on the tensor-core candidate path whose key matrix fits one chunk
 // runs through a plan cached per (device, index, rows, queries, k): the plan
 // owns a stream and its buffers.  Its first call runs the exact pipeline
 // (which settles the candidate count kp), times the tensor-core scan at 32,
 // 64 and 128 queries per tile on a slice of the index and keeps the fastest
-// (the autotuner), then captures the whole pipeline -- split, scan, candidate
+// (the autotuner), then captures the whole pipeline -- query operand, scan, candidate
 // select, margin test, FP64 rescoring, final select, result conversion -- as
 // a CUDA graph with the fixed kp.  Later calls copy the queries in, replay the
 // graph and read back the results and the margin flag; if the flag shows kp
