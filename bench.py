@@ -16,8 +16,8 @@ e2e    : the same step through the public C ABI (ovb_two_stage_search) from
          the timed region.
 plain  : one query per call (device pointers), p50/p99 and QPS, and whether its
          top-100 ids equal the batched form's.
-roofline: the dominant kernel, bitmap_pair_kernel (the stage-1 overlap scan as
-         a u8 GEMM on tcgen05), timed by the stage events of every timed step.
+roofline: the dominant kernel, bitmap_fp4_pair_kernel (the stage-1 overlap scan as
+         a GEMM of 0/1 operands on the FP4 tensor cores), timed by the stage events of every timed step.
 cpu_baseline / --impl reference: the oracle's AVX-512 + OpenMP restatement of
          the reference path (Bitmap::top_m_candidates_batched_chunked in groups
          of 8 queries, then the AVX-512 subset rerank), all host threads, on a
@@ -647,7 +647,7 @@ def serving_run(ob, rq, fs, queries, batched_ids, seconds: float, rate_qps: floa
 # ------------------------------------------------------- profiling cases
 def profile_case(case: str):
     """Small single-kernel workloads for ncu captures (no timing, no JSON):
-      bitmap    Bitmap(768, 192) top-2000 of 1024 queries, N=2M (bitmap_pair_kernel)
+      bitmap    Bitmap(768, 192) top-2000 of 1024 queries, N=2M (bitmap_fp4_pair_kernel)
       bitmap10m the same at N=10M (the headline's stage-1 index only, 0.96 GB)
       popc      the 2M index, one query per call (popc_rows_kernel, wide select)
       rank      RankQuant(1024, 2) exact top-100 of 1024 queries, N=1M (rank_tc_kernel)
@@ -896,10 +896,11 @@ def second_stage1_run(ob, torch, dev, rq, s1, name, words_per_doc, d_q, queries,
             "batched_over_plain": nq / (batch_ms * 1e-3) * statistics.mean(plain_ms) * 1e-3,
             "identical_top100_batched_vs_plain": bool(np.array_equal(p_i.view(P, K).cpu().numpy(), ids[:P])),
             "stages_ms": dict(zip(STAGES, st)), "stages_ms_plain": dict(zip(STAGES, st1)),
-            "roofline_batched_scan": {"bound": "tensor", "kernel": "bitmap_pair_kernel (filter epilogue)",
-                                      "achieved": ops / (st[2] * 1e-3) / 1e12, "peak": 2 * bf16_peak,
-                                      "unit": "TOPS (int8)", "frac": ops / (st[2] * 1e-3) / 1e12 / (2 * bf16_peak),
-                                      "peak_source": f"2 x {peak_kind} bf16 dense TFLOP/s (burst)"},
+            "roofline_batched_scan": {"bound": "tensor", "kernel": "bitmap_fp4_pair_kernel (filter epilogue)",
+                                      "achieved": ops / (st[2] * 1e-3) / 1e12, "peak": 4 * bf16_peak,
+                                      "unit": "TOPS (0/1 operands; FP4 e2m1 MMAs)",
+                                      "frac": ops / (st[2] * 1e-3) / 1e12 / (4 * bf16_peak),
+                                      "peak_source": f"4 x {peak_kind} bf16 dense TFLOP/s (burst)"},
             "roofline_plain_scan": {"bound": "hbm", "kernel": "multibucket_rows_kernel",
                                     "achieved": plain_gbs, "peak": hbm_peak, "unit": "GB/s",
                                     "frac": plain_gbs / hbm_peak, "peak_source": f"{peak_kind} HBM copy"}}

@@ -163,8 +163,9 @@ void run_batch(Server& S, const Route& rt, std::vector<ReqPtr>& batch, uint64_t 
 // Grow this worker's device and pinned buffers to a route's largest batch
 // before it serves requests: buffers only grow, and a growth frees the old
 // allocation, which waits for the whole device and would stall the other
-// workers' batches mid-stream.  Both stage-1 forms are exercised (the CUDA-core
-// scan with its key rows below 8 or 32 queries, and tensor-core batches).
+// workers' batches mid-stream.  The largest batch of each form is exercised: row
+// scores (4 queries), the CUDA-core scan with its key rows below 8 or 32 queries, the
+// whole-GPU select (16 rows), full searches below 64, and tensor-core batches.
 // Two-stage routes also run a ragged batch (requests of different candidate
 // counts: one query at k = 10, the rest at k = 100, the default policy's 320
 // and 3,200 candidates), whose CSR offsets, compacted candidate rows and keys
@@ -188,7 +189,7 @@ void warm_route(Server& S, const Route& rt, HostBuf& hq, HostBuf& hs, HostBuf& h
     }
     return r;
   };
-  for (uint64_t nq : {(uint64_t)7, (uint64_t)31, (uint64_t)S.max_batch}) {
+  for (uint64_t nq : {(uint64_t)4, (uint64_t)7, (uint64_t)16, (uint64_t)31, (uint64_t)63, (uint64_t)S.max_batch}) {
     if (nq > S.max_batch) continue;
     std::vector<ReqPtr> batch(1, make(nq, 100));
     run_batch(S, rt, batch, nq, hq, hs, hi, dq, ds, di);
