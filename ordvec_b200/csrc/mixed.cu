@@ -16,6 +16,10 @@
 // graph and read back the results and the margin flag; if the flag shows kp
 // was too small for some query (its result would not be exact), the call
 // reruns the exact pipeline and the plan is captured again with the larger kp.
+// The exact pipeline shares the plan's workspace, so it may also move a buffer the
+// graph holds (its candidate rows are longer than the filter's sample rows, which
+// a chunk that failed the filter's count check needs without a larger kp): a
+// graph is replayed only while no buffer has moved since its capture.
 #include <cmath>
 #include <limits>
 #include <map>
@@ -39,6 +43,7 @@ struct Plan {
   uint32_t qpt = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  uint64_t moves = 0;  // w->moves at the capture
   uint64_t replays = 0;
   bool no_graph = false;  // capture failed once: keep to the exact pipeline
   std::mutex mu;
@@ -132,6 +137,7 @@ void capture(Plan& p) {
   }
   OVB_CUDA(cudaStreamEndCapture(st, &p.graph));
   OVB_CUDA(cudaGraphInstantiate(&p.exec, p.graph, 0));
+  p.moves = w.moves;
 }
 
 // Runs one group through its plan in two phases, so the groups of a mixed
@@ -150,6 +156,7 @@ bool plan_enqueue(Plan& p, const float* h_q, float* h_s, int64_t* h_i) {
   int64_t* di = (int64_t*)p.di.ensure(p.nq * ke * 8);
   uint32_t* hflag = (uint32_t*)p.hflag.ensure(4);
   OVB_CUDA(cudaMemcpyAsync(dq, h_q, p.nq * ix.dim * 4, cudaMemcpyHostToDevice, st));
+  if (p.exec && p.moves != w.moves) p.drop_graph();  // an earlier call failed after moving a buffer
   if (!p.exec) return false;
   OVB_CUDA(cudaGraphLaunch(p.exec, st));
   OVB_CUDA(cudaMemcpyAsync(hflag, p.dflag.p, 4, cudaMemcpyDeviceToHost, st));
@@ -179,8 +186,8 @@ void plan_finish(Plan& p, bool enqueued, float* h_s, int64_t* h_i) {
   launch_keys_to_results(w.out_keys.as<uint32_t>(), w.out_ids.as<uint32_t>(), p.nq * ke, 0, 0, ds, di, st);
   OVB_CUDA(cudaStreamSynchronize(st));
   check_tc_errors(w);
-  const uint64_t kp = std::max<uint64_t>(w.split_kp, ke);
-  if (!p.no_graph && (!p.exec || kp > p.kp)) {
+  const uint64_t kp = std::max(std::max<uint64_t>(w.split_kp, ke), p.kp);
+  if (!p.no_graph && (!p.exec || kp > p.kp || p.moves != w.moves)) {
     p.drop_graph();
     p.kp = kp;
     if (!p.qpt) p.qpt = autotune_tile(p);

@@ -20,11 +20,14 @@ struct ApiError {
 };
 [[noreturn]] inline void fail(ordvec_status_t s, std::string m) { throw ApiError{s, std::move(m)}; }
 
-// Grow-only device allocation.
+// Grow-only device allocation.  moves (may be null) counts the allocations that
+// were freed for larger ones.
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
+  uint64_t* moves = nullptr;
   DevBuf() = default;
+  explicit DevBuf(uint64_t* count) : moves(count) {}
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() {
@@ -32,7 +35,10 @@ struct DevBuf {
   }
   void* ensure(size_t bytes) {
     if (bytes > cap) {
-      if (p) cudaFree(p);
+      if (p) {
+        cudaFree(p);
+        if (moves) ++*moves;
+      }
       p = nullptr;
       cap = 0;
       OVB_CUDA(cudaMalloc(&p, bytes));
@@ -95,25 +101,34 @@ struct Index {
 struct Workspace {
   int device = 0;
   cudaStream_t stream = nullptr;
-  DevBuf q_raw, q_unit, qbits, lut, bias, invq, keys, sel_keys, sel_ids, off, keys2, out_keys,
-      out_ids, scores, ids, scratch, stage, weights, flag;
+  // Buffers that moved to a larger allocation: a graph captured over this workspace
+  // holds freed pointers once this differs from its value at the capture.  Every
+  // buffer counts (Buf has no default constructor).
+  uint64_t moves = 0;
+  struct Buf : DevBuf {
+    Buf(Workspace* w) : DevBuf(&w->moves) {}
+  };
+  Buf q_raw{this}, q_unit{this}, qbits{this}, lut{this}, bias{this}, invq{this}, keys{this},
+      sel_keys{this}, sel_ids{this}, off{this}, keys2{this}, out_keys{this}, out_ids{this},
+      scores{this}, ids{this}, scratch{this}, stage{this}, weights{this}, flag{this};
   // FastScan threshold filter: sample key matrix, per-query thresholds,
   // kept (key, id) rows, their counts and the failure flag
-  DevBuf smp_keys, thr_keys, thr_ids, f_keys, f_ids, f_cnt, f_flag;
+  Buf smp_keys{this}, thr_keys{this}, thr_ids{this}, f_keys{this}, f_ids{this}, f_cnt{this},
+      f_flag{this};
   // split-BF16 rank scan: [hi; lo] query rows and |q|_1
-  DevBuf q_split, q_l1;
+  Buf q_split{this}, q_l1{this};
   // integer score scans: the queries' byte planes and their error bounds
-  DevBuf q_fix, q_bound;
+  Buf q_fix{this}, q_bound{this};
   // bitmap filter on FP4 tensor cores: the query bits as e2m1 nibbles
-  DevBuf q_nib;
+  Buf q_nib{this};
   // split-BF16 rerank: top-kp split keys / ids per query, their FP64 keys, the margin flag
-  DevBuf rr_keys, rr_ids, rr_keys2, rr_flag;
+  Buf rr_keys{this}, rr_ids{this}, rr_keys2{this}, rr_flag{this};
   HostBuf rr_flag_host;
   // how engine_two_stage reranks (OVB_RERANK_* of ordvec_b200.h; 0 = auto)
   uint32_t rerank_mode = 0;
   // per-query candidate counts of a ragged two-stage batch: CSR offsets and rows
   HostBuf off_host;
-  DevBuf csr_ids;
+  Buf csr_ids{this};
   uint64_t split_kp = 0;  // largest candidate count the last exact split search settled on
   bool cand_unordered = false;  // set while a two-stage search selects its stage-1 set
   HostBuf pinned, f_flag_host;
@@ -130,7 +145,7 @@ struct Workspace {
   } sink;
   HostBuf results;  // small results: device-written pinned memory
   // error word of the tensor-core kernels (zeroed once; checked by host APIs)
-  DevBuf tc_err;
+  Buf tc_err{this};
   bool tc_used = false;
   uint32_t* tc_err_word(cudaStream_t st) {
     if (!tc_err.p) {
