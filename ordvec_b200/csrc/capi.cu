@@ -91,15 +91,17 @@ ordvec_index_info_t info_for(const Index& ix) {
   return info;
 }
 
-// Grow the device code buffer to hold `rows`, keeping existing rows.
-void grow_codes(Index& ix, uint64_t rows) {
+// Grow the device code buffer to hold `rows`, keeping existing rows.  All on the
+// stream of the encoder that follows: it is non-blocking, so nothing orders it
+// behind work on the default stream.
+void grow_codes(Index& ix, uint64_t rows, cudaStream_t st) {
   const uint64_t need = ix.device_bytes(rows), have = ix.device_bytes(ix.n);
   if (need <= ix.codes.cap) return;
   void* p = nullptr;
   uint64_t cap = need > ix.codes.cap + ix.codes.cap / 2 ? need : ix.codes.cap + ix.codes.cap / 2;
   OVB_CUDA(cudaMalloc(&p, cap));
-  if (ix.kind == OVB_INDEX_KIND_FASTSCAN) OVB_CUDA(cudaMemset(p, 0, cap));
-  if (have) OVB_CUDA(cudaMemcpy(p, ix.codes.p, have, cudaMemcpyDeviceToDevice));
+  if (ix.kind == OVB_INDEX_KIND_FASTSCAN) OVB_CUDA(cudaMemsetAsync(p, 0, cap, st));
+  if (have) OVB_CUDA(cudaMemcpyAsync(p, ix.codes.p, have, cudaMemcpyDeviceToDevice, st));
   if (ix.codes.p) cudaFree(ix.codes.p);
   ix.codes.p = p;
   ix.codes.cap = cap;
@@ -123,7 +125,7 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, b
          "FastScan v1: incremental add() not supported (block-32 layout); construct a new index");
   if (ix.kind != OVB_INDEX_KIND_SIGN_BITMAP && ix.dim > kMaxDeviceRankDim)
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "device rank transform supports dim <= 16384");
-  grow_codes(ix, ix.n + n);
+  grow_codes(ix, ix.n + n, w.stream);
   uint32_t *flag = nullptr, *h = nullptr;
   if (check) {
     flag = (uint32_t*)w.flag.ensure(4);
@@ -136,7 +138,10 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, b
   OVB_CUDA(cudaStreamSynchronize(w.stream));
   if (check && *h) {
     // FastScan's last block pads with zeros: a refused add leaves none of its rows there
-    if (ix.kind == OVB_INDEX_KIND_FASTSCAN) OVB_CUDA(cudaMemset(ix.codes.p, 0, ix.codes.cap));
+    if (ix.kind == OVB_INDEX_KIND_FASTSCAN) {
+      OVB_CUDA(cudaMemsetAsync(ix.codes.p, 0, ix.codes.cap, w.stream));
+      OVB_CUDA(cudaStreamSynchronize(w.stream));
+    }
     fail(ORDVEC_STATUS_BAD_ARGUMENT, "ordvec: input contains non-finite (NaN or +-Inf) values");
   }
   ix.n += n;
@@ -635,16 +640,10 @@ ordvec_status_t ovb_index_add(ordvec_index_t* index, const float* vectors, uint6
       OVB_CUDA(cudaMemcpyAsync(d, vectors + r0 * ix.dim, rn * ix.dim * 4, cudaMemcpyHostToDevice, w.stream));
       if (ix.kind == OVB_INDEX_KIND_FASTSCAN && r0 == 0 && rn < n) {
         // FastScan is single-shot: stage the whole corpus through device memory
-        float* all = nullptr;
-        OVB_CUDA(cudaMalloc(&all, n * ix.dim * 4));
-        OVB_CUDA(cudaMemcpy(all, vectors, n * ix.dim * 4, cudaMemcpyHostToDevice));
-        try {
-          add_device_rows(ix, all, n, w);
-        } catch (...) {
-          cudaFree(all);
-          throw;
-        }
-        cudaFree(all);
+        DevBuf all;
+        all.ensure(n * ix.dim * 4);
+        OVB_CUDA(cudaMemcpyAsync(all.p, vectors, n * ix.dim * 4, cudaMemcpyHostToDevice, w.stream));
+        add_device_rows(ix, all.as<float>(), n, w);
         return;
       }
       add_device_rows(ix, d, rn, w);
