@@ -91,20 +91,34 @@ ordvec_index_info_t info_for(const Index& ix) {
   return info;
 }
 
-// Grow the device code buffer to hold `rows`, keeping existing rows.  All on the
-// stream of the encoder that follows: it is non-blocking, so nothing orders it
-// behind work on the default stream.
-void grow_codes(Index& ix, uint64_t rows, cudaStream_t st) {
+// Where the first `rows` rows of ix go: its own code buffer, or, where that is too
+// small, `fresh` with a copy of its rows, which the index takes over by adopt_codes.
+// All on the stream of the encoder that follows: it is non-blocking, so nothing
+// orders it behind work on the default stream.
+void* grown_codes(const Index& ix, uint64_t rows, DevBuf& fresh, cudaStream_t st) {
   const uint64_t need = ix.device_bytes(rows), have = ix.device_bytes(ix.n);
-  if (need <= ix.codes.cap) return;
-  void* p = nullptr;
-  uint64_t cap = need > ix.codes.cap + ix.codes.cap / 2 ? need : ix.codes.cap + ix.codes.cap / 2;
-  OVB_CUDA(cudaMalloc(&p, cap));
-  if (ix.kind == OVB_INDEX_KIND_FASTSCAN) OVB_CUDA(cudaMemsetAsync(p, 0, cap, st));
-  if (have) OVB_CUDA(cudaMemcpyAsync(p, ix.codes.p, have, cudaMemcpyDeviceToDevice, st));
-  if (ix.codes.p) cudaFree(ix.codes.p);
-  ix.codes.p = p;
-  ix.codes.cap = cap;
+  if (need <= ix.codes.cap) return ix.codes.p;
+  fresh.ensure(std::max<uint64_t>(need, ix.codes.cap + ix.codes.cap / 2));
+  if (ix.kind == OVB_INDEX_KIND_FASTSCAN) OVB_CUDA(cudaMemsetAsync(fresh.p, 0, fresh.cap, st));
+  if (have) OVB_CUDA(cudaMemcpyAsync(fresh.p, ix.codes.p, have, cudaMemcpyDeviceToDevice, st));
+  return fresh.p;
+}
+
+void adopt_codes(Index& ix, DevBuf& fresh) {
+  if (!fresh.p) return;
+  std::swap(ix.codes.p, fresh.p);
+  std::swap(ix.codes.cap, fresh.cap);
+}
+
+// Refuses device rows that are not finite.
+void need_finite_rows(const Index& ix, const float* d_vecs, uint64_t n, Workspace& w) {
+  uint32_t* flag = (uint32_t*)w.flag.ensure(4);
+  uint32_t* h = (uint32_t*)w.pinned.ensure(4);
+  OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
+  launch_finite_flag(d_vecs, n * ix.dim, flag, w.stream);
+  OVB_CUDA(cudaMemcpyAsync(h, flag, 4, cudaMemcpyDeviceToHost, w.stream));
+  OVB_CUDA(cudaStreamSynchronize(w.stream));
+  if (*h) fail(ORDVEC_STATUS_BAD_ARGUMENT, "ordvec: input contains non-finite (NaN or +-Inf) values");
 }
 
 bool accepts_rows(const Index& ix, uint64_t n) {
@@ -112,11 +126,13 @@ bool accepts_rows(const Index& ix, uint64_t n) {
          !(ix.kind != OVB_INDEX_KIND_SIGN_BITMAP && ix.dim > kMaxDeviceRankDim);
 }
 
-// Appends n device rows.  With check, a row that is not finite refuses the add:
-// the encoders look at every value anyway, so they raise the flag, and the
-// rows they wrote lie past the index's end until ix.n moves.
+// Appends n device rows.  With check, rows that are not finite refuse the add, before
+// any other reason does: the encoders look at every value anyway, so they raise the
+// flag, and what they wrote lies past the index's end or in a buffer that it does not
+// take over.  Without room for that buffer the rows are looked at on their own.
 void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, bool check = false) {
   if (!n) return;
+  if (check && !accepts_rows(ix, n)) need_finite_rows(ix, d_vecs, n, w);
   if (ix.n + n > kMaxVectors)
     fail(ORDVEC_STATUS_BAD_ARGUMENT, "index would exceed MAX_VECTORS (67108864); had " + std::to_string(ix.n) +
                                          ", adding " + std::to_string(n));
@@ -125,25 +141,34 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, b
          "FastScan v1: incremental add() not supported (block-32 layout); construct a new index");
   if (ix.kind != OVB_INDEX_KIND_SIGN_BITMAP && ix.dim > kMaxDeviceRankDim)
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "device rank transform supports dim <= 16384");
-  grow_codes(ix, ix.n + n, w.stream);
   uint32_t *flag = nullptr, *h = nullptr;
   if (check) {
     flag = (uint32_t*)w.flag.ensure(4);
     h = (uint32_t*)w.pinned.ensure(4);
     OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
   }
-  launch_encode((int)encode_kind(ix.kind), d_vecs, n, ix.dim, ix.bits, ix.n_top, ix.pairs_pad, ix.codes.p, ix.n,
-                flag, w.stream);
+  DevBuf fresh;
+  void* codes;
+  try {
+    codes = grown_codes(ix, ix.n + n, fresh, w.stream);
+  } catch (const CudaError&) {
+    cudaGetLastError();
+    if (check) need_finite_rows(ix, d_vecs, n, w);
+    throw;
+  }
+  launch_encode((int)encode_kind(ix.kind), d_vecs, n, ix.dim, ix.bits, ix.n_top, ix.pairs_pad, codes, ix.n, flag,
+                w.stream);
   if (check) OVB_CUDA(cudaMemcpyAsync(h, flag, 4, cudaMemcpyDeviceToHost, w.stream));
   OVB_CUDA(cudaStreamSynchronize(w.stream));
   if (check && *h) {
     // FastScan's last block pads with zeros: a refused add leaves none of its rows there
-    if (ix.kind == OVB_INDEX_KIND_FASTSCAN) {
+    if (ix.kind == OVB_INDEX_KIND_FASTSCAN && !fresh.p) {
       OVB_CUDA(cudaMemsetAsync(ix.codes.p, 0, ix.codes.cap, w.stream));
       OVB_CUDA(cudaStreamSynchronize(w.stream));
     }
     fail(ORDVEC_STATUS_BAD_ARGUMENT, "ordvec: input contains non-finite (NaN or +-Inf) values");
   }
+  adopt_codes(ix, fresh);
   ix.n += n;
 }
 
@@ -658,15 +683,6 @@ ordvec_status_t ovb_index_add_device(ordvec_index_t* index, const float* d_vecto
     if (n && !d_vectors) fail(ORDVEC_STATUS_NULL_POINTER, "vectors pointer is NULL");
     if (!n) return;
     Workspace& w = workspace();
-    if (!accepts_rows(ix, n)) {  // non-finite input is reported before the other refusals
-      uint32_t* flag = (uint32_t*)w.flag.ensure(4);
-      uint32_t* h = (uint32_t*)w.pinned.ensure(4);
-      OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
-      launch_finite_flag(d_vectors, n * ix.dim, flag, w.stream);
-      OVB_CUDA(cudaMemcpyAsync(h, flag, 4, cudaMemcpyDeviceToHost, w.stream));
-      OVB_CUDA(cudaStreamSynchronize(w.stream));
-      if (*h) fail(ORDVEC_STATUS_BAD_ARGUMENT, "ordvec: input contains non-finite (NaN or +-Inf) values");
-    }
     add_device_rows(ix, d_vectors, n, w, true);
   });
 }
