@@ -749,6 +749,7 @@ void launch_score(ScArgs a, const ScoreOperand& b, uint64_t q0, uint64_t qn, cud
   a.nqt = b.nqt;
   a.n_kb = b.k_bytes / 128;
   const uint32_t nt = C::kPlanes * b.nqt;
+  if (nt % kPairI8StepN) throw std::invalid_argument(std::string(what) + ": bad query tile");
   const uint64_t q_tiles = (qn + b.nqt - 1) / b.nqt, rows = q_tiles * nt;
   const CUtensorMap b_map =
       byte_map((const uint8_t*)b.rows + q0 / b.nqt * nt * (uint64_t)b.k_bytes, b.k_bytes, rows, nt / 2, what);
@@ -804,10 +805,11 @@ ScArgs score_args(const void* rows, uint64_t n, uint32_t dim, uint32_t src) {
   return a;
 }
 
-// queries per tile: the batch rounded up to 16, balanced over tiles of at most `most`
-uint32_t tile_queries(uint64_t nq, uint32_t most) {
+// queries per tile: the batch rounded up to `step`, balanced over tiles of at most `most`
+// (a multiple of it)
+uint32_t tile_queries(uint64_t nq, uint32_t most, uint32_t step) {
   const uint64_t tiles = (nq + most - 1) / most;
-  return (uint32_t)(((nq + tiles - 1) / tiles + 15) / 16 * 16);
+  return (uint32_t)(((nq + tiles - 1) / tiles + step - 1) / step * step);
 }
 
 }  // namespace
@@ -823,7 +825,8 @@ bool score_rank_eligible(uint32_t dim) { return dim % 8 == 0 && dim >= 64 && dim
 ScoreOperand score_operand(uint32_t src, uint64_t nq, uint32_t dim, uint32_t q_per_tile) {
   ScoreOperand b{};
   const bool rank = src == 16;
-  b.nqt = tile_queries(nq, rank ? 64 : q_per_tile ? std::min(q_per_tile, 128u) : 128);
+  // N = planes x nqt is a multiple of kPairI8StepN
+  b.nqt = rank ? tile_queries(nq, 64, 32) : tile_queries(nq, q_per_tile ? std::min(q_per_tile, 128u) : 128, 16);
   b.k_bytes = ((rank ? 2 : 1) * dim + 127) / 128 * 128;
   b.planes = rank ? 3 : 2;
   b.bytes = (nq + b.nqt - 1) / b.nqt * b.nqt * b.planes * (uint64_t)b.k_bytes;

@@ -1515,7 +1515,9 @@ void launch_tc_pair(TcArgs a, const uint8_t* b_rows, cudaStream_t stream, bool p
     const uint64_t qt = (a.nq + tile_n - 1) / tile_n;
     a.nt = (uint32_t)(((a.nq + qt - 1) / qt + 15) / 16 * 16);
   } else {
-    a.nt = a.nq >= kPMaxN ? kPMaxN : (uint32_t)((a.nq + 15) / 16 * 16);  // a multiple of 16 in [16, 256]
+    // a multiple of 32 across the pair, of 16 on one CTA, up to 256
+    const uint32_t step = pair ? kPairI8StepN : 16;
+    a.nt = a.nq >= kPMaxN ? kPMaxN : (uint32_t)((a.nq + step - 1) / step * step);
   }
   CUtensorMap map;
   cuuint64_t gdim[2] = {(cuuint64_t)k_bytes, (cuuint64_t)a.nq};

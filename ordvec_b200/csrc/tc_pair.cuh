@@ -42,6 +42,9 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
       : "memory");
 }
 
+// N of an integer MMA across the pair (M = 256): a multiple of this, up to 256
+constexpr uint32_t kPairI8StepN = 32;
+
 __device__ __forceinline__ void mma_i8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
