@@ -15,6 +15,11 @@
 // then gathers the k winners and a bitonic sort orders them.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+#include <cstdlib>
+#include <map>
+#include <mutex>
+
 #include "ovb_common.cuh"
 #include "ovb_kernels.h"
 
@@ -560,7 +565,6 @@ constexpr uint32_t kGridRows = 16;
 constexpr uint64_t kGridMinN = 32768;
 constexpr int kGridThreads = 512;
 constexpr uint32_t kGridSlice = 4096;   // keys a CTA takes before more CTAs join
-constexpr uint32_t kGridCtas = 148;     // all CTAs of a launch are resident at once
 constexpr uint32_t kGridDigits = 6;     // 32 key bits and 32 id bits, 11 at a time
 constexpr size_t kGridStageBytes = 176 * 1024;
 
@@ -821,25 +825,59 @@ __global__ void __launch_bounds__(kGridThreads) grid_select_kernel(SelectArgs a,
   }
 }
 
-bool use_select_grid(const SelectArgs& a, uint64_t rows, const uint64_t* scratch) {
-  return scratch && !a.row_off && !a.row_len && rows <= kGridRows && a.n >= kGridMinN && a.n < (1ull << 32) &&
-         a.k >= 1 && a.k <= kSelectSmemCap;
+// CTAs a launch may have, all resident at once: one an SM of the current device (a
+// partition has fewer than the whole chip's 148), 0 where it takes no cooperative
+// launch.  OVB_SELECT_CTAS lowers it.
+uint32_t grid_ctas() {
+  static std::mutex mu;
+  static std::map<int, uint32_t> cached;
+  int dev = 0;
+  OVB_CUDA(cudaGetDevice(&dev));
+  uint32_t most;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = cached.find(dev);
+    if (it == cached.end()) {
+      int coop = 0, sms = 0, per_sm = 0;
+      OVB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+      OVB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      allow_dynamic_smem(grid_select_kernel);
+      OVB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_select_kernel, kGridThreads, kGridStageBytes));
+      it = cached.emplace(dev, coop && per_sm > 0 ? (uint32_t)sms : 0u).first;
+    }
+    most = it->second;
+  }
+  if (const char* e = getenv("OVB_SELECT_CTAS")) most = std::min<uint32_t>(most, (uint32_t)strtoul(e, nullptr, 10));
+  return most;
 }
 
-void launch_select_grid(const SelectArgs& a, uint64_t rows, uint64_t* scratch, cudaStream_t stream) {
+bool use_select_grid(const SelectArgs& a, uint64_t rows, const uint64_t* scratch) {
+  return scratch && !a.row_off && !a.row_len && rows <= kGridRows && a.n >= kGridMinN && a.n < (1ull << 32) &&
+         a.k >= 1 && a.k <= kSelectSmemCap && rows <= grid_ctas();
+}
+
+// False when the launch was refused for its size (a stream that may use only some of
+// the SMs): the caller takes another form.
+bool launch_select_grid(const SelectArgs& a, uint64_t rows, uint64_t* scratch, cudaStream_t stream) {
   const GridScratch w = grid_scratch(scratch, rows);
   OVB_CUDA(cudaMemsetAsync(scratch, 0, grid_zero_bytes(rows), stream));
   uint64_t ctas = (a.n + kGridSlice - 1) / kGridSlice;
-  if (ctas > kGridCtas / rows) ctas = kGridCtas / rows;
+  ctas = std::min<uint64_t>(ctas, grid_ctas() / rows);
   const uint64_t per = (a.n + ctas - 1) / ctas, bytes = per * (a.ids ? 8 : 4);
   uint32_t stage = bytes <= kGridStageBytes ? 1u : 0u, c32 = (uint32_t)ctas;
   allow_dynamic_smem(grid_select_kernel);
   SelectArgs args = a;
   GridScratch ws = w;
   void* p[] = {&args, &ws, &c32, &stage};
-  OVB_CUDA(cudaLaunchCooperativeKernel((const void*)grid_select_kernel, dim3((unsigned)(rows * ctas)),
-                                       dim3(kGridThreads), p, stage ? (size_t)bytes : 0, stream));
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)grid_select_kernel, dim3((unsigned)(rows * ctas)),
+                                                    dim3(kGridThreads), p, stage ? (size_t)bytes : 0, stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return false;
+  }
+  OVB_CUDA(e);
   launched();
+  return true;
 }
 
 }  // namespace
@@ -868,8 +906,7 @@ void launch_select_rows(const SelectArgs& a, uint64_t rows, uint64_t* scratch,
       launch_keys_to_results(a.out_keys, a.out_ids, rows * a.k, a.res_mode, a.res_n_top, a.res_scores, a.res_ids,
                              stream, a.err_src, a.err_dst, a.gate);
   };
-  if (select_takes_grid(a, rows, scratch)) {
-    launch_select_grid(a, rows, scratch, stream);
+  if (select_takes_grid(a, rows, scratch) && launch_select_grid(a, rows, scratch, stream)) {
     results();
     return;
   }
