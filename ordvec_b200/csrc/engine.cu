@@ -37,9 +37,9 @@ void select_rows(Workspace& w, const uint32_t* keys, const uint32_t* ids, const 
                  uint64_t ld, uint64_t n, uint64_t rows, uint32_t k, uint32_t key_bits,
                  uint32_t id_bits, uint32_t* out_keys, uint32_t* out_ids, cudaStream_t st,
                  const uint32_t* row_len = nullptr, bool ordered = true, bool final = false,
-                 const uint32_t* gate = nullptr) {
+                 const Redo& redo = Redo()) {
   SelectArgs a{keys, ids, row_off, ld, n, k, key_bits, id_bits, out_keys, out_ids, row_len, ordered ? 0u : 1u};
-  a.gate = gate;
+  a.redo = redo;
   if (final && w.sink.scores) {  // the rows' place in the results is their place in w.out_keys
     const uint64_t at = out_keys - w.out_keys.as<uint32_t>();
     a.res_scores = w.sink.scores + at;
@@ -59,12 +59,18 @@ void select_rows(Workspace& w, const uint32_t* keys, const uint32_t* ids, const 
   launch_select_rows(a, rows, scratch, st);
 }
 
-// scan(q0, qn, keys) writes keys[qn][n]; rows are selected into out[nq][k].  gate (may
-// be null; scan's launches take the same): nothing happens when *gate is 0.
+// A list of nq queries in `buf`, emptied by the preparation of their candidate scores.
+Redo redo_list(DevBuf& buf, uint64_t nq) {
+  uint32_t* p = (uint32_t*)buf.ensure((1 + 2 * nq) * 4);
+  return Redo{p, p + 1, p + 1 + nq, 0, (uint32_t)nq};
+}
+
+// scan(q0, qn, keys, redo) writes keys[qn][n]; rows are selected into out[nq][k].  With a
+// redo list: of its queries only (scan's launches take the chunk's part).
 template <class F>
 void full_scan_select(Workspace& w, uint64_t nq, uint64_t n, uint32_t k, uint32_t key_bits,
                       uint32_t* out_keys, uint32_t* out_ids, cudaStream_t st, F&& scan,
-                      const uint32_t* gate = nullptr) {
+                      const Redo& redo = Redo()) {
   const bool final = out_keys >= w.out_keys.as<uint32_t>() &&
                      out_keys < (uint32_t*)((char*)w.out_keys.p + w.out_keys.cap);  // else stage-1 candidates
   const uint64_t per_q = n * 4;
@@ -75,11 +81,14 @@ void full_scan_select(Workspace& w, uint64_t nq, uint64_t n, uint32_t k, uint32_
   const uint32_t id_bits = bits_for(n - 1);
   for (uint64_t q0 = 0; q0 < nq; q0 += qc) {
     const uint64_t qn = nq - q0 < qc ? nq - q0 : qc;
-    scan(q0, qn, keys);
-    if (!gate) w.mark(st, 2);
+    Redo part = redo;
+    part.first += (uint32_t)q0;
+    part.count = (uint32_t)qn;
+    scan(q0, qn, keys, part);
+    if (!redo.word) w.mark(st, 2);
     select_rows(w, keys, nullptr, nullptr, n, n, qn, k, key_bits, id_bits, out_keys + q0 * k,
-                out_ids + q0 * k, st, nullptr, !w.cand_unordered, final, gate);
-    if (!gate) w.mark(st, 3);
+                out_ids + q0 * k, st, nullptr, !w.cand_unordered, final, part);
+    if (!redo.word) w.mark(st, 3);
   }
 }
 
@@ -180,7 +189,7 @@ void filtered_select(Workspace& w, uint64_t n, uint64_t nq, uint32_t me, const F
     OVB_CUDA(cudaMemsetAsync(cnt, 0, qn * 4, st));
     OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
     filter(q0, qn, tk + (fp.r - 1), ti + (fp.r - 1), cnt, fk, fi);
-    launch_filter_check(cnt, qn, me, fp.cap, flag, st);
+    launch_filter_check(cnt, qn, me, fp.cap, Redo{flag}, st);
     OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
     OVB_CUDA(cudaStreamSynchronize(st));
     if (*flag_h) {
@@ -227,7 +236,7 @@ void bitmap_tc_candidates(const Index& s1, const uint64_t* qb, uint32_t qpv, uin
   uint32_t* err = w.tc_err_word(st);
   auto dense = [&](uint64_t qa, uint64_t qn) {
     full_scan_select(w, qn, n, me, key_bits, sk + qa * me, si + qa * me, st,
-                     [&](uint64_t q0, uint64_t qm, uint32_t* keys) {
+                     [&](uint64_t q0, uint64_t qm, uint32_t* keys, const Redo&) {
                        launch_bitmap_scan_tc(words, n, qpv, key_kind, s1.n_top, qpop ? qpop + qa + q0 : nullptr,
                                              qx + (qa + q0) * row, qm, 1, keys, n, err, st);
                      });
@@ -329,12 +338,12 @@ struct CandScores {
   float* l1 = nullptr;
   CandScores(const Index& ix, float inv, bool half, uint32_t qpt)
       : rq(ix), inv_norm(inv), fixed(score_rankquant_eligible(ix.dim, ix.bits)), half_steps(half), q_per_tile(qpt) {}
-  void prepare(const float* qu, uint64_t qn, Workspace& w, cudaStream_t st) {
+  void prepare(const float* qu, uint64_t qn, Workspace& w, cudaStream_t st, const Redo& list = Redo()) {
     if (fixed) {
       op = score_operand(rq.bits, qn, rq.dim, q_per_tile);
       op.rows = w.q_fix.ensure(op.bytes);
       bound = (double*)w.q_bound.ensure(qn * 16);
-      launch_fix_rankquant(qu, qn, rq.dim, rq.bits, half_steps, op, bound, st);
+      launch_fix_rankquant(qu, qn, rq.dim, rq.bits, half_steps, op, bound, list, st);
     } else {
       qs = (uint16_t*)w.q_split.ensure(qn * 2 * rq.dim * 2);
       l1 = (float*)w.q_l1.ensure(qn * 4);
@@ -357,11 +366,11 @@ struct CandScores {
       launch_rank_filter_tc(codes, rq.n, rq.dim, rq.bits, qs, qn, inv_norm, thr, thr_stride, cnt, cap, fk, fi,
                             q_per_tile, err, st);
   }
-  void margin(const uint32_t* sel, uint64_t qn, uint32_t kp, uint32_t ke, uint32_t* flag, cudaStream_t st) const {
+  void margin(const uint32_t* sel, uint64_t qn, uint32_t kp, uint32_t ke, const Redo& failed, cudaStream_t st) const {
     if (fixed)
-      launch_score_margin(sel, qn, kp, ke, bound, rq.bits, flag, st);
+      launch_score_margin(sel, qn, kp, ke, bound, rq.bits, failed, st);
     else
-      launch_split_margin(sel, qn, kp, ke, l1, split_error_bound(rq.dim, rq.bits, inv_norm), flag, st);
+      launch_split_margin(sel, qn, kp, ke, l1, split_error_bound(rq.dim, rq.bits, inv_norm), failed, st);
   }
 };
 
@@ -369,14 +378,14 @@ struct CandScores {
 // synchronisation, graph-capturable): sample scan, each query's r-th sample
 // key as threshold, filtered scan, top-kp of the kept docs by candidate score,
 // margin test, exact rescoring of the kp (rescore(candidate ids) -> keys), top-ke
-// into out_keys / out_ids.  *d_flag |= 1 when some query kept fewer than kp or
-// more than cap docs, or its kp-th candidate score is within the error bounds of
-// its k-th: the result is then not known to be exact and the caller redoes the
-// rows.  Kept sets are prefixes of the candidate order, so their top-kp is the
+// into out_keys / out_ids.  `failed` marks a query that kept fewer than kp or
+// more than cap docs, or whose kp-th candidate score is within the error bounds of
+// its k-th: its result is then not known to be exact and the caller redoes the
+// row.  Kept sets are prefixes of the candidate order, so their top-kp is the
 // whole index's.
 template <class Scores, class Rescore>
 static void filtered_candidates(const Scores& sc, uint64_t n, uint64_t qn, uint32_t ke, uint32_t kp,
-                                const FilterPlan& fp, uint32_t* d_flag, uint32_t* out_keys, uint32_t* out_ids,
+                                const FilterPlan& fp, const Redo& failed, uint32_t* out_keys, uint32_t* out_ids,
                                 Workspace& w, cudaStream_t st, Rescore&& rescore) {
   const uint32_t id_bits = bits_for(n - 1);
   uint32_t* err = w.tc_err_word(st);
@@ -391,13 +400,13 @@ static void filtered_candidates(const Scores& sc, uint64_t n, uint64_t qn, uint3
   uint32_t* fi = (uint32_t*)w.f_ids.ensure(qn * fp.cap * 4);
   OVB_CUDA(cudaMemsetAsync(cnt, 0, qn * 4, st));
   sc.filter(qn, tk + (fp.r - 1), fp.r, cnt, fp.cap, fk, fi, err, st);
-  launch_filter_check(cnt, qn, kp, fp.cap, d_flag, st);
+  launch_filter_check(cnt, qn, kp, fp.cap, failed, st);
   w.mark(st, 2);
   uint32_t* ck = (uint32_t*)w.sel_keys.ensure(qn * kp * 4);
   uint32_t* ci = (uint32_t*)w.sel_ids.ensure(qn * kp * 4);
   select_rows(w, fk, fi, nullptr, fp.cap, fp.cap, qn, kp, 32, id_bits, ck, ci, st, cnt);
   launch_clamp_ids(ci, qn * kp, (uint32_t)n, st);  // a row that kept < kp docs ends in sentinels
-  sc.margin(ck, qn, kp, ke, d_flag, st);
+  sc.margin(ck, qn, kp, ke, failed, st);
   w.mark(st, 3);
   uint32_t* k2 = (uint32_t*)w.keys2.ensure(qn * kp * 4);
   rescore(ci, k2);
@@ -413,12 +422,12 @@ static void rescore_rankquant(const Index& rq, const float* qu, float inv_norm, 
 }
 
 // The end of a candidate pipeline outside the filtered form: margin test of the kp
-// candidates ck / ci of each query (*d_flag |= 1: the result is not known to be exact),
+// candidates ck / ci of each query (`failed` marks those whose result is not known to be exact),
 // FP64 rescoring, top-ke into w.out_keys / out_ids.
 static void rescored_top_k(const CandScores& sc, const Index& rq, const float* qu, float inv_norm, uint64_t nq,
-                           uint32_t kp, uint32_t ke, const uint32_t* ck, const uint32_t* ci, uint32_t* d_flag,
+                           uint32_t kp, uint32_t ke, const uint32_t* ck, const uint32_t* ci, const Redo& failed,
                            Workspace& w, cudaStream_t st) {
-  sc.margin(ck, nq, kp, ke, d_flag, st);
+  sc.margin(ck, nq, kp, ke, failed, st);
   uint32_t* k2 = (uint32_t*)w.rr_keys2.ensure(nq * kp * 4);
   rescore_rankquant(rq, qu, inv_norm, nq, kp, ci, k2, st);
   select_rows(w, k2, ci, nullptr, kp, kp, nq, ke, 32, bits_for(rq.n - 1), w.out_keys.as<uint32_t>(),
@@ -458,7 +467,7 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, b
       const uint64_t qn = nq - q0 < fc ? nq - q0 : fc;
       OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
       sc.prepare(qu + q0 * dim, qn, w, st);
-      filtered_candidates(sc, n, qn, ke, (uint32_t)kp0, fp, flag, ok + q0 * ke, oi + q0 * ke, w, st,
+      filtered_candidates(sc, n, qn, ke, (uint32_t)kp0, fp, Redo{flag}, ok + q0 * ke, oi + q0 * ke, w, st,
                           [&](const uint32_t* ids, uint32_t* keys) {
                             rescore_rankquant(rq, qu + q0 * dim, inv_norm, qn, (uint32_t)kp0, ids, keys, st);
                           });
@@ -499,7 +508,7 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, b
       select_rows(w, keys, nullptr, nullptr, n, n, qn, (uint32_t)kp, 32, id_bits, tk, ti, st);
       if (kp == n) break;
       OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
-      sc.margin(tk, qn, (uint32_t)kp, ke, flag, st);
+      sc.margin(tk, qn, (uint32_t)kp, ke, Redo{flag}, st);
       OVB_CUDA(cudaMemcpyAsync(flag_h, flag, 4, cudaMemcpyDeviceToHost, st));
       OVB_CUDA(cudaStreamSynchronize(st));
       if (!*flag_h) break;
@@ -554,7 +563,7 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   uint32_t* ok = (uint32_t*)w.out_keys.ensure(nq * ke * 4);
   uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
   if (filtered) {
-    filtered_candidates(sc, n, nq, ke, (uint32_t)kp, fp, d_flag, ok, oi, w, st,
+    filtered_candidates(sc, n, nq, ke, (uint32_t)kp, fp, Redo{d_flag}, ok, oi, w, st,
                         [&](const uint32_t* ids, uint32_t* keys) {
                           rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ids, keys, st);
                         });
@@ -565,7 +574,7 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   uint32_t* tk = (uint32_t*)w.thr_keys.ensure(nq * kp * 4);
   uint32_t* ti = (uint32_t*)w.thr_ids.ensure(nq * kp * 4);
   select_rows(w, keys, nullptr, nullptr, n, n, nq, (uint32_t)kp, 32, id_bits, tk, ti, st);
-  if (kp < n) sc.margin(tk, nq, (uint32_t)kp, ke, d_flag, st);
+  if (kp < n) sc.margin(tk, nq, (uint32_t)kp, ke, Redo{d_flag}, st);
   uint32_t* k2 = (uint32_t*)w.keys2.ensure(nq * kp * 4);
   rescore_rankquant(rq, qu, inv_norm, nq, (uint32_t)kp, ti, k2, st);
   select_rows(w, k2, ti, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true);
@@ -607,8 +616,8 @@ static SmallForm small_form(const Index& rq, uint64_t nq, uint64_t kp, cudaStrea
 }
 
 // Exact search of prepared query rows qu (as in split_search).  The candidate forms are
-// followed by the FP64 table scan of every document behind their flag: it does nothing
-// unless the margin test failed for some query, so no form waits on the host.
+// followed by the FP64 table scan of every document for the queries whose margin test
+// failed, listed on the device: no form waits on the host.
 static void exact_search(const Index& rq, const float* qu, float inv_norm, bool half_steps, uint64_t nq, uint32_t ke,
                          Workspace& w, cudaStream_t st) {
   const uint64_t n = rq.n, kp64 = std::max<uint64_t>(2ull * ke, ke + 64ull);
@@ -617,12 +626,11 @@ static void exact_search(const Index& rq, const float* qu, float inv_norm, bool 
   uint32_t* oi = (uint32_t*)w.out_ids.ensure(nq * ke * 4);
   FilterPlan fp;
   const SmallForm form = small_form(rq, nq, kp64, st, fp);
-  uint32_t* flag = nullptr;
+  Redo redo;
   if (form != SmallForm::kTables) {
-    flag = (uint32_t*)w.f_flag.ensure(4);
-    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
+    redo = redo_list(w.f_flag, nq);
     CandScores sc(rq, inv_norm, half_steps, 0);
-    sc.prepare(qu, nq, w, st);
+    sc.prepare(qu, nq, w, st, redo);
     if (form == SmallForm::kRows) {
       uint32_t* keys = (uint32_t*)w.keys.ensure(nq * n * 4);
       launch_score_rows(rq.codes.p, n, rq.dim, rq.bits, sc.op, nq, keys, n, st);
@@ -631,19 +639,19 @@ static void exact_search(const Index& rq, const float* qu, float inv_norm, bool 
       uint32_t* ci = (uint32_t*)w.thr_ids.ensure(nq * kp * 4);
       select_rows(w, keys, nullptr, nullptr, n, n, nq, kp, 32, bits_for(n - 1), ck, ci, st);
       w.mark(st, 3);
-      rescored_top_k(sc, rq, qu, inv_norm, nq, kp, ke, ck, ci, flag, w, st);
+      rescored_top_k(sc, rq, qu, inv_norm, nq, kp, ke, ck, ci, redo, w, st);
     } else {
-      filtered_candidates(sc, n, nq, ke, kp, fp, flag, ok, oi, w, st, [&](const uint32_t* ids, uint32_t* keys) {
+      filtered_candidates(sc, n, nq, ke, kp, fp, redo, ok, oi, w, st, [&](const uint32_t* ids, uint32_t* keys) {
         rescore_rankquant(rq, qu, inv_norm, nq, kp, ids, keys, st);
       });
     }
   }
   full_scan_select(
       w, nq, n, ke, 32, ok, oi, st,
-      [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
-        launch_asym_scan(rq.codes.as<uint8_t>(), n, rq.dim, rq.bits, qu + q0 * rq.dim, qn, inv_norm, keys, n, st, flag);
+      [&](uint64_t q0, uint64_t qn, uint32_t* keys, const Redo& part) {
+        launch_asym_scan(rq.codes.as<uint8_t>(), n, rq.dim, rq.bits, qu + q0 * rq.dim, qn, inv_norm, keys, n, st, part);
       },
-      flag);
+      redo);
 }
 
 uint32_t engine_rankquant_full(const Index& rq, const float* d_q, uint64_t nq, uint64_t k,
@@ -682,11 +690,11 @@ struct RankScores {
   const Index& rk;
   ScoreOperand op{};
   double* bound = nullptr;
-  void prepare(bool sym, const void* q, uint64_t qn, Workspace& w, cudaStream_t st) {
+  void prepare(bool sym, const void* q, uint64_t qn, Workspace& w, cudaStream_t st, const Redo& list) {
     op = score_operand(16, qn, rk.dim, 0);
     op.rows = w.q_fix.ensure(op.bytes);
     bound = (double*)w.q_bound.ensure(qn * 16);
-    launch_fix_rank(sym, q, qn, rk.dim, op, bound, st);
+    launch_fix_rank(sym, q, qn, rk.dim, op, bound, list, st);
   }
   void scan(uint64_t qn, uint32_t stride, uint32_t* keys, uint64_t ld, uint32_t* err, cudaStream_t st) const {
     launch_score_scan(rk.codes.p, rk.n, rk.dim, 16, op, qn, stride, keys, ld, err, st);
@@ -695,8 +703,8 @@ struct RankScores {
               uint32_t* fi, uint32_t* err, cudaStream_t st) const {
     launch_score_filter(rk.codes.p, rk.n, rk.dim, 16, op, qn, thr, thr_stride, cnt, cap, fk, fi, err, st);
   }
-  void margin(const uint32_t* sel, uint64_t qn, uint32_t kp, uint32_t ke, uint32_t* flag, cudaStream_t st) const {
-    launch_score_margin(sel, qn, kp, ke, bound, 16, flag, st);
+  void margin(const uint32_t* sel, uint64_t qn, uint32_t kp, uint32_t ke, const Redo& failed, cudaStream_t st) const {
+    launch_score_margin(sel, qn, kp, ke, bound, 16, failed, st);
   }
 };
 
@@ -736,39 +744,38 @@ uint32_t engine_rank_full(const Index& rk, const float* d_q, uint64_t nq, uint64
     launch_encode(5, d_q, nq, dim, 0, 0, 0, qr, 0, nullptr, st);
   }
   // rows [q0, q0 + qn) through the key matrix of exact scores
-  auto full = [&](uint64_t qa, uint64_t qn, const uint32_t* gate) {
+  auto full = [&](uint64_t qa, uint64_t qn, const Redo& redo) {
     full_scan_select(
         w, qn, rk.n, ke, 32, ok + qa * ke, oi + qa * ke, st,
-        [&](uint64_t q0, uint64_t qm, uint32_t* keys) {
+        [&](uint64_t q0, uint64_t qm, uint32_t* keys, const Redo& part) {
           const uint64_t q = qa + q0;
           if (asymmetric)
-            launch_rank_asym_scan(ranks, rk.n, dim, qu + q * dim, qsum + q, qm, keys, rk.n, st, gate);
+            launch_rank_asym_scan(ranks, rk.n, dim, qu + q * dim, qsum + q, qm, keys, rk.n, st, part);
           else
-            launch_rank_sym_scan(ranks, rk.n, dim, qr + q * dim, qm, keys, rk.n, st, gate);
+            launch_rank_sym_scan(ranks, rk.n, dim, qr + q * dim, qm, keys, rk.n, st, part);
         },
-        gate);
+        redo);
   };
   const uint64_t kp = std::min<uint64_t>(std::max<uint64_t>(2ull * ke, ke + 64ull), rk.n);
   FilterPlan fp;
   if (!use_rank_scores(rk, nq, kp, st, fp)) {
-    full(0, nq, nullptr);
+    full(0, nq, Redo());
     return ke;
   }
-  uint32_t* flag = (uint32_t*)w.f_flag.ensure(4);
   uint64_t fc = keys_budget() / split_filter_bytes_per_query(fp, kp);
   if (fc < 1) fc = 1;
   RankScores sc{rk};
   for (uint64_t q0 = 0; q0 < nq; q0 += fc) {
     const uint64_t qn = nq - q0 < fc ? nq - q0 : fc;
     const void* q = asymmetric ? (const void*)(qu + q0 * dim) : (const void*)(qr + q0 * dim);
-    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
-    sc.prepare(!asymmetric, q, qn, w, st);
-    filtered_candidates(sc, rk.n, qn, ke, (uint32_t)kp, fp, flag, ok + q0 * ke, oi + q0 * ke, w, st,
+    const Redo redo = redo_list(w.f_flag, qn);
+    sc.prepare(!asymmetric, q, qn, w, st, redo);
+    filtered_candidates(sc, rk.n, qn, ke, (uint32_t)kp, fp, redo, ok + q0 * ke, oi + q0 * ke, w, st,
                         [&](const uint32_t* ids, uint32_t* keys) {
                           launch_rank_subset(!asymmetric, ranks, dim, q, asymmetric ? qsum + q0 : nullptr, qn, ids,
                                              (uint32_t)kp, keys, st);
                         });
-    full(q0, qn, flag);  // does nothing unless the flag is set
+    full(q0, qn, redo);  // for the listed queries
   }
   return ke;
 }
@@ -815,7 +822,7 @@ uint32_t engine_candidates(const Index& s1, const float* d_q, uint64_t nq, uint6
         break;
       }
       w.mark(st, 6);  // no sampling stage
-      full_scan_select(w, nq, n, me, key_bits, sk, si, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
+      full_scan_select(w, nq, n, me, key_bits, sk, si, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys, const Redo&) {
         launch_popc_scan(mode, s1.codes.as<uint64_t>(), n, s1.qpv(), qb + q0 * s1.qpv(), qn, s1.n_top, keys,
                          n, st);
       });
@@ -834,7 +841,7 @@ uint32_t engine_candidates(const Index& s1, const float* d_q, uint64_t nq, uint6
       // rows [qa, qa + qn) through the full key matrix
       auto dense_rows = [&](uint64_t qa, uint64_t qn) {
         full_scan_select(w, qn, n, me, 32, sk + qa * me, si + qa * me, st,
-                         [&](uint64_t q0, uint64_t qm, uint32_t* keys) {
+                         [&](uint64_t q0, uint64_t qm, uint32_t* keys, const Redo&) {
                            const uint64_t qg = qa + q0;
                            if (use_fastscan_tc(qm))
                              launch_fastscan_scan_tc(codes, n, s1.pairs_pad, lut + qg * lut_row, bias + qg,
@@ -886,7 +893,7 @@ uint32_t engine_candidates(const Index& s1, const float* d_q, uint64_t nq, uint6
         OVB_CUDA(cudaStreamSynchronize(st));
         wts = dw;
       }
-      full_scan_select(w, nq, n, me, 32, sk, si, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys) {
+      full_scan_select(w, nq, n, me, 32, sk, si, st, [&](uint64_t q0, uint64_t qn, uint32_t* keys, const Redo&) {
         launch_multibucket_scan(s1.codes.as<uint64_t>(), n, qpb, nb, qb + q0 * nb * qpb, wts, qn, keys, n, st);
       });
       break;
@@ -992,7 +999,7 @@ static bool split_rerank(const Index& rq, const float* qu, uint64_t nq, uint32_t
   uint32_t* flag_h = (uint32_t*)w.rr_flag_host.ensure(4);
   select_rows(w, keys, cand, nullptr, me, me, nq, kp, 32, id_bits, ck, ci, st);
   OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
-  launch_split_margin(ck, nq, kp, ke, l1, split_error_bound(dim, bits, inv_norm), flag, st);
+  launch_split_margin(ck, nq, kp, ke, l1, split_error_bound(dim, bits, inv_norm), Redo{flag}, st);
   uint32_t* k2 = (uint32_t*)w.rr_keys2.ensure(nq * kp * 4);
   launch_asym_subset(codes, dim, bits, qu, nq, nullptr, ci, kp, inv_norm, k2, st);
   select_rows(w, k2, ci, nullptr, kp, kp, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true);
@@ -1033,26 +1040,24 @@ uint32_t engine_two_stage(const Index& rq, const Index& s1, const float* d_q, ui
   if (mode != OVB_RERANK_FP64 && split_rerank(rq, qu, nq, me, ke, inv_norm, mode == OVB_RERANK_SPLIT_RAW, w, st))
     return ke;
   uint32_t* keys = (uint32_t*)w.keys2.ensure(nq * me * 4);
-  const uint32_t* gate = nullptr;
+  Redo redo;
   if (w.rerank_mode == OVB_RERANK_AUTO && use_subset_scores(rq, nq, me, ke, st)) {
     // integer scores of all candidates, FP64 scores of the best kp; the FP64 rerank of all
     // of them below runs only where the margin test failed for some query
     const uint32_t kp = std::max<uint32_t>(2 * ke, ke + 64);
-    uint32_t* flag = (uint32_t*)w.rr_flag.ensure(4);
-    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
+    redo = redo_list(w.rr_flag, nq);
     CandScores sc(rq, inv_norm, false, 0);
-    sc.prepare(qu, nq, w, st);
+    sc.prepare(qu, nq, w, st, redo);
     launch_score_subset(rq.codes.p, rq.dim, rq.bits, sc.op, nq, cand, me, keys, st);
     uint32_t* ck = (uint32_t*)w.rr_keys.ensure(nq * kp * 4);
     uint32_t* ci = (uint32_t*)w.rr_ids.ensure(nq * kp * 4);
     select_rows(w, keys, cand, nullptr, me, me, nq, kp, 32, id_bits, ck, ci, st);
-    rescored_top_k(sc, rq, qu, inv_norm, nq, kp, ke, ck, ci, flag, w, st);
-    gate = flag;
+    rescored_top_k(sc, rq, qu, inv_norm, nq, kp, ke, ck, ci, redo, w, st);
   }
-  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, nq, nullptr, cand, me, inv_norm, keys, st, gate);
+  launch_asym_subset(rq.codes.as<uint8_t>(), rq.dim, rq.bits, qu, nq, nullptr, cand, me, inv_norm, keys, st, redo);
   w.mark(st, 4);
   // rows are uniform (me candidates each): the strided form, not offsets
-  select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true, gate);
+  select_rows(w, keys, cand, nullptr, me, me, nq, ke, 32, id_bits, ok, oi, st, nullptr, true, true, redo);
   w.mark(st, 5);
   return ke;
 }

@@ -91,7 +91,7 @@ uint32_t autotune_tile(Plan& p) {
       op = score_operand(ix.bits, p.nq, ix.dim, qpt);
       op.rows = w.q_fix.ensure(op.bytes);
       launch_fix_rankquant(w.q_unit.as<float>(), p.nq, ix.dim, ix.bits, false, op,
-                           (double*)w.q_bound.ensure(p.nq * 16), w.stream);
+                           (double*)w.q_bound.ensure(p.nq * 16), Redo(), w.stream);
     }
     auto scan = [&] {
       if (fixed)

@@ -94,6 +94,64 @@ __device__ __forceinline__ float key_score(uint32_t key, int mode, uint32_t n_to
   return mode == 0 ? desc_key_to_float(key) : (float)(n_top - key);
 }
 
+// The queries whose candidate result is not known to be exact, on the device: the count
+// and margin tests list them, and the exact pass that follows takes them from there, so
+// nothing waits on the host and the others' work is not done again.  A launch that is
+// given one (word not null) serves the listed queries in [first, first + count) only,
+// its query 0 being `first`.
+struct Redo {
+  uint32_t* word = nullptr;   // how many are listed; with list null, whether any failed
+  uint32_t* flags = nullptr;  // per query: it is listed
+  uint32_t* list = nullptr;   // in no order
+  uint32_t first = 0, count = 0;
+};
+
+// empties the list, a thread for each query
+__device__ __forceinline__ void redo_clear(const Redo& r, uint64_t q) {
+  if (!r.list) return;
+  r.flags[q] = 0;
+  if (q == 0) *r.word = 0;
+}
+__device__ __forceinline__ void redo_mark(const Redo& r, uint32_t q) {
+  if (!r.list)
+    atomicOr(r.word, 1u);
+  else if (!atomicExch(&r.flags[q], 1u))
+    r.list[atomicAdd(r.word, 1u)] = q;
+}
+
+// entry u of the list as a query of the launch; false when it is another chunk's
+__device__ __forceinline__ bool redo_query(const Redo& r, uint64_t u, uint64_t& q) {
+  q = (uint64_t)r.list[u] - r.first;
+  return q < r.count;
+}
+// nothing is listed: the launch has nothing to do (nor to report, which costs a write to the host)
+__device__ __forceinline__ bool redo_idle(const Redo& r) { return r.word && !*r.word; }
+__device__ __forceinline__ bool redo_skips(const Redo& r, uint64_t q) { return r.word && !r.flags[r.first + q]; }
+
+// A CTA's share of the rows of the listed units (queries, or groups of `per_unit` of them):
+// `rows` each, laid end to end and divided evenly over the launch's CTAs, whatever the
+// number of units is.
+struct RedoWalk {
+  uint64_t at, stop, len;
+  __device__ __forceinline__ RedoWalk(const Redo& r, uint32_t per_unit, uint64_t rows) : at(0), stop(0), len(rows) {
+    const uint32_t listed = *r.word;
+    if (!listed) return;
+    const uint64_t total = (uint64_t)((listed + per_unit - 1) / per_unit) * rows;
+    const uint64_t per = ((total + gridDim.x - 1) / gridDim.x + 31) / 32 * 32;
+    at = per * blockIdx.x < total ? per * blockIdx.x : total;
+    stop = at + per < total ? at + per : total;
+  }
+  // the next unit and its rows [lo, hi)
+  __device__ __forceinline__ bool next(uint64_t& unit, uint64_t& lo, uint64_t& hi) {
+    if (at >= stop) return false;
+    unit = at / len;
+    lo = at - unit * len;
+    hi = stop - unit * len < len ? stop - unit * len : len;
+    at += hi - lo;
+    return true;
+  }
+};
+
 constexpr uint32_t kSentinelKey = 0xFFFFFFFFu;
 constexpr uint32_t kSentinelId = 0xFFFFFFFFu;
 

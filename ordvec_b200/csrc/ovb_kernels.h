@@ -6,6 +6,8 @@
 
 #include <cstddef>
 
+#include "ovb_common.cuh"
+
 namespace ovb {
 
 // ---- K7 select (select.cu) ---------------------------------------------------
@@ -33,7 +35,7 @@ struct SelectArgs {
   uint32_t res_n_top;
   const uint32_t* err_src;  // copied to *err_dst once the results are written (either may be null)
   uint32_t* err_dst;
-  const uint32_t* gate;  // the launch does nothing when *gate is 0 (may be null)
+  Redo redo;  // with it, only the listed queries' rows are selected
 };
 // u64 scratch elements launch_select_rows may use for `rows` rows of length n
 // (0 for ragged rows): global sort buffers for k > kSelectSmemCap, and the
@@ -126,8 +128,8 @@ void launch_bitmap_filter_tc(const uint64_t* words, uint64_t n, uint32_t qpv, ui
                              const uint32_t* thr, const uint32_t* thr_pos, uint32_t smp_stride, uint64_t thr_stride,
                              uint32_t* cnt, uint32_t cap, uint32_t* f_keys, uint32_t* f_ids, uint32_t* err,
                              cudaStream_t stream);
-// *flag |= 1 when some cnt[q] < need or > cap.
-void launch_filter_check(const uint32_t* cnt, uint64_t nq, uint32_t need, uint32_t cap, uint32_t* flag,
+// marks the queries with cnt[q] < need or > cap
+void launch_filter_check(const uint32_t* cnt, uint64_t nq, uint32_t need, uint32_t cap, const Redo& failed,
                          cudaStream_t stream);
 void launch_fastscan_relayout(const uint8_t* ref_blocks, uint64_t n, uint32_t pairs,
                               uint32_t pairs_pad, uint8_t* dev_blocks, cudaStream_t stream);
@@ -152,9 +154,9 @@ void launch_rank_filter_tc(const uint8_t* codes, uint64_t n, uint32_t dim, uint3
                            uint64_t nq, float inv_norm, const uint32_t* thr, uint64_t thr_stride, uint32_t* cnt,
                            uint32_t cap, uint32_t* f_keys, uint32_t* f_ids, uint32_t q_per_tile, uint32_t* err,
                            cudaStream_t stream);
-// flag |= 1 if some row's kp-th key is not below its k-th minus twice the bound
+// marks the queries whose kp-th key is not below their k-th minus twice the bound
 void launch_split_margin(const uint32_t* sel_keys, uint64_t nq, uint32_t kp, uint32_t k, const float* l1,
-                         float bound_per_l1, uint32_t* flag, cudaStream_t stream);
+                         float bound_per_l1, const Redo& failed, cudaStream_t stream);
 
 // ---- K5-TC split-BF16 candidate rerank on tcgen05 (rerank_tc.cu) ---------------
 // dim % 64 == 0 and 16 <= dim * bits / 8 <= 256, a multiple of 16
@@ -170,25 +172,38 @@ void launch_wait_probe(uint32_t* d_out, cudaStream_t stream);
 
 // ---- K9 Rank (u16) index scans (scan_rank_full.cu) -> key32 [nq][ld] ------------
 float rank_norm_f32(uint32_t dim);
-// gate (here and below, may be null): the launch does nothing when *gate is 0 on the device
+// CTAs of a launch for listed queries, which divide their rows evenly (RedoWalk).  Most
+// often nothing is listed and the launch is its CTAs' starts, so they are two an SM (two to
+// four measure the same within 3 %).  Whole calls over 1M rows of dim 768 (us; none, one and
+// all of the queries listed; in brackets the same launch for all queries behind one flag,
+// and exact scores alone): RankQuant b=2, 4 queries 229 / 430 / 813 (227 / 769 / 771, 717 to
+// 766), 48: 267 / 727 for two / 6,747 (267 / 6,481 / 6,892, 6,919 to 7,239); Rank, 64 queries
+// 390 / 1,165 / 6,065 (391 / 5,728 / 6,282, 5,031 to 5,430).
+inline unsigned redo_grid(uint64_t queries, uint64_t rows) {
+  const uint64_t want = (queries * rows + 255) / 256, most = 148 * 2;
+  return (unsigned)(want < most ? want : most);
+}
+
+// redo (here and below): with one, only for the listed queries (Rank: dim % 8 == 0; candidate
+// rows: offsets null)
 // Rank::search: q_ranks = the queries' u16 ranks (nq x dim)
 void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const uint16_t* q_ranks, uint64_t nq,
-                          uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate = nullptr);
-// Rank::search_asymmetric: q_unit rows; q_sum (nq floats) is scratch the launch fills
+                          uint32_t* keys, uint64_t ld, cudaStream_t stream, const Redo& redo = Redo());
+// Rank::search_asymmetric: q_unit rows; q_sum: their sums (launch_rank_row_sum)
 void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, const float* q_sum,
                            uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream,
-                           const uint32_t* gate = nullptr);
+                           const Redo& redo = Redo());
 
 // ---- K4/K5 asymmetric RankQuant scoring (scan_asym.cu) ---------------------------
 void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t bits,
                       const float* q_unit, uint64_t nq, float inv_norm, uint32_t* keys,
-                      uint64_t ld, cudaStream_t stream, const uint32_t* gate = nullptr);
+                      uint64_t ld, cudaStream_t stream, const Redo& redo = Redo());
 // rows: query i's candidates cands[offsets[i] .. offsets[i + 1]) (at most max_row), or
 // with offsets null exactly max_row each; keys[] like cands[]
 void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const float* q_unit,
                         uint64_t nq, const uint64_t* offsets, const uint32_t* cands,
                         uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream,
-                        const uint32_t* gate = nullptr);
+                        const Redo& redo = Redo());
 
 // ---- integer score scans on CTA pairs (scan_score_pair.cu) ---------------------------
 // src: 1, 2, 4 = RankQuant bits, 16 = Rank.  The operand's rows (bytes of device
@@ -202,13 +217,14 @@ bool score_rankquant_eligible(uint32_t dim, uint32_t bits);
 bool score_rank_eligible(uint32_t dim);
 // shape of the operand for nq queries (rows unset); q_per_tile (RankQuant): at most this many, 0 = 128
 ScoreOperand score_operand(uint32_t src, uint64_t nq, uint32_t dim, uint32_t q_per_tile);
-// fill the operand and bound[2 nq] (launch_score_margin's); q: what the scores sum;
-// half_steps: multiples of 1/2, which a power-of-two scale holds exactly
+// fill the operand and bound[2 nq] (launch_score_margin's), and empty `list`, which the tests that
+// follow fill; q: what the scores sum; half_steps: multiples of 1/2, which a power-of-two scale
+// holds exactly
 void launch_fix_rankquant(const float* q, uint64_t nq, uint32_t dim, uint32_t bits, bool half_steps,
-                          const ScoreOperand& b, double* bound, cudaStream_t stream);
+                          const ScoreOperand& b, double* bound, const Redo& list, cudaStream_t stream);
 // sym: q = u16 query ranks, else f32 unit queries
 void launch_fix_rank(bool sym, const void* q, uint64_t nq, uint32_t dim, const ScoreOperand& b, double* bound,
-                     cudaStream_t stream);
+                     const Redo& list, cudaStream_t stream);
 // keys[q * ld + u] of the (sampled) documents; smaller is better
 void launch_score_scan(const void* rows, uint64_t n, uint32_t dim, uint32_t src, const ScoreOperand& b, uint64_t nq,
                        uint32_t block_stride, uint32_t* keys, uint64_t ld, uint32_t* err, cudaStream_t stream);
@@ -224,13 +240,12 @@ void launch_score_rows(const void* codes, uint64_t n, uint32_t dim, uint32_t bit
                        uint32_t* keys, uint64_t ld, cudaStream_t stream);
 void launch_score_subset(const void* codes, uint32_t dim, uint32_t bits, const ScoreOperand& b, uint64_t nq,
                          const uint32_t* cands, uint64_t row_len, uint32_t* keys, cudaStream_t stream);
-// *flag |= 1 when a document outside some query's kp selected keys could belong to its top k
+// marks the queries with a document outside the kp selected keys that could belong to their top k
 void launch_score_margin(const uint32_t* sel_keys, uint64_t nq, uint32_t kp, uint32_t k, const double* bound,
-                         uint32_t src, uint32_t* flag, cudaStream_t stream);
+                         uint32_t src, const Redo& failed, cudaStream_t stream);
 // exact Rank scores of kp candidates per query (ids below n): keys[q * kp + i]
 void launch_rank_subset(bool sym, const uint16_t* ranks, uint32_t dim, const void* q, const float* q_sum, uint64_t nq,
                         const uint32_t* cands, uint32_t kp, uint32_t* keys, cudaStream_t stream);
-float rank_norm_f32(uint32_t dim);
 void launch_rank_row_sum(const float* q, uint64_t nq, uint32_t dim, float* out, cudaStream_t stream);
 
 // ---- encoders (encode.cu) ----------------------------------------------------------
@@ -252,10 +267,10 @@ void launch_prefix_compact(const uint32_t* src, uint64_t ld, const uint64_t* off
                            cudaStream_t stream);
 // ids[i] >= n (sentinels of underfull select rows) -> 0, so a gather stays in bounds
 void launch_clamp_ids(uint32_t* ids, uint64_t count, uint32_t n, cudaStream_t stream);
-// (with err_dst, *err_dst = err_src ? *err_src : 0)
+// (with err_dst, *err_dst = err_src ? *err_src : 0; with redo, rows of row_len entries of the listed queries)
 void launch_keys_to_results(const uint32_t* keys, const uint32_t* ids, uint64_t count,
                             int mode, uint32_t n_top, float* scores, int64_t* out_ids,
                             cudaStream_t stream, const uint32_t* err_src = nullptr, uint32_t* err_dst = nullptr,
-                            const uint32_t* gate = nullptr);
+                            const Redo& redo = Redo(), uint32_t row_len = 0);
 
 }  // namespace ovb

@@ -133,11 +133,11 @@ __global__ void keys_to_results_kernel(const uint32_t* __restrict__ keys,
                                        const uint32_t* __restrict__ ids, uint64_t count,
                                        int mode, uint32_t n_top, float* __restrict__ scores,
                                        int64_t* __restrict__ out_ids, const uint32_t* err_src, uint32_t* err_dst,
-                                       const uint32_t* gate) {
-  if (gate && !*gate) return;
+                                       Redo redo, uint32_t row_len) {
   uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (redo_idle(redo)) return;
   if (t == 0 && err_dst) *err_dst = err_src ? *err_src : 0u;
-  if (t >= count) return;
+  if (t >= count || (redo.word && redo_skips(redo, t / row_len))) return;
   const uint32_t id = ids[t];
   const bool none = id == kSentinelId;
   scores[t] = none ? __int_as_float(0xff800000) : key_score(keys[t], mode, n_top);
@@ -210,10 +210,11 @@ void launch_prefix_compact(const uint32_t* src, uint64_t ld, const uint64_t* off
 
 void launch_keys_to_results(const uint32_t* keys, const uint32_t* ids, uint64_t count,
                             int mode, uint32_t n_top, float* scores, int64_t* out_ids,
-                            cudaStream_t stream, const uint32_t* err_src, uint32_t* err_dst, const uint32_t* gate) {
+                            cudaStream_t stream, const uint32_t* err_src, uint32_t* err_dst, const Redo& redo,
+                            uint32_t row_len) {
   if (!count) return;
   keys_to_results_kernel<<<ceil_div(count, 256), 256, 0, stream>>>(keys, ids, count, mode, n_top, scores, out_ids,
-                                                                   err_src, err_dst, gate);
+                                                                   err_src, err_dst, redo, row_len);
   launched();
 }
 

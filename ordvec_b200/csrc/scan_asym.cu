@@ -109,9 +109,9 @@ template <int BITS, int W>
 __global__ void __launch_bounds__(kThreads)
     asym_scan_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
                      const float* __restrict__ q_unit, float inv_norm,
-                     uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
-  if (gate && !*gate) return;
+                     uint32_t* __restrict__ keys, uint64_t ld, Redo redo) {
   const uint64_t qi = blockIdx.y;
+  if (redo_skips(redo, qi)) return;
   const uint32_t words = dim * BITS / 32;
   const int lane = threadIdx.x & 31;
   double qs[W][32 / BITS];
@@ -130,9 +130,9 @@ __global__ void __launch_bounds__(kThreads)
     asym_subset_kernel(const uint8_t* __restrict__ codes, uint32_t dim,
                        const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                        const uint32_t* __restrict__ cands, float inv_norm,
-                       uint32_t* __restrict__ keys, const uint32_t* gate) {
-  if (gate && !*gate) return;
+                       uint32_t* __restrict__ keys, Redo redo) {
   const uint64_t qi = blockIdx.y;
+  if (redo_skips(redo, qi)) return;
   const uint64_t s = off ? off[qi] : qi * row_len, e = off ? off[qi + 1] : s + row_len;
   const uint32_t words = dim * BITS / 32;
   const int lane = threadIdx.x & 31;
@@ -180,9 +180,9 @@ __device__ __forceinline__ double generic_row_dot(const uint8_t* row, uint32_t d
 __global__ void __launch_bounds__(kThreads)
     asym_scan_generic(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim, uint32_t bits,
                       const float* __restrict__ q_unit, float inv_norm,
-                      uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
-  if (gate && !*gate) return;
+                      uint32_t* __restrict__ keys, uint64_t ld, Redo redo) {
   const uint64_t qi = blockIdx.y;
+  if (redo_skips(redo, qi)) return;
   const uint32_t bpv = dim * bits / 8;
   const uint64_t gw = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) / 32;
   const uint64_t nw = (uint64_t)gridDim.x * kThreads / 32;
@@ -196,9 +196,9 @@ __global__ void __launch_bounds__(kThreads)
     asym_subset_generic(const uint8_t* __restrict__ codes, uint32_t dim, uint32_t bits,
                         const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
                         const uint32_t* __restrict__ cands, float inv_norm,
-                        uint32_t* __restrict__ keys, const uint32_t* gate) {
-  if (gate && !*gate) return;
+                        uint32_t* __restrict__ keys, Redo redo) {
   const uint64_t qi = blockIdx.y;
+  if (redo_skips(redo, qi)) return;
   const uint64_t s = off ? off[qi] : qi * row_len, e = off ? off[qi + 1] : s + row_len;
   const uint32_t bpv = dim * bits / 8;
   const uint64_t gw = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) / 32;
@@ -261,34 +261,16 @@ __device__ __forceinline__ double lds_f64(uint32_t addr) {
   return v;
 }
 
+// Scores of rows [start, end) (SUBSET: the candidates there) by the table at t_base:
+// keys[i].  `warp` of `warps` warps, 32 rows each at a time.
 template <int BITS, bool SUBSET>
-__global__ void __launch_bounds__(kTabThreads)
-    asym_table_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
-                      const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
-                      const uint32_t* __restrict__ cands, float inv_norm, uint32_t* __restrict__ keys,
-                      uint64_t ld, const uint32_t* gate) {
-  if (gate && !*gate) return;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
-  double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
-  const uint64_t qi = blockIdx.y;
-  const float* q = q_unit + qi * dim;
-  build_table<BITS, kTabThreads>(T, q, dim);
-  __syncthreads();
-
-  uint64_t start, end;
-  if (SUBSET) {
-    start = off ? off[qi] : qi * row_len;
-    end = off ? off[qi + 1] : start + row_len;
-  } else {
-    start = 0;
-    end = n;
-  }
+__device__ __forceinline__ void table_rows(const uint8_t* __restrict__ codes, uint32_t dim, uint32_t t_base,
+                                           const uint32_t* __restrict__ cands, float inv_norm,
+                                           uint32_t* __restrict__ keys, uint64_t start, uint64_t end, uint64_t warp,
+                                           uint64_t warps) {
   const uint32_t bpv = dim * BITS / 8, chunks = bpv / 16;
   const int lane = threadIdx.x & 31;
-  const uint64_t gw = ((uint64_t)blockIdx.x * kTabThreads + threadIdx.x) / 32;
-  const uint64_t nw = (uint64_t)gridDim.x * kTabThreads / 32;
-  for (uint64_t base = start + gw * 32; base < end; base += nw * 32) {
+  for (uint64_t base = start + warp * 32; base < end; base += warps * 32) {
     const uint64_t i = base + lane;
     const bool valid = i < end;
     const uint64_t row = valid ? (SUBSET ? (uint64_t)cands[i] : i) : 0;
@@ -314,13 +296,48 @@ __global__ void __launch_bounds__(kTabThreads)
         }
       }
     }
-    if (valid) {
-      const float sc = (float)(((acc[0] + acc[1]) + (acc[2] + acc[3])) * (double)inv_norm);
-      if (SUBSET)
-        keys[i] = desc_key(sc);
-      else
-        keys[qi * ld + i] = desc_key(sc);
-    }
+    if (valid) keys[i] = desc_key((float)(((acc[0] + acc[1]) + (acc[2] + acc[3])) * (double)inv_norm));
+  }
+}
+
+template <int BITS, bool SUBSET>
+__global__ void __launch_bounds__(kTabThreads)
+    asym_table_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
+                      const float* __restrict__ q_unit, const uint64_t* __restrict__ off, uint64_t row_len,
+                      const uint32_t* __restrict__ cands, float inv_norm, uint32_t* __restrict__ keys,
+                      uint64_t ld) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
+  double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
+  const uint64_t qi = blockIdx.y;
+  build_table<BITS, kTabThreads>(T, q_unit + qi * dim, dim);
+  __syncthreads();
+  const uint64_t start = !SUBSET ? 0 : off ? off[qi] : qi * row_len;
+  const uint64_t end = !SUBSET ? n : off ? off[qi + 1] : start + row_len;
+  table_rows<BITS, SUBSET>(codes, dim, t_base, cands, inv_norm, keys + (SUBSET ? 0 : qi * ld), start, end,
+                           ((uint64_t)blockIdx.x * kTabThreads + threadIdx.x) / 32,
+                           (uint64_t)gridDim.x * kTabThreads / 32);
+}
+
+// The same scores of the listed queries.
+template <int BITS, bool SUBSET>
+__global__ void __launch_bounds__(kTabThreads)
+    asym_table_redo_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
+                           const float* __restrict__ q_unit, uint64_t row_len, const uint32_t* __restrict__ cands,
+                           float inv_norm, uint32_t* __restrict__ keys, uint64_t ld, Redo redo) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
+  double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
+  RedoWalk walk(redo, 1, SUBSET ? row_len : n);
+  uint64_t u, lo, hi, qi;
+  while (walk.next(u, lo, hi)) {
+    if (!redo_query(redo, u, qi)) continue;
+    build_table<BITS, kTabThreads>(T, q_unit + qi * dim, dim);
+    __syncthreads();
+    const uint64_t at = SUBSET ? qi * row_len : 0;
+    table_rows<BITS, SUBSET>(codes, dim, t_base, cands, inv_norm, keys + (SUBSET ? 0 : qi * ld), at + lo, at + hi,
+                             threadIdx.x / 32, kTabThreads / 32);
+    __syncthreads();  // the next query's table
   }
 }
 
@@ -336,12 +353,12 @@ template <int BITS>
 __global__ void __launch_bounds__(kTab4Threads)
     asym_table4_kernel(const uint8_t* __restrict__ codes, uint32_t dim, const float* __restrict__ q_unit,
                        const uint64_t* __restrict__ off, uint64_t row_len, const uint32_t* __restrict__ cands,
-                       float inv_norm, uint32_t* __restrict__ keys, const uint32_t* gate) {
-  if (gate && !*gate) return;
+                       float inv_norm, uint32_t* __restrict__ keys, Redo redo) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t t_base = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 4095u) & ~4095u;
   double* T = reinterpret_cast<double*>(smem_raw + (t_base - (uint32_t)__cvta_generic_to_shared(smem_raw)));
   const uint64_t qi = blockIdx.y;
+  if (redo_skips(redo, qi)) return;
   const float* q = q_unit + qi * dim;
   const uint64_t start = off ? off[qi] : qi * row_len, end = off ? off[qi + 1] : start + row_len;
   const uint32_t bpv = dim * BITS / 8, chunks = bpv / 16, r = threadIdx.x & 3;
@@ -393,12 +410,18 @@ bool table_ok(uint32_t dim, uint32_t bits) {
 template <bool SUBSET>
 void launch_table(uint32_t bits, dim3 grid, size_t smem, cudaStream_t st, const uint8_t* codes, uint64_t n,
                   uint32_t dim, const float* qu, const uint64_t* off, uint64_t row_len, const uint32_t* cands,
-                  float inv_norm, uint32_t* keys, uint64_t ld, const uint32_t* gate) {
-#define OVB_TAB(B)                                                                                     \
-  do {                                                                                                 \
-    allow_dynamic_smem(asym_table_kernel<B, SUBSET>);                                                  \
-    asym_table_kernel<B, SUBSET><<<grid, kTabThreads, smem, st>>>(codes, n, dim, qu, off, row_len, cands, \
-                                                                  inv_norm, keys, ld, gate);                     \
+                  float inv_norm, uint32_t* keys, uint64_t ld, const Redo& redo) {
+#define OVB_TAB(B)                                                                                              \
+  do {                                                                                                          \
+    if (redo.word) {                                                                                            \
+      allow_dynamic_smem(asym_table_redo_kernel<B, SUBSET>);                                                    \
+      asym_table_redo_kernel<B, SUBSET><<<grid, kTabThreads, smem, st>>>(codes, n, dim, qu, row_len, cands,     \
+                                                                         inv_norm, keys, ld, redo);             \
+    } else {                                                                                                    \
+      allow_dynamic_smem(asym_table_kernel<B, SUBSET>);                                                         \
+      asym_table_kernel<B, SUBSET><<<grid, kTabThreads, smem, st>>>(codes, n, dim, qu, off, row_len, cands,     \
+                                                                    inv_norm, keys, ld);                        \
+    }                                                                                                           \
   } while (0)
   if (bits == 1)
     OVB_TAB(1);
@@ -409,11 +432,11 @@ void launch_table(uint32_t bits, dim3 grid, size_t smem, cudaStream_t st, const 
 #undef OVB_TAB
 }
 
-// CTAs a query.  A gated launch, which most often does nothing, takes two CTAs an SM
-// in all (or one a query): the rows loop.
-unsigned grid_x(uint64_t rows_per_cta, uint64_t n, const uint32_t* gate, uint64_t queries) {
+// CTAs a query.  A launch for listed queries starts them for every query, and most often
+// none is listed: two an SM.
+unsigned grid_x(uint64_t rows_per_cta, uint64_t n, const Redo& redo) {
   uint64_t g = (n + rows_per_cta - 1) / rows_per_cta;
-  const uint64_t most = gate ? 148 * 2 / queries : 148 * 8;
+  const uint64_t most = redo.word ? 148 * 2 : 148 * 8;
   if (g > most) g = most;
   if (g < 1) g = 1;
   return (unsigned)g;
@@ -432,14 +455,14 @@ int plan_w(uint32_t dim, uint32_t bits) {
 template <int BITS>
 void dispatch_bits(int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t* codes, uint64_t n,
                    uint32_t dim, const float* qu, float inv_norm, uint32_t* keys, uint64_t ld,
-                   const uint64_t* off, uint64_t row_len, const uint32_t* cands, const uint32_t* gate) {
+                   const uint64_t* off, uint64_t row_len, const uint32_t* cands, const Redo& redo) {
 #define OVB_ASYM_CASE(WV)                                                                                  \
   if (W == WV) {                                                                                           \
     if (subset)                                                                                            \
       asym_subset_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, dim, qu, off, row_len, cands,         \
-                                                              inv_norm, keys, gate);                       \
+                                                              inv_norm, keys, redo);                       \
     else                                                                                                   \
-      asym_scan_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, n, dim, qu, inv_norm, keys, ld, gate);  \
+      asym_scan_kernel<BITS, WV><<<grid, kThreads, 0, st>>>(codes, n, dim, qu, inv_norm, keys, ld, redo);  \
     return;                                                                                                \
   }
   if constexpr (BITS == 1) {
@@ -457,42 +480,50 @@ void dispatch_bits(int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t
 
 void dispatch(uint32_t bits, int W, bool subset, dim3 grid, cudaStream_t st, const uint8_t* codes,
               uint64_t n, uint32_t dim, const float* qu, float inv_norm, uint32_t* keys, uint64_t ld,
-              const uint64_t* off, uint64_t row_len, const uint32_t* cands, const uint32_t* gate) {
+              const uint64_t* off, uint64_t row_len, const uint32_t* cands, const Redo& redo) {
   if (bits == 1)
-    dispatch_bits<1>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, gate);
+    dispatch_bits<1>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, redo);
   else if (bits == 2)
-    dispatch_bits<2>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, gate);
+    dispatch_bits<2>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, redo);
   else
-    dispatch_bits<4>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, gate);
+    dispatch_bits<4>(W, subset, grid, st, codes, n, dim, qu, inv_norm, keys, ld, off, row_len, cands, redo);
 }
 
 }  // namespace
 
 void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t bits,
                       const float* q_unit, uint64_t nq, float inv_norm, uint32_t* keys,
-                      uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
+                      uint64_t ld, cudaStream_t stream, const Redo& redo) {
   if (!n || !nq) return;
   if (table_ok(dim, bits)) {
+    if (redo.word) {
+      launch_table<false>(bits, redo_grid(nq, n), table_smem(dim, bits), stream, codes, n, dim, q_unit, nullptr, 0,
+                          nullptr, inv_norm, keys, ld, redo);
+      launched();
+      return;
+    }
     // ~1024 rows per CTA: the table build stays a few percent of the scoring
     for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
       unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-      dim3 grid(grid_x(1024, n, gate, gy), gy);
+      dim3 grid(grid_x(1024, n, redo), gy);
       launch_table<false>(bits, grid, table_smem(dim, bits), stream, codes, n, dim, q_unit + q0 * dim, nullptr,
-                           0, nullptr, inv_norm, keys + q0 * ld, ld, gate);
+                           0, nullptr, inv_norm, keys + q0 * ld, ld, redo);
       launched();
     }
     return;
   }
   const int W = plan_w(dim, bits);
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
+    Redo r = redo;
+    r.first += (uint32_t)q0;
     unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-    dim3 grid(grid_x(kThreads / 32, n, gate, gy), gy);
+    dim3 grid(grid_x(kThreads / 32, n, redo), gy);
     if (W)
       dispatch(bits, W, false, grid, stream, codes, n, dim, q_unit + q0 * dim, inv_norm, keys + q0 * ld, ld,
-               nullptr, 0, nullptr, gate);
+               nullptr, 0, nullptr, r);
     else
       asym_scan_generic<<<grid, kThreads, 0, stream>>>(codes, n, dim, bits, q_unit + q0 * dim, inv_norm,
-                                                       keys + q0 * ld, ld, gate);
+                                                       keys + q0 * ld, ld, r);
     launched();
   }
 }
@@ -500,8 +531,9 @@ void launch_asym_scan(const uint8_t* codes, uint64_t n, uint32_t dim, uint32_t b
 void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const float* q_unit,
                         uint64_t nq, const uint64_t* offsets, const uint32_t* cands,
                         uint64_t max_row, float inv_norm, uint32_t* keys, cudaStream_t stream,
-                        const uint32_t* gate) {
+                        const Redo& redo) {
   if (!nq || !max_row) return;
+  if (redo.word && offsets) throw std::invalid_argument("candidate rows of listed queries must be uniform");
   // one arithmetic for every batch size, so a query scores the same alone and
   // inside a batch
   if (table_ok(dim, bits)) {
@@ -515,7 +547,7 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
   do {                                                                                                          \
     allow_dynamic_smem(asym_table4_kernel<B>);                                                                  \
     asym_table4_kernel<B><<<grid, kTab4Threads, smem, stream>>>(codes, dim, q_unit, offsets, max_row, cands,    \
-                                                                inv_norm, keys, gate);                          \
+                                                                inv_norm, keys, redo);                          \
   } while (0)
       if (bits == 1)
         OVB_TAB4(1);
@@ -529,12 +561,18 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
     }
     // 512 rows per CTA (two per lane) with many queries, fewer with few
     const uint64_t rows_per_cta = nq >= 64 ? 512 : 128;
+    if (redo.word) {
+      launch_table<true>(bits, redo_grid(nq, max_row), table_smem(dim, bits), stream, codes, 0, dim, q_unit, nullptr,
+                         max_row, cands, inv_norm, keys, 0, redo);
+      launched();
+      return;
+    }
     for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
       unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-      dim3 grid(grid_x(rows_per_cta, max_row, gate, gy), gy);
+      dim3 grid(grid_x(rows_per_cta, max_row, redo), gy);
       launch_table<true>(bits, grid, table_smem(dim, bits), stream, codes, 0, dim, q_unit + q0 * dim,
                          offsets ? offsets + q0 : nullptr, max_row, cands + (offsets ? 0 : q0 * max_row), inv_norm,
-                         keys + (offsets ? 0 : q0 * max_row), 0, gate);
+                         keys + (offsets ? 0 : q0 * max_row), 0, redo);
       launched();
     }
     return;
@@ -545,16 +583,18 @@ void launch_asym_subset(const uint8_t* codes, uint32_t dim, uint32_t bits, const
   const uint64_t rows_per_warp = nq >= 64 ? 32 : 4;
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     unsigned gy = (unsigned)((nq - q0) < 65535 ? (nq - q0) : 65535);
-    dim3 grid(grid_x((kThreads / 32) * rows_per_warp, max_row, gate, gy), gy);
+    dim3 grid(grid_x((kThreads / 32) * rows_per_warp, max_row, redo), gy);
     const uint64_t* off = offsets ? offsets + q0 : nullptr;
     const uint32_t* c = cands + (offsets ? 0 : q0 * max_row);
     uint32_t* k = keys + (offsets ? 0 : q0 * max_row);
+    Redo r = redo;
+    r.first += (uint32_t)q0;
     if (W)
       dispatch(bits, W, true, grid, stream, codes, 0, dim, q_unit + q0 * dim, inv_norm, k, 0, off, max_row, c,
-               gate);
+               r);
     else
       asym_subset_generic<<<grid, kThreads, 0, stream>>>(codes, dim, bits, q_unit + q0 * dim, off, max_row, c,
-                                                         inv_norm, k, gate);
+                                                         inv_norm, k, r);
     launched();
   }
 }

@@ -548,11 +548,11 @@ __global__ void expand_query_nibbles_kernel(const uint64_t* __restrict__ qbits, 
 }
 
 __global__ void filter_check_kernel(const uint32_t* __restrict__ cnt, uint64_t nq, uint32_t need, uint32_t cap,
-                                    uint32_t* __restrict__ flag) {
+                                    Redo failed) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nq) {
     const uint32_t c = cnt[i];
-    if (c < need || c > cap) atomicOr(flag, 1u);
+    if (c < need || c > cap) redo_mark(failed, (uint32_t)i);
   }
 }
 
@@ -749,10 +749,10 @@ void launch_bitmap_filter_tc(const uint64_t* words, uint64_t n, uint32_t qpv, ui
   launch_tc<1>(a, q_bytes, stream);
 }
 
-void launch_filter_check(const uint32_t* cnt, uint64_t nq, uint32_t need, uint32_t cap, uint32_t* flag,
+void launch_filter_check(const uint32_t* cnt, uint64_t nq, uint32_t need, uint32_t cap, const Redo& failed,
                          cudaStream_t stream) {
   if (!nq) return;
-  filter_check_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, stream>>>(cnt, nq, need, cap, flag);
+  filter_check_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, stream>>>(cnt, nq, need, cap, failed);
   launched();
 }
 

@@ -38,29 +38,28 @@ constexpr int kRfWarps = kRfThreads / 32;
 constexpr int kChunk = 32;                 // coordinates per staged chunk
 constexpr int kRowWords = kChunk / 2 + 1;  // 16 rank pairs + 1 pad word
 
+// Scores of documents [lo, hi) against a group of QT queries; query(t, qi) names query t, or
+// says that there is none.  CTA `part` of `parts`.
 // SYM: q holds u16 ranks, staged as qv[j * QT + t] u32; !SYM: f32 unit-query values.
-template <bool SYM, int QT, bool WIDE>
-__global__ void __launch_bounds__(kRfThreads)
-    rank_tile_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim, const void* __restrict__ q,
-                     const float* __restrict__ q_sum, uint64_t nq, float mean, float scale,
-                     uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
-  if (gate && !*gate) return;
+template <bool SYM, int QT, bool WIDE, class Query>
+__device__ __forceinline__ void rank_tile(uint32_t* smem, const uint16_t* __restrict__ ranks, uint32_t dim,
+                                          const void* __restrict__ q, const float* __restrict__ q_sum, float mean,
+                                          float scale, uint32_t* __restrict__ keys, uint64_t ld, uint64_t lo,
+                                          uint64_t hi, uint64_t part, uint64_t parts, Query&& query) {
   using Acc = typename std::conditional<WIDE, unsigned long long, uint32_t>::type;
-  extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* rows = smem;                            // [warp][32][kRowWords]
   uint32_t* qv = smem + kRfWarps * 32 * kRowWords;  // [dim][QT]
-  const uint64_t g0 = (uint64_t)blockIdx.x * QT;    // first query of the group
   for (uint32_t e = threadIdx.x; e < dim * QT; e += kRfThreads) {
     const uint32_t j = e / QT, t = e % QT;
-    const uint64_t qi = g0 + t < nq ? g0 + t : nq - 1;  // padding queries repeat the last
+    uint64_t qi = 0;
+    query(t, qi);  // padding queries repeat another
     qv[e] = SYM ? (uint32_t)((const uint16_t*)q)[qi * dim + j] : __float_as_uint(((const float*)q)[qi * dim + j]);
   }
   __syncthreads();
   const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
   uint32_t* wrow = rows + warp * 32 * kRowWords;
   const uint32_t n_chunks = (dim + kChunk - 1) / kChunk;
-  for (uint64_t d0 = ((uint64_t)blockIdx.y * kRfWarps + warp) * 32; d0 < n;
-       d0 += (uint64_t)gridDim.y * kRfWarps * 32) {
+  for (uint64_t d0 = lo + (part * kRfWarps + warp) * 32; d0 < hi; d0 += parts * kRfWarps * 32) {
     Acc dot[QT];
     float acc[QT];
 #pragma unroll
@@ -76,7 +75,7 @@ __global__ void __launch_bounds__(kRfThreads)
       for (int i = 0; i < 4; i++) {
         const uint32_t r = (uint32_t)lane / 4 + 8 * i, p = (uint32_t)lane % 4;
         const uint64_t doc = d0 + r;
-        buf[i] = (doc < n && p < pieces) ? __ldg(reinterpret_cast<const uint4*>(ranks + doc * dim + c0 + 8 * p))
+        buf[i] = (doc < hi && p < pieces) ? __ldg(reinterpret_cast<const uint4*>(ranks + doc * dim + c0 + 8 * p))
                                          : make_uint4(0, 0, 0, 0);
       }
     };
@@ -114,12 +113,12 @@ __global__ void __launch_bounds__(kRfThreads)
       }
     }
     const uint64_t doc = d0 + lane;
-    if (doc < n) {
+    if (doc < hi) {
       const long long base = (long long)dim * (long long)(dim - 1) * (long long)(dim - 1);
 #pragma unroll
       for (int t = 0; t < QT; t++) {
-        const uint64_t qi = g0 + t;
-        if (qi < nq) {
+        uint64_t qi;
+        if (query(t, qi)) {
           float s;
           if (SYM) {
             const long long a = 4 * (long long)dot[t] - base;
@@ -134,12 +133,54 @@ __global__ void __launch_bounds__(kRfThreads)
   }
 }
 
+template <bool SYM, int QT, bool WIDE>
+__global__ void __launch_bounds__(kRfThreads)
+    rank_tile_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim, const void* __restrict__ q,
+                     const float* __restrict__ q_sum, uint64_t nq, float mean, float scale,
+                     uint32_t* __restrict__ keys, uint64_t ld) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  const uint64_t g0 = (uint64_t)blockIdx.x * QT;  // first query of the group
+  rank_tile<SYM, QT, WIDE>(smem, ranks, dim, q, q_sum, mean, scale, keys, ld, 0, n, blockIdx.y, gridDim.y,
+                           [&](uint32_t t, uint64_t& qi) {
+                             qi = g0 + t < nq ? g0 + t : nq - 1;
+                             return g0 + t < nq;
+                           });
+}
+
+// The same scores of the listed queries, QT of the list at a time.
+template <bool SYM, int QT>
+__global__ void __launch_bounds__(kRfThreads)
+    rank_redo_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim, const void* __restrict__ q,
+                     const float* __restrict__ q_sum, float mean, float scale, uint32_t* __restrict__ keys,
+                     uint64_t ld, Redo redo) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  const uint32_t total = *redo.word;
+  RedoWalk walk(redo, QT, n);
+  uint64_t group, lo, hi;
+  while (walk.next(group, lo, hi)) {
+    const uint32_t g0 = (uint32_t)group * QT;
+    auto query = [&](uint32_t t, uint64_t& qi) {
+      uint64_t x;
+      const bool mine = g0 + t < total && redo_query(redo, g0 + t, x);
+      if (mine) qi = x;
+      return mine;
+    };
+    bool any = false;
+    for (uint32_t t = 0; t < QT; t++) {
+      uint64_t qi;
+      any |= query(t, qi);
+    }
+    if (!any) continue;  // listed for another chunk
+    rank_tile<SYM, QT, false>(smem, ranks, dim, q, q_sum, mean, scale, keys, ld, lo, hi, 0, 1, query);
+    __syncthreads();  // the next group's values
+  }
+}
+
 // Scalar forms for dims that are not a multiple of 8 (rows not 16-byte aligned).
 __global__ void __launch_bounds__(kRfThreads)
     rank_sym_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim,
                     const uint16_t* __restrict__ q_ranks, float inv_norm_sq, uint32_t* __restrict__ keys,
-                    uint64_t ld, const uint32_t* gate) {
-  if (gate && !*gate) return;
+                    uint64_t ld) {
   extern __shared__ int32_t qc[];  // 2 q_r - (D - 1)
   const uint64_t qi = blockIdx.y;
   const int32_t m2 = (int32_t)dim - 1;
@@ -161,8 +202,7 @@ __global__ void __launch_bounds__(kRfThreads)
 __global__ void __launch_bounds__(kRfThreads)
     rank_asym_kernel(const uint16_t* __restrict__ ranks, uint64_t n, uint32_t dim,
                      const float* __restrict__ q_unit, const float* __restrict__ q_sum, float mean,
-                     float inv_norm, uint32_t* __restrict__ keys, uint64_t ld, const uint32_t* gate) {
-  if (gate && !*gate) return;
+                     float inv_norm, uint32_t* __restrict__ keys, uint64_t ld) {
   extern __shared__ float qs[];
   const uint64_t qi = blockIdx.y;
   for (uint32_t j = threadIdx.x; j < dim; j += blockDim.x) qs[j] = q_unit[qi * dim + j];
@@ -206,12 +246,10 @@ __global__ void row_sum_kernel(const float* __restrict__ q, uint64_t nq, uint32_
   if (lane == 0) out[i] = s;
 }
 
-// CTAs a query; a gated launch, which most often does nothing, takes two an SM in all
-unsigned rf_grid(uint64_t units, uint64_t per_cta, const uint32_t* gate, uint64_t queries) {
+unsigned rf_grid(uint64_t units, uint64_t per_cta) {
   uint64_t g = (units + per_cta - 1) / per_cta;
-  const uint64_t most = gate ? 148 * 2 / queries : 148 * 16;
-  if (g > most) g = most;
   if (g < 1) g = 1;
+  if (g > 148 * 16) g = 148 * 16;
   return (unsigned)g;
 }
 
@@ -225,14 +263,25 @@ int rank_qt(uint64_t nq, uint32_t dim) {
 
 template <bool SYM, int QT, bool WIDE>
 void launch_tile(const uint16_t* ranks, uint64_t n, uint32_t dim, const void* q, const float* q_sum, uint64_t nq,
-                 float mean, float scale, uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
+                 float mean, float scale, uint32_t* keys, uint64_t ld, cudaStream_t stream, const Redo& redo) {
   const size_t smem = ((size_t)kRfWarps * 32 * kRowWords + (size_t)dim * QT) * 4;
+  const uint64_t groups = (nq + QT - 1) / QT;
+  if (redo.word) {
+    if constexpr (WIDE) {
+      throw std::invalid_argument("Rank scan of listed queries: dim too large");
+    } else {
+      auto kern = rank_redo_kernel<SYM, QT>;
+      allow_dynamic_smem(kern);
+      kern<<<redo_grid(groups, n), kRfThreads, smem, stream>>>(ranks, n, dim, q, q_sum, mean, scale, keys, ld, redo);
+      launched();
+      return;
+    }
+  }
   auto kern = rank_tile_kernel<SYM, QT, WIDE>;
   allow_dynamic_smem(kern);
-  const uint64_t groups = (nq + QT - 1) / QT;
   uint64_t gy = (n + kRfWarps * 32 - 1) / (kRfWarps * 32);
   // enough CTAs to fill every SM several times over; documents beyond that loop
-  const uint64_t want = gate ? 148 * 2 : 148 * 32;
+  const uint64_t want = 148ull * 32;
   if (gy * groups > want) gy = (want + groups - 1) / groups;
   if (gy < 1) gy = 1;
   if (gy > 65535) gy = 65535;
@@ -241,8 +290,7 @@ void launch_tile(const uint16_t* ranks, uint64_t n, uint32_t dim, const void* q,
     const uint64_t q0 = g0 * QT;
     const void* qp = SYM ? (const void*)((const uint16_t*)q + q0 * dim) : (const void*)((const float*)q + q0 * dim);
     kern<<<dim3((unsigned)gn, (unsigned)gy), kRfThreads, smem, stream>>>(
-        ranks, n, dim, qp, q_sum ? q_sum + q0 : nullptr, nq - q0, mean, scale, keys + q0 * ld, ld,
-        gate);
+        ranks, n, dim, qp, q_sum ? q_sum + q0 : nullptr, nq - q0, mean, scale, keys + q0 * ld, ld);
     launched();
   }
 }
@@ -250,13 +298,13 @@ void launch_tile(const uint16_t* ranks, uint64_t n, uint32_t dim, const void* q,
 template <bool SYM, bool WIDE>
 void launch_tiled(int qt, const uint16_t* ranks, uint64_t n, uint32_t dim, const void* q, const float* q_sum,
                   uint64_t nq, float mean, float scale, uint32_t* keys, uint64_t ld, cudaStream_t stream,
-                  const uint32_t* gate) {
+                  const Redo& redo) {
   if (qt == 8)
-    launch_tile<SYM, 8, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, gate);
+    launch_tile<SYM, 8, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, redo);
   else if (qt == 4)
-    launch_tile<SYM, 4, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, gate);
+    launch_tile<SYM, 4, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, redo);
   else
-    launch_tile<SYM, 1, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, gate);
+    launch_tile<SYM, 1, WIDE>(ranks, n, dim, q, q_sum, nq, mean, scale, keys, ld, stream, redo);
 }
 
 }  // namespace
@@ -274,7 +322,7 @@ void launch_rank_row_sum(const float* q, uint64_t nq, uint32_t dim, float* out, 
 }
 
 void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const uint16_t* q_ranks, uint64_t nq,
-                          uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
+                          uint32_t* keys, uint64_t ld, cudaStream_t stream, const Redo& redo) {
   if (!n || !nq) return;
   const float norm = rank_norm_f32(dim);
   const float inv_norm_sq = 1.0f / (norm * norm);
@@ -282,38 +330,40 @@ void launch_rank_sym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const
     const int qt = rank_qt(nq, dim);
     if (dim <= 2048)
       launch_tiled<true, false>(qt, ranks, n, dim, q_ranks, nullptr, nq, 0.0f, inv_norm_sq, keys, ld, stream,
-                                gate);
+                                redo);
     else
       launch_tiled<true, true>(qt, ranks, n, dim, q_ranks, nullptr, nq, 0.0f, inv_norm_sq, keys, ld, stream,
-                                gate);
+                                redo);
     return;
   }
+  if (redo.word) throw std::invalid_argument("Rank scan of listed queries: dim must be a multiple of 8");
   const size_t smem = (size_t)dim * 4;
   allow_dynamic_smem(rank_sym_kernel);
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     const unsigned gy = (unsigned)(nq - q0 < 65535 ? nq - q0 : 65535);
-    rank_sym_kernel<<<dim3(rf_grid(n, kRfThreads / 32, gate, gy), gy), kRfThreads, smem, stream>>>(
-        ranks, n, dim, q_ranks + q0 * dim, inv_norm_sq, keys + q0 * ld, ld, gate);
+    rank_sym_kernel<<<dim3(rf_grid(n, kRfThreads / 32), gy), kRfThreads, smem, stream>>>(
+        ranks, n, dim, q_ranks + q0 * dim, inv_norm_sq, keys + q0 * ld, ld);
     launched();
   }
 }
 
 void launch_rank_asym_scan(const uint16_t* ranks, uint64_t n, uint32_t dim, const float* q_unit, const float* q_sum,
-                           uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream, const uint32_t* gate) {
+                           uint64_t nq, uint32_t* keys, uint64_t ld, cudaStream_t stream, const Redo& redo) {
   if (!n || !nq) return;
   const float inv_norm = 1.0f / rank_norm_f32(dim);
   const float mean = ((float)dim - 1.0f) / 2.0f;
   if (dim % 8 == 0) {
     launch_tiled<false, false>(rank_qt(nq, dim), ranks, n, dim, q_unit, q_sum, nq, mean, inv_norm, keys, ld, stream,
-                               gate);
+                               redo);
     return;
   }
+  if (redo.word) throw std::invalid_argument("Rank scan of listed queries: dim must be a multiple of 8");
   const size_t smem = (size_t)dim * 4;
   allow_dynamic_smem(rank_asym_kernel);
   for (uint64_t q0 = 0; q0 < nq; q0 += 65535) {
     const unsigned gy = (unsigned)(nq - q0 < 65535 ? nq - q0 : 65535);
-    rank_asym_kernel<<<dim3(rf_grid(n, kRfThreads, gate, gy), gy), kRfThreads, smem, stream>>>(
-        ranks, n, dim, q_unit + q0 * dim, q_sum + q0, mean, inv_norm, keys + q0 * ld, ld, gate);
+    rank_asym_kernel<<<dim3(rf_grid(n, kRfThreads), gy), kRfThreads, smem, stream>>>(
+        ranks, n, dim, q_unit + q0 * dim, q_sum + q0, mean, inv_norm, keys + q0 * ld, ld);
     launched();
   }
 }

@@ -419,17 +419,17 @@ __global__ void split_queries_kernel(const float* __restrict__ qu, uint64_t nq, 
   }
 }
 
-// Margin test of the split-BF16 candidates: flag |= 1 when a query's kp-th
-// best split score is not below its k-th best minus twice the error bound.
+// Margin test of the split-BF16 candidates: marks a query whose kp-th best
+// split score is not below its k-th best minus twice the error bound.
 __global__ void split_margin_kernel(const uint32_t* __restrict__ sel_keys, uint64_t nq, uint32_t kp, uint32_t k,
-                                    const float* __restrict__ l1, float bound_per_l1, uint32_t* __restrict__ flag) {
+                                    const float* __restrict__ l1, float bound_per_l1, Redo failed) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
   const float tk = desc_key_to_float(sel_keys[i * kp + (k - 1)]);
   const float last = desc_key_to_float(sel_keys[i * kp + (kp - 1)]);
   const float eps = l1[i] * bound_per_l1;
   // written so that NaN anywhere fails the test
-  if (!(last < tk - 2.0f * eps - 4.0f * fabsf(tk) * 1.1920929e-7f)) atomicOr(flag, 1u);
+  if (!(last < tk - 2.0f * eps - 4.0f * fabsf(tk) * 1.1920929e-7f)) redo_mark(failed, (uint32_t)i);
 }
 
 }  // namespace
@@ -453,9 +453,9 @@ void launch_split_queries(const float* q_unit, uint64_t nq, uint32_t dim, void* 
 }
 
 void launch_split_margin(const uint32_t* sel_keys, uint64_t nq, uint32_t kp, uint32_t k, const float* l1,
-                         float bound_per_l1, uint32_t* flag, cudaStream_t stream) {
+                         float bound_per_l1, const Redo& failed, cudaStream_t stream) {
   if (!nq) return;
-  split_margin_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, stream>>>(sel_keys, nq, kp, k, l1, bound_per_l1, flag);
+  split_margin_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, stream>>>(sel_keys, nq, kp, k, l1, bound_per_l1, failed);
   launched();
 }
 

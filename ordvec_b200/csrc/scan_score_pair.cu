@@ -532,7 +532,8 @@ __device__ __forceinline__ uint64_t b_row(uint64_t q, uint32_t nqt, uint32_t pla
 // distinct in the final f32 rounding, so the best kp by (T, id) begin with the answer
 // whatever ties there are: a bound of minus infinity passes the margin test.
 __global__ void fix_rankquant_kernel(const float* __restrict__ qu, uint32_t dim, uint32_t bits, bool half_steps,
-                                     uint32_t nqt, uint32_t k_bytes, int8_t* __restrict__ out, double* __restrict__ bound) {
+                                     uint32_t nqt, uint32_t k_bytes, int8_t* __restrict__ out, double* __restrict__ bound,
+                                     Redo list) {
   __shared__ float fpart[32];
   __shared__ double dpart[32];
   const uint64_t q = blockIdx.x;
@@ -566,6 +567,7 @@ __global__ void fix_rankquant_kernel(const float* __restrict__ qu, uint32_t dim,
   off = block_sum(off, dpart);
   sum = block_sum(sum, dpart);
   if (threadIdx.x == 0) {
+    redo_clear(list, q);
     const double c = ((double)(1u << bits) - 1.0) * 0.5;
     // |fl(S q) - S q| <= 32640 * 2^-24 < 0.002
     bound[2 * q] = bad || flat ? (double)INFINITY : half_steps ? -(double)INFINITY : 2.0 * c * (off + 0.002 * dim);
@@ -584,7 +586,7 @@ __global__ void fix_rankquant_kernel(const float* __restrict__ qu, uint32_t dim,
 //     (2 dim + 8) 2^-24 |q|_1 dim in units of sum q d, times F = L / (max - min).
 template <bool SYM>
 __global__ void fix_rank_kernel(const void* __restrict__ src, uint32_t dim, uint32_t nqt, uint32_t k_bytes,
-                                float levels, uint8_t* __restrict__ out, double* __restrict__ bound) {
+                                float levels, uint8_t* __restrict__ out, double* __restrict__ bound, Redo list) {
   __shared__ float fpart[32];
   __shared__ double dpart[32];
   const uint64_t q = blockIdx.x;
@@ -629,6 +631,7 @@ __global__ void fix_rank_kernel(const void* __restrict__ src, uint32_t dim, uint
   off = block_sum(off, dpart);
   l1 = block_sum(l1, dpart);
   if (threadIdx.x == 0) {
+    redo_clear(list, q);
     const double d = dim;
     if (SYM)
       bound[2 * q] = 2.0 * (1.0 + 2.5e-7 * d * (d * d - 1.0) / 12.0);
@@ -641,18 +644,18 @@ __global__ void fix_rank_kernel(const void* __restrict__ src, uint32_t dim, uint
   }
 }
 
-// flag |= 1 when a query's kp-th best value does not lie below its k-th best by
+// Marks a query whose kp-th best value does not lie below its k-th best by
 // the bound: some document outside the kp could then belong to the top k.
 // `centre`: RankQuant's final f32 rounding, 4 ulp of the centred value, is added.
 __global__ void score_margin_kernel(const uint32_t* __restrict__ sel, uint64_t nq, uint32_t kp, uint32_t k,
                                     const double* __restrict__ bound, uint32_t flip, bool centre,
-                                    uint32_t* __restrict__ flag) {
+                                    Redo failed) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
   const uint32_t a = sel[i * kp + (k - 1)] ^ flip, b = sel[i * kp + (kp - 1)] ^ flip;
   const double vk = centre ? (double)(int32_t)a : (double)a, vp = centre ? (double)(int32_t)b : (double)b;
   const double slack = bound[2 * i] + (centre ? 4.8e-7 * fabs(vk - bound[2 * i + 1]) : 0.0);
-  if (!(vp < vk - slack)) atomicOr(flag, 1u);
+  if (!(vp < vk - slack)) redo_mark(failed, (uint32_t)i);
 }
 
 // ---- exact rescoring of Rank candidates --------------------------------------------------
@@ -834,23 +837,24 @@ ScoreOperand score_operand(uint32_t src, uint64_t nq, uint32_t dim, uint32_t q_p
 }
 
 void launch_fix_rankquant(const float* q, uint64_t nq, uint32_t dim, uint32_t bits, bool half_steps,
-                          const ScoreOperand& b, double* bound, cudaStream_t stream) {
+                          const ScoreOperand& b, double* bound, const Redo& list, cudaStream_t stream) {
   if (!nq) return;
   fix_rankquant_kernel<<<(unsigned)nq, 256, 0, stream>>>(q, dim, bits, half_steps, b.nqt, b.k_bytes, (int8_t*)b.rows,
-                                                      bound);
+                                                      bound, list);
   launched();
 }
 
 void launch_fix_rank(bool sym, const void* q, uint64_t nq, uint32_t dim, const ScoreOperand& b, double* bound,
-                     cudaStream_t stream) {
+                     const Redo& list, cudaStream_t stream) {
   if (!nq) return;
   if (sym) {
-    fix_rank_kernel<true><<<(unsigned)nq, 256, 0, stream>>>(q, dim, b.nqt, b.k_bytes, 0.0f, (uint8_t*)b.rows, bound);
+    fix_rank_kernel<true><<<(unsigned)nq, 256, 0, stream>>>(q, dim, b.nqt, b.k_bytes, 0.0f, (uint8_t*)b.rows, bound,
+                                                      list);
   } else {
     const uint64_t sum_d = (uint64_t)dim * (dim - 1) / 2;
     const uint64_t levels = std::min<uint64_t>(65535, 0xFFFFFFFFull / sum_d);
     fix_rank_kernel<false><<<(unsigned)nq, 256, 0, stream>>>(q, dim, b.nqt, b.k_bytes, (float)levels,
-                                                             (uint8_t*)b.rows, bound);
+                                                             (uint8_t*)b.rows, bound, list);
   }
   launched();
 }
@@ -880,10 +884,10 @@ void launch_score_filter(const void* rows, uint64_t n, uint32_t dim, uint32_t sr
 }
 
 void launch_score_margin(const uint32_t* sel_keys, uint64_t nq, uint32_t kp, uint32_t k, const double* bound,
-                         uint32_t src, uint32_t* flag, cudaStream_t stream) {
+                         uint32_t src, const Redo& failed, cudaStream_t stream) {
   if (!nq) return;
   score_margin_kernel<<<(unsigned)((nq + 255) / 256), 256, 0, stream>>>(
-      sel_keys, nq, kp, k, bound, src == 16 ? SC<16>::kFlip : SC<1>::kFlip, src != 16, flag);
+      sel_keys, nq, kp, k, bound, src == 16 ? SC<16>::kFlip : SC<1>::kFlip, src != 16, failed);
   launched();
 }
 

@@ -82,7 +82,8 @@ __device__ void bitonic_sort(uint64_t* buf, uint32_t len) {
 template <int T, uint32_t CAP>
 __global__ void __launch_bounds__(T)
     select_rows_kernel(SelectArgs a, uint64_t* gbuf, uint32_t gbuf_stride) {
-  if (a.gate && !*a.gate) return;
+  if (a.err_dst && blockIdx.x == 0 && threadIdx.x == 0 && !redo_idle(a.redo)) *a.err_dst = a.err_src ? *a.err_src : 0u;
+  if (redo_skips(a.redo, blockIdx.x)) return;
   constexpr int BPT = kHistBins / T;  // histogram bins per thread in the scan
   __shared__ uint32_t hist[kHistBins];
   __shared__ uint32_t warp_tot[T / 32];
@@ -118,7 +119,6 @@ __global__ void __launch_bounds__(T)
       out_i[j] = id;
     }
   };
-  if (a.err_dst && row == 0 && threadIdx.x == 0) *a.err_dst = a.err_src ? *a.err_src : 0u;
   for (uint32_t j = k_eff + threadIdx.x; j < a.k; j += blockDim.x) put(j, kSentinelKey, kSentinelId);
   if (k_eff == 0) return;
 
@@ -325,7 +325,7 @@ constexpr uint64_t kClusterStageBytes = 160 * 1024;
 
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kSelThreads)
     select_rows_cluster_kernel(SelectArgs a, uint32_t stage) {
-  if (a.gate && !*a.gate) return;
+  if (redo_skips(a.redo, blockIdx.x / kClusterCtas)) return;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ uint32_t hist[kHistBins];
@@ -670,7 +670,7 @@ __device__ void grid_find_bin(const uint32_t (&h)[4], uint32_t need, uint32_t* o
 
 __global__ void __launch_bounds__(kGridThreads) grid_select_kernel(SelectArgs a, GridScratch w, uint32_t ctas,
                                                                    uint32_t stage) {
-  if (a.gate && !*a.gate) return;
+  if (redo_skips(a.redo, blockIdx.x / ctas)) return;
   // this CTA's candidates, then the row's; during the digits four copies of the
   // histogram (the first digits of float scores fall into few bins)
   __shared__ __align__(16) uint64_t buf[kSelectSmemCap];
@@ -904,7 +904,7 @@ void launch_select_rows(const SelectArgs& a, uint64_t rows, uint64_t* scratch,
   auto results = [&] {  // for the forms that leave keys
     if (a.res_scores)
       launch_keys_to_results(a.out_keys, a.out_ids, rows * a.k, a.res_mode, a.res_n_top, a.res_scores, a.res_ids,
-                             stream, a.err_src, a.err_dst, a.gate);
+                             stream, a.err_src, a.err_dst, a.redo, a.k);
   };
   if (select_takes_grid(a, rows, scratch) && launch_select_grid(a, rows, scratch, stream)) {
     results();
