@@ -8,11 +8,10 @@
 // Keys with equal (score, id) (duplicate candidate rows) are interchangeable:
 // any `need` of them give identical output, so no slot order is required.
 //
-// One CTA per row.  Per digit (11 bits at a time, most significant first,
-// skipping bits that are zero in every key) the CTA histograms the keys that
-// still match the fixed prefix, finds the bin holding the k-th key, and stops
-// as soon as that bin holds exactly the keys still needed.  A collect pass
-// then gathers the k winners and a bitonic sort orders them.
+// Forms: a CTA a row (even bins over the row's own keys), a cluster of eight CTAs a row
+// and the whole GPU for few long rows (digits of 11 bits, most significant first).  All
+// count keys into histograms until the bin of the k-th entry holds few enough, gather
+// what lies up to it and order the winners by a bitonic sort.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -74,13 +73,14 @@ __device__ void bitonic_sort(uint64_t* buf, uint32_t len) {
 // are all equal, by ids.  Bound by the passes over the row and the final sort; four loads
 // are in flight a thread, and a histogram of few bins has copies for the lanes.  Fixed
 // digits of 11 bits put most float keys of a row into a few bins (atomics on one
-// address) and took four to seven passes.  All launches of a call, us, then and now:
-// FastScan two-stage of 1,000 queries 146 / 106, multi-bucket 106 / 59, three RankQuant
-// searches of 1,024 / 2,048 / 1,024 queries 808 / 552, Rank of 64 59 / 48; integer keys of a
-// 10M-document bitmap batch (1,024 rows of 39,063 and of 10,000) 298 / 322, with the
-// reranks' 361 / 370.
+// address) and took four to seven passes.  Registers are held to what lets two CTAs of
+// 1,024 threads, or five of 256, share an SM: integer keys (1,024 rows of 39,063 and of
+// 10,000 of a 10M-document bitmap batch) take 264 us so, 319 with one CTA of 1,024, and
+// 279 in fixed digits; float keys are the same either way.  All launches of a call, us,
+// in fixed digits and now: FastScan two-stage of 1,000 queries 146 / 107, multi-bucket 106 /
+// 58, three RankQuant searches of 1,365 queries each 808 / 569, Rank of 64 59 / 47.
 template <int T, uint32_t CAP>
-__global__ void __launch_bounds__(T)
+__global__ void __launch_bounds__(T, T == 1024 ? 2 : 5)
     select_rows_kernel(SelectArgs a, uint64_t* gbuf, uint32_t gbuf_stride) {
   if (a.err_dst && blockIdx.x == 0 && threadIdx.x == 0 && !redo_idle(a.redo)) *a.err_dst = a.err_src ? *a.err_src : 0u;
   if (redo_skips(a.redo, blockIdx.x)) return;
