@@ -141,12 +141,6 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, b
          "FastScan v1: incremental add() not supported (block-32 layout); construct a new index");
   if (ix.kind != OVB_INDEX_KIND_SIGN_BITMAP && ix.dim > kMaxDeviceRankDim)
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "device rank transform supports dim <= 16384");
-  uint32_t *flag = nullptr, *h = nullptr;
-  if (check) {
-    flag = (uint32_t*)w.flag.ensure(4);
-    h = (uint32_t*)w.pinned.ensure(4);
-    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
-  }
   DevBuf fresh;
   void* codes;
   try {
@@ -155,6 +149,12 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, b
     cudaGetLastError();
     if (check) need_finite_rows(ix, d_vecs, n, w);
     throw;
+  }
+  uint32_t *flag = nullptr, *h = nullptr;
+  if (check) {
+    flag = (uint32_t*)w.flag.ensure(4);
+    h = (uint32_t*)w.pinned.ensure(4);
+    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
   }
   launch_encode((int)encode_kind(ix.kind), d_vecs, n, ix.dim, ix.bits, ix.n_top, ix.pairs_pad, codes, ix.n, flag,
                 w.stream);
