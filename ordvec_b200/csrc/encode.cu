@@ -25,12 +25,17 @@
 // boundary are resolved.  One warp takes a row up to dim 1024 (eight rows per
 // CTA, no CTA barrier), four warps one up to 4096.  Rows that bin badly (a
 // crowded bin: heavy ties or outliers; a zero range; non-finite values) are
-// flagged and done by the whole CTA with the bitonic sort of the sorted form,
-// which also serves dim > 4096.
+// sorted instead, in the same launch: by their warp up to dim 512, by the whole
+// CTA above; dim > 4096 is always sorted.
 // What bounds it: issue slots (66 % busy) and shared-memory wavefronts (58 %)
-// of the histogram, about 50 instructions per 32 values at dim 768.
+// of the histogram, about 50 instructions per 32 values at dim 768; registers, hence
+// the CTAs an SM (rank_bins_kernel of dim 768 b=2: 86 us for 40,000 rows at three
+// CTAs of 80 registers, 104 at two of 111); in the sorted form its shuffles.
 // Measured, 120,000 rows of dim 768, RankQuant b=2: 0.25 ms = 1.5 TB/s of
-// input, from 4.8 ms by sorting every row.
+// input, from 4.8 ms by sorting every row through shared memory.  40,000 rows that are all
+// sorted (values below zero set to zero; us, all rows through shared memory and now): dim
+// 768 b=2 1,563 / 860, dim 1024 multi-bucket b=2 1,822 / 1,030, dim 512 Rank 678 / 254; 10,000
+// of dim 4096 b=4 2,023 / 920.
 #include "ovb_common.cuh"
 #include "ovb_kernels.h"
 
@@ -38,20 +43,54 @@ namespace ovb {
 
 namespace {
 
-__device__ void enc_bitonic(uint64_t* buf, uint32_t len) {
-  for (uint32_t size = 2; size <= len; size <<= 1)
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t t = threadIdx.x; t < len / 2; t += blockDim.x) {
-        uint32_t i = 2 * t - (t & (stride - 1)), j = i + stride;
-        bool up = (i & size) == 0;
-        uint64_t a = buf[i], b = buf[j];
-        if ((a > b) == up) {
-          buf[i] = b;
-          buf[j] = a;
+// Bitonic sort of EL keys a thread over T threads (t = 0 .. T - 1: a warp, or a CTA of a
+// power of two of threads).  Key e of thread t is entry t * EL + e: steps of fewer than
+// EL entries stay in a thread's registers, steps of fewer than 32 EL are shuffles, and
+// only the longer ones go through `ex` (T * EL keys) between barriers.
+template <int EL>
+__device__ __forceinline__ void enc_sort(uint64_t (&x)[EL], uint32_t t, uint32_t T, uint64_t* ex) {
+  auto order = [&](uint64_t& lo, uint64_t& hi, bool up) {
+    if ((lo > hi) == up) {
+      const uint64_t y = lo;
+      lo = hi;
+      hi = y;
+    }
+  };
+#pragma unroll
+  for (int size = 2; size <= EL; size <<= 1)
+#pragma unroll
+    for (int stride = size / 2; stride > 0; stride >>= 1)
+#pragma unroll
+      for (int e = 0; e < EL; e++)
+        if (!(e & stride)) order(x[e], x[e | stride], size < EL ? !(e & size) : !(t & 1));
+  for (uint32_t ts = 2; ts <= T; ts <<= 1) {  // threads a sorted run takes
+    const bool up = !(t & ts);
+    for (uint32_t d = ts / 2; d > 0; d >>= 1) {
+      const bool low = up == !(t & d);  // this thread keeps the smaller of each two
+      if (d >= 32) {
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < EL; e++) ex[e * T + t] = x[e];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < EL; e++) {
+          const uint64_t y = ex[e * T + (t ^ d)];
+          x[e] = (x[e] < y) == low ? x[e] : y;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < EL; e++) {
+          const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, (unsigned long long)x[e], d);
+          x[e] = (x[e] < y) == low ? x[e] : y;
         }
       }
-      __syncthreads();
     }
+#pragma unroll
+    for (int stride = EL / 2; stride > 0; stride >>= 1)
+#pragma unroll
+      for (int e = 0; e < EL; e++)
+        if (!(e & stride)) order(x[e], x[e | stride], up);
+  }
 }
 
 struct EncArgs {
@@ -84,33 +123,45 @@ __device__ __forceinline__ uint32_t bucket_end(const EncArgs& a, uint32_t bucket
 // the value that is ranked ascending: -0.0 equals +0.0
 __device__ __forceinline__ float ranked_value(const EncArgs& a, float v) { return (a.kind == 7 ? -v : v) + 0.0f; }
 
-// Sorted form of one row by the whole CTA: bitonic sort of (value key, index),
-// sorted position = rank, then emission.  sk: len (power of two >= dim) keys
-// and dim u16 ranks.
-__device__ void encode_row_sorted(const EncArgs& a, uint64_t d, uint32_t len, uint64_t* sk) {
-  uint16_t* rank = (uint16_t*)(sk + len);
+__host__ __device__ constexpr uint32_t enc_rank_pad(uint32_t dim) { return (dim + 7) / 8 * 8; }
+
+// Sorted form of one row by a warp (WARP) or the whole CTA, T threads, T * EL >= dim: sort of
+// (value key, index), sorted position = rank, then emission.  rank: dim u16, then (CTA)
+// from the next multiple of 16 bytes T * EL keys.  Out of line: the binned form's registers are
+// not its.
+template <int EL, bool WARP>
+__device__ __noinline__ void encode_row_sorted(const EncArgs a, uint64_t d, uint16_t* rank) {
+  const uint32_t tid = WARP ? threadIdx.x & 31 : threadIdx.x, T = WARP ? 32 : blockDim.x;
+  auto sync = [] {
+    if (WARP)
+      __syncwarp();
+    else
+      __syncthreads();
+  };
   const int kind = a.kind;
   const uint32_t dim = a.dim, bits = a.bits, pairs_pad = a.pairs_pad;
   void* out = a.out;
   const float* v = a.vecs + d * dim;
   const uint64_t doc = a.first_doc + d;
-  for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) {
-    if (j < dim) {
-      float x = v[j];
-      x = x == 0.0f ? 0.0f : x;
-      sk[j] = ((uint64_t)(kind == 7 ? desc_key(x) : asc_key(x)) << 32) | j;
-    } else {
-      sk[j] = ~0ull;
-    }
+  uint64_t key[EL];
+#pragma unroll
+  for (int e = 0; e < EL; e++) {
+    const uint32_t j = e * T + tid;
+    const float x = j < dim ? ranked_value(a, v[j]) : 0.0f;
+    key[e] = j < dim ? ((uint64_t)asc_key(x) << 32) | j : ~0ull;
   }
-  __syncthreads();
-  enc_bitonic(sk, len);
-  for (uint32_t p = threadIdx.x; p < dim; p += blockDim.x) rank[(uint32_t)sk[p]] = (uint16_t)p;
-  __syncthreads();
+  enc_sort<EL>(key, tid, T, (uint64_t*)(rank + enc_rank_pad(dim)));
+  sync();  // the warp form: what lay there is no longer read
+#pragma unroll
+  for (int e = 0; e < EL; e++) {
+    const uint32_t p = tid * EL + e;
+    if (p < dim) rank[(uint32_t)key[e]] = (uint16_t)p;
+  }
+  sync();
   if (kind == 0) {
     const uint32_t cpb = 8 / bits, bpv = dim * bits / 8;
     uint8_t* o = (uint8_t*)out + doc * bpv;
-    for (uint32_t t = threadIdx.x; t < bpv; t += blockDim.x) {
+    for (uint32_t t = tid; t < bpv; t += T) {
       uint32_t byte = 0;
       for (uint32_t i = 0; i < cpb; i++) {
         uint32_t j = t * cpb + i;
@@ -120,19 +171,16 @@ __device__ void encode_row_sorted(const EncArgs& a, uint64_t d, uint32_t len, ui
       o[t] = (uint8_t)byte;
     }
   } else if (kind == 2 || kind == 7) {
-    const uint32_t qpv = dim / 64;
-    uint64_t* o = (uint64_t*)out + doc * qpv;
-    for (uint32_t w = threadIdx.x; w < qpv; w += blockDim.x) {
-      uint64_t word = 0;
-      for (int j = 0; j < 64; j++)
-        if (bucket_of(a, rank[w * 64 + j])) word |= 1ull << j;
-      o[w] = word;
+    uint32_t* o = (uint32_t*)out + doc * (dim / 32);
+    for (uint32_t j = tid; j < dim; j += T) {  // whole warps: dim % 64 == 0
+      const uint32_t word = __ballot_sync(0xFFFFFFFFu, bucket_of(a, rank[j]));
+      if (j % 32 == 0) o[j / 32] = word;
     }
   } else if (kind == 3) {
     const uint32_t pairs = dim / 2;
     const uint64_t blk = doc / 32, lane = doc % 32;
     uint8_t* o = (uint8_t*)out + blk * (uint64_t)pairs_pad * 16;
-    for (uint32_t t = threadIdx.x; t < pairs_pad / 2; t += blockDim.x) {
+    for (uint32_t t = tid; t < pairs_pad / 2; t += T) {
       uint32_t g = t / 16, b = t % 16, nib[2];
       for (int h = 0; h < 2; h++) {
         uint32_t p = g * 32 + 2 * b + h;
@@ -148,35 +196,34 @@ __device__ void encode_row_sorted(const EncArgs& a, uint64_t d, uint32_t len, ui
     }
   } else if (kind == 5) {
     uint16_t* o = (uint16_t*)out + doc * dim;
-    for (uint32_t j = threadIdx.x; j < dim; j += blockDim.x) o[j] = rank[j];
+    for (uint32_t j = tid; j < dim; j += T) o[j] = rank[j];
   } else if (kind == 6) {
     float* o = (float*)out + doc * dim;
     const float centre = ((float)(1u << bits) - 1.0f) / 2.0f;
-    for (uint32_t j = threadIdx.x; j < dim; j += blockDim.x)
+    for (uint32_t j = tid; j < dim; j += T)
       o[j] = (float)(uint32_t)(((uint64_t)rank[j] << bits) / dim) - centre;
   } else {  // kind 4
-    const uint32_t qpb = dim / 64, nb = 1u << bits;
-    uint64_t* o = (uint64_t*)out + doc * (uint64_t)nb * qpb;
-    for (uint32_t t = threadIdx.x; t < nb * qpb; t += blockDim.x) {
-      const uint32_t bucket = t / qpb, w = t % qpb;
-      uint64_t word = 0;
-      for (int j = 0; j < 64; j++) {
-        uint32_t b = (uint32_t)(((uint64_t)rank[w * 64 + j] << bits) / dim);
-        if (b == bucket) word |= 1ull << j;
+    const uint32_t nb = 1u << bits;
+    uint32_t* o = (uint32_t*)out + doc * (uint64_t)nb * (dim / 32);
+    for (uint32_t j = tid; j < dim; j += T) {
+      const uint32_t code = bucket_of(a, rank[j]);
+      for (uint32_t b = 0; b < nb; b++) {
+        const uint32_t word = __ballot_sync(0xFFFFFFFFu, code == b);
+        if (j % 32 == 0) o[b * (dim / 32) + j / 32] = word;
       }
-      o[t] = word;
     }
   }
 }
 
-__global__ void rank_encode_kernel(EncArgs a, uint32_t len) {
-  extern __shared__ __align__(16) uint64_t sk[];
+template <int EL>
+__global__ void __launch_bounds__(512) rank_encode_kernel(EncArgs a) {
+  extern __shared__ __align__(16) uint16_t ranks[];
   if (a.flag) {
     bool bad = false;
     for (uint32_t j = threadIdx.x; j < a.dim; j += blockDim.x) bad |= !isfinite(a.vecs[(uint64_t)blockIdx.x * a.dim + j]);
     if (bad) atomicOr(a.flag, 1u);
   }
-  encode_row_sorted(a, blockIdx.x, len, sk);
+  encode_row_sorted<EL, false>(a, blockIdx.x, ranks);
 }
 
 constexpr uint32_t kListCap = 128;  // values of boundary bins a row resolves by comparison
@@ -191,10 +238,24 @@ __host__ __device__ constexpr uint32_t enc_row_bytes(int W, int NI, int BPT, boo
   return enc_tab_words(W, BPT) * 4 + (full ? 32u * W * NI * 8 : 32u * W * NI + kListCap * 10) + 64;
 }
 
+// The sorted form in the same launch: rows of up to 512 by their own warp, in its part of the
+// shared memory (its keys fit the registers); longer ones by the CTA, one after another.
+__host__ __device__ constexpr bool enc_warp_sorts(int W, int NI) { return W == 1 && NI <= 16; }
+__host__ __device__ constexpr int enc_sort_keys(int W, int NI) {  // a thread
+  int keys = 1;
+  while (keys * (enc_warp_sorts(W, NI) ? 32 : W == 1 ? 256 : 32 * W) < 32 * W * NI) keys *= 2;
+  return keys;
+}
+
+// CTAs an SM that the binned form's registers leave room for
+__host__ __device__ constexpr int enc_ctas(int W, int NI) {
+  return W == 1 ? (NI <= 16 ? 4 : NI == 24 ? 3 : 2) : NI == 16 ? 8 : 4;
+}
+
 // W warps per row, NI values per thread (dim <= 32 W NI, EXACT: equal), BPT
 // bins per thread.
 template <int W, int NI, int BPT, bool FULL, bool EXACT>
-__global__ void __launch_bounds__(W == 1 ? 256 : 32 * W) rank_bins_kernel(EncArgs a, uint32_t len) {
+__global__ void __launch_bounds__(W == 1 ? 256 : 32 * W, enc_ctas(W, NI)) rank_bins_kernel(EncArgs a) {
   constexpr int T = 32 * W, GROUPS = W == 1 ? 8 : 1;
   constexpr uint32_t B = enc_bins(W, BPT), CAP = 32u * W * NI;
   extern __shared__ __align__(16) uint8_t smem[];
@@ -477,12 +538,19 @@ uint32_t held = 0;  // W == 1: values in the list so far
       }
     }
   }
-  if (tid == 0) s_slow[group] = slow ? 1u : 0u;
-  __syncthreads();
-  for (int g = 0; g < GROUPS; g++) {
-    if (!s_slow[g]) continue;  // uniform
-    encode_row_sorted(a, (uint64_t)blockIdx.x * GROUPS + g, len, (uint64_t*)smem);
+  constexpr int KEYS = enc_sort_keys(W, NI);
+  if constexpr (enc_warp_sorts(W, NI)) {
+    static_assert(enc_row_bytes(W, NI, BPT, FULL) >= 64u * W * NI, "the ranks of a row");
+    __syncwarp();
+    if (slow) encode_row_sorted<KEYS, true>(a, d, (uint16_t*)tab);  // uniform over the warp
+  } else {
+    if (tid == 0) s_slow[group] = slow ? 1u : 0u;
     __syncthreads();
+    for (int g = 0; g < GROUPS; g++) {
+      if (!s_slow[g]) continue;  // uniform
+      encode_row_sorted<KEYS, false>(a, (uint64_t)blockIdx.x * GROUPS + g, (uint16_t*)smem);
+      __syncthreads();
+    }
   }
 }
 
@@ -525,15 +593,24 @@ void launch_multibucket_query(const float* q, uint64_t nq, uint32_t dim, uint32_
 
 namespace {
 template <int W, int NI, int BPT, bool FULL>
-void launch_bins_as(const EncArgs& a, uint32_t len, cudaStream_t stream) {
+void launch_bins_as(const EncArgs& a, cudaStream_t stream) {
   const bool exact = W == 1 && a.dim == 32u * W * NI;
   auto kernel = exact ? rank_bins_kernel<W, NI, BPT, FULL, W == 1> : rank_bins_kernel<W, NI, BPT, FULL, false>;
   allow_dynamic_smem(kernel);
   const uint32_t groups = W == 1 ? 8 : 1;
   size_t smem = (size_t)groups * enc_row_bytes(W, NI, BPT, FULL);
-  const size_t sorted = (size_t)len * 8 + (size_t)a.dim * 2;
-  if (smem < sorted) smem = sorted;
-  kernel<<<ceil_div(a.n, groups), W == 1 ? 256 : 32 * W, smem, stream>>>(a, len);
+  const unsigned threads = W == 1 ? 256 : 32 * W;
+  const size_t sorted = (size_t)threads * enc_sort_keys(W, NI) * 8 + (size_t)enc_rank_pad(a.dim) * 2;
+  if (!enc_warp_sorts(W, NI) && smem < sorted) smem = sorted;
+  kernel<<<ceil_div(a.n, groups), threads, smem, stream>>>(a);
+  launched();
+}
+
+template <int EL>
+void launch_sorted(const EncArgs& a, cudaStream_t stream) {
+  auto kernel = rank_encode_kernel<EL>;
+  allow_dynamic_smem(kernel);
+  kernel<<<(unsigned)a.n, 512, 512 * EL * 8 + (size_t)enc_rank_pad(a.dim) * 2, stream>>>(a);
   launched();
 }
 
@@ -541,14 +618,14 @@ void launch_bins_as(const EncArgs& a, uint32_t len, cudaStream_t stream) {
 // Up to four buckets resolve three bins at most, so half as many bins, whose
 // prefix sum costs half, do.
 template <int W, int NI, int BPT>
-void launch_bins(const EncArgs& a, uint32_t len, cudaStream_t stream) {
+void launch_bins(const EncArgs& a, cudaStream_t stream) {
   const bool bitmap = a.kind == 2 || a.kind == 7;
   if (a.kind == 5)
-    launch_bins_as<W, NI, BPT, true>(a, len, stream);
+    launch_bins_as<W, NI, BPT, true>(a, stream);
   else if (bitmap || a.bits <= 2)
-    launch_bins_as<W, NI, (BPT > 8 ? BPT / 2 : BPT), false>(a, len, stream);
+    launch_bins_as<W, NI, (BPT > 8 ? BPT / 2 : BPT), false>(a, stream);
   else
-    launch_bins_as<W, NI, BPT, false>(a, len, stream);
+    launch_bins_as<W, NI, BPT, false>(a, stream);
 }
 }  // namespace
 
@@ -560,34 +637,29 @@ void launch_encode(int kind, const float* vecs, uint64_t n, uint32_t dim, uint32
     launch_sign_encode(vecs, n, dim, (uint64_t*)out + first_doc * (dim / 64), flag, stream);
     return;
   }
-  uint32_t len = 1;
-  while (len < dim) len <<= 1;
-  const size_t smem = (size_t)len * 8 + (size_t)dim * 2;
-  if (smem > 227 * 1024) throw std::invalid_argument("dim too large for the device rank transform");
-  allow_dynamic_smem(rank_encode_kernel);
-  const unsigned threads = len >= 1024 ? 512 : 256;
+  if (dim > 16384) throw std::invalid_argument("dim too large for the device rank transform");
   for (uint64_t d0 = 0; d0 < n; d0 += 0x7FFFFFFF) {
     const uint64_t cnt = n - d0 < 0x7FFFFFFF ? n - d0 : 0x7FFFFFFF;
     const EncArgs a{kind, vecs + d0 * dim, cnt, dim, bits, n_top, pairs_pad, out, first_doc + d0,
                     0xFFFFFFFFu / dim + 1u, flag};
     if (dim <= 256)
-      launch_bins<1, 8, 8>(a, len, stream);
+      launch_bins<1, 8, 8>(a, stream);
     else if (dim <= 384)
-      launch_bins<1, 12, 16>(a, len, stream);
+      launch_bins<1, 12, 16>(a, stream);
     else if (dim <= 512)
-      launch_bins<1, 16, 16>(a, len, stream);
+      launch_bins<1, 16, 16>(a, stream);
     else if (dim <= 768)
-      launch_bins<1, 24, 32>(a, len, stream);
+      launch_bins<1, 24, 32>(a, stream);
     else if (dim <= 1024)
-      launch_bins<1, 32, 32>(a, len, stream);
+      launch_bins<1, 32, 32>(a, stream);
     else if (dim <= 2048)
-      launch_bins<4, 16, 16>(a, len, stream);
+      launch_bins<4, 16, 16>(a, stream);
     else if (dim <= 4096)
-      launch_bins<4, 32, 32>(a, len, stream);
-    else {
-      rank_encode_kernel<<<(unsigned)cnt, threads, smem, stream>>>(a, len);
-      launched();
-    }
+      launch_bins<4, 32, 32>(a, stream);
+    else if (dim <= 8192)
+      launch_sorted<16>(a, stream);
+    else
+      launch_sorted<32>(a, stream);
   }
 }
 
