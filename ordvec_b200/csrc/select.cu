@@ -67,18 +67,21 @@ __device__ void bitonic_sort(uint64_t* buf, uint32_t len) {
 //
 // The k-th smallest (key, id) is found by histograms of 2,048 bins that divide the
 // row's own range of keys evenly: the first pass over the row takes its minimum and
-// maximum (keys of at most 11 bits need none), the second the histogram, and where the
-// bin of the k-th entry then holds at most kSelTies entries a third collects what lies
-// below it and ranks the bin's.  A fuller bin is divided again, by keys and, where they
-// are all equal, by ids.  Bound by the passes over the row and the final sort; four loads
-// are in flight a thread, and a histogram of few bins has copies for the lanes.  Fixed
-// digits of 11 bits put most float keys of a row into a few bins (atomics on one
-// address) and took four to seven passes.  Registers are held to what lets two CTAs of
-// 1,024 threads, or five of 256, share an SM: integer keys (1,024 rows of 39,063 and of
-// 10,000 of a 10M-document bitmap batch) take 264 us so, 319 with one CTA of 1,024, and
-// 279 in fixed digits; float keys are the same either way.  All launches of a call, us,
-// in fixed digits and now: FastScan two-stage of 1,000 queries 146 / 107, multi-bucket 106 /
-// 58, three RankQuant searches of 1,365 queries each 808 / 569, Rank of 64 59 / 47.
+// maximum (keys of at most 11 bits need none), the second the histogram, and a third
+// collects what lies up to the bin of the k-th entry where that is no more than the final
+// sort takes anyway (the next power of two of k), or, where the bin holds at most
+// kSelTies entries, what lies below it and the bin's, ranked.  A fuller bin is divided
+// again, by keys and, where they are all equal, by ids.  Four loads are in flight a
+// thread, a warp votes once for its four collects (one atomic where it has any), ids are
+// read for what is kept only, and a histogram of few bins has copies for the lanes.
+// Bound by the passes over the row and the final sort.  Fixed digits of 11 bits put most
+// float keys of a row into a few bins (atomics on one address) and took four to seven
+// passes.  Registers are held to what lets two CTAs of 1,024 threads, or five of 256, share
+// an SM (one of 1,024: 319 us for the integer keys below; six or eight of 256: 1 to 9 %
+// slower).  All launches of a call, us, in fixed digits and now: integer keys of a
+// 10M-document bitmap batch (1,024 rows of 39,063 and of 10,000) 279 / 230, FastScan
+// two-stage of 1,000 queries 146 / 101, multi-bucket 106 / 54, three RankQuant searches of
+// 1,365 queries each 808 / 466, Rank of 64 59 / 39.
 template <int T, uint32_t CAP>
 __global__ void __launch_bounds__(T, T == 1024 ? 2 : 5)
     select_rows_kernel(SelectArgs a, uint64_t* gbuf, uint32_t gbuf_stride) {
@@ -92,18 +95,19 @@ __global__ void __launch_bounds__(T, T == 1024 ? 2 : 5)
   __shared__ uint64_t tbuf[kSelTies];
 
   const uint64_t row = blockIdx.x;
-  uint64_t start, n;
+  uint64_t start;
+  uint32_t n;  // counts are 32 bits
   if (a.row_off) {
     start = a.row_off[row];
-    n = a.row_off[row + 1] - start;
+    n = (uint32_t)(a.row_off[row + 1] - start);
   } else {
     start = row * a.ld;
-    n = a.n;
+    n = (uint32_t)a.n;
     if (a.row_len && a.row_len[row] < n) n = a.row_len[row];
   }
   const uint32_t* keys = a.keys + start;
   const uint32_t* ids = a.ids ? a.ids + start : nullptr;
-  const uint32_t k_eff = (uint32_t)(n < a.k ? n : a.k);
+  const uint32_t k_eff = n < a.k ? n : a.k;
   uint32_t* out_k = a.out_keys + row * (uint64_t)a.k;
   uint32_t* out_i = a.out_ids + row * (uint64_t)a.k;
 
@@ -124,36 +128,39 @@ __global__ void __launch_bounds__(T, T == 1024 ? 2 : 5)
 
   uint64_t* buf = (k_eff <= CAP) ? sbuf : gbuf + row * (uint64_t)gbuf_stride;
 
-  // f(key, id) for every entry of the row (id only with want_ids), four loads in flight;
-  // whole warps call f together
-  auto each = [&](bool want_ids, auto&& f) {
-    const uint64_t padded = (n + 31) / 32 * 32;
-    for (uint64_t i0 = threadIdx.x; i0 < padded; i0 += 4 * T) {
-      uint32_t kk[4], ii[4];
+  // f(keys, first) for every entry of the row, four loads in flight: entry j of four is
+  // first + j T (past the row where first + j T >= n); whole warps call f together
+  auto each = [&](auto&& f) {
+    const uint32_t padded = (n + 31) / 32 * 32;
+    for (uint32_t i0 = threadIdx.x; i0 < padded; i0 += 4 * T) {
+      uint32_t kk[4];
 #pragma unroll
-      for (uint32_t j = 0; j < 4; j++) {
-        const uint64_t i = i0 + j * T;
-        kk[j] = i < n ? keys[i] : 0u;
-        ii[j] = want_ids && i < n ? (ids ? ids[i] : (uint32_t)i) : 0u;
-      }
-#pragma unroll
-      for (uint32_t j = 0; j < 4; j++)
-        if (i0 + j * T < padded) f(kk[j], ii[j], i0 + j * T < n);
+      for (uint32_t j = 0; j < 4; j++) kk[j] = i0 + j * T < n ? keys[i0 + j * T] : 0u;
+      f(kk, i0);
     }
   };
+  auto id_of = [&](uint32_t i) -> uint32_t { return ids ? ids[i] : i; };
   const uint32_t t = threadIdx.x;
   const int lane = t & 31, w = t >> 5;
   const bool take_all = k_eff == n;
   // part 0: keys in [base, base + 2^sh) hold the need-th of the entries not below them;
   // part 1: so do ids, of the entries whose key is `same`
-  uint32_t part = 0, base = 0, same = 0, sh = 0, need = k_eff;
+  uint32_t part = 0, base = 0, same = 0, sh = 0, need = k_eff, in_bin = k_eff;
+  // the entries up to the bin's end are no more than the final sort takes anyway
+  uint32_t len = 1;
+  while (len < k_eff) len <<= 1;
+  auto sorts_all = [&]() { return !a.unordered && k_eff - need + in_bin <= len; };
   if (!take_all) {
     uint32_t used = 1u << (a.key_bits < 11 ? a.key_bits : 11);  // bins that can be hit
     if (a.key_bits > 11) {
       uint32_t mn = 0xFFFFFFFFu, mx = 0;
-      each(false, [&](uint32_t key, uint32_t, bool in) {
-        mn = in && key < mn ? key : mn;
-        mx = in && key > mx ? key : mx;
+      each([&](const uint32_t (&kk)[4], uint32_t i0) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) {
+          const bool in = i0 + j * T < n;
+          mn = in && kk[j] < mn ? kk[j] : mn;
+          mx = in && kk[j] > mx ? kk[j] : mx;
+        }
       });
       mn = __reduce_min_sync(0xFFFFFFFFu, mn);
       mx = __reduce_max_sync(0xFFFFFFFFu, mx);
@@ -178,9 +185,13 @@ __global__ void __launch_bounds__(T, T == 1024 ? 2 : 5)
       // few bins: 2^copies of each, the lanes in turn, so that equal keys of a warp meet less
       const uint32_t copies = used <= kHistBins / 4 ? min(31 - __clz(kHistBins / used), 5) : 0;
       const uint32_t copy = lane & ((1u << copies) - 1);
-      each(part != 0, [&](uint32_t key, uint32_t id, bool in) {
-        const uint32_t x = part ? id : key, bin = (x - base) >> sh;
-        if (in && (!part || key == same) && x >= base && bin < kHistBins) atomicAdd(&hist[bin << copies | copy], 1u);
+      each([&](const uint32_t (&kk)[4], uint32_t i0) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) {
+          if (i0 + j * T >= n || (part && kk[j] != same)) continue;
+          const uint32_t x = part ? id_of(i0 + j * T) : kk[j], bin = (x - base) >> sh;
+          if (x >= base && bin < kHistBins) atomicAdd(&hist[bin << copies | copy], 1u);
+        }
       });
       __syncthreads();
       if (copies) {  // used <= 512
@@ -240,9 +251,9 @@ __global__ void __launch_bounds__(T, T == 1024 ? 2 : 5)
       __syncthreads();
       need -= s_before;
       base += s_bin << sh;
-      const uint32_t in_bin = s_in_bin;
+      in_bin = s_in_bin;
       __syncthreads();
-      if (in_bin == need || in_bin <= kSelTies) break;
+      if (in_bin == need || in_bin <= kSelTies || sorts_all()) break;
       if (sh) {
         sh = sh > 11 ? sh - 11 : 0;
       } else if (!part) {
@@ -256,51 +267,69 @@ __global__ void __launch_bounds__(T, T == 1024 ? 2 : 5)
     }
   }
 
-  // collect: what lies below the bin, then the bin's `need` smallest
+  // collect: what lies below the bin, and the bin's entries: all of them with the others
+  // (they are all needed, or the sort sorts them out), or apart, to rank them
   if (t == 0) {
     s_cnt_below = 0;
     s_cnt_tie = 0;
   }
   __syncthreads();
-  const uint32_t below_total = take_all ? k_eff : k_eff - need;
-  const bool rank_ties = !take_all && s_in_bin <= kSelTies && s_in_bin != need;
+  const bool together = take_all || in_bin == need || sorts_all(), rank_ties = !together && in_bin <= kSelTies;
+  const uint32_t below_total = take_all ? k_eff : together ? k_eff - need + in_bin : k_eff - need;
   uint32_t lt;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-  each(true, [&](uint32_t key, uint32_t id, bool in) {
-    const uint32_t x = part ? id : key;
-    const bool here = !part || key == same;  // the bin's range applies
-    const bool below = in && (take_all || (here ? x < base : key < same));
-    const bool tie = in && !take_all && here && x >= base && (x - base) >> sh == 0;
-    const uint32_t bb = __ballot_sync(0xFFFFFFFFu, below);
-    if (bb) {
-      uint32_t at = 0;
-      if (lane == 0) at = atomicAdd(&s_cnt_below, (uint32_t)__popc(bb));
-      at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(bb & lt);
-      if (below && at < below_total) buf[at] = ((uint64_t)key << 32) | id;
+  each([&](const uint32_t (&kk)[4], uint32_t i0) {
+    uint32_t hit = 0;  // bit j: entry j is below, bit 4 + j: in the bin
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+      if (i0 + j * T >= n) continue;
+      const bool here = !part || kk[j] == same;  // the bin's range applies
+      const uint32_t x = part && here ? id_of(i0 + j * T) : kk[j];
+      const bool below = take_all || (here ? x < base : kk[j] < same);
+      const bool tie = !below && here && (x - base) >> sh == 0;
+      hit |= ((uint32_t)(below || (tie && together)) | (uint32_t)(tie && !together) << 4) << j;
     }
-    if (tie) {
-      const uint32_t tk = atomicAdd(&s_cnt_tie, 1u);
-      if (rank_ties)
-        tbuf[tk] = ((uint64_t)key << 32) | id;  // tk < s_in_bin <= kSelTies
-      else if (tk < need)
-        buf[below_total + tk] = ((uint64_t)key << 32) | id;
+    if (!__any_sync(0xFFFFFFFFu, hit != 0)) return;
+    uint32_t bb[4], all = 0, at = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+      bb[j] = __ballot_sync(0xFFFFFFFFu, hit >> j & 1);
+      all += __popc(bb[j]);
+    }
+    if (all) {
+      if (lane == 0) at = atomicAdd(&s_cnt_below, all);
+      at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+      if (hit >> j & 17) {
+        const uint64_t entry = ((uint64_t)kk[j] << 32) | id_of(i0 + j * T);
+        if (hit >> j & 1) {
+          const uint32_t slot = at + __popc(bb[j] & lt);
+          if (slot < below_total) buf[slot] = entry;
+        } else {
+          const uint32_t tk = atomicAdd(&s_cnt_tie, 1u);
+          if (rank_ties)
+            tbuf[tk] = entry;  // tk < in_bin <= kSelTies
+          else if (tk < need)
+            buf[below_total + tk] = entry;
+        }
+      }
+      at += __popc(bb[j]);
     }
   });
   __syncthreads();
   if (rank_ties) {
-    const uint32_t c = s_in_bin;
-    if (t < c) {
+    if (t < in_bin) {
       const uint64_t mine = tbuf[t];
       uint32_t rank = 0;
-      for (uint32_t i = 0; i < c; i++) rank += tbuf[i] < mine || (tbuf[i] == mine && i < t);
+      for (uint32_t i = 0; i < in_bin; i++) rank += tbuf[i] < mine || (tbuf[i] == mine && i < t);
       if (rank < need) buf[below_total + rank] = mine;
     }
     __syncthreads();
   }
   if (!a.unordered) {  // a caller that needs only the set skips the sort
-    uint32_t len = 1;
-    while (len < k_eff) len <<= 1;
-    for (uint32_t j = k_eff + threadIdx.x; j < len; j += blockDim.x) buf[j] = ~0ull;
+    for (uint32_t j = (together ? below_total : k_eff) + threadIdx.x; j < len; j += blockDim.x) buf[j] = ~0ull;
     __syncthreads();
     bitonic_sort(buf, len);
   }
