@@ -607,10 +607,10 @@ void launch_bins_as(const EncArgs& a, cudaStream_t stream) {
 }
 
 template <int EL>
-void launch_sorted(const EncArgs& a, cudaStream_t stream) {
+void launch_sorted(const EncArgs& a, unsigned threads, cudaStream_t stream) {
   auto kernel = rank_encode_kernel<EL>;
   allow_dynamic_smem(kernel);
-  kernel<<<(unsigned)a.n, 512, 512 * EL * 8 + (size_t)enc_rank_pad(a.dim) * 2, stream>>>(a);
+  kernel<<<(unsigned)a.n, threads, threads * (size_t)EL * 8 + (size_t)enc_rank_pad(a.dim) * 2, stream>>>(a);
   launched();
 }
 
@@ -642,7 +642,15 @@ void launch_encode(int kind, const float* vecs, uint64_t n, uint32_t dim, uint32
     const uint64_t cnt = n - d0 < 0x7FFFFFFF ? n - d0 : 0x7FFFFFFF;
     const EncArgs a{kind, vecs + d0 * dim, cnt, dim, bits, n_top, pairs_pad, out, first_doc + d0,
                     0xFFFFFFFFu / dim + 1u, flag};
-    if (dim <= 256)
+    // full ranks of a batch of queries: the binned form's one warp a row has a long chain, and
+    // the rows do not fill the GPU (us, binned / sorted: 1 row of dim 1,024 20.1 / 5.8, 256 rows
+    // 26.5 / 8.1, 1,024 rows 26.3 / 20.9; dim 384 7.4 / 4.5, 9.4 / 5.5, 10.0 / 12.7)
+    const bool few_ranks = kind == 5 && cnt <= 592;
+    if (few_ranks && dim > 256 && dim <= 512)
+      launch_sorted<2>(a, 256, stream);
+    else if (few_ranks && dim > 512 && dim <= 1024)
+      launch_sorted<4>(a, 256, stream);
+    else if (dim <= 256)
       launch_bins<1, 8, 8>(a, stream);
     else if (dim <= 384)
       launch_bins<1, 12, 16>(a, stream);
@@ -657,9 +665,9 @@ void launch_encode(int kind, const float* vecs, uint64_t n, uint32_t dim, uint32
     else if (dim <= 4096)
       launch_bins<4, 32, 32>(a, stream);
     else if (dim <= 8192)
-      launch_sorted<16>(a, stream);
+      launch_sorted<16>(a, 512, stream);
     else
-      launch_sorted<32>(a, stream);
+      launch_sorted<32>(a, 512, stream);
   }
 }
 

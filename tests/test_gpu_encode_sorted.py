@@ -46,3 +46,13 @@ def test_bucket_rows(orc, dim):
     got = np.stack(bm.top_m_candidates_batched(docs, 7))  # the queries' bits: descending, ties to the lower index
     want = np.stack([orc.bitmap_top_m(words, len(docs), dim, dim // 4, q, 7) for q in docs])
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 591, 592, 593])
+@pytest.mark.parametrize("dim", [257, 512, 520, 1024])
+def test_ranks_of_a_batch(orc, dim, n):
+    """Both sides of the number of rows from which full ranks are binned."""
+    docs = _docs(dim, n)
+    rk = ob.Rank(dim)
+    rk.add(docs)
+    assert np.array_equal(rk.payload().view(np.uint16), orc.rank_encode(docs, dim))
