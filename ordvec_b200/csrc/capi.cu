@@ -209,19 +209,19 @@ const float* upload_queries(Workspace& w, const float* q, uint64_t nq, uint32_t 
   return d;
 }
 
-// After a synchronised pipeline: surface a timed-out wait of a tensor-core
-// kernel (its results are then incomplete) as INTERNAL, and re-arm the word.
-void check_tc(Workspace& w) {
-  if (!w.tc_used) return;
-  w.tc_used = false;
-  uint32_t* h = (uint32_t*)w.pinned.ensure(4);
-  OVB_CUDA(cudaMemcpyAsync(h, w.tc_err.p, 4, cudaMemcpyDeviceToHost, w.stream));
+// A wait that timed out in a kernel of the pipeline (its results are then incomplete)
+// surfaces as INTERNAL, and the word is re-armed.
+[[noreturn]] void tc_timeout(Workspace& w) {
+  OVB_CUDA(cudaMemsetAsync(w.tc_err.p, 0, 4, w.stream));
   OVB_CUDA(cudaStreamSynchronize(w.stream));
-  if (*h) {
-    OVB_CUDA(cudaMemsetAsync(w.tc_err.p, 0, 4, w.stream));
-    OVB_CUDA(cudaStreamSynchronize(w.stream));
-    fail(ORDVEC_STATUS_INTERNAL, "tensor-core FastScan scan: a bounded wait timed out; results discarded");
-  }
+  fail(ORDVEC_STATUS_INTERNAL, "a bounded wait in a scan or select timed out; results discarded");
+}
+
+// After a synchronised pipeline.
+void check_tc(Workspace& w) {
+  const bool queued = queue_tc_error(w);
+  if (queued) OVB_CUDA(cudaStreamSynchronize(w.stream));
+  check_tc_error(w, queued);
 }
 
 // Results of up to this many bytes are written by the device straight into pinned
@@ -275,12 +275,6 @@ struct DeviceSink {
   ~DeviceSink() { w.sink = Workspace::Sink(); }
 };
 
-[[noreturn]] void tc_timeout(Workspace& w) {
-  OVB_CUDA(cudaMemsetAsync(w.tc_err.p, 0, 4, w.stream));
-  OVB_CUDA(cudaStreamSynchronize(w.stream));
-  fail(ORDVEC_STATUS_INTERNAL, "tensor-core FastScan scan: a bounded wait timed out; results discarded");
-}
-
 // results of the last pipeline (in the sink, or keys in w.out_keys / w.out_ids; count entries) -> host
 void download_results(HostSink& out, uint64_t count, float* scores, int64_t* ids) {
   if (!count) return;
@@ -297,14 +291,11 @@ void download_results(HostSink& out, uint64_t count, float* scores, int64_t* ids
     memcpy(ids, s.ids, count * 8);
     return;
   }
+  const bool queued = queue_tc_error(w);
   OVB_CUDA(cudaMemcpyAsync(scores, s.scores, count * 4, cudaMemcpyDeviceToHost, w.stream));
   OVB_CUDA(cudaMemcpyAsync(ids, s.ids, count * 8, cudaMemcpyDeviceToHost, w.stream));
-  // the tensor-core error word comes back with the results: one synchronisation
-  uint32_t* h_err = w.tc_used ? (uint32_t*)w.pinned.ensure(4) : nullptr;
-  if (h_err) OVB_CUDA(cudaMemcpyAsync(h_err, w.tc_err.p, 4, cudaMemcpyDeviceToHost, w.stream));
   OVB_CUDA(cudaStreamSynchronize(w.stream));
-  w.tc_used = false;
-  if (h_err && *h_err) tc_timeout(w);
+  check_tc_error(w, queued);
 }
 
 void need_queries(const float* q, uint64_t nq) {
@@ -332,6 +323,17 @@ uint32_t bitmap_subset(const Index& bm, const float* d_q, uint64_t nq, const uin
 
 ordvec_status_t api_boundary(const std::function<void()>& f) { return boundary(f); }
 void check_tc_errors(Workspace& w) { check_tc(w); }
+
+bool queue_tc_error(Workspace& w) {
+  if (!w.tc_used) return false;
+  OVB_CUDA(cudaMemcpyAsync(w.pinned.ensure(4), w.tc_err.p, 4, cudaMemcpyDeviceToHost, w.stream));
+  return true;
+}
+
+void check_tc_error(Workspace& w, bool queued) {
+  w.tc_used = false;
+  if (queued && *(uint32_t*)w.pinned.p) tc_timeout(w);
+}
 
 Workspace::Workspace() {
   OVB_CUDA(cudaGetDevice(&device));
@@ -815,9 +817,14 @@ static void top_m_host(const Index& ix, const float* queries, uint64_t nq, uint6
     d_w = dw;
   }
   uint32_t got = engine_candidates(ix, d_q, nq, me, d_w, w, w.stream);
-  OVB_CUDA(cudaMemcpyAsync(out, w.sel_ids.p, nq * got * 4, cudaMemcpyDeviceToHost, w.stream));
+  // small ones by way of pinned memory, with the error word (as in HostSink)
+  const uint64_t bytes = nq * got * 4;
+  const bool queued = queue_tc_error(w);
+  void* to = bytes <= kPinnedResults ? w.results.ensure(kPinnedResults + 16) : out;
+  OVB_CUDA(cudaMemcpyAsync(to, w.sel_ids.p, bytes, cudaMemcpyDeviceToHost, w.stream));
   OVB_CUDA(cudaStreamSynchronize(w.stream));
-  check_tc(w);
+  check_tc_error(w, queued);
+  if (to != out) memcpy(out, to, bytes);
 }
 
 ordvec_status_t ovb_sign_bitmap_top_m(const ordvec_index_t* sign, const float* queries, uint64_t nq, uint64_t m,

@@ -239,5 +239,9 @@ extern thread_local uint64_t tl_last_launches;
 // other files; tensor-core error word check after a synchronised pipeline.
 ordvec_status_t api_boundary(const std::function<void()>& f);
 void check_tc_errors(Workspace& w);
+// The same in two parts, so that the word comes back with the results: queue its copy on
+// w.stream (false: nothing to check) before theirs, and look at it after the synchronisation.
+bool queue_tc_error(Workspace& w);
+void check_tc_error(Workspace& w, bool queued);
 
 }  // namespace ovb

@@ -133,6 +133,7 @@ void run_batch(Server& S, const Route& rt, std::vector<ReqPtr>& batch, uint64_t 
   }
   float* hsp = nullptr;
   int64_t* hip = nullptr;
+  const bool queued = queue_tc_error(w);
   if (ke) {
     float* dsp = (float*)ds.ensure(nq * ke * 4);
     int64_t* dip = (int64_t*)di.ensure(nq * ke * 8);
@@ -143,7 +144,7 @@ void run_batch(Server& S, const Route& rt, std::vector<ReqPtr>& batch, uint64_t 
     OVB_CUDA(cudaMemcpyAsync(hip, dip, nq * ke * 8, cudaMemcpyDeviceToHost, w.stream));
   }
   OVB_CUDA(cudaStreamSynchronize(w.stream));
-  check_tc_errors(w);
+  check_tc_error(w, queued);
   off = 0;
   for (auto& q : batch) {
     // this request's own width: min(k, its candidate count), a prefix of each row
