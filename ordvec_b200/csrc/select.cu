@@ -592,6 +592,8 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kSelThrea
 // overlaps top-2,000 92 -> 33.
 constexpr uint32_t kGridRows = 16;
 constexpr uint64_t kGridMinN = 32768;
+constexpr uint64_t kGridMinFew = 40000;         // up to eight rows
+constexpr uint64_t kGridMinOrderedInt = 98304;  // ... of keys of at most 11 bits, in order
 constexpr int kGridThreads = 512;
 constexpr uint32_t kGridSlice = 4096;   // keys a CTA takes before more CTAs join
 constexpr uint32_t kGridDigits = 6;     // 32 key bits and 32 id bits, 11 at a time
@@ -717,12 +719,16 @@ __global__ void __launch_bounds__(kGridThreads) grid_select_kernel(SelectArgs a,
   const uint32_t* ids = a.ids ? a.ids + row * a.ld + lo : nullptr;
   uint32_t* st_ids = st_keys + per;
   const uint32_t k_eff = (uint32_t)(n < a.k ? n : a.k);
-  // few enough for one CTA: a sort of at most k + k/4 + 64, or, when the order does
-  // not matter, a last bin of at most 256 whose lowest are found by rank
+  // few enough for one CTA: a sort of at most k + k/4 + 64 (from 1,024 on, where twice the
+  // sort takes longer than another digit, of k's next power of two), or, when the order
+  // does not matter, a last bin of at most 256 whose lowest are found by rank
+  uint32_t k_len = 1;
+  while (k_len < k_eff) k_len <<= 1;
+  const uint32_t most = k_len < 1024 ? k_eff + k_eff / 4 + 64 : k_len;
   auto enough = [&](uint32_t need, uint32_t in_bin) -> bool {
     const uint32_t total = k_eff - need + in_bin;
     if (in_bin == need) return true;
-    return total <= kSelectSmemCap && (a.unordered ? in_bin <= 256 : total <= k_eff + k_eff / 4 + 64);
+    return total <= kSelectSmemCap && (a.unordered ? in_bin <= 256 : total <= most);
   };
   if (stage) {  // eight loads in flight per thread
     for (uint32_t i0 = t; i0 < cnt; i0 += 8 * kGridThreads) {
@@ -880,7 +886,13 @@ uint32_t grid_ctas() {
   return most;
 }
 
+// From 32,768 keys a row on, for up to eight rows from 40,000: the launch costs the host a memset and a cooperative launch
+// more than the cluster form (whole calls, us, cluster / grid: Rank top-10 of 33,000 44.8 /
+// 46.6, of 50,000 43.8 / 39.9).  Integer keys have many ties at the cut, which an ordered
+// result resolves by digits of the ids (SignBitmap top-500 of 60,000 66 / 73, top-2,000 78 /
+// 85, of 250,000 79 / 74 and 139 / 129; 16 rows of 60,000 top-500 87 / 80).
 bool use_select_grid(const SelectArgs& a, uint64_t rows, const uint64_t* scratch) {
+  if (rows <= 8 && a.n < (!a.unordered && a.key_bits <= 11 ? kGridMinOrderedInt : kGridMinFew)) return false;
   return scratch && !a.row_off && !a.row_len && rows <= kGridRows && a.n >= kGridMinN && a.n < (1ull << 32) &&
          a.k >= 1 && a.k <= kSelectSmemCap && rows <= grid_ctas();
 }

@@ -46,3 +46,25 @@ def test_unordered_set(monkeypatch, m):
     for i, c in enumerate(cand):
         _, want = rq.search_asymmetric_subset(q[i], np.sort(c).astype(np.uint32), 50)
         assert np.array_equal(got.indices_for_query(i), want)
+
+
+@pytest.mark.parametrize("n", [39_999, 40_000, 98_303, 98_304])
+@pytest.mark.parametrize("nq", [1, 8, 9])
+def test_both_sides_of_the_whole_gpu_rule(monkeypatch, n, nq):
+    """Ordered integer keys, and unordered ones before a rerank; k whose sort is doubled, and not."""
+    dim = 64
+    rng = np.random.default_rng(n + nq)
+    docs = rng.standard_normal((n, dim)).astype(np.float32)
+    q = rng.standard_normal((nq, dim)).astype(np.float32)
+    sb, rq = ob.SignBitmap(dim), ob.RankQuant(dim, 1)
+    sb.add(docs)
+    rq.add(docs)
+    monkeypatch.setenv("OVB_BITMAP_TC", "0")
+    order = [np.lexsort((np.arange(n), dim - sb.score_all(x).astype(np.int64))) for x in q]
+    for k in (100, 800, 1024, 2000, 2048, 4096):
+        for g, want in zip(sb.top_m_candidates_batched(q, k), order):
+            assert np.array_equal(g, want[:k]), k
+    got = ob.two_stage_search(rq, sb, q, 1000, 20)
+    for i in range(nq):
+        _, want = rq.search_asymmetric_subset(q[i], np.sort(order[i][:1000]).astype(np.uint32), 20)
+        assert np.array_equal(got.indices_for_query(i), want)
