@@ -646,7 +646,9 @@ void launch_encode(int kind, const float* vecs, uint64_t n, uint32_t dim, uint32
     // the rows do not fill the GPU (us, binned / sorted: 1 row of dim 1,024 20.1 / 5.8, 256 rows
     // 26.5 / 8.1, 1,024 rows 26.3 / 20.9; dim 384 7.4 / 4.5, 9.4 / 5.5, 10.0 / 12.7)
     const bool few_ranks = kind == 5 && cnt <= 592;
-    if (few_ranks && dim > 256 && dim <= 512)
+    if (few_ranks && dim > 128 && dim <= 256)
+      launch_sorted<1>(a, 256, stream);
+    else if (few_ranks && dim > 256 && dim <= 512)
       launch_sorted<2>(a, 256, stream);
     else if (few_ranks && dim > 512 && dim <= 1024)
       launch_sorted<4>(a, 256, stream);

@@ -49,7 +49,7 @@ def test_bucket_rows(orc, dim):
 
 
 @pytest.mark.parametrize("n", [1, 591, 592, 593])
-@pytest.mark.parametrize("dim", [257, 512, 520, 1024])
+@pytest.mark.parametrize("dim", [128, 129, 256, 257, 512, 520, 1024])
 def test_ranks_of_a_batch(orc, dim, n):
     """Both sides of the number of rows from which full ranks are binned."""
     docs = _docs(dim, n)
