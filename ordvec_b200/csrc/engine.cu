@@ -948,21 +948,22 @@ static uint32_t rerank_mode(const Workspace& w, const Index& rq, uint64_t nq, ui
 }
 
 // Whether a rerank scores its candidates in integers first (scan_score_rows.cu) and
-// only the best kp in FP64: from 2-bit codes and nq me dim bits >= 5e8 on, where the FP64
-// rerank's time is more than the select, margin test and rescoring add.  Measured on
-// whole two-stage calls (us, FP64 / integers first): n = 171,332 dim 1024 b=2: 230 / 250
-// at 61 x 1,600 candidates (2.0e8), 342 / 327 at 256 x 1,000 (5.2e8), 618 / 551 at 1,000 x
-// 1,000, 948 / 775 at 1,024 x 2,000; n = 1M dim 768 b=2: 453 / 464 at 256 x 1,000 (3.9e8),
-// 558 / 538 at 256 x 2,000 (7.9e8), 1,352 / 1,221 at 1,024 x 2,000; n = 1M dim 1024 b=4: 260
-// / 291 at 32 x 1,000 (1.3e8), 368 / 356 at 128 x 1,000 (5.2e8), 762 / 606 at 256 x 2,000;
-// one-bit rows, whose FP64 form reads few tables, stay: 751 / 754 at 1,024 x 2,000 of dim
-// 1024.
+// only the best kp in FP64: from 2-bit codes, 1,024 bits a row and nq me dim bits = 5e8
+// on, where the FP64 rerank's time, which goes with the bits of a candidate, is more than the
+// select, margin test and rescoring add.  Measured on whole two-stage calls (us, FP64 /
+// integers first): n = 60k, 1,000 queries x 1,000 candidates: dim 256 b=2 410 / 432, dim
+// 384 b=2 441 / 457, dim 512 b=2 472 / 468, dim 256 b=4 461 / 447, dim 768 b=2 518 / 484, dim
+// 1024 b=2 586 / 518, b=4 900 / 621; 256 x 2,000: dim 384 b=2 223 / 236, dim 512 b=2 243 / 242,
+// dim 1024 b=2 319 / 272; 256 x 1,000: dim 768 b=2 231 / 245 (3.9e8), dim 1024 b=2 279 / 257
+// (5.2e8); one-bit rows, whose FP64 form reads few tables, stay: dim 1024 477 / 496 and 736 /
+// 726 at 1,000 x 2,000.
 static bool use_subset_scores(const Index& rq, uint64_t nq, uint32_t me, uint32_t ke, cudaStream_t st) {
   const char* e = getenv("OVB_ROW_SCORES");
   if (e && e[0] == '0') return false;
   const uint64_t kp = std::max<uint64_t>(2ull * ke, ke + 64ull);
   if (!score_rows_eligible(rq.dim, rq.bits) || nq > 65535 || me < 4 * kp || capturing(st)) return false;
-  return (e && e[0] == '1') || (rq.bits >= 2 && nq * me * rq.dim * rq.bits >= 500000000ull);
+  const uint64_t row_bits = (uint64_t)rq.dim * rq.bits;
+  return (e && e[0] == '1') || (rq.bits >= 2 && row_bits >= 1024 && nq * me * row_bits >= 500000000ull);
 }
 
 // Split-BF16 rerank of the uniform candidate rows in w.sel_ids (me per query):

@@ -80,7 +80,7 @@ def test_rank(monkeypatch, nq, some):
 
 
 @pytest.mark.parametrize("some", ["none", "some", "all"])
-@pytest.mark.parametrize("bits,nq", [(4, 520), (2, 1000)])
+@pytest.mark.parametrize("bits,nq", [(4, 520), (4, 1000)])  # 1,024 bits a row
 def test_two_stage_rerank(monkeypatch, bits, nq, some):
     docs = _docs(20_000, 1000)
     rq, sb = ob.RankQuant(DIM, bits), ob.SignBitmap(DIM)
