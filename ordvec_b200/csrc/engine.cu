@@ -318,6 +318,20 @@ static bool split_filter_plan(uint64_t n, uint64_t kp, FilterPlan& fp) {
   return kp <= kSelectSmemCap && filter_plan(n, (uint32_t)kp, fp);
 }
 
+// The filter's plan for the candidates of an exact RankQuant batch of nq queries.  Integer
+// scores of up to 256 queries over up to 131,072 rows go through the key matrix instead from
+// kp = n / 160 on: so many kept documents keep the filter's epilogue on its lists, and rows
+// of that length select fast (whole calls of 64 queries, us, filter / key matrix: n =
+// 100k dim 320 b=2, top-300 152 / 137, top-1,000 209 / 165, top-1,500 280 / 194; n = 40k
+// dim 256, top-300 141 / 107; 256 queries 352 / 285, 500 queries 475 / 472; n = 300k dim
+// 768 top-1,000 241 / 432).
+static bool cand_filter_plan(const Index& rq, uint64_t nq, uint64_t kp, FilterPlan& fp) {
+  if (score_rankquant_eligible(rq.dim, rq.bits) && nq <= 256 && rq.n <= 131072 && kp * 160 > rq.n &&
+      nq * rq.n * 4 <= keys_budget())
+    return false;
+  return split_filter_plan(rq.n, kp, fp);
+}
+
 static uint64_t split_filter_bytes_per_query(const FilterPlan& fp, uint64_t kp) {
   return fp.n_s * 4 + (uint64_t)fp.r * 8 + (uint64_t)fp.cap * 8 + 4 + kp * 12 + 8;
 }
@@ -459,7 +473,7 @@ static uint32_t split_search(const Index& rq, const float* qu, float inv_norm, b
   FilterPlan fp;
   // rows that passed the filtered pipeline; the others take the key matrix below
   std::vector<char> done;
-  if (exact && split_filter_plan(n, kp0, fp)) {
+  if (exact && cand_filter_plan(rq, nq, kp0, fp)) {
     uint64_t fc = keys_budget() / split_filter_bytes_per_query(fp, kp0);
     if (fc < 1) fc = 1;
     done.assign(nq, 0);
@@ -539,7 +553,7 @@ bool split_fixed_fits(const Index& rq, uint64_t nq, uint64_t k) {
   const uint64_t n = rq.n, ke = k < n ? k : n;
   const uint64_t kp = std::min<uint64_t>(std::max<uint64_t>(2 * ke, ke + 64), n);
   FilterPlan fp;
-  if (split_filter_plan(n, kp, fp) && nq * split_filter_bytes_per_query(fp, kp) <= keys_budget()) return true;
+  if (cand_filter_plan(rq, nq, kp, fp) && nq * split_filter_bytes_per_query(fp, kp) <= keys_budget()) return true;
   return nq * n * 4 <= keys_budget();
 }
 
@@ -552,7 +566,7 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
   if (kp > n) kp = n;
   if (kp < ke) kp = ke;
   FilterPlan fp;
-  const bool filtered = split_filter_plan(n, kp, fp) && nq * split_filter_bytes_per_query(fp, kp) <= keys_budget();
+  const bool filtered = cand_filter_plan(rq, nq, kp, fp) && nq * split_filter_bytes_per_query(fp, kp) <= keys_budget();
   if (!rank_tc_eligible(rq.dim, rq.bits) || (!filtered && nq * n * 4 > keys_budget()))
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "fixed split search: shape outside the single-chunk form");
   const uint32_t dim = rq.dim, bits = rq.bits, id_bits = bits_for(n - 1);
