@@ -141,6 +141,10 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, b
          "FastScan v1: incremental add() not supported (block-32 layout); construct a new index");
   if (ix.kind != OVB_INDEX_KIND_SIGN_BITMAP && ix.dim > kMaxDeviceRankDim)
     fail(ORDVEC_STATUS_UNSUPPORTED_OPERATION, "device rank transform supports dim <= 16384");
+  // what the workspace keeps is allocated before the codes: a word placed behind the first
+  // small index would split the 2 MB block that later ones are handed out from
+  uint32_t* flag = check ? (uint32_t*)w.flag.ensure(4) : nullptr;
+  uint32_t* h = check ? (uint32_t*)w.pinned.ensure(4) : nullptr;
   DevBuf fresh;
   void* codes;
   try {
@@ -150,12 +154,7 @@ void add_device_rows(Index& ix, const float* d_vecs, uint64_t n, Workspace& w, b
     if (check) need_finite_rows(ix, d_vecs, n, w);
     throw;
   }
-  uint32_t *flag = nullptr, *h = nullptr;
-  if (check) {
-    flag = (uint32_t*)w.flag.ensure(4);
-    h = (uint32_t*)w.pinned.ensure(4);
-    OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
-  }
+  if (check) OVB_CUDA(cudaMemsetAsync(flag, 0, 4, w.stream));
   launch_encode((int)encode_kind(ix.kind), d_vecs, n, ix.dim, ix.bits, ix.n_top, ix.pairs_pad, codes, ix.n, flag,
                 w.stream);
   if (check) OVB_CUDA(cudaMemcpyAsync(h, flag, 4, cudaMemcpyDeviceToHost, w.stream));
