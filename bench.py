@@ -203,7 +203,7 @@ def rerank_report(ob, orc, torch, dev, rq, s1, d_q, queries, m, k, packed, sampl
     sp = torch.cuda.current_stream(dev).cuda_stream
     d_s = torch.empty(nq * k, dtype=torch.float32, device=dev)
     d_i = torch.empty(nq * k, dtype=torch.int64, device=dev)
-    out = {"default_form": "FP64 per-query nibble tables (CUDA cores)",
+    out = {"default_form": "integer row scores, then FP64 of the best behind a bound (CUDA cores); FP64 tables where small",
            "split_form": "split-BF16 tcgen05 (codes exact in BF16, query hi+lo BF16, f32 accumulation) + margin test "
                          "+ FP64 rescoring of the top 2k+32"}
     os.environ["OVB_RERANK_TC"] = "1"
@@ -326,10 +326,10 @@ def mixed_run(ob, nq: int, steps: int):
             info = ob.mixed_plan_info(rq, rows.size, int(ks[rows].max()))
             plans.append({"bits": (1, 2, 4)[j], "queries": int(rows.size), **info})
     sec = float(np.median(times))
-    flops = 2 * 2 * nq * n * dim  # hi and lo products, multiply + add
+    ops = 2 * 2 * nq * n * dim  # products of both s8 planes, multiply + add
     return {"workload": f"N={n} dim={dim} bits {{1,2,4}} k {{10,50,100}}, {nq} mixed queries per call",
             "qps": nq / sec, "s_per_call": sec, "first_call_s": first_s, "calls": reps,
-            "split_bf16_tflops_effective": flops / sec / 1e12, "identical_across_calls": same, "plans": plans,
+            "int8_tops_effective": ops / sec / 1e12, "identical_across_calls": same, "plans": plans,
             "form": "host buffers; 16-bit fixed-point tcgen05 (s8 planes) candidate scan + exact FP64 rescoring; CUDA-graph replay"}
 
 
@@ -650,17 +650,18 @@ def profile_case(case: str):
       bitmap    Bitmap(768, 192) top-2000 of 1024 queries, N=2M (bitmap_fp4_pair_kernel)
       bitmap10m the same at N=10M (the headline's stage-1 index only, 0.96 GB)
       popc      the 2M index, one query per call (popc_rows_kernel, wide select)
-      rank      RankQuant(1024, 2) exact top-100 of 1024 queries, N=1M (rank_tc_kernel)
-      fastscan  the FastScan configuration's top-1000 of 1000 queries (fastscan_tc_kernel)
+      rank      RankQuant(1024, 2) exact top-100 of 1024 queries, N=1M (score_pair_kernel<2>)
+      fastscan  the FastScan configuration's top-1000 of 1000 queries (fastscan_persist_kernel)
       plain     the FastScan two-stage search, one query per call, 12 calls
-                (fastscan_scan_kernel, select_rows_cluster_kernel, rerank)
+                (fastscan_scan_kernel, grid_select_kernel, rerank)
       rankfull  Rank(768) N=1M top-100: symmetric then asymmetric, 1 query and 64
-                queries per call (rank_tile_kernel)
+                queries per call (rank_tile_kernel, score_pair_kernel<16>)
       multibucket MultiBucketBitmap(768, 2) N=2M: diagonal-weight top-2000 of 1
                 query per call (multibucket_rows_kernel), 3 calls
       encode    RankQuant(768, 2).add of 1M docs, twice (rank_bins_kernel)
       rerank    Bitmap(768, 192) top-2000 -> RankQuant b=2 top-100 of 1024 queries,
-                N=2M, twice (rerank_tc_kernel, asym_table_kernel rescoring)
+                N=2M, twice (score_rows_kernel<2, 1, 1>; rerank_tc_kernel under
+                OVB_RERANK_TC=1)
     Each search runs more than once so captures can skip the first call."""
     import ordvec_b200 as ob
 

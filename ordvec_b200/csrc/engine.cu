@@ -609,7 +609,10 @@ uint32_t engine_rankquant_split_fixed(const Index& rq, const float* d_q, uint64_
 // 200k dim 1024 b=1: 91 / 109 / 129 at 3 (6.1e8), 154 / 141 / 136 at 6; b=2: 86 / 90 / 129
 // at 1 (4.1e8), 113 / 99 / 129 at 2 (8.2e8), 266 / 147 / 140 at 6; n = 40k dim 384 b=2: 112
 // / 107 / 103 at 24 (7.4e8), b=4: 89 / 79 / 98 at 8 (4.9e8), 181 / 110 / 106 at 24; n = 10k
-// dim 256: 40 / 80 / 80.
+// dim 256: 40 / 80 / 80.  All of calls on device pointers; from host buffers add about 20.
+// One line in W for all shapes leaves rows of few bytes above it on the slower form: of
+// these, n = 40k takes the tables at 24 queries b=2 (9 us from the best) and at 8
+// queries b=4 (10 us).
 // A capturing stream keeps the tables, whose buffers every search of the size has.
 // OVB_ROW_SCORES=0/1 forces kRows, here and for candidate rows; OVB_RANK_TC=0 leaves
 // kFilter out.
@@ -727,7 +730,8 @@ struct RankScores {
 // RankQuant).  Measured with both forms, symmetric (us, CUDA cores / tensor
 // cores): n = 1M dim 768: 324 / 363 at 1 query, 567 / 364 at 2, 692 / 369 at 8, 3,939
 // / 376 at 48; n = 200k dim 1024: 180 / 216 at 4, 277 / 217 at 5; n = 100k dim 768: 123 /
-// 160 at 8, 192 / 162 at 12; n = 40k dim 384: 107 / 110 at 24, 139 / 111 at 48.
+// 160 at 8, 192 / 162 at 12; n = 40k dim 384: 107 / 110 at 24, 139 / 111 at 48 (7.4e8: one
+// line for all shapes leaves this one on the CUDA cores).
 static bool use_rank_scores(const Index& rk, uint64_t nq, uint64_t kp, cudaStream_t st, FilterPlan& fp) {
   const char* e = getenv("OVB_RANK_TC");
   if (e && e[0] == '0') return false;

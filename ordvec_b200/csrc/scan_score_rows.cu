@@ -14,8 +14,8 @@
 // Bound by issue: at n = 1M, dim 768, 2 bits, one query, 75 % of the issue slots and
 // half the HBM rate (192 MB in 57 us; the FP64 table scan takes 151 us), 12 warps an SM by
 // the stages' shared memory.  Up to four queries share a pass over the rows (1M rows,
-// dim 768, b=2, whole call: 129 us at one query, 157 at 2, 216 at 4); more take a pass
-// for each four.  1,000 x 1,000 candidates of dim 1024, b=2: 70 us, the FP64 rerank 219.
+// dim 768, b=2, whole call on device pointers: 129 us at one query, 157 at 2, 216 at 4; the
+// same call from host buffers 148 at one query); more take a pass for each four.  1,000 x 1,000 candidates of dim 1024, b=2: 70 us, the FP64 rerank 219.
 #include <algorithm>
 
 #include "ovb_common.cuh"

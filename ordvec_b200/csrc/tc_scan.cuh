@@ -138,8 +138,9 @@ __device__ __forceinline__ uint4 load_codes(const uint8_t* p) {
 // MODE 0: FastScan (A = one-hot of nibble codes, B = u8 LUTs, score by the
 // FastScan formula).  MODE 1: bitmap AND-overlap (A = doc bits as 0/1 bytes,
 // B = query bits as 0/1 bytes, acc = overlap, key = n_top - overlap).  MODE 2:
-// the bitmap filter on FP4 tensor cores (A, B = bits as e2m1 nibbles of 1.0 /
-// 0, f32 acc = overlap), CTA pairs only.
+// the bitmap filter on FP4 tensor cores (A = doc bits left where they are in their e2m1
+// nibbles, values 0.5, 1 or 2; B = the reciprocal where the query's bit is set, so each
+// product is 1 and the f32 acc = overlap), CTA pairs only.
 }  // namespace tcs
 
 // Forms of the tensor-core scans: one CTA per 256-doc tile (scan_fastscan_tc.cu),
